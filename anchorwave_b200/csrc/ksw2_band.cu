@@ -554,40 +554,39 @@ struct BtArgs {
     int m, flag, block;
 };
 
-// ksw_backtrack (minimap2/ksw2.h:160-192) over the strip layout with the band's
-// off/off_end forcing, run in lockstep by a warp; stops when the walk ends or leaves the
-// columns >= col_lo.
-template <int NC, class Cache, class Load>
-__device__ void band_walk(int &i, int &j, int &state, int col_lo, WarpCig &cg, Cache &cache, Load &load,
-                          const Geom &g) {
-    while (i >= 0 && j >= 0 && i >= col_lo) {
-        const int r = i + j;
-        int force = -1;
-        if (i < (g.st0(r) & g.bmask)) force = 2;
-        if (i > (g.en0(r) | 15)) force = 1;
-        const uint32_t cellv = force < 0 ? cache.byte(i / NC, j, i % NC, load) : 0u;
-        if (state == 0) state = cellv & 7;
-        else if (!(cellv >> (state + 2) & 1)) state = 0;
-        if (state == 0) state = cellv & 7;
-        if (force >= 0) state = force;
-        if (state == 0) cg.push(0, 1), --i, --j;
-        else if (state == 1 || state == 3) cg.push(2, 1), --i;
-        else cg.push(1, 1), --j;
-    }
+// The move that ksw_backtrack's off/off_end forcing takes outside the computed blocks of the
+// cell's anti-diagonal (1: deletion, 2: insertion), or -1.
+__device__ __forceinline__ int band_force(const Geom &g, int i, int j) {
+    const int r = i + j;
+    return i > (g.en0(r) | 15) ? 1 : i < (g.st0(r) & g.bmask) ? 2 : -1;
 }
 
-constexpr int FIN_WARPS = 4;
+// The stored rows of a column group of a pair's strips (words of WB bytes).
+template <int WB, int NC>
+__device__ __forceinline__ TbGroup band_group(const BandStripDev *strips, const uint8_t *tb, int tlen, int col_lo,
+                                              int gg) {
+    if (gg < 0 || gg * NC >= tlen || gg * NC < col_lo) return TbGroup{tb, 0, -1};
+    const BandStripDev St = strips[gg >> 5];
+    const int L = gg & 31;
+    return TbGroup{tb + St.tb_off + ((int64_t)L * 32 + L) * WB, St.jlo, St.jend};
+}
+
+// Warps per block of the finishing kernel: the Singletrack words are twice as large, and its
+// gap search has two tiles of its own.
+template <bool ST>
+constexpr int fin_warps() { return ST ? 1 : 4; }
 
 // Result record of one pair, then ksw_backtrack (minimap2/ksw2.h:160-192) with the
 // off/off_end forcing of the band, or the Singletrack reconstruction
-// (minimap2/ksw2_singletrack.cpp:63-176); one warp per pair walks with the tile cache.
+// (minimap2/ksw2_singletrack.cpp:63-176); one warp per pair walks in runs (tb_walk.cuh).
 template <bool ST, int NC>
-__global__ void __launch_bounds__(32 * FIN_WARPS) ksw_band_finish_kernel(BtArgs A) {
+__global__ void __launch_bounds__(32 * fin_warps<ST>()) ksw_band_finish_kernel(BtArgs A) {
     constexpr int WB = ST ? 2 * NC : NC;  // bytes per lane-word: NC columns (v then u for Singletrack)
-    using Cache = TileCache<WB, 32, 64 / NC>;  // 32 rows x 64 columns
-    __shared__ typename Cache::Word tiles[FIN_WARPS][2 * Cache::NW];
+    using Window = TbWindow<WB, NC, ST ? 1 : 0, true>;
+    using Probe = TbWindow<WB, NC, 0, false>;  // the rows and columns of a Singletrack gap search
+    __shared__ __align__(16) uint8_t tiles[fin_warps<ST>()][Window::BYTES + (ST ? Probe::BYTES : 0)];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int pi = blockIdx.x * FIN_WARPS + warp;
+    const int pi = blockIdx.x * fin_warps<ST>() + warp;
     if (pi >= A.npair) return;
     const BandPairDev P = A.pairs[pi];
     const BandRes R = A.res[pi];
@@ -617,18 +616,9 @@ __global__ void __launch_bounds__(32 * FIN_WARPS) ksw_band_finish_kernel(BtArgs 
     const bool cigar = !(flag & AW_EZ_SCORE_ONLY);
     const BandStripDev *strips = A.strips + P.strip0;
     const uint8_t *tb = A.tb;
-    Cache cache;
-    cache.init(tiles[warp]);
-    // the stored lane-word of column group gg (NC columns), row jj (zero outside the stored rows)
-    auto load = [&](int gg, int jj) -> typename Cache::Word {
-        typename Cache::Word z{};
-        if (gg < 0 || jj < 0 || gg * NC >= tlen) return z;
-        const int s = gg >> 5, L = gg & 31;
-        const BandStripDev St = strips[s];
-        if (jj < St.jlo || jj > St.jend) return z;
-        const uint8_t *p = tb + St.tb_off + ((int64_t)(jj - St.jlo + L) * 32 + L) * WB;
-        return __ldcs(reinterpret_cast<const typename Cache::Word *>(p));
-    };
+    Window win;
+    win.init(tiles[warp], 32 * WB);
+    auto grp = [&](int gg) -> TbGroup { return band_group<WB, NC>(strips, tb, tlen, 0, gg); };
     auto stB = [&](int r) { return g.st0(r) & g.bmask; };
     auto en16 = [&](int r) { return (g.en0(r) & ~15) + 15; };
     WarpCig cg{A.cig + P.cig_off, 0, 0, 0};
@@ -638,55 +628,85 @@ __global__ void __launch_bounds__(32 * FIN_WARPS) ksw_band_finish_kernel(BtArgs 
         if (!o.zdropped && (sse_st || !(flag & (AW_EZ_EXTZ_ONLY | AW_EZ_SEMIGLOBAL_END)))) {
             const uint8_t *qs = A.qcodes + P.qoff, *ts = A.tcodes + P.toff;
             const int o1 = -A.sc.q, g1 = -A.sc.e, o2 = -A.sc.q2, g2 = -A.sc.e2;
-            // track value (0 = v, 1 = u), the matrix-edge difference, or NEG_INF outside the stored band
-            auto diff = [&](int part, int i, int j) -> int {
-                if (i < 0 || j < 0) {
-                    const int c = i < 0 ? j : i;
-                    return st_gap(c + 1, o1, g1, o2, g2) - st_gap(c, o1, g1, o2, g2);
-                }
+            // the difference along the matrix edge for edge cell c
+            auto edge = [&](int c) { return st_gap(c + 1, o1, g1, o2, g2) - st_gap(c, o1, g1, o2, g2); };
+            auto stored = [&](int i, int j) {
                 const int d = i + j;
-                if (i < stB(d) || i > en16(d)) return AW_NEG_INF;
-                return sx8(cache.byte(i / NC, j, (i % NC) + NC * part, load));
+                return i >= stB(d) && i <= en16(d);
             };
-            auto fin = [](int v) { return v > AW_NEG_INF / 2 && v < -AW_NEG_INF / 2; };
-            bool in_m = true, valid = true;
-            int i = tlen - 1, j = qlen - 1, l = 0, dd = 0, di = 0;
+            Probe probe;
+            probe.init(tiles[warp] + Window::BYTES, 32 * WB);
+            bool valid = true;
+            int i = tlen - 1, j = qlen - 1;
             while (i >= 0 && j >= 0) {
                 const int dg = i + j;
-                if (i < stB(dg)) { cg.push(1, 1); --j; in_m = true; continue; }
-                if (i > en16(dg)) { cg.push(2, 1); --i; in_m = true; continue; }
-                if (in_m) {
-                    const int h = diff(0, i, j), v = diff(1, i, j - 1);
-                    const int cost = A.mat[ts[i] * A.m + qs[j]];
-                    if (fin(h) && fin(v) && (long long)h + v == cost) {
-                        cg.push(0, 1);
-                        --i, --j;
-                    } else {
-                        in_m = false, l = 0;
-                        di = diff(0, i, j);
-                        dd = diff(1, i, j);
-                    }
-                } else {
-                    ++l;
-                    if (l > i + 1 && l > j + 1) { valid = false; break; }
-                    const int a1 = o1 + l * g1, a2 = o2 + l * g2, jn = j - l, id = i - l;
-                    if (id >= -1 && (dd == a1 || dd == a2)) {
-                        cg.push(2, l);
-                        i = id, in_m = true;
-                    } else if (jn >= -1 && (di == a1 || di == a2)) {
-                        cg.push(1, l);
-                        j = jn, in_m = true;
-                    } else {
-                        if (jn >= 0) {
-                            const int Hh = diff(0, i, jn);
-                            di = (fin(di) && fin(Hh)) ? di + Hh : AW_NEG_INF;
-                        }
-                        if (id >= 0) {
-                            const int V = diff(1, id, j);
-                            dd = (fin(dd) && fin(V)) ? dd + V : AW_NEG_INF;
-                        }
-                    }
+                if (i < stB(dg)) { cg.push(1, 1); --j; continue; }
+                if (i > en16(dg)) { cg.push(2, 1); --i; continue; }
+                // the run of diagonal moves: v(i, j) + u(i, j-1) is the cell's substitution score
+                win.ensure(i, j, grp);
+                const int li = i - lane, lj = j - lane;
+                const bool in = li >= 0 && lj >= 0 && win.has(li, lj) && stored(li, lj);
+                bool on = in;
+                if (in) {
+                    const int h = sx8(win.at(li, lj, 0));
+                    const bool fin = lj == 0 || stored(li, lj - 1);
+                    const int v = lj == 0 ? edge(li) : fin ? sx8(win.at(li, lj - 1, 1)) : 0;
+                    on = fin && h + v == A.mat[ts[li] * A.m + qs[lj]];
                 }
+                const unsigned off = __ballot_sync(FULL, !on);
+                const int run = off ? __ffs(off) - 1 : 32;
+                if (run > 0) {
+                    cg.push(0, run);
+                    i -= run, j -= run;
+                }
+                if (run == 32 || !__shfl_sync(FULL, in ? 1 : 0, run)) continue;
+                // the gap that leaves (i, j): the first length l whose summed differences up the
+                // column of rows (insertion) or along the row (deletion) are exactly a gap of l;
+                // 32 lengths at a time, lane k looking at length base + k + 1.  Sums over cells
+                // outside the stored band match no gap (d_ok, i_ok).
+                int base = 0, dsum = 0, isum = 0;
+                bool d_ok = true, i_ok = true;
+                for (;;) {
+                    const int l = base + lane + 1, id = i - l, jn = j - l;
+                    // differences of the l-th cell: u(i-l+1, j) and v(i, j-l+1)
+                    int du = 0, dv = 0;
+                    bool uf = true, vf = true;
+                    if (d_ok && i - base >= 0) probe.corner(i - base, j, grp);
+                    if (d_ok && id + 1 >= 0) {
+                        uf = stored(id + 1, j);
+                        if (uf) du = sx8(probe.at(id + 1, j, 1));
+                    }
+                    __syncwarp();
+                    if (i_ok && j - base >= 0) probe.corner(i, j - base, grp);
+                    if (i_ok && jn + 1 >= 0) {
+                        vf = stored(i, jn + 1);
+                        if (vf) dv = sx8(probe.at(i, jn + 1, 0));
+                    }
+                    __syncwarp();
+#pragma unroll
+                    for (int k = 1; k < 32; k <<= 1) {
+                        const int a = __shfl_up_sync(FULL, du, k), b = __shfl_up_sync(FULL, dv, k);
+                        if (lane >= k) du += a, dv += b;
+                    }
+                    const unsigned ub = __ballot_sync(FULL, !uf), vb = __ballot_sync(FULL, !vf);
+                    const unsigned upto = lane == 31 ? FULL : (2u << lane) - 1u;
+                    const int a1 = o1 + l * g1, a2 = o2 + l * g2, dd = dsum + du, di = isum + dv;
+                    const bool dhit = d_ok && !(ub & upto) && id >= -1 && (dd == a1 || dd == a2);
+                    const bool ihit = i_ok && !(vb & upto) && jn >= -1 && (di == a1 || di == a2);
+                    const unsigned end = __ballot_sync(FULL, l > i + 1 && l > j + 1);
+                    const unsigned db = __ballot_sync(FULL, dhit), hit = db | __ballot_sync(FULL, ihit);
+                    if (hit && (!end || __ffs(hit) <= __ffs(end))) {
+                        const int k = __ffs(hit) - 1, len = base + k + 1;
+                        if (db >> k & 1u) cg.push(2, len), i -= len;
+                        else cg.push(1, len), j -= len;
+                        break;
+                    }
+                    if (end) { valid = false; break; }
+                    dsum += __shfl_sync(FULL, du, 31), isum += __shfl_sync(FULL, dv, 31);
+                    d_ok = d_ok && !ub, i_ok = i_ok && !vb;
+                    base += 32;
+                }
+                if (!valid) break;
             }
             if (valid) {
                 if (i >= 0) cg.push(2, i + 1);
@@ -717,7 +737,7 @@ __global__ void __launch_bounds__(32 * FIN_WARPS) ksw_band_finish_kernel(BtArgs 
             }
         } else if (i0 >= 0 || j0 >= 0) {
             int i = i0, j = j0, state = 0;
-            band_walk<NC>(i, j, state, 0, cg, cache, load, g);
+            tb_walk(i, j, state, 0, cg, win, grp, [&](int a, int b) { return band_force(g, a, b); });
             if (i >= 0) cg.push(2, i + 1);
             if (j >= 0) cg.push(1, j + 1);
             o.n_cigar = cg.finish(!(flag & AW_EZ_REV_CIGAR));
@@ -732,8 +752,8 @@ __global__ void __launch_bounds__(32 * FIN_WARPS) ksw_band_finish_kernel(BtArgs 
 // CIGAR length).
 template <int NC>
 __global__ void __launch_bounds__(32) ksw_band_round_walk_kernel(BtArgs A, const BandGroupDev *groups) {
-    using Cache = TileCache<NC, 32, 64 / NC>;
-    __shared__ typename Cache::Word tiles[2 * Cache::NW];
+    using Window = TbWindow<NC, NC, 0, true>;
+    __shared__ __align__(16) uint8_t tiles[Window::BYTES];
     const BandGroupDev G = groups[blockIdx.x];
     const int slot = G.slot, col_lo = G.col_lo;
     BandWalkState w = A.walk[slot];
@@ -751,20 +771,12 @@ __global__ void __launch_bounds__(32) ksw_band_round_walk_kernel(BtArgs A, const
     const int tlen = P.tlen;
     const BandStripDev *strips = A.strips + P.strip0;
     const uint8_t *tb = A.tb;
-    Cache cache;
-    cache.init(tiles);
-    auto load = [&](int gg, int jj) -> typename Cache::Word {
-        typename Cache::Word z{};
-        if (gg < 0 || jj < 0 || gg * NC >= tlen || gg * NC < col_lo) return z;
-        const int s = gg >> 5, L = gg & 31;
-        const BandStripDev St = strips[s];
-        if (jj < St.jlo || jj > St.jend) return z;
-        const uint8_t *p = tb + St.tb_off + ((int64_t)(jj - St.jlo + L) * 32 + L) * NC;
-        return __ldcs(reinterpret_cast<const typename Cache::Word *>(p));
-    };
+    Window win;
+    win.init(tiles, 32 * NC);
+    auto grp = [&](int gg) -> TbGroup { return band_group<NC, NC>(strips, tb, tlen, col_lo, gg); };
     WarpCig cg{A.cig + P.cig_off, w.n, (uint32_t)w.op, w.len};
     int i = w.i, j = w.j, state = w.state;
-    band_walk<NC>(i, j, state, col_lo, cg, cache, load, g);
+    tb_walk(i, j, state, col_lo, cg, win, grp, [&](int a, int b) { return band_force(g, a, b); });
     if (G.last) {
         if (i >= 0) cg.push(2, i + 1);
         if (j >= 0) cg.push(1, j + 1);
@@ -1157,14 +1169,15 @@ cudaError_t band_launch_finish(const BandPlan &bp, int k, const BandDev &D, cons
     memset(b.mat, 0, sizeof(b.mat));
     memcpy(b.mat, mat, (size_t)m * m);
     b.m = m, b.flag = flag, b.block = bp.block;
-    const int grid = (W.npair + FIN_WARPS - 1) / FIN_WARPS;
     const bool stk = singletrack_tracks(flag, b.block) && !(flag & AW_EZ_SCORE_ONLY);
+    const int fw = stk ? fin_warps<true>() : fin_warps<false>();
+    const int grid = (W.npair + fw - 1) / fw;
     if (bp.nc == 4) {
-        if (stk) ksw_band_finish_kernel<true, 4><<<grid, 32 * FIN_WARPS, 0, st>>>(b);
-        else ksw_band_finish_kernel<false, 4><<<grid, 32 * FIN_WARPS, 0, st>>>(b);
+        if (stk) ksw_band_finish_kernel<true, 4><<<grid, 32 * fw, 0, st>>>(b);
+        else ksw_band_finish_kernel<false, 4><<<grid, 32 * fw, 0, st>>>(b);
     } else {
-        if (stk) ksw_band_finish_kernel<true, 8><<<grid, 32 * FIN_WARPS, 0, st>>>(b);
-        else ksw_band_finish_kernel<false, 8><<<grid, 32 * FIN_WARPS, 0, st>>>(b);
+        if (stk) ksw_band_finish_kernel<true, 8><<<grid, 32 * fw, 0, st>>>(b);
+        else ksw_band_finish_kernel<false, 8><<<grid, 32 * fw, 0, st>>>(b);
     }
     return cudaGetLastError();
 }

@@ -586,12 +586,12 @@ constexpr int BT_WARPS = 4;
 
 // ksw_backtrack of minimap2/ksw2.h:160-192 over the strip layout; in full mode
 // every visited cell is a stored cell, so the off/off_end forcing never fires.
-// One warp per pair walks in lockstep and fetches traceback tiles cooperatively.
+// One warp per pair walks in runs over prefetched tiles (tb_walk.cuh).
 __global__ void __launch_bounds__(32 * BT_WARPS)
     ksw_backtrack_full_kernel(const KswPair *pairs, const int32_t *order, int n, const uint8_t *tb_arena,
                               KswOut *out, uint32_t *cig, int flag) {
-    using Cache = TileCache<8>;
-    __shared__ Cache::Word tiles[BT_WARPS][2 * Cache::NW];
+    using Window = TbWindow<KSW_COLS, KSW_COLS, 0, true>;
+    __shared__ __align__(16) uint8_t tiles[BT_WARPS][Window::BYTES];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int pi = blockIdx.x * BT_WARPS + warp;
     if (pi >= n) return;
@@ -599,33 +599,23 @@ __global__ void __launch_bounds__(32 * BT_WARPS)
     const KswPair P = pairs[idx];
     KswOut o = out[idx];
     const int qlen = P.qlen, tlen = P.tlen;
-    int i0 = tlen - 1, j0 = qlen - 1;
+    int i = tlen - 1, j = qlen - 1, state = 0;
     if (o.zdropped || o.stopped) return;
     if (flag & AW_EZ_SEMIGLOBAL_END) {
-        if (o.mqe > o.mte) o.score = o.mqe, i0 = o.mqe_t, j0 = qlen - 1;
-        else o.score = o.mte, i0 = tlen - 1, j0 = o.mte_q;
+        if (o.mqe > o.mte) o.score = o.mqe, i = o.mqe_t, j = qlen - 1;
+        else o.score = o.mte, i = tlen - 1, j = o.mte_q;
     }
     const uint8_t *tb = tb_arena + P.tb_off;
     const int64_t stride_k = qlen + KSW_LAG;
-    Cache cache;
-    cache.init(tiles[warp]);
-    auto load = [&](int gg, int jj) -> uint2 {
-        if (gg < 0 || jj < 0 || jj >= qlen || (gg << 3) >= tlen) return make_uint2(0, 0);
+    Window win;
+    win.init(tiles[warp], KSW_GROUPS * KSW_COLS);
+    auto grp = [&](int gg) -> TbGroup {
+        if (gg < 0 || gg * KSW_COLS >= tlen) return TbGroup{tb, 0, -1};
         const int s = gg / KSW_GROUPS, L = gg % KSW_GROUPS;
-        return __ldcs(reinterpret_cast<const uint2 *>(
-            tb + (((int64_t)s * stride_k + jj + L) * KSW_GROUPS + L) * KSW_COLS));
+        return TbGroup{tb + (((int64_t)s * stride_k + L) * KSW_GROUPS + L) * KSW_COLS, 0, qlen - 1};
     };
     WarpCigar w{cig + P.cig_off, 0, 0, 0};
-    int i = i0, j = j0, state = 0;
-    while (i >= 0 && j >= 0) {
-        const uint32_t cellv = cache.byte(i >> 3, j, i & 7, load);
-        if (state == 0) state = cellv & 7;
-        else if (!(cellv >> (state + 2) & 1)) state = 0;
-        if (state == 0) state = cellv & 7;
-        if (state == 0) w.push(0, 1), --i, --j;
-        else if (state == 1 || state == 3) w.push(2, 1), --i;
-        else w.push(1, 1), --j;
-    }
+    tb_walk(i, j, state, 0, w, win, grp, [](int, int) { return -1; });
     if (i >= 0) w.push(2, i + 1);
     if (j >= 0) w.push(1, j + 1);
     o.n_cigar = w.finish(!(flag & AW_EZ_REV_CIGAR));

@@ -1,13 +1,21 @@
 // Warp-cooperative traceback reads for the strip layouts.
 //
 // A traceback walk (ksw_backtrack, the Singletrack reconstruction) is a chain of
-// dependent one-byte reads that move up and left through the matrix; read one by
-// one from HBM each costs a full memory latency.  Here all 32 lanes of a warp run
-// the same walk in lockstep (the walk is uniform), and a miss makes the warp fetch
-// a whole tile of lane-words around the missing cell in one parallel round:
-// TR rows (or anti-diagonals) x TG column groups of 8 target columns, the rows and
-// groups at and before the miss, which is where the walk goes next.  Two tile slots, so the
-// vertical and horizontal probes of a Singletrack gap search stay cached together.
+// dependent decisions that moves up and left through the matrix.  Read one byte at a time
+// it costs a shared-memory latency and a branch per cell (125 ns measured).  Here the 32
+// lanes of a warp look at the next 32 cells of the walk's current direction at once: down
+// the diagonal while the state is M, along the row or column inside a gap; a ballot gives
+// the length of the run that the serial walk would take, so the walk advances a whole run
+// per round and only changes of state are serial.
+//
+// The cells come from tiles of 32 rows x 64 columns in shared memory.  A walk mostly
+// follows the diagonal, so while a tile is walked the next three down the diagonal are on
+// their way (cp.async, one group per tile); each is placed 16 columns ahead of the
+// diagonal, so that it still covers the walk after a drift of 16 columns either way.  A
+// larger drift is a miss: the tile at the walk's position is fetched and the tiles ahead of
+// it again.  Bound by the tiles' latency; measured against byte-by-byte walks over tiles
+// fetched on a miss: one 5 kb pair 1.25 -> 0.14 ms, 768 pairs of 0.2-20 kb 6.8 -> 0.8 ms, four
+// banded pairs of 60-160 kb 85 -> 6.8 ms, 128 Singletrack pairs of 2-8 kb 6.6 -> 0.65 ms.
 #pragma once
 #include <stdint.h>
 #include <climits>
@@ -15,55 +23,152 @@
 
 namespace aw {
 
-// WB: bytes per lane-word, 4 or 8 (state bytes) or 16 (Singletrack v|u tracks); a tile is
-// TR_ rows (matrix rows, or anti-diagonals for the anti-diagonal layout) x TG_ groups.
-template <int WB, int TR_ = 32, int TG_ = 8>
-struct TileCache {
-    static constexpr int TR = TR_, TG = TG_, NW = TR * TG;
-    using Word = typename std::conditional<WB == 16, uint4,
-                                           typename std::conditional<WB == 8, uint2, uint32_t>::type>::type;
-    Word *slot[2];  // shared memory, NW words each
-    int g0[2], j0[2];
-    int next;
+// The stored rows of one column group: row jlo's word lies at p, the others `stride` (of the
+// layout) apart; no row is stored when jhi < jlo.
+struct TbGroup {
+    const uint8_t *p;
+    int jlo, jhi;
+};
 
-    __device__ void init(Word *smem) {
-        slot[0] = smem, slot[1] = smem + NW;
-        g0[0] = g0[1] = INT_MIN / 2, j0[0] = j0[1] = INT_MIN / 2;
-        next = 0;
+template <int WB>
+__device__ __forceinline__ void tb_copy(uint32_t dst, const uint8_t *src, bool ok) {
+    // zero bytes read (the word becomes zero) when the cell is not stored
+    asm volatile("cp.async.ca.shared.global [%0], [%1], %2, %3;" ::"r"(dst), "l"(src), "n"(WB), "r"(ok ? WB : 0)
+                 : "memory");
+}
+__device__ __forceinline__ void tb_wait(int pending) {
+    if (pending <= 0) asm volatile("cp.async.wait_group 0;" ::: "memory");
+    else if (pending == 1) asm volatile("cp.async.wait_group 1;" ::: "memory");
+    else if (pending == 2) asm volatile("cp.async.wait_group 2;" ::: "memory");
+    else asm volatile("cp.async.wait_group 3;" ::: "memory");
+}
+
+// WB: bytes per word (4, 8 or 16) covering CPW columns (Singletrack words hold the v bytes,
+// then the u bytes); DEPTH: rows below a cell's own that a look at it needs as well.
+// AHEAD: fetch the tiles down the diagonal ahead of the walk (four slots, else two).
+template <int WB, int CPW, int DEPTH, bool AHEAD>
+struct TbWindow {
+    static constexpr int TR = 32, TG = 64 / CPW, PITCH = TR - DEPTH;
+    static constexpr int RS = TG * WB + (WB == 16 ? 16 : 8);  // row stride: a diagonal spreads over the banks
+    static constexpr int NS = AHEAD ? 4 : 2, SLOT = TR * RS, BYTES = NS * SLOT;
+    const uint8_t *sm;
+    uint32_t sa;
+    int64_t stride;   // bytes between a group's rows in the layout
+    int cur, cg, cj;  // the current tile: slot, last column group, last row
+    int og, oj, oseq; // lane s < NS: the same of slot s, and its number
+    int issued;       // tiles fetched so far (tile n lies in slot n % NS)
+
+    __device__ void init(uint8_t *smem, int64_t row_stride) {
+        sm = smem, sa = (uint32_t)__cvta_generic_to_shared(smem), stride = row_stride;
+        cur = 0, cg = cj = INT_MIN / 2, og = oj = INT_MIN / 2, oseq = -1, issued = 0;
     }
 
-    // Byte c (0..WB-1) of the lane-word covering column group g = i >> 3 and row j.
-    // LOAD(g, j) returns the word (zero when the cell is not stored).
-    template <class LOAD>
-    __device__ uint32_t byte(int g, int j, int c, LOAD &&load) {
-        int k = -1;
-#pragma unroll
-        for (int t = 0; t < 2; ++t)
-            if (g <= g0[t] && g > g0[t] - TG && j <= j0[t] && j > j0[t] - TR) k = t;
-        if (k < 0) {  // uniform across the warp: every lane runs the same walk
-            k = next;
-            next ^= 1;
-            g0[k] = g, j0[k] = j;
-            const int lane = threadIdx.x & 31;
-            Word *dst = slot[k];
-            __syncwarp();
+    // Starts the copy of the tile whose last cell is (group g, row j); GRP(gg) describes group gg.
+    template <class GRP>
+    __device__ void fetch(int g, int j, GRP &&grp) {
+        const int lane = threadIdx.x & 31, slot = issued % NS;
+        if (j >= 0) {
+            const TbGroup G = grp(g - lane % TG);
+            constexpr int RPI = 32 / TG;
+            const uint32_t dst = sa + slot * SLOT + (lane / TG) * RS + (lane % TG) * WB;
 #pragma unroll 4
-            for (int w = lane; w < NW; w += 32) dst[w] = load(g - (w % TG), j - (w / TG));
-            __syncwarp();
+            for (int it = 0; it < TR / RPI; ++it) {
+                const int row = j - (it * RPI + lane / TG);
+                const bool ok = row >= G.jlo && row <= G.jhi;
+                tb_copy<WB>(dst + it * RPI * RS, G.p + (ok ? (int64_t)(row - G.jlo) * stride : 0), ok);
+            }
         }
-        const Word wd = slot[k][(j0[k] - j) * TG + (g0[k] - g)];
-        uint32_t x;
-        if (WB == 16) {
-            const uint4 &q = reinterpret_cast<const uint4 &>(wd);
-            x = c < 4 ? q.x : c < 8 ? q.y : c < 12 ? q.z : q.w;
-        } else if (WB == 8) {
-            const uint2 &q = reinterpret_cast<const uint2 &>(wd);
-            x = c < 4 ? q.x : q.y;
+        asm volatile("cp.async.commit_group;" ::: "memory");
+        if (lane == slot) og = g, oj = j, oseq = issued;
+        ++issued;
+    }
+
+    // Makes the tile that covers (i, j) and (i, j - DEPTH) the current one.
+    template <class GRP>
+    __device__ void ensure(int i, int j, GRP &&grp) {
+        const int g = i / CPW, jd = max(j - DEPTH, 0);
+        if (g <= cg && g > cg - TG && j <= cj && jd > cj - TR) return;
+        const int lane = threadIdx.x & 31;
+        __syncwarp();
+        const unsigned b = __ballot_sync(0xffffffffu, lane < NS && g <= og && g > og - TG && j <= oj && jd > oj - TR);
+        int seq;
+        if (b) {
+            cur = __ffs(b) - 1;
+            seq = __shfl_sync(0xffffffffu, oseq, cur);
+            cg = __shfl_sync(0xffffffffu, og, cur), cj = __shfl_sync(0xffffffffu, oj, cur);
         } else {
-            x = reinterpret_cast<const uint32_t &>(wd);
+            tb_wait(0);  // a slot may only be refilled once its copy is done
+            __syncwarp();
+            seq = issued, cur = issued % NS, cg = g, cj = j;
+            fetch(g, j, grp);
         }
-        return (x >> (8 * (c & 3))) & 0xffu;
+        if (AHEAD) {
+            // older tiles are complete with this one, so their slots are free again
+            if (b) tb_wait(issued - 1 - seq), __syncwarp();
+            while (issued - 1 - seq < NS - 1) {
+                const int row = cj - PITCH * (issued - seq);
+                fetch(max(i - (j - row) + 16, 0) / CPW, row, grp);
+            }
+            if (!b) tb_wait(issued - 1 - seq);
+        } else {
+            tb_wait(0);
+        }
+        __syncwarp();
+    }
+
+    // Makes the tile whose last cell is (i, j)'s group and row the current one.
+    template <class GRP>
+    __device__ void corner(int i, int j, GRP &&grp) {
+        const int g = i / CPW;
+        if (g == cg && j == cj) return;
+        __syncwarp();
+        const unsigned b = __ballot_sync(0xffffffffu, (threadIdx.x & 31) < NS && g == og && j == oj);
+        cur = b ? __ffs(b) - 1 : issued % NS, cg = g, cj = j;
+        if (!b) fetch(g, j, grp), tb_wait(0);
+        __syncwarp();
+    }
+
+    // Whether (i, j) and (i, j - DEPTH) lie in the current tile (rows above the matrix count).
+    __device__ __forceinline__ bool has(int i, int j) const {
+        return i / CPW > cg - TG && max(j - DEPTH, 0) > cj - TR;
+    }
+    // Byte of the cell (i, j) of the current tile (part 1: the second half of the word).
+    __device__ __forceinline__ uint32_t at(int i, int j, int part = 0) const {
+        return sm[cur * SLOT + (cj - j) * RS + (cg - i / CPW) * WB + part * CPW + i % CPW];
     }
 };
+
+constexpr unsigned TB_ALL = 0xffffffffu;
+
+// ksw_backtrack (minimap2/ksw2.h:160-192) from (i, j) until the walk leaves the matrix or the
+// columns >= col_lo, in runs.  FORCE(i, j): the move forced outside the computed band (1:
+// deletion, 2: insertion) or -1.
+template <class Window, class GRP, class FORCE, class Cig>
+__device__ void tb_walk(int &i, int &j, int &state, int col_lo, Cig &cg, Window &win, GRP &&grp, FORCE &&force) {
+    const int lane = threadIdx.x & 31;
+    while (i >= 0 && j >= 0 && i >= col_lo) {
+        win.ensure(i, j, grp);
+        const int di = state == 0 || state == 1 || state == 3, dj = state == 0 || state == 2 || state == 4;
+        const int li = i - (di ? lane : 0), lj = j - (dj ? lane : 0);
+        const bool in = li >= 0 && lj >= 0 && li >= col_lo && win.has(li, lj);
+        const int fc = in ? force(li, lj) : -1;
+        const uint32_t c = in && fc < 0 ? win.at(li, lj) : 0u;
+        // the cell takes the walk's state on: an M cell in state 0, a continued gap otherwise
+        const bool on = in && fc < 0 && (state == 0 ? (c & 7u) == 0 : ((c >> (state + 2)) & 1u) != 0);
+        const unsigned off = __ballot_sync(TB_ALL, !on);
+        const int run = off ? __ffs(off) - 1 : 32;
+        if (run > 0) {
+            cg.push(state == 0 ? 0u : di ? 2u : 1u, run);
+            i -= di ? run : 0, j -= dj ? run : 0;
+        }
+        // the cell that ends the run, if it is there: a forced move, or its own state
+        if (run == 32 || !__shfl_sync(TB_ALL, in ? 1 : 0, run)) continue;
+        const int f = __shfl_sync(TB_ALL, fc, run);
+        state = f >= 0 ? f : (int)(__shfl_sync(TB_ALL, c, run) & 7u);
+        if (state == 0) continue;  // an M cell after a gap: the next round takes its run
+        if (state == 1 || state == 3) cg.push(2, 1), --i;
+        else cg.push(1, 1), --j;
+    }
+}
 
 }  // namespace aw
