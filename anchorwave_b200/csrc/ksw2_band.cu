@@ -25,22 +25,34 @@
 //     on the last anti-diagonal; the anti-diagonal loop stops at the first empty
 //     band (:151-154, zdropped = 1).
 // Rows above the matrix (j < 0) only refresh the stale score; rows below it and
-// columns right of it never reach a cell of the matrix.  Rows where a lane's 8
-// cells all lie strictly inside the band take the full-matrix cell arithmetic
-// unchanged (the fast path); the rest go through the per-cell rules above.
+// columns right of it never reach a cell of the matrix.
+//
+// Three forms of a step (one row of every lane), chosen for the whole warp:
+//   * interior: every cell strictly inside the band, the full-matrix arithmetic unchanged;
+//     the steps where that holds for all lanes are one range of k, solved once per strip;
+//   * edge: the rules above from closed forms in the distance of a cell to the band's
+//     right edge, e = j + w - t.  The band edge crosses a strip during its first rows and
+//     the strip on the right cannot start before, so these steps are the chain that bounds
+//     long pairs;
+//   * corner (rows 0 and qlen-1, rows above the matrix, and the anti-diagonals where the
+//     rule for st0 changes): the same rules from st0 and en0 of every cell.
+// The stale scores are kept as the last fill of each column in a register of its own, which
+// interior steps refresh for nothing.
 //
 // Work decomposition: every (pair, strip) is a unit of a device queue, ordered so
-// that a strip is always taken after the strip on its left; a warp takes a unit,
-// waits (bounded) for the left strip's published rows in global memory and sweeps
-// its rows with the one-row lane skew of the full-matrix kernel.  Many warps,
-// across CTAs, work on one pair at once, so a single long interval fills the GPU.
+// that a strip is always taken after the strip on its left; a warp takes a unit and
+// sweeps its rows with the one-row lane skew of the full-matrix kernel, reading its left
+// column as the strip on the left writes it.  Many warps, across CTAs, work on one pair at
+// once, so a single long interval fills the GPU.  An entry of a boundary column carries a
+// mark that says it is written (the columns are cleared before the first pass), so a strip
+// reads eight rows ahead and waits (bounded) only for entries that are not there yet: no
+// fence and no counter between the strips.
 #include "ksw2_band.h"
 #include "tb_walk.cuh"
 
 #include <algorithm>
 #include <climits>
 #include <cstring>
-#include <cuda/atomic>
 
 namespace aw {
 
@@ -138,7 +150,7 @@ struct BandArgs {
     const BandStripDev *strips;
     const int2 *units;
     int32_t n_units;
-    int32_t *queue, *progress, *error;
+    int32_t *queue, *error;
     uint8_t *tb;
     uint2 *bnd;
     BandRes *res;
@@ -155,10 +167,21 @@ struct BandArgs {
 };
 
 constexpr uint64_t WAIT_NS = 20ull * 1000 * 1000 * 1000;  // bounded wait on the left strip
-// rows per publication of a strip's boundary column: the strip on the right starts a row once
-// the PUB rows from it are published (lane 31 finishes row j 31 steps after lane 0), so a hop
-// between strips costs strip width + 31 + PUB lane-steps
+// Rows of the left column read at a time: a strip starts a row once the group it lies in is
+// written (lane 31 finishes row j 31 steps after lane 0), so a hop between strips costs strip
+// width + 31 + PUB lane-steps.
 constexpr int PUB = 8;
+// Mark of a written boundary entry: the byte above its x, v and x2.
+constexpr uint32_t BND_MARK = 0x80000000u;
+
+__device__ __forceinline__ uint2 bnd_load(const uint2 *p) {
+    uint64_t v;
+    asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
+    return make_uint2((uint32_t)v, (uint32_t)(v >> 32));
+}
+__device__ __forceinline__ void bnd_store(uint2 *p, uint32_t x, uint32_t h) {
+    asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p), "l"((uint64_t)h << 32 | (x | BND_MARK)) : "memory");
+}
 
 // NC target columns per lane (strips of 32*NC columns): 8 for throughput, 4 for a shorter
 // pipeline lag between strips when few long pairs run.
@@ -186,7 +209,7 @@ __global__ void __launch_bounds__(256, 2) ksw_band_kernel(BandArgs A) {
         const int s = un.y;
         const BandStripDev St = A.strips[P.strip0 + s];
         // the last row this pass needs: the strip's last band row, or in a recompute round the
-        // walk's row (the same limit for every strip of the pair, producers included)
+        // walk's row
         int wlim = INT_MAX;
         if (A.walk) {
             const BandWalkState wk = A.walk[un.x];
@@ -197,33 +220,42 @@ __global__ void __launch_bounds__(256, 2) ksw_band_kernel(BandArgs A) {
         volatile int32_t *stop_word = &A.res[un.x].stopped;
         if (A.deadline && *stop_word) continue;  // the pair stopped at the deadline
         const Geom g{P.qlen, P.tlen, P.w, P.qlen + P.tlen - 1, P.rb, ~(B - 1)};
-        const int qlen = P.qlen, tlen = P.tlen, qm1 = qlen - 1, tm1 = tlen - 1;
+        const int qlen = P.qlen, tlen = P.tlen, qm1 = qlen - 1, tm1 = tlen - 1, w = P.w;
         const int rlim = min(g.nd, g.rb);
         const uint8_t *qs = A.qcodes + P.qoff, *ts = A.tcodes + P.toff;
         const int col0 = s * 32 * C + lane * C;
         const bool last_strip = s + 1 == P.nstrip;
-        // the strip on the left: its published rows and its final H (an empty strip
+        // the strip on the left: its stored rows and, after them, its final H (an empty strip
         // computes nothing, so its column keeps the initial values)
         int prod_lo = 0, prod_hi = -1;
         const uint2 *bnd_prod = nullptr;
-        int32_t *prog_prod = nullptr;
         if (s > 0) {
             const BandStripDev Pr = A.strips[P.strip0 + s - 1];
             if (min(Pr.jend, wlim) >= Pr.jlo) {
                 prod_lo = Pr.jlo, prod_hi = min(Pr.jend, wlim);
                 bnd_prod = A.bnd + Pr.bnd_off;
-                prog_prod = A.progress + PROG_STRIDE * (P.strip0 + s - 1);
             }
         }
-        uint2 *bnd_me = A.bnd + St.bnd_off;
-        int32_t *prog_me = A.progress + PROG_STRIDE * (P.strip0 + s);
-        uint8_t *tbp = CIGAR ? A.tb + St.tb_off : nullptr;
+        // a recompute round reads the columns of the first pass and writes none
+        uint2 *bnd_me = lane == 31 && !last_strip && !A.walk ? A.bnd + St.bnd_off : nullptr;
         const bool store_tb = CIGAR && (!P.ckpt || A.store_ckpt);  // this strip's traceback is kept
+        // this lane's traceback word of step k: tbp + k * 32 * CB
+        uint8_t *tbp = CIGAR ? A.tb + St.tb_off + ((int64_t)(jstart - jlo) * 32 + lane) * CB : nullptr;
         BandRes *R = A.res + un.x;
         // lane constants of the closed-form bounds: floor16 and the block end of the lane's columns
         const int F16 = col0 & ~15, XB = (col0 & g.bmask) + B - 1;
+        // Score fill right of the band while st0 = (r-w+1)>>1: en0-st0+1 is w+1 where e is even
+        // and w where it is odd, so the fill reaches the columns with e >= -2 pad (even) and
+        // e >= 1 - 2 pad (odd), pad = what rounds that length up to 16.
+        const int fill_even = A.generic ? 0 : 2 * (-(w + 1) & 15), fill_odd = A.generic ? -1 : 2 * (-w & 15) - 1;
+        // rows where the lane's cells all lie strictly inside the band, with natural neighbours
+        const int fa = max(1, col0 + C + 1 - w);
+        const int fb = col0 + C > tm1 ? -1 : min(min(qlen - 2, rlim - col0 - C), col0 > 0 ? col0 + w - 2 : w);
+        // steps where that holds for every lane
+        const int kf0 = (int)__reduce_max_sync(FULL, max(fa, jstart) + lane) - jstart;
+        const int kf1 = (int)__reduce_min_sync(FULL, min(fb, jend) + lane) - jstart + 1;
 
-        int ut[C], yt[C], y2t[C], H[C];
+        int ut[C], yt[C], y2t[C], H[C], ss[C];
         uint32_t rlo[C], rhi[C];
 #pragma unroll
         for (int c = 0; c < C; ++c) {
@@ -233,266 +265,290 @@ __global__ void __launch_bounds__(256, 2) ksw_band_kernel(BandArgs A) {
             rhi[c] = S.tab_hi[tc];
             ut[c] = -S.qe, yt[c] = -S.qe, y2t[c] = -S.qe2;
             H[c] = AW_NEG_INF;
+            ss[c] = 0;
         }
-        uint32_t sreg0 = 0, sreg1 = 0;  // stale score bytes of columns 0-3 / 4-7
-        int lastfast = INT_MIN;          // row of the latest fast step (all 8 scores fresh there)
         const uint32_t init_pack = pack3(-S.qe, -S.qe, -S.qe2, 0);
-        uint32_t carry = 0, qchunk = 0;
+        uint32_t carry = 0;
         int Hcarry = AW_NEG_INF;
-        uint2 bchunk = make_uint2(init_pack, (uint32_t)AW_NEG_INF);
-        int seen = INT_MIN;  // lane 0: the left strip's progress count last read
-        bool failed = false;
+        unsigned long long mte_key = 0;  // last strip: the lane that owns the last column
+        const int pm = A.sse_st ? INT_MAX : 0;  // strict end rule: mirrored positions
+        // lane 0's left values of row jr: x, v, x2 with the mark, and the H on the left
+        auto left_of = [&](int jr) -> uint2 {
+            if (s == 0) return make_uint2(pack3(-S.qe, edge_diff(jr, S), -S.qe2, 0) | BND_MARK, (uint32_t)AW_NEG_INF);
+            if (!bnd_prod || jr < prod_lo) return make_uint2(init_pack | BND_MARK, (uint32_t)AW_NEG_INF);
+            return bnd_load(bnd_prod + (min(jr, prod_hi + 1) - prod_lo));
+        };
+        auto code_of = [&](int jr) -> uint32_t { return jr >= 0 && jr < qlen ? qs[jr] : 0u; };
+        // lane i holds what lane 0 needs for row jstart + (k & ~31) + i: the next group's entries
+        // and the next 32 query codes are on their way while the current ones are used
+        uint2 ahead = make_uint2(BND_MARK, 0u);
+        if (lane < PUB) ahead = left_of(jstart + lane);
+        uint32_t qnext = code_of(jstart + lane), qcur = 0, bx = 0;
+        int bh = 0;
+        bool failed = false, stopped = false;
         const int nsteps = jend - jstart + 32;
-        for (int k = 0; k < nsteps; ++k) {
-            if ((k & 31) == 0 && A.deadline) {
-                // cooperative stop, polled every 32 rows (ksw2_progress.c:30-38 polls every
-                // 256 anti-diagonals); the pair's other strips see the flag and stop too
-                int st = 0;
-                if (lane == 0) {
-                    st = *stop_word;
-                    if (!st && aw_deadline_passed(A.deadline)) st = 1, atomicExch((int32_t *)stop_word, 1);
+        for (int kb = 0; kb < nsteps; kb += PUB) {
+            if ((kb & 31) == 0) {
+                if (A.deadline) {
+                    // cooperative stop, polled every 32 rows (ksw2_progress.c:30-38 polls every
+                    // 256 anti-diagonals); the pair's other strips see the flag and stop too
+                    int st = 0;
+                    if (lane == 0) {
+                        st = *stop_word;
+                        if (!st && aw_deadline_passed(A.deadline)) st = 1, atomicExch((int32_t *)stop_word, 1);
+                    }
+                    if (__shfl_sync(FULL, st, 0)) {
+                        stopped = true;
+                        break;
+                    }
                 }
-                if (__shfl_sync(FULL, st, 0)) break;
+                qcur = qnext;
+                qnext = code_of(jstart + kb + 32 + lane);
             }
-            if ((k & 31) == 0) {
-                const int J = jstart + k, jr = J + lane;
-                qchunk = (jr >= 0 && jr < qlen) ? qs[jr] : 0u;
-            }
-            if (prog_prod && (k & (PUB - 1)) == 0) {
-                // rows J..J+PUB-1 of the left strip (published rows, or past its last row its
-                // final H with the initial x/v/x2), loaded by the lanes that hold them in the
-                // 32-row chunk the step shuffles from (lane L holds row jstart + (k & ~31) + L)
-                const int J = jstart + k, jr = jstart + (k & ~31) + lane;
-                const int need = J + PUB - 1 > prod_hi ? prod_hi + 2 : J + PUB;
-                if (J + PUB - 1 >= prod_lo && lane == 0 && seen < need) {
-                    // one poller per warp with back-off; the bound and the error flag
-                    // (another warp gave up) are checked every 32 polls
-                    cuda::atomic_ref<int32_t, cuda::thread_scope_device> pr(*prog_prod);
-                    seen = pr.load(cuda::memory_order_acquire);
-                    if (seen < need) {
-                        const uint64_t t0 = globaltimer();
-                        unsigned ns = 32, polls = 0;
-                        while ((seen = pr.load(cuda::memory_order_acquire)) < need) {
-                            __nanosleep(ns);
-                            ns = ns < 1024 ? ns * 2 : ns;
-                            if (A.deadline && *stop_word) break;  // the left strip stopped
-                            if ((++polls & 31) == 0 &&
-                                (globaltimer() - t0 > WAIT_NS || *(volatile int32_t *)A.error)) {
-                                failed = true;
-                                break;
-                            }
+            const bool mine = (lane & ~(PUB - 1)) == (kb & 31);
+            if (!__all_sync(FULL, !mine || (ahead.x & BND_MARK))) {
+                // the left strip is not there yet: poll with back-off; the bound and the error
+                // flag (another warp gave up) are checked every 32 polls
+                const uint64_t t0 = globaltimer();
+                unsigned ns = 16, polls = 0;
+                for (;;) {
+                    if (mine && !(ahead.x & BND_MARK)) ahead = left_of(jstart + (kb & ~31) + lane);
+                    if (__all_sync(FULL, !mine || (ahead.x & BND_MARK))) break;
+                    if (A.deadline && __shfl_sync(FULL, lane == 0 ? *stop_word : 0, 0)) {
+                        stopped = true;  // the left strip stopped
+                        break;
+                    }
+                    if ((++polls & 31) == 0) {
+                        const int bad = globaltimer() - t0 > WAIT_NS || *(volatile int32_t *)A.error;
+                        if (__any_sync(FULL, bad)) {
+                            failed = true;
+                            break;
                         }
                     }
+                    __nanosleep(ns);
+                    ns = ns < 256 ? ns * 2 : ns;
                 }
-                failed = __shfl_sync(FULL, failed, 0);
-                if (failed) {
-                    if (lane == 0) atomicExch(A.error, 1);
-                    break;
-                }
-                if (A.deadline && __shfl_sync(FULL, lane == 0 ? *stop_word : 0, 0)) break;
-                if ((lane & ~(PUB - 1)) == (k & 31)) {
-                    if (jr >= prod_lo && jr <= prod_hi) bchunk = __ldcg(bnd_prod + (jr - prod_lo));
-                    else if (jr > prod_hi) bchunk = make_uint2(init_pack, __ldcg(bnd_prod + (prod_hi - prod_lo + 1)).y);
-                    else bchunk = make_uint2(init_pack, (uint32_t)AW_NEG_INF);
-                }
+                if (failed && lane == 0) atomicExch(A.error, 1);
+                if (failed || stopped) break;
             }
-            const uint32_t qv = __shfl_sync(FULL, qchunk, k & 31);
-            const uint32_t bx = __shfl_sync(FULL, bchunk.x, k & 31);
-            const int bh = (int)__shfl_sync(FULL, bchunk.y, k & 31);
-            const uint32_t in = __shfl_up_sync(FULL, carry, 1);
-            const int Hin = __shfl_up_sync(FULL, Hcarry, 1);
-            const int j = jstart + k - lane;
-            int xs, vs, x2s, Hl;
-            uint32_t qc;
-            if (lane == 0) {
-                qc = qv;
-                if (s == 0) xs = -S.qe, vs = edge_diff(j, S), x2s = -S.qe2, Hl = AW_NEG_INF;
-                else xs = sx8(bx), vs = sx8(bx >> 8), x2s = sx8(bx >> 16), Hl = bh;
-            } else {
-                qc = in >> 24;
-                xs = sx8(in), vs = sx8(in >> 8), x2s = sx8(in >> 16), Hl = Hin;
-            }
-            const bool active = j >= jstart && j <= jend;
-            const int r0 = col0 + j;
-            // all 8 cells strictly inside the band, with natural neighbours: the fast path
-            const bool fast = active && j > 0 && col0 > g.st0(r0) && col0 + C - 1 < g.en0(r0 + C - 1) &&
-                              r0 + C - 1 < rlim;
-            // one path for the whole warp, so an edge step costs the edge code once
-            const bool warp_fast = __all_sync(FULL, fast || !active);
-            uint32_t w0 = 0, w1 = 0, w2 = 0, w3 = 0;  // traceback bytes of this lane-step
-            if (active) {
-                if (warp_fast && ARGMAX && !store_tb) {
-                    // no traceback is kept for this strip (a recomputed pair's first pass, or a
-                    // pair whose band empties): the cells without their state bytes
-                    const uint32_t sel = qc * 0x1111u + 0x8880u;
-#pragma unroll
-                    for (int c = 0; c < C; ++c) {
-                        int d = 0;
-                        const int sc = prmt_sx(rlo[c], rhi[c], sel);
-                        cell<false, RIGHT>(sc, xs, vs, x2s, ut[c], yt[c], y2t[c], d, S);
-                        H[c] += vs;
-                    }
-                    lastfast = j;
-                    carry = pack3(xs, vs, x2s, qc);
-                    Hcarry = H[C - 1];
-                } else if (warp_fast) {
-                    const uint32_t sel = qc * 0x1111u + 0x8880u;
-#pragma unroll
-                    for (int c = 0; c < C; ++c) {
-                        int d = 0;
-                        const int sc = prmt_sx(rlo[c], rhi[c], sel);
-                        cell<ARGMAX, RIGHT>(sc, xs, vs, x2s, ut[c], yt[c], y2t[c], d, S);
-                        H[c] += vs;
-                        if (ARGMAX) {
-                            if (c < 4) w0 |= (uint32_t)d << (8 * c);
-                            else w1 |= (uint32_t)d << (8 * (c - 4));
-                        } else if (ST) {
-                            if (c < 4) w0 |= (uint32_t)(vs & 0xff) << (8 * c), w2 |= (uint32_t)(ut[c] & 0xff) << (8 * c);
-                            else w1 |= (uint32_t)(vs & 0xff) << (8 * (c - 4)), w3 |= (uint32_t)(ut[c] & 0xff) << (8 * (c - 4));
-                        }
-                    }
-                    lastfast = j;
-                    carry = pack3(xs, vs, x2s, qc);
-                    Hcarry = H[C - 1];
-                } else {
-                    if (lastfast != INT_MIN) {
-                        // the fast steps refreshed every score of this lane; rebuild the stale bytes
-                        const uint32_t sl = (uint32_t)qs[lastfast] * 0x1111u + 0x8880u;
-                        sreg0 = sreg1 = 0;
+            if (mine) bx = (ahead.x & 0xffffffu) | qcur << 24, bh = (int)ahead.y;
+            if ((lane & ~(PUB - 1)) == ((kb + PUB) & 31)) ahead = left_of(jstart + ((kb + PUB) & ~31) + lane);
+            const int kend = min(kb + PUB, nsteps);
+            int k = kb;
+            if (k >= kf0 && kend <= kf1) {
+                // interior: no tests inside the group
+#pragma unroll 1
+                for (; k < kend; ++k) {
+                    uint32_t in = __shfl_up_sync(FULL, carry, 1);
+                    const uint32_t b = __shfl_sync(FULL, bx, k & 31);
+                    if (lane == 0) in = b;
+                    int xs = sx8(in), vs = sx8(in >> 8), x2s = sx8(in >> 16);
+                    const uint32_t qc = in >> 24, sel = qc * 0x1111u + 0x8880u;
+                    uint32_t w0 = 0, w1 = 0, w2 = 0, w3 = 0;
+                    if (ARGMAX && !store_tb) {
+                        // no traceback is kept for this strip (a recomputed pair's first pass, or a
+                        // pair whose band empties): the cells without their state bytes
 #pragma unroll
                         for (int c = 0; c < C; ++c) {
-                            const uint32_t b = (uint32_t)prmt_sx(rlo[c], rhi[c], sl) & 0xffu;
-                            if (c < 4) sreg0 |= b << (8 * c);
-                            else sreg1 |= b << (8 * (c - 4));
+                            int d = 0;
+                            ss[c] = prmt_sx(rlo[c], rhi[c], sel);
+                            cell<false, RIGHT>(ss[c], xs, vs, x2s, ut[c], yt[c], y2t[c], d, S);
+                            H[c] += vs;
                         }
-                        lastfast = INT_MIN;
-                    }
-                    const uint32_t selj = (j < 0 ? 0u : qc) * 0x1111u + 0x8880u;
-                    int fx = xs, fv = vs, fx2 = x2s, Hf = Hl;
-                    if (j < 0) {
-                        // above the matrix: only the score fill of the reference runs here
-#pragma unroll
-                        for (int c = 0; c < C; ++c) {
-                            const int t = col0 + c, r = r0 + c;
-                            if (t <= tm1 && r >= 0 && r < rlim) {
-                                const int st0 = g.st0(r), en0 = g.en0(r);
-                                const int fe = A.generic ? en0 : st0 + ((en0 - st0 + 16) & ~15) - 1;
-                                if (st0 <= t && t <= fe) {
-                                    const uint32_t b = (uint32_t)prmt_sx(rlo[c], rhi[c], selj) & 0xffu;
-                                    if (c < 4) sreg0 = (sreg0 & ~(0xffu << (8 * c))) | (b << (8 * c));
-                                    else sreg1 = (sreg1 & ~(0xffu << (8 * (c - 4)))) | (b << (8 * (c - 4)));
-                                }
-                            }
-                        }
-                        fx = -S.qe, fv = -S.qe, fx2 = -S.qe2, Hf = H[C - 1];
                     } else {
-                        // Closed forms of the per-cell geometry over this lane-step (cell c: t = col0+c,
-                        // r = r0+c): in band  <=> cB <= c <= cE;  computed (stB <= t <= en16) <=>
-                        // cRlo <= c <= cRhi;  right band edge (t == en0) <=> in band and
-                        // (t == tlen-1 or j == 0 or t >= j+w-1).
-                        const int cB = max(0, j - g.w - col0);
-                        const int cE = min(min(tm1 - col0, j + g.w - col0), min(rlim - 1 - r0, C - 1));
-                        const int cRlo = max(0, 2 * F16 - col0 - j - g.w);
-                        const int cRhi = min(min(XB + qm1 - r0, 2 * XB + g.w - r0), min(min(tm1 - col0, rlim - 1 - r0), C - 1));
-                        const int redge = j + g.w - 1 - col0;  // c >= redge: t >= j+w-1
+#pragma unroll
+                        for (int c = 0; c < C; ++c) {
+                            int d = 0;
+                            ss[c] = prmt_sx(rlo[c], rhi[c], sel);
+                            cell<ARGMAX, RIGHT>(ss[c], xs, vs, x2s, ut[c], yt[c], y2t[c], d, S);
+                            H[c] += vs;
+                            if (ARGMAX) {
+                                if (c < 4) w0 |= (uint32_t)d << (8 * c);
+                                else w1 |= (uint32_t)d << (8 * (c - 4));
+                            } else if (ST) {
+                                if (c < 4) w0 |= (uint32_t)(vs & 0xff) << (8 * c), w2 |= (uint32_t)(ut[c] & 0xff) << (8 * c);
+                                else w1 |= (uint32_t)(vs & 0xff) << (8 * (c - 4)), w3 |= (uint32_t)(ut[c] & 0xff) << (8 * (c - 4));
+                            }
+                        }
+                        if (store_tb) {
+                            uint8_t *dst = tbp + (int64_t)k * (32 * CB);
+                            if (C == 8) {
+                                if (ST) __stcs(reinterpret_cast<uint4 *>(dst), make_uint4(w0, w1, w2, w3));
+                                else __stcs(reinterpret_cast<uint2 *>(dst), make_uint2(w0, w1));
+                            } else {
+                                if (ST) __stcs(reinterpret_cast<uint2 *>(dst), make_uint2(w0, w2));
+                                else __stcs(reinterpret_cast<uint32_t *>(dst), w0);
+                            }
+                        }
+                    }
+                    carry = pack3(xs, vs, x2s, qc);
+                    Hcarry = H[C - 1];
+                    if (src_lane && k >= kf1 - 16) ring[warp][k & 15][lane] = carry;  // the wrap looks 16 rows back
+                    if (bnd_me) bnd_store(bnd_me + (jstart + k - 31 - jlo), carry & 0xffffffu, (uint32_t)Hcarry);
+                }
+                __syncwarp();
+                continue;
+            }
+#pragma unroll 1
+            for (; k < kend; ++k) {
+                uint32_t in = __shfl_up_sync(FULL, carry, 1);
+                int Hl = __shfl_up_sync(FULL, Hcarry, 1);
+                const uint32_t b = __shfl_sync(FULL, bx, k & 31);
+                const int hb = __shfl_sync(FULL, bh, k & 31);
+                if (lane == 0) in = b, Hl = hb;
+                const int j = jstart + k - lane, r0 = col0 + j;
+                int xs = sx8(in), vs = sx8(in >> 8), x2s = sx8(in >> 16);
+                const uint32_t qc = in >> 24, sel = (j < 0 ? 0u : qc) * 0x1111u + 0x8880u;
+                const bool active = j >= jstart && j <= jend;
+                // Closed forms of the per-cell geometry over this lane-step (cell c: t = col0+c,
+                // r = r0+c, e = e0-c): in band <=> cB <= c <= cE; computed (stB <= t <= en16) <=>
+                // cRlo <= c <= cRhi; score filled <=> cB <= c <= fill0 (even c), fill1 (odd c).
+                const int e0 = j + w - col0, cB = j - w - col0;
+                const int cmax = min(tm1 - col0, rlim - 1 - r0), cE = min(e0, cmax);
+                const int cRlo = 2 * (F16 - col0) - cB - 2 * w;
+                const int cRhi = min(min(XB + qm1, 2 * XB + w) - r0, cmax);
+                // the rule for st0: r-qlen+1 once it is above (r-w+1)>>1, where the fill's length
+                // rounds up with the rows left below
+                const bool tail0 = r0 - qm1 > ((r0 - w + 1) >> 1), tail1 = r0 + C - 1 - qm1 > ((r0 + C - w) >> 1);
+                const bool corner = active && (j < 1 || j >= qm1 || (tail0 != tail1 && cRhi > cE));
+                uint32_t w0 = 0, w1 = 0, w2 = 0, w3 = 0;  // traceback bytes of this lane-step
+                if (!__any_sync(FULL, corner)) {
+                    if (active) {
+                        const int f = tail0 ? (A.generic ? 0 : 2 * ((qm1 - j) & 15)) : 0;
+                        const bool odd = e0 & 1;
+                        const int fill0 = e0 + (tail0 ? f : odd ? fill_odd : fill_even);
+                        const int fill1 = e0 + (tail0 ? f : odd ? fill_even : fill_odd);
                         // the band-edge lane st16 and the block wrap stB can only be column col0 (c = 0)
                         if (r0 < rlim) {
                             const int st0 = g.st0(r0), st16 = st0 & ~15, stB = st0 & g.bmask;
                             if (col0 == st16) {
-                                if (st16 == 0) fx = -S.qe, fv = edge_diff(j, S), fx2 = -S.qe2;
-                                else if ((g.st0(r0 - 1) & ~15) == st16) fx = -S.qe, fv = -S.qe, fx2 = -S.qe2;
+                                if (st16 == 0) xs = -S.qe, vs = edge_diff(j, S), x2s = -S.qe2;
+                                else if ((g.st0(r0 - 1) & ~15) == st16) xs = -S.qe, vs = -S.qe, x2s = -S.qe2;
                             } else if (col0 == stB) {
                                 const uint32_t wv = ring[warp][(k + D) & 15][lane + D];
-                                fx = sx8(wv), fv = sx8(wv >> 8), fx2 = sx8(wv >> 16);
+                                xs = sx8(wv), vs = sx8(wv >> 8), x2s = sx8(wv >> 16);
                             }
                         }
-                        // score fill right of the band (st0 <= t <= fe, fe <= en0+15 <= (r+w)/2+15,
-                        // i.e. t <= j+w+30): per cell, in the lanes that reach it
-                        if (cE < C - 1 && col0 + cE + 1 <= j + g.w + 30) {
-#pragma unroll
-                            for (int c = 0; c < C; ++c) {
-                                const int t = col0 + c, r = r0 + c;
-                                if (c > cE && t <= tm1 && r < rlim) {
-                                    const int st0 = g.st0(r), en0 = g.en0(r);
-                                    const int fe = A.generic ? en0 : st0 + ((en0 - st0 + 16) & ~15) - 1;
-                                    if (t <= fe) {
-                                        const uint32_t b = (uint32_t)prmt_sx(rlo[c], rhi[c], selj) & 0xffu;
-                                        if (c < 4) sreg0 = (sreg0 & ~(0xffu << (8 * c))) | (b << (8 * c));
-                                        else sreg1 = (sreg1 & ~(0xffu << (8 * (c - 4)))) | (b << (8 * (c - 4)));
-                                    }
-                                }
-                            }
-                        }
-                        const bool top = j == 0;
+                        const int ctm = tm1 - col0;
 #pragma unroll
                         for (int c = 0; c < C; ++c) {
-                            const int t = col0 + c;
                             const bool inBand = c >= cB && c <= cE;
                             const bool inR = c >= cRlo && c <= cRhi;
-                            uint32_t &sw = c < 4 ? sreg0 : sreg1;
-                            const int sh = 8 * (c & 3);
-                            const uint32_t fresh = (uint32_t)prmt_sx(rlo[c], rhi[c], selj) & 0xffu;
-                            if (inBand) sw = (sw & ~(0xffu << sh)) | (fresh << sh);
-                            const int z0 = sx8(sw >> sh);
-                            int lx = fx, lv = fv, lx2 = fx2;
-                            int uu = top ? edge_diff(t, S) : ut[c];
-                            int yy = top ? -S.qe : yt[c], yy2 = top ? -S.qe2 : y2t[c];
-                            int d = 0;
-                            cell<ARGMAX, RIGHT>(z0, lx, lv, lx2, uu, yy, yy2, d, S);
-                            if (inR) ut[c] = uu, yt[c] = yy, y2t[c] = yy2;
-                            fx = inR ? lx : -S.qe, fv = inR ? lv : -S.qe, fx2 = inR ? lx2 : -S.qe2;
-                            const bool re = t == tm1 || top || c >= redge;
-                            const int hn = r0 + c == 0 ? lv - S.qe_pre : (re && t > 0) ? Hf + uu : H[c] + lv;
-                            if (inBand) {
-                                H[c] = hn;
-                                // end tracking straight into the pair's record (rare cells; the
-                                // packed keys make the ">=" later-wins rule an unsigned max, and
-                                // the strict earlier-wins rule one on the mirrored position)
-                                const int pm = A.sse_st ? INT_MAX : 0;
-                                if (re && t == tm1) atomicMax(&R->mte_key, end_key(hn, pm ^ j));
-                                if (j == qm1) atomicMax(&R->mqe_key, end_key(hn, pm ^ t));
-                                if (j == qm1 && t == tm1) R->score = hn, R->has_score = 1;
-                            }
+                            const bool fresh = c >= cB && c <= ((c & 1) ? fill1 : fill0);
+                            const int sc = prmt_sx(rlo[c], rhi[c], sel);
+                            ss[c] = fresh ? sc : ss[c];
+                            int uu = ut[c], yy = yt[c], yy2 = y2t[c], d = 0;
+                            cell<ARGMAX, RIGHT>(ss[c], xs, vs, x2s, uu, yy, yy2, d, S);
+                            // H[en0] = H[en0-1] + u on the right edge of the band, else H += v
+                            const bool re = (c >= e0 - 1 || c == ctm) && (c > 0 || col0 > 0);
+                            const int hn = re ? Hl + uu : H[c] + vs;
+                            H[c] = inBand ? hn : H[c];
+                            Hl = H[c];
+                            ut[c] = inR ? uu : ut[c], yt[c] = inR ? yy : yt[c], y2t[c] = inR ? yy2 : y2t[c];
                             if (ARGMAX) {
                                 const uint32_t dd = inR ? (uint32_t)d : 0u;
                                 if (c < 4) w0 |= dd << (8 * c);
                                 else w1 |= dd << (8 * (c - 4));
                             } else if (ST) {
-                                const uint32_t bv = inR ? (uint32_t)(lv & 0xff) : 0u, bu = inR ? (uint32_t)(uu & 0xff) : 0u;
+                                const uint32_t bv = inR ? (uint32_t)(vs & 0xff) : 0u, bu = inR ? (uint32_t)(uu & 0xff) : 0u;
                                 if (c < 4) w0 |= bv << (8 * c), w2 |= bu << (8 * c);
                                 else w1 |= bv << (8 * (c - 4)), w3 |= bu << (8 * (c - 4));
                             }
-                            Hf = H[c];
+                            xs = inR ? xs : -S.qe, vs = inR ? vs : -S.qe, x2s = inR ? x2s : -S.qe2;
+                        }
+                        if (last_strip) {
+                            // H of the last column in band: the largest, later rows on a tie
+#pragma unroll
+                            for (int c = 0; c < C; ++c)
+                                if (c == ctm && c >= cB && c <= cE) {
+                                    const unsigned long long key = end_key(H[c], pm ^ j);
+                                    mte_key = key > mte_key ? key : mte_key;
+                                }
+                        }
+                        carry = pack3(xs, vs, x2s, qc);
+                        Hcarry = Hl;
+                    }
+                } else if (active) {
+                    int fx = xs, fv = vs, fx2 = x2s, Hf = Hl;
+                    if (r0 < rlim && j >= 0) {
+                        const int st0 = g.st0(r0), st16 = st0 & ~15, stB = st0 & g.bmask;
+                        if (col0 == st16) {
+                            if (st16 == 0) fx = -S.qe, fv = edge_diff(j, S), fx2 = -S.qe2;
+                            else if ((g.st0(r0 - 1) & ~15) == st16) fx = -S.qe, fv = -S.qe, fx2 = -S.qe2;
+                        } else if (col0 == stB) {
+                            const uint32_t wv = ring[warp][(k + D) & 15][lane + D];
+                            fx = sx8(wv), fv = sx8(wv >> 8), fx2 = sx8(wv >> 16);
                         }
                     }
+                    const bool top = j == 0;
+#pragma unroll
+                    for (int c = 0; c < C; ++c) {
+                        const int t = col0 + c, r = r0 + c;
+                        if (t <= tm1 && r >= 0 && r < rlim) {
+                            const int st0 = g.st0(r), en0 = g.en0(r);
+                            const int fe = A.generic ? en0 : st0 + ((en0 - st0 + 16) & ~15) - 1;
+                            if (st0 <= t && t <= fe) ss[c] = prmt_sx(rlo[c], rhi[c], sel);
+                        }
+                        if (j < 0) continue;  // above the matrix: only the score fill of the reference runs here
+                        const bool inBand = c >= cB && c <= cE;
+                        const bool inR = c >= cRlo && c <= cRhi;
+                        int lx = fx, lv = fv, lx2 = fx2;
+                        int uu = top ? edge_diff(t, S) : ut[c];
+                        int yy = top ? -S.qe : yt[c], yy2 = top ? -S.qe2 : y2t[c];
+                        int d = 0;
+                        cell<ARGMAX, RIGHT>(ss[c], lx, lv, lx2, uu, yy, yy2, d, S);
+                        if (inR) ut[c] = uu, yt[c] = yy, y2t[c] = yy2;
+                        fx = inR ? lx : -S.qe, fv = inR ? lv : -S.qe, fx2 = inR ? lx2 : -S.qe2;
+                        const bool re = t == tm1 || top || c >= e0 - 1;
+                        const int hn = r == 0 ? lv - S.qe_pre : (re && t > 0) ? Hf + uu : H[c] + lv;
+                        if (inBand) {
+                            H[c] = hn;
+                            // end tracking straight into the pair's record (rare cells; the
+                            // packed keys make the ">=" later-wins rule an unsigned max, and
+                            // the strict earlier-wins rule one on the mirrored position)
+                            if (re && t == tm1) atomicMax(&R->mte_key, end_key(hn, pm ^ j));
+                            if (j == qm1) atomicMax(&R->mqe_key, end_key(hn, pm ^ t));
+                            if (j == qm1 && t == tm1) R->score = hn, R->has_score = 1;
+                        }
+                        if (ARGMAX) {
+                            const uint32_t dd = inR ? (uint32_t)d : 0u;
+                            if (c < 4) w0 |= dd << (8 * c);
+                            else w1 |= dd << (8 * (c - 4));
+                        } else if (ST) {
+                            const uint32_t bv = inR ? (uint32_t)(lv & 0xff) : 0u, bu = inR ? (uint32_t)(uu & 0xff) : 0u;
+                            if (c < 4) w0 |= bv << (8 * c), w2 |= bu << (8 * c);
+                            else w1 |= bv << (8 * (c - 4)), w3 |= bu << (8 * (c - 4));
+                        }
+                        Hf = H[c];
+                    }
+                    if (j < 0) fx = -S.qe, fv = -S.qe, fx2 = -S.qe2, Hf = H[C - 1];
                     carry = pack3(fx, fv, fx2, qc);
                     Hcarry = Hf;
                 }
-                if (src_lane) ring[warp][k & 15][lane] = carry;
-                if (store_tb && j >= jlo) {
-                    uint8_t *dst = tbp + ((int64_t)(j - jlo + lane) * 32 + lane) * CB;
-                    if (C == 8) {
-                        if (ST) __stcs(reinterpret_cast<uint4 *>(dst), make_uint4(w0, w1, w2, w3));
-                        else __stcs(reinterpret_cast<uint2 *>(dst), make_uint2(w0, w1));
-                    } else {
-                        if (ST) __stcs(reinterpret_cast<uint2 *>(dst), make_uint2(w0, w2));
-                        else __stcs(reinterpret_cast<uint32_t *>(dst), w0);
+                if (active) {
+                    if (src_lane) ring[warp][k & 15][lane] = carry;
+                    if (j >= jlo) {
+                        if (store_tb) {
+                            uint8_t *dst = tbp + (int64_t)k * (32 * CB);
+                            if (C == 8) {
+                                if (ST) __stcs(reinterpret_cast<uint4 *>(dst), make_uint4(w0, w1, w2, w3));
+                                else __stcs(reinterpret_cast<uint2 *>(dst), make_uint2(w0, w1));
+                            } else {
+                                if (ST) __stcs(reinterpret_cast<uint2 *>(dst), make_uint2(w0, w2));
+                                else __stcs(reinterpret_cast<uint32_t *>(dst), w0);
+                            }
+                        }
+                        if (bnd_me) bnd_store(bnd_me + (j - jlo), carry & 0xffffffu, (uint32_t)Hcarry);
                     }
                 }
-                if (lane == 31 && !last_strip && j >= jlo) bnd_me[j - jlo] = make_uint2(carry & 0xffffffu, (uint32_t)Hcarry);
+                if (B > 16) __syncwarp();
             }
-            if (lane == 31 && !last_strip) {
-                const int jj = jstart + k - 31;
-                if (jj >= jlo && jj <= jend && (((jj - jlo) & (PUB - 1)) == PUB - 1 || jj == jend)) {
-                    if (jj == jend) bnd_me[jend - jlo + 1] = make_uint2(init_pack, (uint32_t)Hcarry);
-                    // the release store orders this lane's boundary writes before the count
-                    cuda::atomic_ref<int32_t, cuda::thread_scope_device> pw(*prog_me);
-                    pw.store(jj == jend ? jj + 2 : jj + 1, cuda::memory_order_release);
-                }
-            }
-            if (B > 16) __syncwarp();
         }
         if (failed) break;
+        if (stopped) continue;
+        // the strip's final H, for the rows below its last one
+        if (bnd_me) bnd_store(bnd_me + (jend - jlo + 1), init_pack, (uint32_t)Hcarry);
+        if (mte_key) atomicMax(&R->mte_key, mte_key);
     }
 }
 
@@ -793,15 +849,6 @@ __global__ void __launch_bounds__(32) ksw_band_round_walk_kernel(BtArgs A, const
     }
 }
 
-// Progress counters of a round (one block per group): the group's strips start from zero, the
-// strip on its left (not recomputed: its boundary column is stored from the first pass) counts
-// as done.
-__global__ void band_round_progress_kernel(int32_t *progress, const BandGroupDev *groups) {
-    const BandGroupDev G = groups[blockIdx.x];
-    for (int k = G.s_first + (int)threadIdx.x; k < G.s_end; k += blockDim.x) progress[PROG_STRIDE * k] = 0;
-    if (threadIdx.x == 0 && G.left >= 0) progress[PROG_STRIDE * G.left] = INT_MAX / 2;
-}
-
 template <bool CIGAR, bool RIGHT, bool ST>
 void *kernel_ptr() {
     return (void *)ksw_band_kernel<CIGAR, RIGHT, ST, 8>;
@@ -1078,10 +1125,9 @@ int band_plan_build(BandPlan &bp, const std::vector<int32_t> &ids, const std::ve
                 const int s0 = groups[c][r].first, s1 = groups[c][r].second;
                 BandGroupDev gd;
                 gd.slot = slot, gd.s_first = pd.strip0 + s0, gd.s_end = pd.strip0 + s1;
-                gd.left = s0 > 0 ? pd.strip0 + s0 - 1 : -1;
                 gd.col_lo = s0 * SW;
                 gd.last = r + 1 == groups[c].size() ? 1 : 0;
-                gd.pad0 = gd.pad1 = 0;
+                gd.pad = 0;
                 bp.groups.push_back(gd);
                 int64_t o = off;
                 for (int s = s0; s < s1; ++s) {
@@ -1118,9 +1164,8 @@ cudaError_t band_launch_dp(const BandPlan &bp, int k, const BandDev &D, const ui
                            const uint8_t *tcodes, const KswScore &S, int flag, int ctas, cudaStream_t st) {
     const BandWave &W = bp.waves[k];
     cudaError_t e;
-    if ((e = cudaMemsetAsync(D.progress + (size_t)PROG_STRIDE * W.strip0, 0,
-                             sizeof(int32_t) * PROG_STRIDE * std::max(W.nstrip, 1), st)) != cudaSuccess)
-        return e;
+    // no boundary entry is written yet
+    if ((e = cudaMemsetAsync(D.bnd, 0, sizeof(uint2) * (size_t)W.bnd_entries, st)) != cudaSuccess) return e;
     if ((e = cudaMemsetAsync(D.res + W.pair0, 0, sizeof(BandRes) * std::max(W.npair, 1), st)) != cudaSuccess)
         return e;
     if ((e = cudaMemsetAsync(D.queue + 64 * k, 0, sizeof(int32_t), st)) != cudaSuccess) return e;
@@ -1128,7 +1173,7 @@ cudaError_t band_launch_dp(const BandPlan &bp, int k, const BandDev &D, const ui
     a.qcodes = qcodes, a.tcodes = tcodes;
     a.pairs = D.pairs, a.strips = D.strips, a.units = D.units + W.unit0;
     a.n_units = W.nunit;
-    a.queue = D.queue + 64 * k, a.progress = D.progress, a.error = D.error;
+    a.queue = D.queue + 64 * k, a.error = D.error;
     a.tb = D.tb, a.bnd = D.bnd, a.res = D.res;
     a.sc = S;
     a.block = bp.block;
@@ -1197,15 +1242,15 @@ cudaError_t band_launch_groups(const BandPlan &bp, int k, const BandDev &D, cons
     for (int ri = W.round0; ri < W.round0 + W.nround; ++ri) {
         const BandRound &R = bp.rounds[ri];
         const BandGroupDev *gd = D.groups + R.group0;
-        band_round_progress_kernel<<<R.ngroup, 256, 0, st>>>(D.progress, gd);
-        if ((e = cudaGetLastError()) != cudaSuccess) return e;
+        // every strip's left column is there from the first pass, so the strips of a round do
+        // not wait for one another
         // this round's counter of the work queue: the wave's slot, reused per round
         if ((e = cudaMemsetAsync(D.queue + 64 * k, 0, sizeof(int32_t), st)) != cudaSuccess) return e;
         BandArgs a;
         a.qcodes = qcodes, a.tcodes = tcodes;
         a.pairs = D.pairs, a.strips = D.strips, a.units = D.units + R.unit0;
         a.n_units = R.nunit;
-        a.queue = D.queue + 64 * k, a.progress = D.progress, a.error = D.error;
+        a.queue = D.queue + 64 * k, a.error = D.error;
         a.tb = D.tb, a.bnd = D.bnd, a.res = D.res;
         a.sc = S;
         a.block = bp.block;

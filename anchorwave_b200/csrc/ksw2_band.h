@@ -59,10 +59,9 @@ struct BandWalkState {
 struct BandGroupDev {
     int32_t slot;             // pair slot
     int32_t s_first, s_end;   // strip descriptors [s_first, s_end) (global indices)
-    int32_t left;             // the strip on the group's left (its stored column is the input), or -1
     int32_t col_lo;           // first target column of the group
     int32_t last;             // 1: the pair's first group (the walk ends here)
-    int32_t pad0, pad1;
+    int32_t pad;
 };
 
 // One recompute round of a wave: one group of every recomputed pair that still has one, run
@@ -103,16 +102,12 @@ int band_plan_build(BandPlan &bp, const std::vector<int32_t> &ids, const std::ve
                     const std::vector<int> &tlen, const std::vector<int> &w, const std::vector<KswPair> &pairs,
                     int flag, int block, int64_t tb_budget, int nc, std::vector<int32_t> *refused);
 
-// Progress counters sit one 128-byte line apart (one line per strip).
-constexpr int PROG_STRIDE = 32;
-
 struct BandDev {
     BandPairDev *pairs;
     BandStripDev *strips;
     int2 *units;
     BandRes *res;
     BandWalkState *walk;  // per pair slot
-    int32_t *progress;  // one counter per strip descriptor, PROG_STRIDE ints apart
     int32_t *queue;     // one counter per wave, 64 ints apart
     uint2 *bnd;
     uint8_t *tb;
