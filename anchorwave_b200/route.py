@@ -45,7 +45,7 @@ class Route:
 
 def _load():
     if not os.path.exists(LIB_PATH):
-        raise ImportError(f"{LIB_PATH} is missing; build it with `make -C anchorwave_b200/frontend REF=<AnchorWave>`")
+        raise ModuleNotFoundError(f"{LIB_PATH} is missing; build it with `make -C anchorwave_b200/frontend REF=<AnchorWave>`")
     lib = C.CDLL(LIB_PATH)
     lib.aw_route_intervals.argtypes = [C.c_int, C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p, C.c_int64,
                                        C.c_int32, C.c_int32, C.c_int32, C.c_int32, C.c_int32, C.c_int,
