@@ -2,9 +2,9 @@
 
 Knobs, each timed on a seeded sample of the caller's own workload (same length
 distribution), the fastest installed or returned:
-  * full-matrix strip kernel (aw_set_tuning): large_warps, how many warps pipeline the strips
-    of one large pair (2, 4 or 8), and large_tlen_threshold, the target length from which a
-    pair counts as large;
+  * full-matrix strip kernel (aw_set_tuning): large_warps (above 1: the strips of a large pair
+    run on a warp each), and large_tlen_threshold, the target length from which a pair counts
+    as large;
   * banded strip kernel (aw_set_band_columns): target columns per lane (4: a shorter pipeline
     lag between strips, for batches bound by their longest pair's chain; 8: less work per
     cell, for batches bound by total work; 0 keeps the per-batch rule);

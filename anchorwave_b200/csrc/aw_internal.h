@@ -51,13 +51,24 @@ struct KswOut {
     int32_t n_cigar, zdropped, reach_end, stopped;
 };
 
+// Per-pair record that the strips of a pair share while they run: the best H of the last row
+// as an ordered key (value, later column on a tie), and the cooperative stop.  Zero before a
+// launch.
+struct KswFullRes {
+    unsigned long long mqe_key;
+    int32_t stopped, pad;
+};
+
 struct KswFullArgs {
     const uint8_t *qcodes, *tcodes;
     const KswPair *pairs;
-    const int32_t *order;     // processing order (largest first)
-    int32_t n;
+    // work units in processing order: (pair, strip), or (pair, -1) for all strips of the pair
+    // one after the other; null: the strips of pair 0
+    const int2 *units;
+    int32_t n;                // units
     uint8_t *tb;              // traceback arena (CIGAR modes)
-    uint32_t *bnd;            // strip-boundary arena
+    uint32_t *bnd;            // strip-boundary arena, zero before a launch
+    KswFullRes *res;
     KswOut *out;
     int32_t *queue;           // work-queue head (device counter)
     int32_t *error;           // set non-zero if a bounded wait gave up
@@ -79,23 +90,28 @@ __device__ __forceinline__ bool aw_deadline_passed(const unsigned long long *d) 
 }
 #endif
 
-// Traceback geometry of the full-matrix strip kernel: strips of KSW_STRIP = 512 target
-// columns in KSW_GROUPS = 64 groups of KSW_COLS = 8; a step of a strip stores one
-// KSW_COLS-byte word per group, the word of group g at row r being stored at step r + g:
-// byte ((strip * (qlen + KSW_LAG) + r + g) * KSW_GROUPS + g) * KSW_COLS + (col & 7).
-constexpr int KSW_COLS = 8;
-constexpr int KSW_GROUPS = 64;
-constexpr int KSW_STRIP = KSW_GROUPS * KSW_COLS;
-constexpr int KSW_LAG = KSW_GROUPS - 1;
+// Traceback geometry of the full-matrix strip kernel.  A strip is 32 lanes of KSW_WIDE or
+// KSW_NARROW target columns; lane L computes row k - 2L in the first half of its columns and
+// row k - 2L - 1 in the second half at step k, so a sweep takes qlen + KSW_LAG steps.
+//   wide: a step stores one 8-byte word per half (group g = 2L + half of 8 columns, row r = k - g)
+//   at byte ((strip * (qlen + KSW_LAG) + k) * 64 + g) * 8;
+//   narrow: the first half of a row waits a step for the second, and one 4-byte word per lane
+//   (row r = k - 2L - 1) goes to byte ((strip * (qlen + KSW_LAG) + k) * 32 + L) * 4.
+// Singletrack words hold the v bytes and then the u bytes of their columns: twice the size.
+constexpr int KSW_WIDE = 16, KSW_NARROW = 4;  // target columns per lane
+constexpr int KSW_LAG = 63;
 
-inline int64_t ksw_full_tb_bytes(int qlen, int tlen) {
-    const int64_t nstrip = (tlen + KSW_STRIP - 1) / KSW_STRIP;
-    return nstrip * (int64_t)(qlen + KSW_LAG) * KSW_STRIP;
+inline int64_t ksw_full_strips(int tlen, bool narrow) {
+    const int w = 32 * (narrow ? KSW_NARROW : KSW_WIDE);
+    return (tlen + (int64_t)w - 1) / w;
+}
+inline int64_t ksw_full_tb_bytes(int qlen, int tlen, bool narrow = false, bool tracks = false) {
+    return ksw_full_strips(tlen, narrow) * (int64_t)(qlen + KSW_LAG) * 32 * (narrow ? KSW_NARROW : KSW_WIDE) *
+           (tracks ? 2 : 1);
 }
 // boundary column of a strip: one 8-byte entry per row and one for the strip's last-row H
-inline int64_t ksw_full_bnd_words(int qlen, int tlen) {
-    const int64_t nstrip = (tlen + KSW_STRIP - 1) / KSW_STRIP;
-    return nstrip * ((int64_t)qlen + 1) * 2;
+inline int64_t ksw_full_bnd_words(int qlen, int tlen, bool narrow = false) {
+    return ksw_full_strips(tlen, narrow) * ((int64_t)qlen + 1) * 2;
 }
 
 // Grow-only device allocation (pooled per host thread or per plan).
@@ -141,13 +157,15 @@ int reserve_thread_tb(int64_t bytes);
 int full_path_params(int qlen, int tlen, int8_t m, const int8_t *mat, int8_t q, int8_t e, int8_t q2,
                      int8_t e2, int flag, KswScore *S);
 
-// Launchers (ksw2_full.cu).
-int ksw_full_occupancy(int flag, int warps_per_pair, int groups_per_cta);
-cudaError_t launch_ksw_full(const KswFullArgs &a, int flag, int warps_per_pair,
-                            int groups_per_cta, int ctas, cudaStream_t st);
+// Launchers (ksw2_full.cu).  narrow: strips of KSW_NARROW columns per lane.
+int ksw_full_warps_per_cta(bool narrow);
+int ksw_full_occupancy(int flag, bool narrow);
+cudaError_t launch_ksw_full(const KswFullArgs &a, int flag, bool narrow, int ctas, cudaStream_t st);
+// Tracebacks of the pairs order[0..n); mat (m x m) is read by the Singletrack reconstruction.
 cudaError_t launch_ksw_backtrack_full(const KswPair *pairs, const int32_t *order, int n,
-                                      const uint8_t *tb, KswOut *out, uint32_t *cig,
-                                      int flag, cudaStream_t st);
+                                      const uint8_t *tb, KswOut *out, uint32_t *cig, int flag, bool narrow,
+                                      const uint8_t *qcodes, const uint8_t *tcodes, const KswScore &S,
+                                      const int8_t *mat, int m, cudaStream_t st);
 // Writes globaltimer + remaining_ns (or "never" for ~0) to *deadline on the stream, so
 // the deadline counts from when the stream reaches this call.
 cudaError_t launch_set_deadline(unsigned long long *deadline, unsigned long long remaining_ns, cudaStream_t st);

@@ -7,8 +7,8 @@
 //   * batch planning: pairs sorted largest first, traceback arenas packed into
 //     waves under an HBM budget (the -M admission envelope of
 //     AlignmentResourceScheduler.cpp:706 restated for device memory);
-//   * per-thread pooled device/pinned buffers (grow-only) and a private stream
-//     pair, so concurrent host threads never share state (the reference's
+//   * per-thread pooled device/pinned buffers (grow-only) and a private
+//     stream, so concurrent host threads never share state (the reference's
 //     one-call-per-worker threading contract: each AnchorTaskExecutor worker
 //     calls ksw_extd2 on its own, src/service/AnchorTaskExecutor.cpp:54, :374);
 //   * CIGAR ownership exactly as ksw_push_cigar (minimap2/ksw2.h:144-154).
@@ -66,9 +66,8 @@ static cudaError_t record_timing(cudaEvent_t e, cudaStream_t st) {
 // ---- tuning ----------------------------------------------------------------
 static int64_t g_tb_budget = 0;           // 0 = 60% of free memory
 static thread_local int64_t tls_tb_budget = 0;  // per-thread override (serving workers)
-static thread_local bool tls_all_large = false;  // single-pair calls: every pair gets a warp group
-// full-matrix pairs on the critical path go to the banded kernel at full width
-// (aw_set_full_pair_routing)
+// full-matrix pairs on the critical path whose traceback exceeds the budget go to the banded
+// kernel at full width, which can recompute it in rounds (aw_set_full_pair_routing)
 static std::atomic<bool> g_band_full_pairs{true};
 static int g_large_warps = 8;
 static int g_large_tlen = 4096;
@@ -97,41 +96,36 @@ struct PinBuf {
 };
 
 struct Buffers {
-    DevBuf qcodes, tcodes, pairs, order, out, cig, packed, packed_off, tb, bnd, queue, error;
+    DevBuf qcodes, tcodes, pairs, order, units, full_res, out, cig, packed, packed_off, tb, bnd, queue, error;
     DevBuf exact_ws, deadline;
     DevBuf band_pairs, band_strips, band_units, band_res, band_bnd, band_queue, band_walk, band_groups;
     PinBuf h_band;
-    PinBuf h_codes, h_pairs, h_order, h_out, h_packed, h_packed_off, h_small;
-    cudaStream_t st = nullptr, st2 = nullptr;
-    cudaEvent_t ev_a = nullptr, ev_b = nullptr, ev_t0 = nullptr, ev_t1 = nullptr;
+    PinBuf h_codes, h_pairs, h_order, h_units, h_out, h_packed, h_packed_off, h_small;
+    cudaStream_t st = nullptr;
+    cudaEvent_t ev_t0 = nullptr, ev_t1 = nullptr;
     std::vector<cudaEvent_t> ev_k;  // per-launch timing events
     int device = -1;
     int sms = 0;
     ~Buffers() {
         qcodes.release(); tcodes.release(); pairs.release(); order.release(); out.release();
+        units.release(); full_res.release();
         cig.release(); packed.release(); packed_off.release(); tb.release(); bnd.release();
         queue.release(); error.release(); exact_ws.release(); deadline.release();
         band_pairs.release(); band_strips.release(); band_units.release(); band_res.release();
         band_bnd.release(); band_queue.release(); band_walk.release(); h_band.release();
         band_groups.release();
-        h_codes.release(); h_pairs.release(); h_order.release(); h_out.release();
+        h_codes.release(); h_pairs.release(); h_order.release(); h_units.release(); h_out.release();
         h_packed.release(); h_packed_off.release(); h_small.release();
         for (auto e : ev_k) cudaEventDestroy(e);
-        if (ev_a) cudaEventDestroy(ev_a);
-        if (ev_b) cudaEventDestroy(ev_b);
         if (ev_t0) cudaEventDestroy(ev_t0);
         if (ev_t1) cudaEventDestroy(ev_t1);
         if (st) cudaStreamDestroy(st);
-        if (st2) cudaStreamDestroy(st2);
     }
     int init() {
         if (st) return AW_OK;
         AW_CUDA(cudaGetDevice(&device));
         AW_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
         AW_CUDA(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking));
-        AW_CUDA(cudaStreamCreateWithFlags(&st2, cudaStreamNonBlocking));
-        AW_CUDA(cudaEventCreateWithFlags(&ev_a, cudaEventDisableTiming));
-        AW_CUDA(cudaEventCreateWithFlags(&ev_b, cudaEventDisableTiming));
         AW_CUDA(cudaEventCreate(&ev_t0));
         AW_CUDA(cudaEventCreate(&ev_t1));
         return AW_OK;
@@ -219,8 +213,12 @@ static KswScore make_score(const Params &P) {
 // the kernel's field biases.
 static bool full_path_ok(const Params &P, int qlen, int tlen, int w) {
     if (exact_stop_enabled()) return false;
-    const int allowed = AW_EZ_SCORE_ONLY | AW_EZ_RIGHT | AW_EZ_GENERIC_SC | AW_EZ_REV_CIGAR |
-                        AW_EZ_SEMIGLOBAL_END;
+    int allowed = AW_EZ_SCORE_ONLY | AW_EZ_RIGHT | AW_EZ_GENERIC_SC | AW_EZ_REV_CIGAR | AW_EZ_SEMIGLOBAL_END;
+    // the Singletrack entries of the AVX builds (blocks of 32 or 64 bytes): their tracks are
+    // those of the matrix cells at full width; with the semiglobal end they report no CIGAR,
+    // which the banded kernel's finishing step does
+    if ((P.flag & AW_EZ_SINGLETRACK) && exact_block() > 16)
+        allowed = AW_EZ_SINGLETRACK | AW_EZ_RIGHT | AW_EZ_GENERIC_SC | AW_EZ_REV_CIGAR;
     if (P.flag & ~allowed) return false;
     if (!(w < 0 || w >= std::max(qlen, tlen))) return false;
     if (P.zdrop >= 0) return false;
@@ -229,7 +227,7 @@ static bool full_path_ok(const Params &P, int qlen, int tlen, int w) {
     if (P.e2 > P.e || P.q2 < P.q) return false;
     const int mag = (P.q2 + P.e2) + (P.q + P.e) + std::abs(P.min_sc) + std::abs((int)P.mat[0]);
     if (mag > 100) return false;
-    const int64_t nstrip = (tlen + KSW_STRIP - 1) / KSW_STRIP;
+    const int64_t nstrip = ksw_full_strips(tlen, false);
     if (nstrip * ((int64_t)qlen + 2) + qlen > INT_MAX / 2) return false;
     return true;
 }
@@ -312,17 +310,19 @@ struct aw_ksw_plan {
     int n = 0;
     std::vector<int> qlen, tlen, w;
     std::vector<int> route;   // 0 = no device work (early return), 1 = strip kernel, 2 = exact kernel, 3 = banded kernel
+    bool narrow = false;      // strip kernel: narrow strips
     std::vector<int> early_zdrop;
     std::vector<KswPair> pairs;
     std::vector<int64_t> qoff, toff;
     int64_t qbytes = 0, tbytes = 0, cig_words = 0;
-    // waves of strip-kernel pairs: order array segments
+    // waves of strip-kernel pairs: their ranges in order[] and units[]
     struct Wave {
-        int begin_small, n_small, begin_large, n_large;  // ranges in order[]
+        int begin, n, unit0, nunit;
         int64_t tb_bytes, bnd_words;
     };
     std::vector<Wave> waves;
     std::vector<int32_t> order;      // strip-kernel processing order, wave by wave
+    std::vector<int2> units;         // work units (KswFullArgs::units)
     std::vector<int32_t> exact_ids;  // pairs for the exact kernel
     std::vector<int32_t> band_ids;   // pairs for the banded kernel
     BandPlan band;
@@ -337,7 +337,6 @@ struct aw_ksw_plan {
     // ones replay it
     int eager_runs = 0;
     bool graph_off = false, graph_used = false;
-    int graph_warps = 0;
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t gexec = nullptr;
     void drop_graph() {
@@ -368,6 +367,22 @@ static int band_columns(const aw_ksw_plan_t *pl) {
     }
     return chain > work ? 4 : 8;
 }
+
+// Seconds that full-matrix pairs take on strips of one width: their cells at the rate of the
+// whole GPU, and half of the longest pair's chain of steps (its rows and the skew of a strip,
+// and a lag of 80 steps per further strip), which the other pairs hide only in part.
+// Measured: a step of a warp alone takes 0.51 us wide and 0.178 us narrow; on all warps
+// 1.0e12 and 0.75e12 cells/s.  One 5 kb pair 3.0 / 1.4 ms (wide / narrow), 8 pairs the same;
+// 24 of 2-20 kb 10.2 / 6.3, 1,000 of 0.2-2 kb 1.7 / 1.2, 32 of 20 kb 22.2 / 20.7, 64 of 20 kb
+// 27.5 / 37, 768 of 0.2-20 kb 33 / 42.  The two widths side by side in one launch were slower
+// than either (64 pairs of 1-8 kb: 6.0 against 4.4 / 2.8): a chain runs at its slowest warp.
+static double strip_seconds(double cells, double longest_chain, bool narrow) {
+    return narrow ? cells / 0.75e12 + 0.5 * 0.178e-6 * longest_chain : cells / 1.0e12 + 0.5 * 0.51e-6 * longest_chain;
+}
+static double chain_steps(double qlen, int tlen, bool narrow) {
+    return qlen + KSW_LAG + 80.0 * (double)(ksw_full_strips(tlen, narrow) - 1);
+}
+static constexpr int64_t kResidentWarps = 2368;  // 148 SMs x 16 warps of wide strips
 
 static int plan_build(aw_ksw_plan_t *pl, int n, const int *qlen, const int *tlen, const int *w) {
     pl->n = n;
@@ -401,24 +416,45 @@ static int plan_build(aw_ksw_plan_t *pl, int n, const int *qlen, const int *tlen
         pl->cells += (int64_t)ql * tl;
     }
     pl->qbytes = qb, pl->tbytes = tbt, pl->cig_words = cw;
-    // A full-matrix pair that would be the batch's critical path goes to the banded strip
-    // kernel at full width instead (w >= max(qlen, tlen) is the reference's full mode, so the
-    // results are the same): the strip kernel pipelines one pair's strips over a group of
-    // 8 warps of one CTA, ceil(strips / 8) sweeps of its rows, while the banded kernel
-    // pipelines them across CTAs, one strip per warp.  Estimates (seconds): strip-kernel
-    // chain ceil(ceil(tlen/512)/8) * (qlen + 600) * 0.35e-6 against the batch's work at
-    // 1e12 cells/s, and the banded kernel's chain (tlen/256 strips * 64 lane-steps * 2e-6, plus
-    // the rows) and the pair's work at 2e11 cells/s.
-    if (g_band_full_pairs.load()) {
-        double work = 0.0;
-        for (int i = 0; i < n; ++i)
-            if (pl->route[i] == 1) work += (double)pl->qlen[i] * pl->tlen[i];
-        const double batch_s = work / 1e12;
-        for (int i = 0; i < n; ++i) {
-            if (pl->route[i] != 1 || !band_path_ok(P, pl->qlen[i], pl->tlen[i])) continue;
-            const double ql = pl->qlen[i], tl = pl->tlen[i];
-            const double k1 = std::ceil(std::ceil(tl / KSW_STRIP) / 8.0) * (ql + 600.0) * 0.35e-6;
-            const double k2 = std::ceil(tl / 256.0) * 64.0 * 2e-6 + ql * 0.3e-6 + ql * tl / 2e11;
+    const bool cigar = !(P.flag & AW_EZ_SCORE_ONLY), tracks = cigar && (P.flag & AW_EZ_SINGLETRACK);
+    int64_t budget = tls_tb_budget;
+    int large_tlen, large_warps;
+    {
+        std::lock_guard<std::mutex> lk(g_cfg_mu);
+        if (budget <= 0) budget = g_tb_budget;
+        large_tlen = g_large_tlen, large_warps = g_large_warps;
+    }
+    if (budget <= 0) {
+        size_t fr = 0, tot = 0;
+        if (cudaMemGetInfo(&fr, &tot) != cudaSuccess) fr = (size_t)16 << 30;
+        // the traceback arena this thread already holds is reused (or freed) by this
+        // batch, so it counts as available: otherwise every call after the first would
+        // see the pooled arena as used memory and split the batch into more waves
+        if (pl->B) fr += pl->B->tb.cap;
+        budget = (int64_t)(fr * 0.6);
+    }
+    double work = 0.0, chain[2] = {0.0, 0.0};
+    for (int i = 0; i < n; ++i) {
+        if (pl->route[i] != 1) continue;
+        work += (double)pl->qlen[i] * pl->tlen[i];
+        for (int c = 0; c < 2; ++c) chain[c] = std::max(chain[c], chain_steps(pl->qlen[i], pl->tlen[i], c));
+    }
+    pl->narrow = strip_seconds(work, chain[1], true) < strip_seconds(work, chain[0], false);
+    const double batch_s = work / 1e12;
+    for (int i = 0; i < n; ++i) {
+        if (pl->route[i] != 1) continue;
+        const int ql = pl->qlen[i], tl = pl->tlen[i];
+        // A traceback that does not fit the budget: the banded kernel at full width (w >=
+        // max(qlen, tlen) is the reference's full mode) recomputes it in rounds, for pairs whose
+        // chain outlasts the batch; Singletrack tracks are its to refuse, from the two thirds of the
+        // budget that it always has for them.
+        const int64_t tb = cigar ? ksw_full_tb_bytes(ql, tl, false, tracks) : 0;
+        if (!band_path_ok(P, ql, tl)) continue;
+        if (tracks && tb > budget / 3 * 2) pl->route[i] = 3;
+        if (!tracks && tb > budget && g_band_full_pairs.load()) {
+            const double strips8 = std::ceil(std::ceil(tl / 512.0) / 8.0);
+            const double k1 = strips8 * (ql + 600.0) * 0.35e-6;
+            const double k2 = std::ceil(tl / 256.0) * 64.0 * 2e-6 + ql * 0.3e-6 + (double)ql * tl / 2e11;
             if (k1 > 1.5 * std::max(batch_s, k2)) pl->route[i] = 3;
         }
     }
@@ -432,29 +468,14 @@ static int plan_build(aw_ksw_plan_t *pl, int n, const int *qlen, const int *tlen
         const int64_t ca = (int64_t)pl->qlen[a] * pl->tlen[a], cb = (int64_t)pl->qlen[b] * pl->tlen[b];
         return ca != cb ? ca > cb : a < b;
     });
-    const bool cigar = !(P.flag & AW_EZ_SCORE_ONLY);
-    int64_t budget = tls_tb_budget;
-    if (budget <= 0) {
-        std::lock_guard<std::mutex> lk(g_cfg_mu);
-        budget = g_tb_budget;
-    }
-    if (budget <= 0) {
-        size_t fr = 0, tot = 0;
-        if (cudaMemGetInfo(&fr, &tot) != cudaSuccess) fr = (size_t)16 << 30;
-        // the traceback arena this thread already holds is reused (or freed) by this
-        // batch, so it counts as available: otherwise every call after the first would
-        // see the pooled arena as used memory and split the batch into more waves
-        if (pl->B) fr += pl->B->tb.cap;
-        budget = (int64_t)(fr * 0.6);
-    }
     // LPT multiway partition of traceback bytes into the fewest waves that fit
     std::vector<std::vector<int32_t>> wv;
     std::vector<int64_t> wload, wbnd;
     for (int32_t i : strip) {
-        const int64_t tbb = cigar ? ksw_full_tb_bytes(pl->qlen[i], pl->tlen[i]) : 0;
-        const int64_t bw = ksw_full_bnd_words(pl->qlen[i], pl->tlen[i]);
+        const int64_t tbb = cigar ? ksw_full_tb_bytes(pl->qlen[i], pl->tlen[i], pl->narrow, tracks) : 0;
+        const int64_t bw = ksw_full_bnd_words(pl->qlen[i], pl->tlen[i], pl->narrow);
         pl->tb_total += tbb;
-        if (tbb > budget) {
+        if (cigar && ksw_full_tb_bytes(pl->qlen[i], pl->tlen[i], false, tracks) > budget) {
             set_error("pair traceback exceeds the HBM traceback budget");
             return AW_E_NOMEM;
         }
@@ -474,22 +495,31 @@ static int plan_build(aw_ksw_plan_t *pl, int n, const int *qlen, const int *tlen
         wbnd[best] += (bw + 63) / 64 * 64;
         wv[best].push_back(i);
     }
-    int large_tlen, large_warps;
-    {
-        std::lock_guard<std::mutex> lk(g_cfg_mu);
-        large_tlen = g_large_tlen, large_warps = g_large_warps;
-    }
+    // Work units: the strips of a pair on as many warps, or the whole pair on one warp (no
+    // waiting between strips, which is the better use of a warp while there are pairs enough).
+    // A pair is split when its strips are narrow, when its target is long (aw_set_tuning), when
+    // all strips of the wave are on warps at once anyway, or when one warp would take longer for
+    // it (0.65 us a step on a full SM) than half the wave's work.
     for (size_t k = 0; k < wv.size(); ++k) {
         aw_ksw_plan::Wave W;
-        std::vector<int32_t> lg, sm;
-        for (int32_t i : wv[k])
-            ((pl->tlen[i] >= large_tlen || tls_all_large) && large_warps > 1 ? lg : sm).push_back(i);
-        W.begin_large = (int)pl->order.size();
-        W.n_large = (int)lg.size();
-        pl->order.insert(pl->order.end(), lg.begin(), lg.end());
-        W.begin_small = (int)pl->order.size();
-        W.n_small = (int)sm.size();
-        pl->order.insert(pl->order.end(), sm.begin(), sm.end());
+        int64_t strips = 0;
+        double cells = 0.0;
+        for (int32_t i : wv[k]) {
+            strips += ksw_full_strips(pl->tlen[i], pl->narrow);
+            cells += (double)pl->qlen[i] * pl->tlen[i];
+        }
+        W.begin = (int)pl->order.size(), W.unit0 = (int)pl->units.size();
+        for (int32_t i : wv[k]) {
+            pl->order.push_back(i);
+            const int ns = (int)ksw_full_strips(pl->tlen[i], pl->narrow);
+            const bool split = pl->narrow || (large_warps > 1 && (pl->tlen[i] >= large_tlen || strips <= kResidentWarps ||
+                                                                  ns * (pl->qlen[i] + 64.0) * 0.65e-6 > 0.5 * cells / 1e12));
+            if (!split || ns == 1) pl->units.push_back(make_int2(i, -1));
+            else
+                for (int u = 0; u < ns; ++u) pl->units.push_back(make_int2(i, u));
+        }
+        W.n = (int)pl->order.size() - W.begin;
+        W.nunit = (int)pl->units.size() - W.unit0;
         W.tb_bytes = wload[k];
         W.bnd_words = wbnd[k];
         pl->tb_cap = std::max(pl->tb_cap, W.tb_bytes);
@@ -533,13 +563,16 @@ static int plan_alloc(aw_ksw_plan_t *pl) {
     AW_CUDA(B->tcodes.ensure(pl->tbytes + 16));
     AW_CUDA(B->pairs.ensure(sizeof(KswPair) * (size_t)std::max(n, 1)));
     AW_CUDA(B->order.ensure(sizeof(int32_t) * (pl->order.size() + pl->exact_ids.size() + 1)));
+    AW_CUDA(B->units.ensure(sizeof(int2) * (pl->units.size() + 1)));
+    AW_CUDA(B->full_res.ensure(sizeof(KswFullRes) * (size_t)std::max(n, 1)));
+    AW_CUDA(B->h_units.ensure(sizeof(int2) * (pl->units.size() + 1)));
     AW_CUDA(B->out.ensure(sizeof(KswOut) * (size_t)std::max(n, 1)));
     AW_CUDA(B->cig.ensure(4 * (size_t)(pl->cig_words + 1)));
     AW_CUDA(B->packed.ensure(4 * (size_t)(pl->cig_words + 1)));
     AW_CUDA(B->packed_off.ensure(8 * (size_t)std::max(n, 1)));
     AW_CUDA(B->tb.ensure((size_t)pl->tb_cap + 256));
     AW_CUDA(B->bnd.ensure(4 * (size_t)pl->bnd_cap + 256));
-    AW_CUDA(B->queue.ensure(sizeof(int32_t) * 64 * (2 * pl->waves.size() + 2)));  // two counters per wave
+    AW_CUDA(B->queue.ensure(sizeof(int32_t) * 64 * (pl->waves.size() + 1)));  // a counter per wave
     AW_CUDA(B->error.ensure(sizeof(int32_t) * 4));
     if (!pl->band_ids.empty()) {
         const BandPlan &bp = pl->band;
@@ -600,6 +633,10 @@ static int plan_upload(aw_ksw_plan_t *pl, const uint8_t *const *query, const uin
     AW_CUDA(cudaMemcpyAsync(B->pairs.p, B->h_pairs.p, sizeof(KswPair) * (size_t)n, cudaMemcpyHostToDevice, B->st));
     AW_CUDA(cudaMemcpyAsync(B->order.p, ho, sizeof(int32_t) * (pl->order.size() + pl->exact_ids.size()),
                             cudaMemcpyHostToDevice, B->st));
+    if (!pl->units.empty()) {
+        memcpy(B->h_units.p, pl->units.data(), sizeof(int2) * pl->units.size());
+        AW_CUDA(cudaMemcpyAsync(B->units.p, B->h_units.p, sizeof(int2) * pl->units.size(), cudaMemcpyHostToDevice, B->st));
+    }
     if (!pl->band_ids.empty()) {
         const BandPlan &bp = pl->band;
         const size_t np = sizeof(BandPairDev) * bp.pairs.size(), ns = sizeof(BandStripDev) * bp.strips.size(),
@@ -624,11 +661,12 @@ static int plan_launch(aw_ksw_plan_t *pl) {
     Buffers *B = pl->B;
     const Params &P = pl->P;
     if (!pl->uploaded) { set_error("plan not uploaded"); return AW_E_INVAL; }
-    const size_t nq = 64 * (2 * pl->waves.size() + 2);  // large + small counter per wave, 256 B apart
+    const size_t nq = 64 * (pl->waves.size() + 1);  // a counter per wave, 256 B apart
     int launches = 0;
     AW_CUDA(cudaMemsetAsync(B->queue.p, 0, sizeof(int32_t) * nq, B->st));
     AW_CUDA(cudaMemsetAsync(B->error.p, 0, sizeof(int32_t) * 4, B->st));
     AW_CUDA(cudaMemsetAsync(B->out.p, 0, sizeof(KswOut) * (size_t)std::max(pl->n, 1), B->st));
+    if (!pl->waves.empty()) AW_CUDA(cudaMemsetAsync(B->full_res.p, 0, sizeof(KswFullRes) * (size_t)pl->n, B->st));
     AW_CUDA(record_timing(B->ev_t0, B->st));
     // the deadline word: globaltimer at the start of this work + the time left
     const unsigned long long *deadline = nullptr;
@@ -640,11 +678,6 @@ static int plan_launch(aw_ksw_plan_t *pl) {
                                     (unsigned long long)std::max(left, 0LL), B->st));
         deadline = B->deadline.as<unsigned long long>();
         ++launches;
-    }
-    int large_warps;
-    {
-        std::lock_guard<std::mutex> lk(g_cfg_mu);
-        large_warps = g_large_warps;
     }
     // per-wave timing events: DP phase start, DP phase end (after the join), backtrack end
     const size_t need_ev = 3 * (pl->waves.size() + pl->band.waves.size()) + 3;
@@ -659,48 +692,26 @@ static int plan_launch(aw_ksw_plan_t *pl) {
         KswFullArgs a;
         a.qcodes = B->qcodes.as<uint8_t>(), a.tcodes = B->tcodes.as<uint8_t>();
         a.pairs = B->pairs.as<KswPair>(), a.out = B->out.as<KswOut>();
+        a.res = B->full_res.as<KswFullRes>();
         a.tb = B->tb.as<uint8_t>(), a.bnd = B->bnd.as<uint32_t>();
         a.error = B->error.as<int32_t>();
         a.sc = pl->S;
         a.deadline = deadline;
         AW_CUDA(record_timing(B->ev_k[3 * k], B->st));
-        // fork: large pairs on st2 (groups of large_warps warps), small on st (single warps)
-        AW_CUDA(cudaEventRecord(B->ev_a, B->st));
-        AW_CUDA(cudaStreamWaitEvent(B->st2, B->ev_a, 0));
-        if (W.n_large > 0) {
-            a.order = B->order.as<int32_t>() + W.begin_large;
-            a.n = W.n_large;
-            a.queue = B->queue.as<int32_t>() + 64 * (2 * k);
-            const int groups = 8 / large_warps;
-            const int occ = std::max(1, ksw_full_occupancy(P.flag, large_warps, groups));
-            const int ctas = std::min(W.n_large / groups + 1, occ * B->sms);
-            AW_CUDA(launch_ksw_full(a, P.flag, large_warps, groups, ctas, B->st2));
-            ++launches;
-        }
-        if (W.n_small > 0) {
-            a.order = B->order.as<int32_t>() + W.begin_small;
-            a.n = W.n_small;
-            a.queue = B->queue.as<int32_t>() + 64 * (2 * k + 1);
-            // warps per small pair: one when the pairs alone fill the resident warps, else
-            // up to 8 so that a small batch still runs on the whole GPU (a pair's strips
-            // then pipeline over its warps instead of running one after another)
-            const int resident = 16 * B->sms;  // 2 CTAs x 8 warps per SM
-            const int64_t used = std::min<int64_t>((int64_t)W.n_large * large_warps, resident);
-            int ws = 1;
-            while (ws < 8 && (int64_t)W.n_small * (2 * ws) <= resident - used) ws *= 2;
-            const int groups = 8 / ws;
-            const int occ = std::max(1, ksw_full_occupancy(P.flag, ws, groups));
-            const int ctas = std::min((W.n_small + groups - 1) / groups, occ * B->sms);
-            AW_CUDA(launch_ksw_full(a, P.flag, ws, groups, ctas, B->st));
-            ++launches;
-        }
-        AW_CUDA(cudaEventRecord(B->ev_b, B->st2));
-        AW_CUDA(cudaStreamWaitEvent(B->st, B->ev_b, 0));
+        AW_CUDA(cudaMemsetAsync(B->bnd.p, 0, 4 * (size_t)W.bnd_words, B->st));
+        a.units = B->units.as<int2>() + W.unit0;
+        a.n = W.nunit;
+        a.queue = B->queue.as<int32_t>() + 64 * k;
+        const int per = ksw_full_warps_per_cta(pl->narrow);
+        const int occ = std::max(1, ksw_full_occupancy(P.flag, pl->narrow));
+        AW_CUDA(launch_ksw_full(a, P.flag, pl->narrow, std::min((a.n + per - 1) / per, occ * B->sms), B->st));
+        ++launches;
         AW_CUDA(record_timing(B->ev_k[3 * k + 1], B->st));
-        if (!(P.flag & AW_EZ_SCORE_ONLY) && W.n_large + W.n_small > 0) {
-            AW_CUDA(launch_ksw_backtrack_full(B->pairs.as<KswPair>(), B->order.as<int32_t>() + W.begin_large,
-                                              W.n_large + W.n_small, B->tb.as<uint8_t>(), B->out.as<KswOut>(),
-                                              B->cig.as<uint32_t>(), P.flag, B->st));
+        if (!(P.flag & AW_EZ_SCORE_ONLY)) {
+            AW_CUDA(launch_ksw_backtrack_full(B->pairs.as<KswPair>(), B->order.as<int32_t>() + W.begin, W.n,
+                                              B->tb.as<uint8_t>(), B->out.as<KswOut>(), B->cig.as<uint32_t>(), P.flag,
+                                              pl->narrow, B->qcodes.as<uint8_t>(), B->tcodes.as<uint8_t>(), pl->S, P.mat,
+                                              P.m, B->st));
             ++launches;
         }
         AW_CUDA(record_timing(B->ev_k[3 * k + 2], B->st));
@@ -905,12 +916,6 @@ int aw_ksw_plan_execute(aw_ksw_plan_t *pl, float *ms) {
     if (pl->graph_off || !pl->uploaded || !pl->exact_ids.empty() || tls_has_deadline ||
         pl->cells > kGraphMaxCells)
         return plan_execute(pl, ms);
-    int lw;
-    {
-        std::lock_guard<std::mutex> lk(g_cfg_mu);
-        lw = g_large_warps;
-    }
-    if (pl->gexec && pl->graph_warps != lw) pl->drop_graph();  // tuning changed: capture again
     if (!pl->gexec) {
         if (pl->eager_runs < 1) {
             ++pl->eager_runs;
@@ -931,7 +936,7 @@ int aw_ksw_plan_execute(aw_ksw_plan_t *pl, float *ms) {
             pl->graph_off = true;
             return plan_execute(pl, ms);
         }
-        pl->graph = g, pl->gexec = ge, pl->graph_warps = lw;
+        pl->graph = g, pl->gexec = ge;
     }
     AW_CUDA(cudaGraphLaunch(pl->gexec, pl->B->st));
     pl->graph_used = true;
@@ -1009,10 +1014,7 @@ static void single_call(void *km, int qlen, const uint8_t *query, int tlen, cons
         ez->zdropped = 1;
         return;
     }
-    // one pair alone: let a whole warp group pipeline its strips whatever its length
-    tls_all_large = true;
     int rc = plan_build(&pl, 1, &qlen, &tlen, &w);
-    tls_all_large = false;
     if (!rc) rc = plan_alloc(&pl);
     if (!rc) rc = plan_upload(&pl, &query, &target);
     if (!rc) rc = plan_execute(&pl, nullptr);
@@ -1066,7 +1068,7 @@ int full_path_params(int qlen, int tlen, int8_t m, const int8_t *mat, int8_t q, 
     Params P;
     if (!make_params(m, mat, q, e, q2, e2, -1, 0, flag, P)) return AW_E_UNSUPPORTED;
     if (P.early_return) return 1;
-    if (!full_path_ok(P, qlen, tlen, -1)) return AW_E_UNSUPPORTED;
+    if ((flag & AW_EZ_SINGLETRACK) || !full_path_ok(P, qlen, tlen, -1)) return AW_E_UNSUPPORTED;
     *S = make_score(P);
     return AW_OK;
 }

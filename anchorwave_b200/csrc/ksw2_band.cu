@@ -554,47 +554,6 @@ __global__ void __launch_bounds__(256, 2) ksw_band_kernel(BandArgs A) {
 
 // ---- traceback --------------------------------------------------------------------
 
-// CIGAR under construction, replicated in every lane of the walking warp: the open
-// run stays in registers and lane 0 writes a run when the next op differs (the
-// merge rule of ksw_push_cigar, minimap2/ksw2.h:144-154).
-struct WarpCig {
-    uint32_t *buf;
-    int n;          // runs written
-    uint32_t op;    // open run
-    int len;        // 0 = no open run
-    __device__ void push(uint32_t o, int l) {
-        if (len > 0 && o == op) {
-            len += l;
-            return;
-        }
-        if (len > 0 && (threadIdx.x & 31) == 0) buf[n] = (uint32_t)len << 4 | op;
-        if (len > 0) ++n;
-        op = o, len = l;
-    }
-    __device__ int finish(bool reverse) {
-        if (len > 0) {
-            if ((threadIdx.x & 31) == 0) buf[n] = (uint32_t)len << 4 | op;
-            ++n, len = 0;
-        }
-        __syncwarp();
-        if (reverse) {
-            const int lane = threadIdx.x & 31;
-            for (int a = lane; a < n / 2; a += 32) {
-                const uint32_t t = buf[a];
-                buf[a] = buf[n - 1 - a], buf[n - 1 - a] = t;
-            }
-            __syncwarp();
-        }
-        return n;
-    }
-};
-
-__device__ __forceinline__ int st_gap(int l, int o1, int e1, int o2, int e2) {
-    if (l <= 0) return 0;
-    const long long a = (long long)o1 + (long long)l * e1, b = (long long)o2 + (long long)l * e2;
-    return (int)(a > b ? a : b);
-}
-
 struct BtArgs {
     const BandPairDev *pairs;
     int npair;
@@ -675,101 +634,20 @@ __global__ void __launch_bounds__(32 * fin_warps<ST>()) ksw_band_finish_kernel(B
     Window win;
     win.init(tiles[warp], 32 * WB);
     auto grp = [&](int gg) -> TbGroup { return band_group<WB, NC>(strips, tb, tlen, 0, gg); };
-    auto stB = [&](int r) { return g.st0(r) & g.bmask; };
-    auto en16 = [&](int r) { return (g.en0(r) & ~15) + 15; };
-    WarpCig cg{A.cig + P.cig_off, 0, 0, 0};
+    WarpCigar cg{A.cig + P.cig_off, 0, 0, 0};
     if (cigar && ST) {
         // ksw_extd2_singletrack_sse reconstructs whatever the EXTZ/SEMIGLOBAL flags
         // (minimap2/ksw2_singletrack.cpp:606-615)
         if (!o.zdropped && (sse_st || !(flag & (AW_EZ_EXTZ_ONLY | AW_EZ_SEMIGLOBAL_END)))) {
             const uint8_t *qs = A.qcodes + P.qoff, *ts = A.tcodes + P.toff;
-            const int o1 = -A.sc.q, g1 = -A.sc.e, o2 = -A.sc.q2, g2 = -A.sc.e2;
-            // the difference along the matrix edge for edge cell c
-            auto edge = [&](int c) { return st_gap(c + 1, o1, g1, o2, g2) - st_gap(c, o1, g1, o2, g2); };
-            auto stored = [&](int i, int j) {
-                const int d = i + j;
-                return i >= stB(d) && i <= en16(d);
-            };
             Probe probe;
             probe.init(tiles[warp] + Window::BYTES, 32 * WB);
-            bool valid = true;
             int i = tlen - 1, j = qlen - 1;
-            while (i >= 0 && j >= 0) {
-                const int dg = i + j;
-                if (i < stB(dg)) { cg.push(1, 1); --j; continue; }
-                if (i > en16(dg)) { cg.push(2, 1); --i; continue; }
-                // the run of diagonal moves: v(i, j) + u(i, j-1) is the cell's substitution score
-                win.ensure(i, j, grp);
-                const int li = i - lane, lj = j - lane;
-                const bool in = li >= 0 && lj >= 0 && win.has(li, lj) && stored(li, lj);
-                bool on = in;
-                if (in) {
-                    const int h = sx8(win.at(li, lj, 0));
-                    const bool fin = lj == 0 || stored(li, lj - 1);
-                    const int v = lj == 0 ? edge(li) : fin ? sx8(win.at(li, lj - 1, 1)) : 0;
-                    on = fin && h + v == A.mat[ts[li] * A.m + qs[lj]];
-                }
-                const unsigned off = __ballot_sync(FULL, !on);
-                const int run = off ? __ffs(off) - 1 : 32;
-                if (run > 0) {
-                    cg.push(0, run);
-                    i -= run, j -= run;
-                }
-                if (run == 32 || !__shfl_sync(FULL, in ? 1 : 0, run)) continue;
-                // the gap that leaves (i, j): the first length l whose summed differences up the
-                // column of rows (insertion) or along the row (deletion) are exactly a gap of l;
-                // 32 lengths at a time, lane k looking at length base + k + 1.  Sums over cells
-                // outside the stored band match no gap (d_ok, i_ok).
-                int base = 0, dsum = 0, isum = 0;
-                bool d_ok = true, i_ok = true;
-                for (;;) {
-                    const int l = base + lane + 1, id = i - l, jn = j - l;
-                    // differences of the l-th cell: u(i-l+1, j) and v(i, j-l+1)
-                    int du = 0, dv = 0;
-                    bool uf = true, vf = true;
-                    if (d_ok && i - base >= 0) probe.corner(i - base, j, grp);
-                    if (d_ok && id + 1 >= 0) {
-                        uf = stored(id + 1, j);
-                        if (uf) du = sx8(probe.at(id + 1, j, 1));
-                    }
-                    __syncwarp();
-                    if (i_ok && j - base >= 0) probe.corner(i, j - base, grp);
-                    if (i_ok && jn + 1 >= 0) {
-                        vf = stored(i, jn + 1);
-                        if (vf) dv = sx8(probe.at(i, jn + 1, 0));
-                    }
-                    __syncwarp();
-#pragma unroll
-                    for (int k = 1; k < 32; k <<= 1) {
-                        const int a = __shfl_up_sync(FULL, du, k), b = __shfl_up_sync(FULL, dv, k);
-                        if (lane >= k) du += a, dv += b;
-                    }
-                    const unsigned ub = __ballot_sync(FULL, !uf), vb = __ballot_sync(FULL, !vf);
-                    const unsigned upto = lane == 31 ? FULL : (2u << lane) - 1u;
-                    const int a1 = o1 + l * g1, a2 = o2 + l * g2, dd = dsum + du, di = isum + dv;
-                    const bool dhit = d_ok && !(ub & upto) && id >= -1 && (dd == a1 || dd == a2);
-                    const bool ihit = i_ok && !(vb & upto) && jn >= -1 && (di == a1 || di == a2);
-                    const unsigned end = __ballot_sync(FULL, l > i + 1 && l > j + 1);
-                    const unsigned db = __ballot_sync(FULL, dhit), hit = db | __ballot_sync(FULL, ihit);
-                    if (hit && (!end || __ffs(hit) <= __ffs(end))) {
-                        const int k = __ffs(hit) - 1, len = base + k + 1;
-                        if (db >> k & 1u) cg.push(2, len), i -= len;
-                        else cg.push(1, len), j -= len;
-                        break;
-                    }
-                    if (end) { valid = false; break; }
-                    dsum += __shfl_sync(FULL, du, 31), isum += __shfl_sync(FULL, dv, 31);
-                    d_ok = d_ok && !ub, i_ok = i_ok && !vb;
-                    base += 32;
-                }
-                if (!valid) break;
-            }
-            if (valid) {
+            if (tb_singletrack(i, j, cg, win, probe, grp, [&](int a, int c) { return band_force(g, a, c); }, A.sc, A.mat,
+                               A.m, qs, ts)) {
                 if (i >= 0) cg.push(2, i + 1);
                 if (j >= 0) cg.push(1, j + 1);
                 o.n_cigar = cg.finish(true);
-            } else {
-                o.n_cigar = 0;
             }
             if (o.n_cigar == 0) o.zdropped = 1;
         } else if (!o.zdropped) {
@@ -830,7 +708,7 @@ __global__ void __launch_bounds__(32) ksw_band_round_walk_kernel(BtArgs A, const
     Window win;
     win.init(tiles, 32 * NC);
     auto grp = [&](int gg) -> TbGroup { return band_group<NC, NC>(strips, tb, tlen, col_lo, gg); };
-    WarpCig cg{A.cig + P.cig_off, w.n, (uint32_t)w.op, w.len};
+    WarpCigar cg{A.cig + P.cig_off, w.n, (uint32_t)w.op, w.len};
     int i = w.i, j = w.j, state = w.state;
     tb_walk(i, j, state, col_lo, cg, win, grp, [&](int a, int b) { return band_force(g, a, b); });
     if (G.last) {

@@ -50,6 +50,7 @@ struct Ctrl {
     int32_t queue;
     int32_t error;
     int32_t pad;
+    KswFullRes res;
     KswOut out;
 };
 static_assert(sizeof(Ctrl) <= CTRL_BYTES, "control block too large");
@@ -91,6 +92,7 @@ __global__ void noalloc_setup_kernel(Ctrl *c, int qlen, int tlen) {
     c->order = 0;
     c->queue = 0;
     c->error = 0;
+    c->res = KswFullRes{0, 0, 0};
     KswOut o = {};
     c->out = o;
 }
@@ -147,8 +149,16 @@ extern "C" int aw_ksw_extd2_device_noalloc(int qlen, const uint8_t *d_query, int
         return AW_E_UNSUPPORTED;
     }
     const bool cigar = !(flag & AW_EZ_SCORE_ONLY);
-    const int64_t bnd_bytes = al256(4 * ksw_full_bnd_words(qlen, tlen));
-    const int64_t tb_bytes = cigar ? al256(ksw_full_tb_bytes(qlen, tlen)) : 0;
+    // narrow strips (the shorter chain of steps, which bounds one pair alone) where their longer
+    // boundary columns fit as well, wide strips otherwise
+    auto sizes = [&](bool narrow, int64_t &bnd, int64_t &tb) {
+        bnd = al256(4 * ksw_full_bnd_words(qlen, tlen, narrow));
+        tb = cigar ? al256(ksw_full_tb_bytes(qlen, tlen, narrow)) : 0;
+        return (int64_t)CTRL_BYTES + bnd + tb <= (int64_t)AW_NOALLOC_SCRATCH_BYTES;
+    };
+    int64_t bnd_bytes = 0, tb_bytes = 0;
+    const bool narrow = sizes(true, bnd_bytes, tb_bytes);
+    if (!narrow) sizes(false, bnd_bytes, tb_bytes);
     if ((int64_t)CTRL_BYTES + bnd_bytes + tb_bytes > (int64_t)AW_NOALLOC_SCRATCH_BYTES) {
         set_error("aw_ksw_extd2_device_noalloc: pair too large for the fixed scratch array "
                   "(traceback + boundary columns exceed AW_NOALLOC_SCRATCH_BYTES)");
@@ -172,17 +182,21 @@ extern "C" int aw_ksw_extd2_device_noalloc(int qlen, const uint8_t *d_query, int
     }
     KswFullArgs a;
     a.qcodes = d_query, a.tcodes = d_target;
-    a.pairs = &ctrl->pair, a.order = &ctrl->order, a.n = 1;
-    a.tb = tb, a.bnd = bnd, a.out = &ctrl->out;
+    a.pairs = &ctrl->pair, a.units = nullptr, a.n = (int32_t)ksw_full_strips(tlen, narrow);
+    a.tb = tb, a.bnd = bnd, a.res = &ctrl->res, a.out = &ctrl->out;
     a.queue = &ctrl->queue, a.error = &ctrl->error;
     a.sc = S;
-    // one pair: one group of eight warps pipelining the strips
-    if (launch_ksw_full(a, flag, 8, 1, 1, st) != cudaSuccess) {
+    // one strip per warp; no boundary entry is written yet.  A strip only waits for units taken
+    // before it, so the grid need not be resident as a whole.
+    const int per = ksw_full_warps_per_cta(narrow);
+    const int ctas = (int)std::min<int64_t>((a.n + (int64_t)per - 1) / per, 148);
+    if (cudaMemsetAsync(bnd, 0, (size_t)bnd_bytes, st) != cudaSuccess ||
+        launch_ksw_full(a, flag, narrow, ctas, st) != cudaSuccess) {
         set_error("aw_ksw_extd2_device_noalloc: DP launch failed");
         return AW_E_CUDA;
     }
-    if (cigar && launch_ksw_backtrack_full(&ctrl->pair, &ctrl->order, 1, tb, &ctrl->out, d_cigar, flag, st) !=
-                     cudaSuccess) {
+    if (cigar && launch_ksw_backtrack_full(&ctrl->pair, &ctrl->order, 1, tb, &ctrl->out, d_cigar, flag, narrow, d_query,
+                                           d_target, S, mat, m, st) != cudaSuccess) {
         set_error("aw_ksw_extd2_device_noalloc: traceback launch failed");
         return AW_E_CUDA;
     }

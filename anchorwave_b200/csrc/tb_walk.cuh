@@ -19,7 +19,7 @@
 #pragma once
 #include <stdint.h>
 #include <climits>
-#include <type_traits>
+#include "aw_internal.h"
 
 namespace aw {
 
@@ -140,6 +140,41 @@ struct TbWindow {
 
 constexpr unsigned TB_ALL = 0xffffffffu;
 
+// CIGAR under construction, replicated in every lane of the walking warp: the open
+// run stays in registers and lane 0 writes a run when the next op differs (the
+// merge rule of ksw_push_cigar, minimap2/ksw2.h:144-154).
+struct WarpCigar {
+    uint32_t *buf;
+    int n;         // runs written
+    uint32_t op;   // open run
+    int len;       // 0 = no open run
+    __device__ void push(uint32_t o, int l) {
+        if (len > 0 && o == op) {
+            len += l;
+            return;
+        }
+        if (len > 0 && (threadIdx.x & 31) == 0) buf[n] = (uint32_t)len << 4 | op;
+        if (len > 0) ++n;
+        op = o, len = l;
+    }
+    __device__ int finish(bool reverse) {
+        if (len > 0) {
+            if ((threadIdx.x & 31) == 0) buf[n] = (uint32_t)len << 4 | op;
+            ++n, len = 0;
+        }
+        __syncwarp();
+        if (reverse) {
+            const int lane = threadIdx.x & 31;
+            for (int a = lane; a < n / 2; a += 32) {
+                const uint32_t t = buf[a];
+                buf[a] = buf[n - 1 - a], buf[n - 1 - a] = t;
+            }
+            __syncwarp();
+        }
+        return n;
+    }
+};
+
 // ksw_backtrack (minimap2/ksw2.h:160-192) from (i, j) until the walk leaves the matrix or the
 // columns >= col_lo, in runs.  FORCE(i, j): the move forced outside the computed band (1:
 // deletion, 2: insertion) or -1.
@@ -169,6 +204,96 @@ __device__ void tb_walk(int &i, int &j, int &state, int col_lo, Cig &cg, Window 
         if (state == 1 || state == 3) cg.push(2, 1), --i;
         else cg.push(1, 1), --j;
     }
+}
+
+__device__ __forceinline__ int tb_sx8(uint32_t w) { return (int)(int8_t)(uint8_t)w; }
+__device__ __forceinline__ int tb_st_gap(int l, int o1, int e1, int o2, int e2) {
+    if (l <= 0) return 0;
+    const long long a = (long long)o1 + (long long)l * e1, b = (long long)o2 + (long long)l * e2;
+    return (int)(a > b ? a : b);
+}
+
+// The Singletrack reconstruction (minimap2/ksw2_singletrack.cpp:63-176) from (i, j) to a matrix
+// edge.  FORCE as above (insertions above the computed blocks of an anti-diagonal, deletions
+// below).  Returns false when no gap explains a cell.  `probe` holds the tiles of a gap search.
+template <class Window, class Probe, class GRP, class FORCE>
+__device__ bool tb_singletrack(int &i, int &j, WarpCigar &cg, Window &win, Probe &probe, GRP &&grp, FORCE &&force,
+                               const KswScore &S, const int8_t *mat, int m, const uint8_t *qs, const uint8_t *ts) {
+    const int lane = threadIdx.x & 31;
+    auto stored = [&](int a, int b) { return force(a, b) < 0; };
+    const int o1 = -S.q, g1 = -S.e, o2 = -S.q2, g2 = -S.e2;
+    // the difference along the matrix edge for edge cell c
+    auto edge = [&](int c) { return tb_st_gap(c + 1, o1, g1, o2, g2) - tb_st_gap(c, o1, g1, o2, g2); };
+    while (i >= 0 && j >= 0) {
+        const int f = force(i, j);
+        if (f == 2) { cg.push(1, 1); --j; continue; }
+        if (f == 1) { cg.push(2, 1); --i; continue; }
+        // the run of diagonal moves: v(i, j) + u(i, j-1) is the cell's substitution score
+        win.ensure(i, j, grp);
+        const int li = i - lane, lj = j - lane;
+        const bool in = li >= 0 && lj >= 0 && win.has(li, lj) && stored(li, lj);
+        bool on = in;
+        if (in) {
+            const int h = tb_sx8(win.at(li, lj, 0));
+            const bool fin = lj == 0 || stored(li, lj - 1);
+            const int v = lj == 0 ? edge(li) : fin ? tb_sx8(win.at(li, lj - 1, 1)) : 0;
+            on = fin && h + v == mat[ts[li] * m + qs[lj]];
+        }
+        const unsigned off = __ballot_sync(TB_ALL, !on);
+        const int run = off ? __ffs(off) - 1 : 32;
+        if (run > 0) {
+            cg.push(0, run);
+            i -= run, j -= run;
+        }
+        if (run == 32 || !__shfl_sync(TB_ALL, in ? 1 : 0, run)) continue;
+        // the gap that leaves (i, j): the first length l whose summed differences up the
+        // column of rows (insertion) or along the row (deletion) are exactly a gap of l;
+        // 32 lengths at a time, lane k looking at length base + k + 1.  Sums over cells
+        // outside the stored band match no gap (d_ok, i_ok).
+        int base = 0, dsum = 0, isum = 0;
+        bool d_ok = true, i_ok = true;
+        for (;;) {
+            const int l = base + lane + 1, id = i - l, jn = j - l;
+            // differences of the l-th cell: u(i-l+1, j) and v(i, j-l+1)
+            int du = 0, dv = 0;
+            bool uf = true, vf = true;
+            if (d_ok && i - base >= 0) probe.corner(i - base, j, grp);
+            if (d_ok && id + 1 >= 0) {
+                uf = stored(id + 1, j);
+                if (uf) du = tb_sx8(probe.at(id + 1, j, 1));
+            }
+            __syncwarp();
+            if (i_ok && j - base >= 0) probe.corner(i, j - base, grp);
+            if (i_ok && jn + 1 >= 0) {
+                vf = stored(i, jn + 1);
+                if (vf) dv = tb_sx8(probe.at(i, jn + 1, 0));
+            }
+            __syncwarp();
+#pragma unroll
+            for (int k = 1; k < 32; k <<= 1) {
+                const int a = __shfl_up_sync(TB_ALL, du, k), b = __shfl_up_sync(TB_ALL, dv, k);
+                if (lane >= k) du += a, dv += b;
+            }
+            const unsigned ub = __ballot_sync(TB_ALL, !uf), vb = __ballot_sync(TB_ALL, !vf);
+            const unsigned upto = lane == 31 ? TB_ALL : (2u << lane) - 1u;
+            const int a1 = o1 + l * g1, a2 = o2 + l * g2, dd = dsum + du, di = isum + dv;
+            const bool dhit = d_ok && !(ub & upto) && id >= -1 && (dd == a1 || dd == a2);
+            const bool ihit = i_ok && !(vb & upto) && jn >= -1 && (di == a1 || di == a2);
+            const unsigned end = __ballot_sync(TB_ALL, l > i + 1 && l > j + 1);
+            const unsigned db = __ballot_sync(TB_ALL, dhit), hit = db | __ballot_sync(TB_ALL, ihit);
+            if (hit && (!end || __ffs(hit) <= __ffs(end))) {
+                const int k = __ffs(hit) - 1, len = base + k + 1;
+                if (db >> k & 1u) cg.push(2, len), i -= len;
+                else cg.push(1, len), j -= len;
+                break;
+            }
+            if (end) return false;
+            dsum += __shfl_sync(TB_ALL, du, 31), isum += __shfl_sync(TB_ALL, dv, 31);
+            d_ok = d_ok && !ub, i_ok = i_ok && !vb;
+            base += 32;
+        }
+    }
+    return true;
 }
 
 }  // namespace aw

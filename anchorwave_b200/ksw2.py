@@ -289,7 +289,8 @@ def set_band_columns(columns: int = 0):
 
 
 def set_full_pair_routing(enabled: bool = True):
-    """aw_set_full_pair_routing: critical-path full-matrix pairs on the banded kernel (default)."""
+    """aw_set_full_pair_routing: critical-path full-matrix pairs beyond the traceback budget on the
+    banded kernel (default)."""
     lib.aw_set_full_pair_routing(1 if enabled else 0)
 
 

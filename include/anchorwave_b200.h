@@ -414,15 +414,18 @@ int aw_ksw_extd2_device_noalloc(int qlen, const uint8_t *d_query, int tlen, cons
  * admission envelope (src/myImportandFunction/AlignmentResourceScheduler.cpp:706).
  * 0 = default (60% of free device memory). */
 void aw_set_traceback_budget(int64_t bytes);
-/* Warps that cooperate on one pair for pairs with tlen >= threshold, and the
- * threshold (autotuner knobs; 0 keeps the current value). */
+/* Full-matrix pairs with tlen >= threshold run their strips on a warp each (large_warps > 1:
+ * 2, 4 or 8) or all on one warp (1); shorter pairs of a batch are split by the batch's work
+ * unless large_warps is 1, and small batches always run on narrow strips, one warp each
+ * (autotuner knobs; 0 keeps the current value).  Results are identical. */
 void aw_set_tuning(int large_warps, int large_tlen_threshold);
 /* Target columns per lane of the banded kernel (4 or 8; 0 = chosen per batch from
  * its work and its longest pair).  No counterpart in the reference (tuning knob). */
 void aw_set_band_columns(int columns);
 /* 1 (default): a full-matrix pair that would be its batch's critical path (a long interval
- * alone or among short ones) runs on the banded kernel at full width, whose strip pipeline
- * spans all SMs; 0: every full-matrix pair runs on the full-matrix strip kernel.  Results
+ * alone or among short ones) and whose traceback exceeds the HBM traceback budget runs on the
+ * banded kernel at full width, which recomputes the traceback in rounds; 0: every full-matrix
+ * pair runs on the full-matrix strip kernel, and such a pair fails with AW_E_NOMEM.  Results
  * are identical either way.  No counterpart in the reference (tuning knob). */
 void aw_set_full_pair_routing(int enabled);
 /* Frees the device and pinned buffers that the calling thread's KSW2 calls keep pooled
