@@ -28,9 +28,13 @@
 // cell and unpacks the blocks oldest first, re-extending the matches
 // (wavefront/wavefront_backtrace.c:767-799, wavefront/wavefront_pcigar.c:222-278).
 //
-// Memory: per-score headers and wavefront arrays come from one device pool by a
-// bump allocator (atomicAdd, 256 KiB chunks).  A pair that finds the pool empty
-// stops with WFA_RETRY and the host re-runs it in a later round with a fresh pool.
+// Memory: per-score headers and wavefront arrays come from one device pool in 256 KiB
+// chunks (larger arrays in several), taken from its end by an atomicAdd.  A finished pair
+// gives its chunks to a free ring, from which the next pairs take theirs first, so a
+// batch needs the memory of the pairs in flight and not of all pairs (16,384 pairs of
+// 0.1-10 kb in a 20 GB pool: 672 -> 123 ms, 33 rounds -> 1).  A pair that finds
+// the pool empty stops with WFA_RETRY and the host re-runs it in a later round with a
+// fresh pool.
 #include "aw_internal.h"
 #include "wfa_internal.h"
 
@@ -41,7 +45,6 @@ namespace {
 
 constexpr int32_t WF_NULL = INT32_MIN / 2;
 constexpr int HDR_CHUNK = 256;               // scores per header chunk
-constexpr int64_t DATA_CHUNK = 256 << 10;    // bytes per data chunk
 
 struct CompHdr {
     int32_t lo, hi, base, pad;
@@ -52,10 +55,14 @@ struct ScoreHdr {
 };
 enum { CM = 0, CI1 = 1, CD1 = 2, CI2 = 3, CD2 = 4 };
 
+// A pair's (or, for piggyback blocks, a warp's) memory: the current chunk's free range and the
+// chunks taken, linked through their first 16 bytes (previous chunk, size).  In shared memory:
+// one lane of a warp uses it, and every lane would pay for its registers.
 struct Alloc {
     int64_t cur, end;
-    bool ok;
-    int64_t used;  // bytes taken from the pool (lane 0's copy)
+    int64_t used;   // bytes taken from the pool
+    int64_t list;
+    __device__ void init() { cur = end = used = 0, list = -1; }
 };
 
 // Packed CIGAR of the piggyback modes (wavefront/wavefront_pcigar.h:44-71): 2 bits per
@@ -65,50 +72,112 @@ constexpr uint32_t BT_NULL = 0xFFFFFFFFu;          // no earlier block
 constexpr int PIG_U = 2;                           // diagonals per lane in flight
 constexpr uint32_t LANE_BLOCKS = 32;               // blocks a lane reserves at a time
 
-__device__ __forceinline__ int64_t pool_grab(const WfaArgs &A, int64_t bytes) {
-    const unsigned long long b = atomicAdd(A.pool_head, (unsigned long long)bytes);
-    if ((int64_t)(b + bytes) > A.pool_bytes) return -1;
+// The pool as the allocating functions (out of line, so no reference to the kernel's arguments)
+// take it.
+struct Pool {
+    uint8_t *base;
+    int64_t bytes;
+    WfaPoolCtl *ctl;
+    int32_t *ring;
+    uint32_t slots;
+};
+__device__ __forceinline__ Pool pool_of(const WfaArgs &A) {
+    return Pool{A.pool, A.pool_bytes, A.ctl, A.free_ring, A.free_slots};
+}
+
+__device__ __forceinline__ int64_t pool_grab(const Pool &A, int64_t bytes) {
+    const unsigned long long b = atomicAdd(&A.ctl->head, (unsigned long long)bytes);
+    if ((int64_t)(b + bytes) > A.bytes) return -1;
     return (int64_t)b;
 }
 
-// Lane-0 bump allocation inside the warp's current chunk; broadcast to the warp.
-__device__ int64_t warp_alloc(const WfaArgs &A, Alloc &al, int64_t bytes, int lane) {
+// A chunk of a finished pair, or -1.  The ring holds `avail` complete entries; the entry at the
+// taken position may still be on its way from the thread that reserved it, hence the wait.
+__device__ __forceinline__ int64_t free_pop(const Pool &A) {
+    if (*(volatile int32_t *)&A.ctl->avail <= 0) return -1;
+    if (atomicSub(&A.ctl->avail, 1) <= 0) {
+        atomicAdd(&A.ctl->avail, 1);
+        return -1;
+    }
+    int32_t *slot = A.ring + atomicAdd(&A.ctl->popped, 1u) % A.slots;
+    int32_t v = 0;
+    for (int spins = 0; spins < (1 << 20) && (v = atomicExch(slot, 0)) == 0; ++spins) __nanosleep(20);
+    __threadfence();  // the previous owner's accesses come before ours
+    return v ? (int64_t)(v - 1) * WFA_CHUNK : -1;
+}
+__device__ __forceinline__ void free_push(const Pool &A, int64_t off) {
+    int32_t *slot = A.ring + atomicAdd(&A.ctl->pushed, 1u) % A.slots;
+    for (int spins = 0; atomicCAS(slot, 0, (int32_t)(off / WFA_CHUNK) + 1) != 0; ++spins) {
+        if (spins > (1 << 20)) return;  // never with a slot per chunk; the chunk is lost for the round
+        __nanosleep(20);
+    }
+    __threadfence();
+    atomicAdd(&A.ctl->avail, 1);
+}
+
+// One thread: a chunk that holds `bytes`, linked to the allocation's list; false if there is none.
+__device__ __noinline__ bool take_chunk(Pool A, Alloc &al, int64_t bytes) {
+    const int64_t sz = (bytes + 16 + WFA_CHUNK - 1) / WFA_CHUNK * WFA_CHUNK;
+    int64_t b = sz == WFA_CHUNK ? free_pop(A) : -1;
+    if (b < 0) b = pool_grab(A, sz);
+    if (b < 0 && sz == WFA_CHUNK) b = free_pop(A);  // given back meanwhile
+    if (b < 0) return false;
+    int64_t *h = (int64_t *)(A.base + b);
+    h[0] = al.list, h[1] = sz;
+    al.list = b, al.cur = b + 16, al.end = b + sz;
+    al.used += bytes > WFA_CHUNK ? bytes : WFA_CHUNK;
+    return true;
+}
+
+// One thread, after every access to the allocation: its chunks back to the pool.
+__device__ __noinline__ void give_back(Pool A, Alloc &al) {
+    __threadfence();
+    for (int64_t b = al.list; b >= 0;) {
+        const int64_t *h = (const int64_t *)(A.base + b);
+        const int64_t prev = h[0], sz = h[1];
+        for (int64_t o = 0; o < sz; o += WFA_CHUNK) free_push(A, b + o);
+        b = prev;
+    }
+    al.list = -1;
+}
+
+// Lane-0 bump allocation inside the current chunk; broadcast to the warp (-1: none left).
+__device__ __forceinline__ int64_t warp_alloc(const WfaArgs &A, Alloc &al, int64_t bytes, int lane) {
     bytes = (bytes + 15) & ~(int64_t)15;
     int64_t r = -1;
-    if (lane == 0) {
-        if (al.ok) {
-            if (al.cur + bytes > al.end) {
-                const int64_t sz = bytes > DATA_CHUNK ? bytes : DATA_CHUNK;
-                const int64_t b = pool_grab(A, sz);
-                if (b < 0) al.ok = false;
-                else al.cur = b, al.end = b + sz, al.used += sz;
-            }
-            if (al.ok) {
-                r = al.cur;
-                al.cur += bytes;
-            }
-        }
+    if (lane == 0 && (al.cur + bytes <= al.end || take_chunk(pool_of(A), al, bytes))) {
+        r = al.cur;
+        al.cur = r + bytes;
     }
-    r = __shfl_sync(0xffffffffu, r, 0);
-    al.ok = __shfl_sync(0xffffffffu, al.ok ? 1 : 0, 0);
-    al.cur = __shfl_sync(0xffffffffu, al.cur, 0);
-    al.end = __shfl_sync(0xffffffffu, al.end, 0);
-    return r;
+    return __shfl_sync(0xffffffffu, r, 0);
 }
 
 __device__ __forceinline__ ScoreHdr *hdr_ptr(const WfaArgs &A, const int64_t *ctab, int s) {
     return (ScoreHdr *)(A.pool + ctab[s / HDR_CHUNK]) + (s % HDR_CHUNK);
 }
 
-// The forward pass reads the headers of the last max_score_scope scores only; each warp
-// keeps them in a shared-memory ring of RS (a power of two above the scope) as well as in
-// the pool (the backtrace reads all of them from the pool).  RS = 0: pool only.
+// The forward pass reads M's headers of the last max_score_scope scores, I1/D1's of the last
+// e1 and I2/D2's of the last e2; each warp (or CTA) keeps them in shared-memory rings (powers
+// of two, masks mm, m1, m2) as well as in the pool (the backtrace reads all of them from the
+// pool).  mm < 0: pool only.
+struct RingShape {
+    int mm, m1, m2;
+    __host__ __device__ int entries() const { return mm < 0 ? 0 : mm + 1 + 2 * (m1 + 1) + 2 * (m2 + 1); }
+};
 struct HdrRing {
-    ScoreHdr *ring;
-    int rs;
-    __device__ __forceinline__ const ScoreHdr *get(const WfaArgs &A, const int64_t *ctab, int sc, int s) const {
-        if (rs && sc > s - rs) return ring + (sc & (rs - 1));
-        return hdr_ptr(A, ctab, sc);
+    CompHdr *ring;
+    RingShape sh;
+    __device__ __forceinline__ CompHdr *at(int c, int sc) const {
+        if (c == CM) return ring + (sc & sh.mm);
+        CompHdr *r = ring + sh.mm + 1;
+        if (c <= CD1) return r + (c - CI1) * (sh.m1 + 1) + (sc & sh.m1);
+        return r + 2 * (sh.m1 + 1) + (c - CI2) * (sh.m2 + 1) + (sc & sh.m2);
+    }
+    __device__ __forceinline__ CompHdr get(const WfaArgs &A, const int64_t *ctab, int c, int sc) const {
+        return sh.mm >= 0 ? *at(c, sc) : hdr_ptr(A, ctab, sc)->c[c];
+    }
+    __device__ __forceinline__ void put(int c, int sc, const CompHdr &h) const {
+        if (sh.mm >= 0) *at(c, sc) = h;
     }
 };
 
@@ -290,7 +359,7 @@ __device__ void finish_pair(const WfaArgs &A, const WfaPairDev &PR, int idx, con
             // reverse the links from the end cell in place, then unpack the blocks
             // oldest first: before every operation taken in M the run of matches
             // is re-extended; the mismatch that closes a gap is dropped
-            const CompHdr m = HR.get(A, ctab, end_score, end_score)->c[CM];
+            const CompHdr m = HR.get(A, ctab, CM, end_score);
             const uint32_t *md = (const uint32_t *)(A.pool + m.off) + (k_end - m.base);
             const uint32_t pc_end = md[m.pad];
             uint32_t cur = md[2 * m.pad], prv = BT_NULL;
@@ -587,62 +656,70 @@ struct WidePlan {
     int op, lo, hi, mask;  // mask: components allocated at the planned score (bit c)
     CompHdr in[7];         // M[s-x], M[s-o1-e1], I1[s-e1], D1[s-e1], M[s-o2-e2], I2[s-e2], D2[s-e2]
     CompHdr out[5];
+    InHdr view[7];         // the same inputs as the compute step of the high memory modes reads them
+    int32_t *dst[5];       // and where it writes diagonal lo (null: not stored)
 };
-struct WidePart {
-    int kmin[5], kmax[5], reached, pad;
-    int retry, pad2;          // a warp found the pool exhausted (CTA-cooperative piggyback mode)
+// Maxima over a CTA's diagonals, folded by atomicMax: k[c] the highest diagonal of component
+// c in the matrix, k[5 + c] minus the lowest, k[10] 1 when the end cell was reached.
+struct __align__(16) WidePart {
+    int k[12];
+    int retry, pad;           // a warp found the pool exhausted (CTA-cooperative piggyback mode)
     unsigned long long used;  // pool bytes of the warps' block reservations (the same)
 };
 
-__device__ __forceinline__ void part_reset(WidePart &p) {
-    for (int c = 0; c < 5; ++c) p.kmin[c] = INT_MAX, p.kmax[c] = INT_MIN;
-    p.reached = 0;
+__device__ __forceinline__ void part_reset(WidePart &p, int lane) {
+    if (lane < 12) p.k[lane] = INT_MIN;
 }
 
-// The input headers of score s from the header ring (null below score 0).
-__device__ __forceinline__ void plan_inputs(const WfaArgs &A, const int64_t *ctab, const HdrRing &HR, int s,
-                                            CompHdr (&in)[7]) {
-    const WfaPen P = A.pen;
-    const CompHdr NUL{1, -1, 0, 0, 0};
-    const int sm = s - P.x, so1 = s - P.o1 - P.e1, se1 = s - P.e1, so2 = s - P.o2 - P.e2, se2 = s - P.e2;
-    in[0] = sm >= 0 ? HR.get(A, ctab, sm, s)->c[CM] : NUL;
-    in[1] = so1 >= 0 ? HR.get(A, ctab, so1, s)->c[CM] : NUL;
-    in[2] = se1 >= 0 ? HR.get(A, ctab, se1, s)->c[CI1] : NUL;
-    in[3] = se1 >= 0 ? HR.get(A, ctab, se1, s)->c[CD1] : NUL;
-    in[4] = so2 >= 0 ? HR.get(A, ctab, so2, s)->c[CM] : NUL;
-    in[5] = se2 >= 0 ? HR.get(A, ctab, se2, s)->c[CI2] : NUL;
-    in[6] = se2 >= 0 ? HR.get(A, ctab, se2, s)->c[CD2] : NUL;
+// Planning a score takes one warp: lane j < 7 holds the j-th input of the compute step (M[s-x],
+// M[s-o1-e1], I1[s-e1], D1[s-e1], M[s-o2-e2], I2[s-e2], D2[s-e2]): its component, its distance
+// in scores, and how it moves the limits.  A null input contributes lo=1, hi=-1.
+struct PlanLane {
+    int comp, dist, dlo, dhi;
+};
+__device__ __forceinline__ PlanLane plan_lane(const WfaPen &P, int lane) {
+    switch (lane) {
+    case 0: return PlanLane{CM, P.x, 0, 0};
+    case 1: return PlanLane{CM, P.o1 + P.e1, -1, 1};
+    case 2: return PlanLane{CI1, P.e1, 1, 1};
+    case 3: return PlanLane{CD1, P.e1, -1, -1};
+    case 4: return PlanLane{CM, P.o2 + P.e2, -1, 1};
+    case 5: return PlanLane{CI2, P.e2, 1, 1};
+    case 6: return PlanLane{CD2, P.e2, -1, -1};
+    default: return PlanLane{CM, 0, 0, 0};
+    }
 }
-
-// The limits of the compute step over its inputs (null inputs contribute lo=1, hi=-1) and
-// which I/D outputs exist (one of their inputs exists).
-__device__ __forceinline__ void plan_limits(const CompHdr (&in)[7], int &lo, int &hi, int &mask) {
-    bool isnull[7];
-    for (int j = 0; j < 7; ++j) isnull[j] = in[j].lo > in[j].hi;
-    lo = in[0].lo, hi = in[0].hi;
-    lo = min(lo, in[1].lo - 1), hi = max(hi, in[1].hi + 1);
-    lo = min(lo, in[2].lo + 1), hi = max(hi, in[2].hi + 1);
-    lo = min(lo, in[3].lo - 1), hi = max(hi, in[3].hi - 1);
-    lo = min(lo, in[4].lo - 1), hi = max(hi, in[4].hi + 1);
-    lo = min(lo, in[5].lo + 1), hi = max(hi, in[5].hi + 1);
-    lo = min(lo, in[6].lo - 1), hi = max(hi, in[6].hi - 1);
+// Lane j's input header of score s; returns the lanes whose input is not null.
+__device__ __forceinline__ unsigned plan_input(const WfaArgs &A, const int64_t *ctab, const HdrRing &HR, const PlanLane &L,
+                                               int s, int lane, CompHdr &h) {
+    h = CompHdr{1, -1, 0, 0, 0};
+    if (lane < 7 && s - L.dist >= 0) h = HR.get(A, ctab, L.comp, s - L.dist);
+    return __ballot_sync(0xffffffffu, lane < 7 && h.lo <= h.hi);
+}
+// The limits of the compute step and which I/D outputs exist (one of their inputs exists).
+__device__ __forceinline__ void plan_limits(const PlanLane &L, int lane, const CompHdr &h, unsigned some, int &lo, int &hi,
+                                            int &mask) {
+    lo = __reduce_min_sync(0xffffffffu, lane < 7 ? h.lo + L.dlo : INT_MAX);
+    hi = __reduce_max_sync(0xffffffffu, lane < 7 ? h.hi + L.dhi : INT_MIN);
     mask = 1;
-    if (!isnull[1] || !isnull[2]) mask |= 1 << CI1;
-    if (!isnull[1] || !isnull[3]) mask |= 1 << CD1;
-    if (!isnull[4] || !isnull[5]) mask |= 1 << CI2;
-    if (!isnull[4] || !isnull[6]) mask |= 1 << CD2;
+    if (some & (1u << 1 | 1u << 2)) mask |= 1 << CI1;
+    if (some & (1u << 1 | 1u << 3)) mask |= 1 << CD1;
+    if (some & (1u << 4 | 1u << 5)) mask |= 1 << CI2;
+    if (some & (1u << 4 | 1u << 6)) mask |= 1 << CD2;
 }
 
 // A warp's trimmed ends and end check, folded into its CTA's partials.
 __device__ __forceinline__ void fold_partials(const int (&kmin)[5], const int (&kmax)[5], bool reached, WidePart &pp) {
     const int lane = threadIdx.x & 31;
+    int v = __any_sync(0xffffffffu, reached) ? 1 : INT_MIN;
 #pragma unroll
     for (int c = 0; c < 5; ++c) {
         const int th = __reduce_max_sync(0xffffffffu, kmax[c]);
-        const int tl = __reduce_min_sync(0xffffffffu, kmin[c]);
-        if (lane == 0 && th != INT_MIN) atomicMax(&pp.kmax[c], th), atomicMin(&pp.kmin[c], tl);
+        const int tl = __reduce_max_sync(0xffffffffu, -kmin[c]);
+        if (lane == c) v = th;
+        if (lane == 5 + c) v = tl;
     }
-    if (__any_sync(0xffffffffu, reached) && lane == 0) pp.reached = 1;
+    if (lane < 11 && v != INT_MIN) atomicMax(&pp.k[lane], v);
 }
 
 // First array of component c at score sc in the piggyback rings: M's last SR scores, then
@@ -665,15 +742,11 @@ template <bool L2>
 __device__ __forceinline__ void plan_compute(const WfaArgs &A, const WfaPairDev &PR, const uint8_t *pat,
                                              const uint8_t *txt, const WidePlan &Q, int g0, int G, WidePart &pp) {
     const int plen = PR.plen, tlen = PR.tlen, k_end = tlen - plen;
-    const int lo = Q.lo, hi = Q.hi, mask = Q.mask;
-    const InHdr m_misms = in_hdr(A, Q.in[0]), m_open1 = in_hdr(A, Q.in[1]), i1 = in_hdr(A, Q.in[2]),
-                d1 = in_hdr(A, Q.in[3]), m_open2 = in_hdr(A, Q.in[4]), i2 = in_hdr(A, Q.in[5]),
-                d2 = in_hdr(A, Q.in[6]);
-    int32_t *oM = (int32_t *)(A.pool + Q.out[CM].off);
-    int32_t *oI1 = (mask & 2) ? (int32_t *)(A.pool + Q.out[CI1].off) : nullptr;
-    int32_t *oD1 = (mask & 4) ? (int32_t *)(A.pool + Q.out[CD1].off) : nullptr;
-    int32_t *oI2 = (mask & 8) ? (int32_t *)(A.pool + Q.out[CI2].off) : nullptr;
-    int32_t *oD2 = (mask & 16) ? (int32_t *)(A.pool + Q.out[CD2].off) : nullptr;
+    const int lo = Q.lo, hi = Q.hi;
+    if (lo + (g0 & ~31) > hi) return;  // no diagonal for this warp
+    const InHdr m_misms = Q.view[0], m_open1 = Q.view[1], i1 = Q.view[2], d1 = Q.view[3], m_open2 = Q.view[4],
+                i2 = Q.view[5], d2 = Q.view[6];
+    int32_t *oM = Q.dst[CM], *oI1 = Q.dst[CI1], *oD1 = Q.dst[CD1], *oI2 = Q.dst[CI2], *oD2 = Q.dst[CD2];
     int kmin[5], kmax[5];
     bool reached = false;
 #pragma unroll
@@ -727,32 +800,23 @@ __device__ __forceinline__ void plan_compute(const WfaArgs &A, const WfaPairDev 
     fold_partials(kmin, kmax, reached, pp);
 }
 
-// Thread-0 bump allocation for the CTA-cooperative mode.
-__device__ int64_t cta_alloc(const WfaArgs &A, Alloc &al, int64_t bytes) {
-    bytes = (bytes + 15) & ~(int64_t)15;
-    if (!al.ok) return -1;
-    if (al.cur + bytes > al.end) {
-        const int64_t sz = bytes > DATA_CHUNK ? bytes : DATA_CHUNK;
-        const int64_t b = pool_grab(A, sz);
-        if (b < 0) {
-            al.ok = false;
-            return -1;
-        }
-        al.cur = b, al.end = b + sz, al.used += sz;
-    }
-    const int64_t r = al.cur;
-    al.cur += bytes;
-    return r;
-}
-
-// CTA-cooperative mode: one long pair on all threads of a CTA.  Thread 0 plans
-// every score (the headers in the CTA's header ring and the pool, the allocations) and all
-// threads compute and extend the diagonals lo + tid + NT*u; two CTA barriers per score.  A
-// pair whose wavefront grows too wide stops with WFA_WIDE for the cluster kernel.  The cell arithmetic, the limits, the trimming and the backtrace are the warp's.
-// In the piggyback modes every warp reserves its own block runs; no pair moves to the
-// cluster kernel.
+// CTA-cooperative mode: one long pair on all threads of a CTA.  Warp 0 plans every score, a
+// lane per input and per output component (the headers in the CTA's header ring and the pool,
+// the allocations), and all threads compute and extend the diagonals lo + tid + NT*u; two
+// CTA barriers per score.  A pair whose wavefront grows too wide stops with WFA_WIDE for
+// the cluster kernel.  The cell arithmetic, the limits, the trimming and the backtrace are the
+// warp's.  In the piggyback modes every warp reserves its own block runs; no pair moves to
+// the cluster kernel.
+struct CtaPlanner {  // warp 0's state (shared memory)
+    int s, num_null, status, end_score;
+    int64_t ring, hdr_off;
+    int64_t rbase;  // piggyback rings: their place and the elements of a slot's array
+    int rcap, pad;
+    Alloc al;
+};
 template <bool PIG>
-__device__ void cta_pair(const WfaArgs &A, int idx, const HdrRing &HR, WidePlan &plan, WidePart &part) {
+__device__ void cta_pair(const WfaArgs &A, int idx, const HdrRing &HR, WidePlan &plan, WidePart &part, CtaPlanner &Q,
+                         Alloc &wal) {
     const int tid = threadIdx.x, NT = blockDim.x, lane = tid & 31;
     const WfaPen P = A.pen;
     const WfaPairDev PR = A.pairs[idx];
@@ -760,26 +824,24 @@ __device__ void cta_pair(const WfaArgs &A, int idx, const HdrRing &HR, WidePlan 
     const uint8_t *pat = A.pat + PR.poff, *txt = A.txt + PR.toff;
     int64_t *ctab = A.ctab + PR.ctab_off;
     const CompHdr NUL{1, -1, 0, 0, 0};
-    // thread 0's state
-    int s = 0, num_null = 0, status = 0, end_score = -1;
     const int smax = PR.ctab_cap * HDR_CHUNK - 1;
     const int R = (P.e1 > P.e2 ? P.e1 : P.e2) + 1, ring_cap = plen + tlen + 8;
-    int64_t ring = -1;
-    Alloc al{0, 0, true, 0};
-    // piggyback rings (thread 0) and every warp's block reservations
+    // piggyback rings, and every warp's block reservations
     const int SR = A.max_score_scope, R1 = P.e1 + 1, R2 = P.e2 + 1;
     const int64_t ring_arrays = 3 * (int64_t)(SR + 2 * R1 + 2 * R2);
-    int rcap = 32;
-    int64_t rbase = -1;
-    Alloc wal{0, 0, true, 0};
     uint32_t bnext = 0, bend = 0;
-    auto set_hdr = [&](int sc, const CompHdr (&o)[5]) {
-        ScoreHdr *OH = hdr_ptr(A, ctab, sc);
-        for (int c = 0; c < 5; ++c) OH->c[c] = o[c];
-        if (HR.rs)
-            for (int c = 0; c < 5; ++c) HR.ring[sc & (HR.rs - 1)].c[c] = o[c];
+    if (lane == 0) wal.init();
+    // lane c < 5: component c's header of score sc
+    auto set_hdr = [&](int sc, const CompHdr &o) {
+        if (lane < 5) {
+            ((ScoreHdr *)(A.pool + Q.hdr_off))[sc % HDR_CHUNK].c[lane] = o;
+            HR.put(lane, sc, o);
+        }
+        __syncwarp();
     };
     auto plan_next = [&]() {
+        const PlanLane L = plan_lane(P, lane);
+        int s = Q.s, num_null = Q.num_null, status = 0;
         for (;;) {
             ++s;
             if (s > smax) {
@@ -787,20 +849,18 @@ __device__ void cta_pair(const WfaArgs &A, int idx, const HdrRing &HR, WidePlan 
                 break;
             }
             if (s % HDR_CHUNK == 0) {
-                const int64_t hb = cta_alloc(A, al, (int64_t)sizeof(ScoreHdr) * HDR_CHUNK);
+                const int64_t hb = warp_alloc(A, Q.al, (int64_t)sizeof(ScoreHdr) * HDR_CHUNK, lane);
                 if (hb < 0) {
                     status = WFA_RETRY;
                     break;
                 }
-                ctab[s / HDR_CHUNK] = hb;
+                if (lane == 0) Q.hdr_off = hb, ctab[s / HDR_CHUNK] = hb;
+                __syncwarp();
             }
-            CompHdr in[7];
-            plan_inputs(A, ctab, HR, s, in);
-            bool all_null = true;
-            for (int j = 0; j < 7; ++j) all_null &= in[j].lo > in[j].hi;
-            if (all_null) {
-                const CompHdr o[5] = {NUL, NUL, NUL, NUL, NUL};
-                set_hdr(s, o);
+            CompHdr in;
+            const unsigned some = plan_input(A, ctab, HR, L, s, lane, in);
+            if (!some) {
+                set_hdr(s, NUL);
                 if (++num_null > A.max_score_scope) {  // the top of the next step: M[s] is empty
                     status = -3;
                     break;
@@ -809,93 +869,111 @@ __device__ void cta_pair(const WfaArgs &A, int idx, const HdrRing &HR, WidePlan 
             }
             num_null = 0;
             int lo, hi, mask;
-            plan_limits(in, lo, hi, mask);
+            plan_limits(L, lane, in, some, lo, hi, mask);
             const int width = hi - lo + 1;
+            const bool mine = lane < 5 && (mask >> lane & 1);
+            CompHdr out = NUL;
             if constexpr (PIG) {
-                if (width > rcap) {
-                    const int nc = max(2 * rcap, (width + 3) & ~3);
-                    const int64_t nb = cta_alloc(A, al, ring_arrays * nc * 4);
+                if (width > Q.rcap) {
+                    const int nc = max(2 * Q.rcap, (width + 3) & ~3);
+                    const int64_t nb = warp_alloc(A, Q.al, ring_arrays * nc * 4, lane);
                     if (nb < 0) {
                         status = WFA_RETRY;
                         break;
                     }
-                    rcap = nc, rbase = nb;
+                    __syncwarp();
+                    if (lane == 0) Q.rcap = nc, Q.rbase = nb;
+                    __syncwarp();
                 }
-                for (int c = 0; c < 5; ++c)
-                    plan.out[c] = (mask & (1 << c)) ? CompHdr{lo, hi, lo, rcap, rbase + pig_slot(c, s, SR, R1, R2) * rcap * 4}
-                                                     : NUL;
-                for (int j = 0; j < 7; ++j) plan.in[j] = in[j];
-                plan.op = WOP_COMPUTE, plan.lo = lo, plan.hi = hi, plan.mask = mask;
-                return;
-            }
-            // a wavefront too wide for the CTA: the cluster kernel re-runs the pair (past
-            // wide_width_cta always; past wide_width_tail in the call's tail, checked every 32
-            // scores: every pair started and few still running)
-            if (A.wide_width_cta > 0 && width > A.wide_width_tail) {
-                bool wide = width > A.wide_width_cta;
-                if (!wide && (s & 31) == 0)
-                    wide = *(volatile int32_t *)(A.queue + 2) >= A.n_long && *(volatile int32_t *)A.queue >= A.n &&
-                           *(volatile int32_t *)(A.queue + 1) <= A.wide_tail_pairs;
-                if (wide) {
-                    status = WFA_WIDE;
+                if (mine) out = CompHdr{lo, hi, lo, Q.rcap, Q.rbase + pig_slot(lane, s, SR, R1, R2) * Q.rcap * 4};
+            } else {
+                // a wavefront too wide for the CTA: the cluster kernel re-runs the pair (past
+                // wide_width_cta always; past wide_width_tail in the call's tail, checked every 32
+                // scores: every pair started and few still running)
+                if (A.wide_width_cta > 0 && width > A.wide_width_tail) {
+                    bool wide = width > A.wide_width_cta;
+                    if (!wide && (s & 31) == 0)
+                        wide = __all_sync(0xffffffffu, *(volatile int32_t *)(A.queue + 3) >= A.n_all &&
+                                                           *(volatile int32_t *)(A.queue + 1) <= A.wide_tail_pairs);
+                    if (wide) {
+                        status = WFA_WIDE;
+                        break;
+                    }
+                }
+                if (A.singletrack && width > ring_cap) {
+                    status = WFA_OVERFLOW;
                     break;
                 }
+                const int64_t wb = (((int64_t)width * 4) + 15) & ~(int64_t)15;
+                const int64_t blk = warp_alloc(A, Q.al, wb * (A.singletrack ? 1 : __popc(mask)), lane);
+                if (blk < 0) {
+                    status = WFA_RETRY;
+                    break;
+                }
+                if (mine) {
+                    const int64_t place = lane == CM || !A.singletrack
+                                              ? blk + wb * __popc(mask & ((1 << lane) - 1))
+                                              : Q.ring + ((int64_t)((s % R) * 4 + (lane - 1)) * ring_cap) * 4;
+                    out = CompHdr{lo, hi, lo, 0, place};
+                }
             }
-            if (A.singletrack && width > ring_cap) {
-                status = WFA_OVERFLOW;
-                break;
+            if constexpr (PIG) {
+                if (lane < 7) plan.in[lane] = in;
+            } else {
+                if (lane < 7) plan.view[lane] = in_hdr(A, in);
+                if (lane < 5) plan.dst[lane] = mine ? (int32_t *)(A.pool + out.off) : nullptr;
             }
-            const int64_t wb = (((int64_t)width * 4) + 15) & ~(int64_t)15;
-            const int64_t blk = cta_alloc(A, al, wb * (A.singletrack ? 1 : __popc(mask)));
-            if (blk < 0) {
-                status = WFA_RETRY;
-                break;
+            if (lane < 5) plan.out[lane] = out;
+            if (lane == 0) {
+                plan.op = WOP_COMPUTE, plan.lo = lo, plan.hi = hi, plan.mask = mask;
+                Q.s = s, Q.num_null = 0;
             }
-            int64_t o = blk;
-            for (int c = 0; c < 5; ++c) {
-                plan.out[c] = NUL;
-                if (!(mask & (1 << c))) continue;
-                int64_t place;
-                if (c == CM || !A.singletrack) place = o, o += wb;
-                else place = ring + ((int64_t)((s % R) * 4 + (c - 1)) * ring_cap) * 4;
-                plan.out[c] = CompHdr{lo, hi, lo, 0, place};
-            }
-            for (int j = 0; j < 7; ++j) plan.in[j] = in[j];
-            plan.op = WOP_COMPUTE, plan.lo = lo, plan.hi = hi, plan.mask = mask;
             return;
         }
-        plan.op = WOP_DONE;
+        if (lane == 0) plan.op = WOP_DONE, Q.s = s, Q.status = status;
     };
-    if (tid == 0) {
-        atomicAdd(A.queue + 1, 1);  // pairs running
-        part_reset(part);
-        part.retry = 0, part.used = 0;
+    if (tid < 32) {
+        int status = 0, end_score = -1;
+        int64_t ring = -1, rbase = -1;
+        constexpr int rcap = 32;
+        if (lane == 0) Q.al.init(), Q.s = Q.num_null = 0, Q.rcap = rcap;
+        __syncwarp();
+        if (lane == 0) atomicAdd(A.queue + 1, 1), atomicAdd(A.queue + 3, 1);  // pairs running, started
+        part_reset(part, lane);
+        if (lane == 0) part.retry = 0, part.used = 0;
         if (!PIG && A.singletrack) {
-            ring = cta_alloc(A, al, (int64_t)R * 4 * ring_cap * 4);
+            ring = warp_alloc(A, Q.al, (int64_t)R * 4 * ring_cap * 4, lane);
             if (ring < 0) status = WFA_RETRY;
         }
         if (PIG) {
-            rbase = cta_alloc(A, al, ring_arrays * rcap * 4);
+            rbase = warp_alloc(A, Q.al, ring_arrays * rcap * 4, lane);
             if (rbase < 0) status = WFA_RETRY;
         }
-        const int64_t h0 = status == 0 ? cta_alloc(A, al, (int64_t)sizeof(ScoreHdr) * HDR_CHUNK) : -1;
-        const int64_t d0 = h0 < 0 ? -1 : PIG ? rbase : cta_alloc(A, al, 16);  // piggyback: slot 0 of M
+        const int64_t h0 = status == 0 ? warp_alloc(A, Q.al, (int64_t)sizeof(ScoreHdr) * HDR_CHUNK, lane) : -1;
+        const int64_t d0 = h0 < 0 ? -1 : PIG ? rbase : warp_alloc(A, Q.al, 16, lane);  // piggyback: slot 0 of M
         if (status == 0 && d0 < 0) status = WFA_RETRY;
         if (status == 0) {
             // M[0] = {0} on diagonal 0, extended
             const int32_t o0 = (int32_t)lcp1(A, PR, pat, txt, 0, 0);
-            ctab[0] = h0;
-            *(int32_t *)(A.pool + d0) = o0;
-            if (PIG) {
-                ((uint32_t *)(A.pool + d0))[rcap] = 0u;
-                ((uint32_t *)(A.pool + d0))[2 * rcap] = BT_NULL;  // the start (0, 0)
+            if (lane == 0) {
+                Q.hdr_off = h0, Q.ring = ring, Q.rbase = rbase;
+                ctab[0] = h0;
+                *(int32_t *)(A.pool + d0) = o0;
+                if (PIG) {
+                    ((uint32_t *)(A.pool + d0))[rcap] = 0u;
+                    ((uint32_t *)(A.pool + d0))[2 * rcap] = BT_NULL;  // the start (0, 0)
+                }
             }
-            const CompHdr o[5] = {CompHdr{0, 0, 0, PIG ? rcap : 0, d0}, NUL, NUL, NUL, NUL};
-            set_hdr(0, o);
+            __syncwarp();
+            set_hdr(0, lane == 0 ? CompHdr{0, 0, 0, PIG ? rcap : 0, d0} : NUL);
             if (tlen - plen == 0 && o0 >= tlen) end_score = 0;
         }
-        if (status != 0 || end_score == 0) plan.op = WOP_DONE;
-        else plan_next();
+        if (lane == 0) Q.status = status, Q.end_score = end_score;
+        if (status != 0 || end_score == 0) {
+            if (lane == 0) plan.op = WOP_DONE;
+        } else {
+            plan_next();
+        }
     }
     __syncthreads();
     while (plan.op == WOP_COMPUTE) {
@@ -904,7 +982,8 @@ __device__ void cta_pair(const WfaArgs &A, int idx, const HdrRing &HR, WidePlan 
             bool reached = false, ok = true;
 #pragma unroll
             for (int c = 0; c < 5; ++c) kmin[c] = INT_MAX, kmax[c] = INT_MIN;
-            for (int kb = plan.lo; kb <= plan.hi && ok; kb += NT * PIG_U)
+            // a warp whose first diagonal lies beyond the wavefront has none in the trip
+            for (int kb = plan.lo; kb + (tid & ~31) <= plan.hi && ok; kb += NT * PIG_U)
                 ok = pig_trip(A, PR, pat, txt, kb, tid, NT, plan.lo, plan.hi, plan.in, plan.out, plan.mask,
                               plan.out[CM].pad, wal, bnext, bend, kmin, kmax, reached);
             fold_partials(kmin, kmax, reached, part);
@@ -913,26 +992,25 @@ __device__ void cta_pair(const WfaArgs &A, int idx, const HdrRing &HR, WidePlan 
             plan_compute<false>(A, PR, pat, txt, plan, tid, NT, part);
         }
         __syncthreads();
-        if (tid == 0 && part.retry) {
-            status = WFA_RETRY;
-            plan.op = WOP_DONE;
-        } else if (tid == 0) {
-            CompHdr out[5];
-            for (int c = 0; c < 5; ++c) {
-                out[c] = plan.out[c];
-                if (!(plan.mask & (1 << c))) continue;
-                // no diagonal in the matrix: the empty range [lo, lo-1] of the scan
-                if (part.kmax[c] == INT_MIN) out[c].hi = out[c].lo - 1;
-                else out[c].lo = part.kmin[c], out[c].hi = part.kmax[c];
-            }
-            const bool reached = part.reached != 0;
-            part_reset(part);
-            set_hdr(s, out);
-            if (reached) {
-                end_score = s;
-                plan.op = WOP_DONE;
+        if (tid < 32) {
+            if (part.retry) {
+                if (lane == 0) plan.op = WOP_DONE, Q.status = WFA_RETRY;
             } else {
-                plan_next();
+                CompHdr out = lane < 5 ? plan.out[lane] : NUL;
+                if (lane < 5 && (plan.mask >> lane & 1)) {
+                    // no diagonal in the matrix: the empty range [lo, lo-1] of the scan
+                    if (part.k[lane] == INT_MIN) out.hi = out.lo - 1;
+                    else out.lo = -part.k[5 + lane], out.hi = part.k[lane];
+                }
+                const bool reached = part.k[10] == 1;
+                __syncwarp();
+                part_reset(part, lane);
+                set_hdr(Q.s, out);
+                if (reached) {
+                    if (lane == 0) plan.op = WOP_DONE, Q.end_score = Q.s;
+                } else {
+                    plan_next();
+                }
             }
         }
         __syncthreads();
@@ -940,10 +1018,12 @@ __device__ void cta_pair(const WfaArgs &A, int idx, const HdrRing &HR, WidePlan 
     if (PIG && lane == 0) atomicAdd(&part.used, (unsigned long long)wal.used);
     __syncthreads();
     if (tid == 0) {
-        finish_pair<PIG>(A, PR, idx, pat, txt, ctab, HR, status, end_score, s, al.used + (int64_t)part.used);
+        finish_pair<PIG>(A, PR, idx, pat, txt, ctab, HR, Q.status, Q.end_score, Q.s, Q.al.used + (int64_t)part.used);
         atomicSub(A.queue + 1, 1);
     }
     __syncthreads();
+    if (tid == 0) give_back(pool_of(A), Q.al);
+    if (PIG && lane == 0) give_back(pool_of(A), wal);
 }
 
 // Build-time tuning of the warp kernel: CTAs per SM the registers are sized for (4 warps
@@ -956,39 +1036,42 @@ __device__ void cta_pair(const WfaArgs &A, int idx, const HdrRing &HR, WidePlan 
 #endif
 constexpr int WU = AW_WFA_WARP_U;
 
-template <bool PIG>
-__global__ void __launch_bounds__(128, AW_WFA_MINB) wfa_kernel(WfaArgs A, int rs) {
+template <bool PIG, int NT>
+__global__ void __launch_bounds__(NT, AW_WFA_MINB * WFA_CTA / NT) wfa_kernel(WfaArgs A, RingShape rs) {
     const int lane = threadIdx.x & 31;
     const WfaPen P = A.pen;
-    extern __shared__ ScoreHdr hring_all[];
+    extern __shared__ CompHdr hring_all[];
+    __shared__ Alloc allocs[NT / 32];
+    Alloc &al = allocs[threadIdx.x >> 5];
     {
         // the long pairs first, each on the whole CTA (warp 0's header ring serves the
         // planner; the warps take their own rings afterwards)
         __shared__ WidePlan cplan;
         __shared__ WidePart cpart;
+        __shared__ CtaPlanner cstate;
         __shared__ int cpi;
         for (;;) {
-            if (threadIdx.x == 0) cpi = A.n_long > 0 ? atomicAdd(A.queue + 2, 1) : A.n_long;
+            if (threadIdx.x == 0) cpi = A.n_long > 0 ? atomicAdd(A.queue + A.q_long, 1) : A.n_long;
             __syncthreads();
             const int pi = cpi;
             __syncthreads();
             if (pi >= A.n_long) break;
-            cta_pair<PIG>(A, A.order_long[pi], HdrRing{hring_all, rs}, cplan, cpart);
+            cta_pair<PIG>(A, A.order_long[pi], HdrRing{hring_all, rs}, cplan, cpart, cstate, al);
         }
     }
-    const HdrRing HR{hring_all + (threadIdx.x >> 5) * rs, rs};
-    for (;;) {
+    const HdrRing HR{hring_all + (threadIdx.x >> 5) * rs.entries(), rs};
+    for (; A.n > 0;) {
         int pi = 0;
         if (lane == 0) pi = atomicAdd(A.queue, 1);
         pi = __shfl_sync(0xffffffffu, pi, 0);
         if (pi >= A.n) break;
-        if (lane == 0) atomicAdd(A.queue + 1, 1);  // pairs running on warps
+        if (lane == 0) atomicAdd(A.queue + 1, 1), atomicAdd(A.queue + 3, 1);  // pairs running, started
         const int idx = A.order[pi];
         const WfaPairDev PR = A.pairs[idx];
         const int plen = PR.plen, tlen = PR.tlen;
         const uint8_t *pat = A.pat + PR.poff, *txt = A.txt + PR.toff;
         int64_t *ctab = A.ctab + PR.ctab_off;
-        Alloc al{0, 0, true, 0};
+        if (lane == 0) al.init();
         uint32_t bnext = 0, bend = 0;  // this lane's reserved piggyback blocks
         int status = 0, end_score = -1;
         // piggyback rings, each slot three arrays (offsets, packed CIGARs, links) of rcap
@@ -1033,7 +1116,7 @@ __global__ void __launch_bounds__(128, AW_WFA_MINB) wfa_kernel(WfaArgs A, int rs
                 ((uint32_t *)(A.pool + d0))[rcap] = 0u;
                 ((uint32_t *)(A.pool + d0))[2 * rcap] = BT_NULL;  // the start (0, 0)
             }
-            if (HR.rs) HR.ring[0] = *H;
+            for (int c = 0; c < 5; ++c) HR.put(c, 0, H->c[c]);
         }
         __syncwarp();
         const int k_end = tlen - plen;
@@ -1044,7 +1127,7 @@ __global__ void __launch_bounds__(128, AW_WFA_MINB) wfa_kernel(WfaArgs A, int rs
             // ---- extend M[s] and check the end.  The compute step below extends M[s] as it
             // computes it (fused), so here only M[0] is extended.
             {
-                const CompHdr m = HR.get(A, ctab, s, s)->c[CM];
+                const CompHdr m = HR.get(A, ctab, CM, s);
                 bool reached = false;
                 if (m.lo <= m.hi) {
                     if (s == 0) {
@@ -1095,22 +1178,19 @@ __global__ void __launch_bounds__(128, AW_WFA_MINB) wfa_kernel(WfaArgs A, int rs
             ScoreHdr *OH = hdr_ptr(A, ctab, s);
             const CompHdr NUL{1, -1, 0, 0, 0};
             const int sm = s - P.x, so1 = s - P.o1 - P.e1, se1 = s - P.e1, so2 = s - P.o2 - P.e2, se2 = s - P.e2;
-            const CompHdr m_misms = sm >= 0 ? HR.get(A, ctab, sm, s)->c[CM] : NUL;
-            const CompHdr m_open1 = so1 >= 0 ? HR.get(A, ctab, so1, s)->c[CM] : NUL;
-            const CompHdr i1 = se1 >= 0 ? HR.get(A, ctab, se1, s)->c[CI1] : NUL;
-            const CompHdr d1 = se1 >= 0 ? HR.get(A, ctab, se1, s)->c[CD1] : NUL;
-            const CompHdr m_open2 = so2 >= 0 ? HR.get(A, ctab, so2, s)->c[CM] : NUL;
-            const CompHdr i2 = se2 >= 0 ? HR.get(A, ctab, se2, s)->c[CI2] : NUL;
-            const CompHdr d2 = se2 >= 0 ? HR.get(A, ctab, se2, s)->c[CD2] : NUL;
+            const CompHdr m_misms = sm >= 0 ? HR.get(A, ctab, CM, sm) : NUL;
+            const CompHdr m_open1 = so1 >= 0 ? HR.get(A, ctab, CM, so1) : NUL;
+            const CompHdr i1 = se1 >= 0 ? HR.get(A, ctab, CI1, se1) : NUL;
+            const CompHdr d1 = se1 >= 0 ? HR.get(A, ctab, CD1, se1) : NUL;
+            const CompHdr m_open2 = so2 >= 0 ? HR.get(A, ctab, CM, so2) : NUL;
+            const CompHdr i2 = se2 >= 0 ? HR.get(A, ctab, CI2, se2) : NUL;
+            const CompHdr d2 = se2 >= 0 ? HR.get(A, ctab, CD2, se2) : NUL;
             const bool n_mm = m_misms.lo > m_misms.hi, n_o1 = m_open1.lo > m_open1.hi, n_i1 = i1.lo > i1.hi,
                        n_d1 = d1.lo > d1.hi, n_o2 = m_open2.lo > m_open2.hi, n_i2 = i2.lo > i2.hi,
                        n_d2 = d2.lo > d2.hi;
             if (n_mm && n_o1 && n_i1 && n_d1 && n_o2 && n_i2 && n_d2) {
-                if (lane == 0) {
-                    for (int c = 0; c < 5; ++c) OH->c[c] = NUL;
-                    if (HR.rs)
-                        for (int c = 0; c < 5; ++c) HR.ring[s & (HR.rs - 1)].c[c] = NUL;
-                }
+                if (lane == 0)
+                    for (int c = 0; c < 5; ++c) OH->c[c] = NUL, HR.put(c, s, NUL);
                 __syncwarp();
                 ++num_null;
                 fused_reached = false;
@@ -1135,7 +1215,7 @@ __global__ void __launch_bounds__(128, AW_WFA_MINB) wfa_kernel(WfaArgs A, int rs
             if (!PIG && A.wide_width > 0 && width > A.wide_width_tail) {
                 int drained = 0;
                 if (lane == 0)
-                    drained = *(volatile int32_t *)A.queue >= A.n &&
+                    drained = *(volatile int32_t *)(A.queue + 3) >= A.n_all &&
                               *(volatile int32_t *)(A.queue + 1) <= A.wide_tail_pairs;
                 drained = __shfl_sync(0xffffffffu, drained, 0);
                 if (width > A.wide_width || drained) {
@@ -1263,11 +1343,8 @@ __global__ void __launch_bounds__(128, AW_WFA_MINB) wfa_kernel(WfaArgs A, int rs
                 if (th == INT_MIN) out[c].hi = out[c].lo - 1;
                 else out[c].lo = tl, out[c].hi = th;
             }
-            if (lane == 0) {
-                for (int c = 0; c < 5; ++c) OH->c[c] = out[c];
-                if (HR.rs)
-                    for (int c = 0; c < 5; ++c) HR.ring[s & (HR.rs - 1)].c[c] = out[c];
-            }
+            if (lane == 0)
+                for (int c = 0; c < 5; ++c) OH->c[c] = out[c], HR.put(c, s, out[c]);
             __syncwarp();
         }
         // ---- backtrace (lane 0)
@@ -1276,6 +1353,7 @@ __global__ void __launch_bounds__(128, AW_WFA_MINB) wfa_kernel(WfaArgs A, int rs
             atomicSub(A.queue + 1, 1);
         }
         __syncwarp();
+        if (lane == 0) give_back(pool_of(A), al);
     }
 }
 
@@ -1288,10 +1366,11 @@ __global__ void __launch_bounds__(128, AW_WFA_MINB) wfa_kernel(WfaArgs A, int rs
 //      trimmed ends per component, and whether the end cell was reached, into its CTA's
 //      partials;
 //   2. cluster barrier;
-//   3. warp 0 of every CTA gathers all CTAs' partials through distributed shared memory,
-//      and its lane 0 (the CTA's planner) finishes the score's headers and plans the next
-//      score.  Every planner holds the same state (the headers of the last scores in a
-//      shared-memory ring, the pool position), so all plans agree without being exchanged.
+//   3. warp 0 of every CTA (the CTA's planner) gathers all CTAs' partials through
+//      distributed shared memory, four lanes per CTA, finishes the score's headers and plans the
+//      next score, a lane per input and per component.  Every planner holds the same state
+//      (the headers of the last scores in shared-memory rings, the pool position), so all
+//      plans agree without being exchanged.
 // Pool space is carved deterministically out of reserve chunks that thread 0 of the first
 // CTA (the leader) takes from the pool one score ahead of need and announces to every CTA
 // through distributed shared memory before the barrier; the leader alone writes the pool
@@ -1309,7 +1388,7 @@ struct WideAnn {
     int64_t off, len;
 };
 
-// The planner's state (lane 0 of warp 0 in every CTA; identical in all of them).
+// The planner's state (the same in all lanes of warp 0 of every CTA).
 struct WidePlanner {
     int pi, idx;  // queue position and pair
     int s, num_null, status, end_score, smax, R, ring_cap;
@@ -1326,14 +1405,14 @@ __device__ __forceinline__ int64_t wide_chunk(const WfaArgs &A, int64_t need) {
     return ((max(base, 2 * need) + 255) & ~(int64_t)255);
 }
 
-__global__ void __launch_bounds__(WIDE_NT, 1) wfa_wide_kernel(WfaArgs A, int rs) {
+__global__ void __launch_bounds__(WIDE_NT, 1) wfa_wide_kernel(WfaArgs A, RingShape rs) {
     namespace cg = cooperative_groups;
     cg::cluster_group cl = cg::this_cluster();
     const int CL = (int)cl.num_blocks();
     const int rank = (int)cl.block_rank();
     const int tid = threadIdx.x, lane = tid & 31;
     const int GT = CL * WIDE_NT, gtid = rank * WIDE_NT + tid;
-    const bool planner = tid == 0;
+    const bool planner = tid < 32;
     const bool leader = rank == 0 && tid == 0;
     const WfaPen P = A.pen;
     __shared__ WidePlan plan;
@@ -1342,18 +1421,19 @@ __global__ void __launch_bounds__(WIDE_NT, 1) wfa_wide_kernel(WfaArgs A, int rs)
     __shared__ WideAnn pstart[2];  // the pair of the np-th pair start (np & 1): tag = queue position,
                                    // seq = pair, off/len = its first chunk
     __shared__ int64_t qoff[WIDE_CHUNKS], qlen[WIDE_CHUNKS];  // the planner's chunks
-    extern __shared__ ScoreHdr wring[];
+    extern __shared__ CompHdr wring[];
     const HdrRing HR{wring, rs};
-    if (tid < 2) {
-        part_reset(part[tid]);
-        ann[tid] = WideAnn{-1, -1, -1, 0};
+    const PlanLane L = plan_lane(P, lane);
+    if (planner) {
+        part_reset(part[0], lane), part_reset(part[1], lane);
+        if (lane < 2) ann[lane] = WideAnn{-1, -1, -1, 0};
     }
     const CompHdr NUL{1, -1, 0, 0, 0};
     WidePlanner W{};
     int64_t used = 0;  // the leader's pool bytes for the pair
     int it = 0, np = 0;
 
-    // ---- planner helpers (lane 0 of warp 0)
+    // ---- planner helpers (all lanes of warp 0)
     auto carve = [&](int64_t bytes) -> int64_t {
         bytes = (bytes + 15) & ~(int64_t)15;
         while (W.cur + bytes > W.end) {
@@ -1381,13 +1461,13 @@ __global__ void __launch_bounds__(WIDE_NT, 1) wfa_wide_kernel(WfaArgs A, int rs)
         for (int j = W.cidx + 1; j < W.nchunks; ++j) ok |= qlen[j % WIDE_CHUNKS] >= need;
         return ok;
     };
-    auto set_hdr = [&](int sc, const CompHdr (&o)[5]) {
-        if (leader) {
-            ScoreHdr *OH = (ScoreHdr *)(A.pool + W.hdr_off) + (sc % HDR_CHUNK);
-            for (int c = 0; c < 5; ++c) OH->c[c] = o[c];
+    // lane c < 5: component c's header of score sc (the first CTA's planner writes the pool copy)
+    auto set_hdr = [&](int sc, const CompHdr &o) {
+        if (lane < 5) {
+            if (rank == 0) ((ScoreHdr *)(A.pool + W.hdr_off))[sc % HDR_CHUNK].c[lane] = o;
+            HR.put(lane, sc, o);
         }
-        if (HR.rs)
-            for (int c = 0; c < 5; ++c) HR.ring[sc & (HR.rs - 1)].c[c] = o[c];
+        __syncwarp();
     };
     // plans the next score with a non-null input; op = DONE with W.status set if the pair stops
     auto plan_next = [&]() {
@@ -1406,14 +1486,12 @@ __global__ void __launch_bounds__(WIDE_NT, 1) wfa_wide_kernel(WfaArgs A, int rs)
                 }
                 W.hdr_off = hb;
                 if (leader) A.ctab[W.ctab_off + s / HDR_CHUNK] = hb;
+                __syncwarp();
             }
-            CompHdr in[7];
-            plan_inputs(A, A.ctab + W.ctab_off, HR, s, in);
-            bool all_null = true;
-            for (int j = 0; j < 7; ++j) all_null &= in[j].lo > in[j].hi;
-            if (all_null) {
-                const CompHdr o[5] = {NUL, NUL, NUL, NUL, NUL};
-                set_hdr(s, o);
+            CompHdr in;
+            const unsigned some = plan_input(A, A.ctab + W.ctab_off, HR, L, s, lane, in);
+            if (!some) {
+                set_hdr(s, NUL);
                 // the top of the next step: M[s] is empty
                 if (++W.num_null > A.max_score_scope) {
                     W.status = -3;
@@ -1423,34 +1501,33 @@ __global__ void __launch_bounds__(WIDE_NT, 1) wfa_wide_kernel(WfaArgs A, int rs)
             }
             W.num_null = 0;
             int lo, hi, mask;
-            plan_limits(in, lo, hi, mask);
+            plan_limits(L, lane, in, some, lo, hi, mask);
             W.lo_all = min(W.lo_all, lo), W.hi_all = max(W.hi_all, hi);
             const int width = hi - lo + 1;
             const int64_t wb = (((int64_t)width * 4) + 15) & ~(int64_t)15;
-            const int nstore = A.singletrack ? 1 : __popc(mask);
             if (A.singletrack && width > W.ring_cap) {
                 W.status = WFA_OVERFLOW;
                 break;
             }
-            const int64_t blk = carve(wb * nstore);
+            const int64_t blk = carve(wb * (A.singletrack ? 1 : __popc(mask)));
             if (blk < 0) {
                 W.status = WFA_RETRY;
                 break;
             }
-            int64_t o = blk;
-            for (int c = 0; c < 5; ++c) {
-                plan.out[c] = NUL;
-                if (!(mask & (1 << c))) continue;
-                int64_t place;
-                if (c == CM || !A.singletrack) place = o, o += wb;
-                else place = W.ring + ((int64_t)((s % W.R) * 4 + (c - 1)) * W.ring_cap) * 4;
-                plan.out[c] = CompHdr{lo, hi, lo, 0, place};
+            if (lane < 5) {
+                CompHdr out = NUL;
+                if (mask >> lane & 1)
+                    out = CompHdr{lo, hi, lo, 0,
+                                  lane == CM || !A.singletrack ? blk + wb * __popc(mask & ((1 << lane) - 1))
+                                                               : W.ring + ((int64_t)((s % W.R) * 4 + (lane - 1)) * W.ring_cap) * 4};
+                plan.out[lane] = out;
+                plan.dst[lane] = mask >> lane & 1 ? (int32_t *)(A.pool + out.off) : nullptr;
             }
-            for (int j = 0; j < 7; ++j) plan.in[j] = in[j];
-            plan.op = WOP_COMPUTE, plan.lo = lo, plan.hi = hi, plan.mask = mask;
+            if (lane < 7) plan.view[lane] = in_hdr(A, in);
+            if (lane == 0) plan.op = WOP_COMPUTE, plan.lo = lo, plan.hi = hi, plan.mask = mask;
             return;
         }
-        plan.op = WOP_DONE;
+        if (lane == 0) plan.op = WOP_DONE;
     };
 
     for (;;) {
@@ -1464,7 +1541,7 @@ __global__ void __launch_bounds__(WIDE_NT, 1) wfa_wide_kernel(WfaArgs A, int rs)
                 const int R = (P.e1 > P.e2 ? P.e1 : P.e2) + 1;
                 const int64_t ring_b = A.singletrack ? (int64_t)R * 4 * (PR.plen + PR.tlen + 8) * 4 + 16 : 0;
                 const int64_t len = wide_chunk(A, ring_b + (int64_t)sizeof(ScoreHdr) * HDR_CHUNK + 4096);
-                a = WideAnn{pi, idx, pool_grab(A, len), len};
+                a = WideAnn{pi, idx, pool_grab(pool_of(A), len), len};
                 used = a.off >= 0 ? len : 0;
             }
             for (int c = 0; c < CL; ++c) *cl.map_shared_rank(&pstart[np & 1], c) = a;
@@ -1473,7 +1550,7 @@ __global__ void __launch_bounds__(WIDE_NT, 1) wfa_wide_kernel(WfaArgs A, int rs)
         if (planner) {
             const WideAnn a = pstart[np & 1];
             if (a.tag >= A.n) {
-                plan.op = WOP_EXIT;
+                if (lane == 0) plan.op = WOP_EXIT;
             } else {
                 const WfaPairDev PR = A.pairs[a.seq];
                 W = WidePlanner{};
@@ -1483,7 +1560,8 @@ __global__ void __launch_bounds__(WIDE_NT, 1) wfa_wide_kernel(WfaArgs A, int rs)
                 W.ring_cap = PR.plen + PR.tlen + 8;
                 W.end_score = -1, W.lo_all = 0, W.hi_all = 0;
                 W.ring = -1;
-                qoff[0] = a.off, qlen[0] = a.len;
+                if (lane == 0) qoff[0] = a.off, qlen[0] = a.len;
+                __syncwarp();
                 W.nchunks = 1, W.cidx = 0, W.cur = a.off, W.end = a.off + a.len;
                 W.exhausted = a.off < 0;
                 if (a.off < 0) W.status = WFA_RETRY;
@@ -1499,13 +1577,16 @@ __global__ void __launch_bounds__(WIDE_NT, 1) wfa_wide_kernel(WfaArgs A, int rs)
                     const int32_t o0 = (int32_t)lcp1(A, PR, A.pat + PR.poff, A.txt + PR.toff, 0, 0);
                     W.hdr_off = h0;
                     if (leader) A.ctab[PR.ctab_off] = h0;
-                    *(int32_t *)(A.pool + d0) = o0;
-                    const CompHdr o[5] = {CompHdr{0, 0, 0, 0, d0}, NUL, NUL, NUL, NUL};
-                    set_hdr(0, o);
+                    if (lane == 0) *(int32_t *)(A.pool + d0) = o0;
+                    __syncwarp();
+                    set_hdr(0, lane == 0 ? CompHdr{0, 0, 0, 0, d0} : NUL);
                     if (PR.tlen - PR.plen == 0 && o0 >= PR.tlen) W.end_score = 0;
                 }
-                if (W.status != 0 || W.end_score == 0) plan.op = WOP_DONE;
-                else plan_next();
+                if (W.status != 0 || W.end_score == 0) {
+                    if (lane == 0) plan.op = WOP_DONE;
+                } else {
+                    plan_next();
+                }
             }
         }
         __syncthreads();
@@ -1521,50 +1602,52 @@ __global__ void __launch_bounds__(WIDE_NT, 1) wfa_wide_kernel(WfaArgs A, int rs)
             // the leader reserves the next plan's space ahead of need
             if (leader && !W.exhausted && W.nchunks - W.cidx < WIDE_CHUNKS - 1 && !reserve_ok()) {
                 const int64_t len = wide_chunk(A, need_next());
-                const int64_t off = pool_grab(A, len);
+                const int64_t off = pool_grab(pool_of(A), len);
                 if (off >= 0) used += len;
                 const WideAnn a{W.pi, W.nchunks, off, off >= 0 ? len : 0};
                 for (int c = 0; c < CL; ++c) *cl.map_shared_rank(&ann[it & 1], c) = a;
             }
             cl.sync();
             // ---- 3. gather, finish the score, plan the next one (warp 0 of every CTA)
-            if (tid < 32) {
-                int gmin[5], gmax[5], gr = 0;
+            if (planner) {
+                // lane 4r + q: the q-th quadruple of CTA r's partials, then the maxima over the CTAs
+                int4 v = make_int4(INT_MIN, INT_MIN, INT_MIN, INT_MIN);
+                if ((lane >> 2) < CL && (lane & 3) < 3)
+                    v = *reinterpret_cast<const int4 *>(cl.map_shared_rank(part[it & 1].k, lane >> 2) + 4 * (lane & 3));
 #pragma unroll
-                for (int c = 0; c < 5; ++c) gmin[c] = INT_MAX, gmax[c] = INT_MIN;
-                if (lane < CL) {
-                    const WidePart *rp = cl.map_shared_rank(&part[it & 1], lane);
-#pragma unroll
-                    for (int c = 0; c < 5; ++c) gmin[c] = rp->kmin[c], gmax[c] = rp->kmax[c];
-                    gr = rp->reached;
+                for (int o = 4; o < 32; o <<= 1) {
+                    v.x = max(v.x, __shfl_xor_sync(0xffffffffu, v.x, o)), v.y = max(v.y, __shfl_xor_sync(0xffffffffu, v.y, o));
+                    v.z = max(v.z, __shfl_xor_sync(0xffffffffu, v.z, o)), v.w = max(v.w, __shfl_xor_sync(0xffffffffu, v.w, o));
                 }
-#pragma unroll
-                for (int c = 0; c < 5; ++c)
-                    gmin[c] = __reduce_min_sync(0xffffffffu, gmin[c]), gmax[c] = __reduce_max_sync(0xffffffffu, gmax[c]);
-                gr = __any_sync(0xffffffffu, gr != 0);
-                if (planner) {
-                    part_reset(part[(it + 1) & 1]);
-                    const WideAnn a = ann[it & 1];
-                    if (a.tag == W.pi && a.seq == W.nchunks) {
-                        qoff[W.nchunks % WIDE_CHUNKS] = a.off, qlen[W.nchunks % WIDE_CHUNKS] = a.len;
-                        ++W.nchunks;
-                        if (a.off < 0) W.exhausted = true;
-                    }
-                    CompHdr out[5];
-                    for (int c = 0; c < 5; ++c) {
-                        out[c] = plan.out[c];
-                        if (!(plan.mask & (1 << c))) continue;
-                        // no diagonal in the matrix: the empty range [lo, lo-1] of the scan
-                        if (gmax[c] == INT_MIN) out[c].hi = out[c].lo - 1;
-                        else out[c].lo = gmin[c], out[c].hi = gmax[c];
-                    }
-                    set_hdr(W.s, out);
-                    if (gr) {
-                        W.end_score = W.s;
-                        plan.op = WOP_DONE;
-                    } else {
-                        plan_next();
-                    }
+                // value i of the quadruples: field i & 3 of lane i >> 2
+                auto value = [&](int i) {
+                    const int x = __shfl_sync(0xffffffffu, v.x, i >> 2), y = __shfl_sync(0xffffffffu, v.y, i >> 2);
+                    const int z = __shfl_sync(0xffffffffu, v.z, i >> 2), w = __shfl_sync(0xffffffffu, v.w, i >> 2);
+                    return (i & 3) == 0 ? x : (i & 3) == 1 ? y : (i & 3) == 2 ? z : w;
+                };
+                const int c5 = min(lane, 4), top = value(c5), bottom = value(5 + c5);
+                const bool reached = __shfl_sync(0xffffffffu, v.z, 2) == 1;
+                part_reset(part[(it + 1) & 1], lane);
+                const WideAnn a = ann[it & 1];
+                if (a.tag == W.pi && a.seq == W.nchunks) {
+                    if (lane == 0) qoff[W.nchunks % WIDE_CHUNKS] = a.off, qlen[W.nchunks % WIDE_CHUNKS] = a.len;
+                    __syncwarp();
+                    ++W.nchunks;
+                    if (a.off < 0) W.exhausted = true;
+                }
+                CompHdr out = lane < 5 ? plan.out[lane] : NUL;
+                if (lane < 5 && (plan.mask >> lane & 1)) {
+                    // no diagonal in the matrix: the empty range [lo, lo-1] of the scan
+                    if (top == INT_MIN) out.hi = out.lo - 1;
+                    else out.lo = -bottom, out.hi = top;
+                }
+                __syncwarp();
+                set_hdr(W.s, out);
+                if (reached) {
+                    W.end_score = W.s;
+                    if (lane == 0) plan.op = WOP_DONE;
+                } else {
+                    plan_next();
                 }
             }
             __syncthreads();
@@ -1579,29 +1662,37 @@ __global__ void __launch_bounds__(WIDE_NT, 1) wfa_wide_kernel(WfaArgs A, int rs)
 
 }  // namespace
 
-// Header ring size for a score scope: the smallest power of two above it, 32..128
-// (shared memory of 4 warps x 128 x 120 B at most), or 0 (pool reads) beyond.
-static int ring_size(int scope) {
-    int rs = 32;
-    while (rs <= scope && rs < 256) rs <<= 1;
-    return rs <= 128 ? rs : 0;
+// Header rings for a penalty set: powers of two above each component's reach; no rings (pool
+// reads) when they would take more than `cap` bytes.
+static RingShape ring_shape(const WfaPen &P, int scope, int cap) {
+    auto mask = [](int reach) {
+        int n = 2;
+        while (n <= reach && n < (1 << 20)) n <<= 1;
+        return n - 1;
+    };
+    const RingShape r{mask(scope), mask(P.e1), mask(P.e2)};
+    if ((int64_t)r.entries() * (int64_t)sizeof(CompHdr) > cap) return RingShape{-1, 0, 0};
+    return r;
 }
+constexpr int WARP_RING_BYTES = 8 * 1024, WIDE_RING_BYTES = 96 * 1024;
 
-template <bool PIG>
+template <bool PIG, int NT>
 static cudaError_t launch_wfa_t(const WfaArgs &a, int ctas, cudaStream_t st) {
-    const int rs = ring_size(a.max_score_scope);
-    const size_t smem = (size_t)4 * rs * sizeof(ScoreHdr);
+    const RingShape rs = ring_shape(a.pen, a.max_score_scope, WARP_RING_BYTES);
+    const size_t smem = (size_t)(NT / 32) * rs.entries() * sizeof(CompHdr);
     if (smem > 48 * 1024) {
         const cudaError_t e =
-            cudaFuncSetAttribute(wfa_kernel<PIG>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+            cudaFuncSetAttribute(wfa_kernel<PIG, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return e;
     }
-    wfa_kernel<PIG><<<ctas, 128, smem, st>>>(a, rs);
+    wfa_kernel<PIG, NT><<<ctas, NT, smem, st>>>(a, rs);
     return cudaGetLastError();
 }
 
-cudaError_t launch_wfa(const WfaArgs &a, int ctas, cudaStream_t st) {
-    return a.piggyback ? launch_wfa_t<true>(a, ctas, st) : launch_wfa_t<false>(a, ctas, st);
+cudaError_t launch_wfa(const WfaArgs &a, int threads, int ctas, cudaStream_t st) {
+    if (threads == WFA_BIG_CTA)
+        return a.piggyback ? launch_wfa_t<true, WFA_BIG_CTA>(a, ctas, st) : launch_wfa_t<false, WFA_BIG_CTA>(a, ctas, st);
+    return a.piggyback ? launch_wfa_t<true, WFA_CTA>(a, ctas, st) : launch_wfa_t<false, WFA_CTA>(a, ctas, st);
 }
 
 static cudaLaunchConfig_t wide_config(int ctas, int cl, size_t smem, cudaStream_t st, cudaLaunchAttribute *at) {
@@ -1619,18 +1710,10 @@ static cudaLaunchConfig_t wide_config(int ctas, int cl, size_t smem, cudaStream_
     return cfg;
 }
 
-// Header ring of the cluster kernel's planners: the smallest power of two above the score
-// scope, 32..1024 (0: scope too large for the cluster kernel).
-static int wide_ring_size(int scope) {
-    int rs = 32;
-    while (rs <= scope && rs <= 1024) rs <<= 1;
-    return rs <= 1024 ? rs : 0;
-}
-
 cudaError_t launch_wfa_wide(const WfaArgs &a, int clusters, int cl, cudaStream_t st) {
-    const int rs = wide_ring_size(a.max_score_scope);
-    if (rs == 0) return cudaErrorInvalidValue;
-    const size_t smem = (size_t)rs * sizeof(ScoreHdr);
+    const RingShape rs = ring_shape(a.pen, a.max_score_scope, WIDE_RING_BYTES);
+    if (rs.mm < 0) return cudaErrorInvalidValue;
+    const size_t smem = (size_t)rs.entries() * sizeof(CompHdr);
     if (smem > 48 * 1024) {
         const cudaError_t e = cudaFuncSetAttribute(wfa_wide_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return e;
@@ -1641,10 +1724,10 @@ cudaError_t launch_wfa_wide(const WfaArgs &a, int clusters, int cl, cudaStream_t
     return e != cudaSuccess ? e : cudaGetLastError();
 }
 
-int wfa_wide_clusters(int cl, int scope) {
-    const int rs = wide_ring_size(scope);
-    if (rs == 0) return 0;
-    const size_t smem = (size_t)rs * sizeof(ScoreHdr);
+int wfa_wide_clusters(int cl, const WfaPen &pen, int scope) {
+    const RingShape rs = ring_shape(pen, scope, WIDE_RING_BYTES);
+    if (rs.mm < 0) return 0;
+    const size_t smem = (size_t)rs.entries() * sizeof(CompHdr);
     if (smem > 48 * 1024 &&
         cudaFuncSetAttribute(wfa_wide_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
         return 0;
@@ -1707,11 +1790,14 @@ cudaError_t launch_wfa_pack(const uint8_t *pat, int64_t pbytes, uint64_t *ppat, 
     return cudaGetLastError();
 }
 
-int wfa_occupancy(bool piggyback) {
+int wfa_occupancy(bool piggyback, int threads, const WfaPen &pen, int scope) {
+    const size_t smem = (size_t)(threads / 32) * ring_shape(pen, scope, WARP_RING_BYTES).entries() * sizeof(CompHdr);
+    const void *k = threads == WFA_BIG_CTA
+                        ? (piggyback ? (const void *)wfa_kernel<true, WFA_BIG_CTA> : (const void *)wfa_kernel<false, WFA_BIG_CTA>)
+                        : (piggyback ? (const void *)wfa_kernel<true, WFA_CTA> : (const void *)wfa_kernel<false, WFA_CTA>);
+    if (smem > 48 * 1024) cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     int nb = 0;
-    const cudaError_t e =
-        piggyback ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, wfa_kernel<true>, 128, 4 * 32 * sizeof(ScoreHdr))
-                  : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, wfa_kernel<false>, 128, 4 * 32 * sizeof(ScoreHdr));
+    const cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k, threads, smem);
     return e == cudaSuccess ? nb : 1;
 }
 

@@ -13,6 +13,7 @@
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
+#include <iterator>
 #include <string>
 #include <vector>
 
@@ -54,9 +55,9 @@ std::atomic<int> g_long_sum{1536};
 
 struct wavefront_aligner_gpu {
     wavefront_gpu_attr_t attr;
-    cudaStream_t st = nullptr;
-    cudaEvent_t e0 = nullptr, e1 = nullptr;
-    DevBuf d_pat, d_txt, d_pairs, d_order, d_pool, d_head, d_ctab, d_ops, d_out, d_queue;
+    cudaStream_t st = nullptr, st2 = nullptr;  // st2: the big CTAs, beside the others on st
+    cudaEvent_t e0 = nullptr, e1 = nullptr, fork = nullptr, join = nullptr;
+    DevBuf d_pat, d_txt, d_pairs, d_order, d_pool, d_ctl, d_free, d_ctab, d_ops, d_out, d_queue;
     DevBuf d_ppat, d_ptxt;  // 2-bit copies of the sequence arenas
     PinBuf h_pat, h_txt, h_ops;
     std::vector<WfaPairDev> pairs;
@@ -71,11 +72,14 @@ struct wavefront_aligner_gpu {
     int last_cluster_launches = 0, last_cluster_pairs = 0;
     ~wavefront_aligner_gpu() {
         d_pat.release(), d_txt.release(), d_pairs.release(), d_order.release(), d_pool.release();
-        d_head.release(), d_ctab.release(), d_ops.release(), d_out.release(), d_queue.release();
+        d_ctl.release(), d_free.release(), d_ctab.release(), d_ops.release(), d_out.release(), d_queue.release();
         d_ppat.release(), d_ptxt.release();
         if (e0) cudaEventDestroy(e0);
         if (e1) cudaEventDestroy(e1);
+        if (fork) cudaEventDestroy(fork);
+        if (join) cudaEventDestroy(join);
         if (st) cudaStreamDestroy(st);
+        if (st2) cudaStreamDestroy(st2);
     }
 };
 
@@ -87,6 +91,35 @@ struct wavefront_aligner_gpu {
             return AW_E_CUDA;                                               \
         }                                                                   \
     } while (0)
+
+constexpr int64_t kClusterSum = 8000;  // pattern + text of a pair that starts on the cluster kernel
+
+// How many of the long pairs (largest first) run on big CTAs.  A pair's work grows with the
+// square of its length; a batch takes as long as its longest pair or as its work over all CTA
+// slots, and big CTAs shorten the first at the cost of the second.  Measured (small CTAs
+// only / this rule): 2,048 pairs of 0.1-10 kb in medium memory 97 / 45 ms, 4,096 in high
+// memory 66 / 43 ms; 8,192 and 16,384 pairs choose no or few big CTAs.  A speedup of 1.5 in its
+// place gave 72 / 45 ms, 2.5 54 / 45 ms.
+static int big_pairs(const std::vector<int32_t> &longest, const int *plen, const int *tlen, int sms) {
+    const double kSpeedup = 4.0;       // a pair on a big CTA against one on a small CTA
+    std::vector<double> cost(longest.size());
+    double rest = 0.0;
+    for (size_t k = 0; k < longest.size(); ++k) {
+        const double len = (double)plen[longest[k]] + tlen[longest[k]];
+        rest += cost[k] = len * len;
+    }
+    double best = 0.0, big = 0.0;
+    int n_big = 0;
+    for (size_t k = 0; k <= longest.size(); ++k) {
+        // k pairs on big CTAs; the small ones have the SMs' other slots
+        const double t_big = k ? std::max(cost[0] / kSpeedup, big / kSpeedup / sms) : 0.0;
+        const double t_small = k < longest.size() ? std::max(cost[k], (rest + big * 4 / kSpeedup) / (4.0 * sms)) : 0.0;
+        const double t = std::max(t_big, t_small);
+        if (k == 0 || t < 0.98 * best) best = t, n_big = (int)k;
+        if (k < longest.size()) big += cost[k], rest -= cost[k];
+    }
+    return n_big;
+}
 
 static int run_batch(wavefront_aligner_gpu *al, int n, const char *const *pattern, const int *plen,
                      const char *const *text, const int *tlen) {
@@ -137,7 +170,7 @@ static int run_batch(wavefront_aligner_gpu *al, int n, const char *const *patter
     WCUDA(al->d_ops.ensure((size_t)ob + 64));
     WCUDA(al->d_out.ensure(sizeof(WfaOutDev) * (size_t)n));
     WCUDA(al->d_queue.ensure(64));
-    WCUDA(al->d_head.ensure(64));
+    WCUDA(al->d_ctl.ensure(sizeof(WfaPoolCtl)));
     // device pool: 85% of free memory (capped by max_memory_abort when set)
     if (al->d_pool.cap == 0) {
         size_t fr = 0, tot = 0;
@@ -148,6 +181,7 @@ static int run_batch(wavefront_aligner_gpu *al, int n, const char *const *patter
         if (A.memory_mode != 0) want = std::min<int64_t>(want, ((int64_t)1 << 35) - ((int64_t)1 << 20));
         want = std::max<int64_t>(want, (int64_t)64 << 20);
         WCUDA(al->d_pool.ensure((size_t)want));
+        WCUDA(al->d_free.ensure(sizeof(int32_t) * (al->d_pool.cap / (size_t)WFA_CHUNK + 1)));
     }
     WCUDA(cudaMemcpyAsync(al->d_pat.p, hp, (size_t)pb, cudaMemcpyHostToDevice, al->st));
     WCUDA(cudaMemcpyAsync(al->d_txt.p, ht, (size_t)tb, cudaMemcpyHostToDevice, al->st));
@@ -161,7 +195,8 @@ static int run_batch(wavefront_aligner_gpu *al, int n, const char *const *patter
     W.ppat = al->d_ppat.as<uint64_t>(), W.ptxt = al->d_ptxt.as<uint64_t>();
     W.pairs = al->d_pairs.as<WfaPairDev>();
     W.pool = al->d_pool.as<uint8_t>(), W.pool_bytes = (int64_t)al->d_pool.cap;
-    W.pool_head = al->d_head.as<unsigned long long>();
+    W.ctl = al->d_ctl.as<WfaPoolCtl>();
+    W.free_ring = al->d_free.as<int32_t>(), W.free_slots = (uint32_t)(al->d_pool.cap / (size_t)WFA_CHUNK + 1);
     W.ctab = al->d_ctab.as<int64_t>();
     W.ops = al->d_ops.as<char>();
     W.out = al->d_out.as<WfaOutDev>();
@@ -171,11 +206,12 @@ static int run_batch(wavefront_aligner_gpu *al, int n, const char *const *patter
     W.singletrack = A.singletrack && !W.piggyback ? 1 : 0;
     const int scope = std::max(A.gap_opening1 + A.gap_extension1, A.gap_opening2 + A.gap_extension2);
     W.max_score_scope = std::max(scope, A.mismatch) + 1;
-    const int occ = std::max(1, wfa_occupancy(W.piggyback != 0));
+    const int occ = std::max(1, wfa_occupancy(W.piggyback != 0, WFA_CTA, W.pen, W.max_score_scope));
+    const int occ_big = std::max(1, wfa_occupancy(W.piggyback != 0, WFA_BIG_CTA, W.pen, W.max_score_scope));
     // Pairs whose wavefront outgrows a warp (high memory only) stop with WFA_WIDE and run
     // again, from score 0, on the cluster kernel once the warp phase is over.
     const int cl = std::min(8, std::max(1, g_wide_cluster.load()));
-    const int wide_clusters = W.piggyback ? 0 : wfa_wide_clusters(cl, W.max_score_scope);
+    const int wide_clusters = W.piggyback ? 0 : wfa_wide_clusters(cl, W.pen, W.max_score_scope);
     W.wide_width = wide_clusters > 0 ? std::max(0, g_wide_width.load()) : 0;
     W.wide_width_tail = std::min(W.wide_width, std::max(0, g_wide_tail.load()));
     W.wide_tail_pairs = std::max(1, wide_clusters);
@@ -191,20 +227,31 @@ static int run_batch(wavefront_aligner_gpu *al, int n, const char *const *patter
     al->last_cluster_launches = 0;
     float total_ms = 0.f;
     int launches = 0;
+    // A call of a few pairs: its long ones start on the cluster kernel, where they would end up
+    // (10 kb at 5%: 15.8 ms against 17.5 by way of a CTA and 23 on a CTA to the end; at small
+    // scores the two cost about the same per score).
+    std::vector<int32_t> first = order;
+    if (W.wide_width > 0 && n <= wide_clusters) {
+        auto is_long = [&](int32_t i) { return (int64_t)plen[i] + tlen[i] >= kClusterSum; };
+        std::copy_if(order.begin(), order.end(), std::back_inserter(wide), is_long);
+        first.erase(std::remove_if(first.begin(), first.end(), is_long), first.end());
+    }
     for (int phase = 0; phase < 2; ++phase) {
-        std::vector<int32_t> pending = phase == 0 ? order : wide;
+        std::vector<int32_t> pending = phase == 0 ? first : wide;
         size_t chunk = pending.size();
         while (!pending.empty()) {
             const size_t take = std::min(chunk, pending.size());
             std::vector<int32_t> batch(pending.begin(), pending.begin() + (std::ptrdiff_t)take);
             // warp phase: the long pairs (still largest first) ahead of the others, each taken by
-            // a whole CTA before the CTAs' warps take the others one each
-            int32_t n_long = 0;
+            // a whole CTA before the CTAs' warps take the others one each; of the long ones, the
+            // first n_big on big CTAs of their own launch
+            int32_t n_long = 0, n_big = 0;
             staged.clear();
             if (phase == 0 && long_sum > 0) {
                 for (int32_t i : batch)
                     if ((int64_t)plen[i] + tlen[i] >= long_sum) staged.push_back(i);
                 n_long = (int32_t)staged.size();
+                n_big = big_pairs(staged, plen, tlen, al->sms);
                 for (int32_t i : batch)
                     if ((int64_t)plen[i] + tlen[i] < long_sum) staged.push_back(i);
             } else {
@@ -212,22 +259,48 @@ static int run_batch(wavefront_aligner_gpu *al, int n, const char *const *patter
             }
             WCUDA(cudaMemcpyAsync(al->d_order.p, staged.data(), sizeof(int32_t) * staged.size(), cudaMemcpyHostToDevice,
                                   al->st));
-            WCUDA(cudaMemsetAsync(al->d_queue.p, 0, 16, al->st));
-            WCUDA(cudaMemsetAsync(al->d_head.p, 0, 8, al->st));
-            W.order_long = al->d_order.as<int32_t>();
-            W.n_long = n_long;
-            W.order = al->d_order.as<int32_t>() + n_long;
-            W.n = (int32_t)staged.size() - n_long;
+            WCUDA(cudaMemsetAsync(al->d_queue.p, 0, 32, al->st));
+            WCUDA(cudaMemsetAsync(al->d_ctl.p, 0, sizeof(WfaPoolCtl), al->st));
+            WCUDA(cudaMemsetAsync(al->d_free.p, 0, sizeof(int32_t) * W.free_slots, al->st));
+            W.n_all = (int32_t)staged.size();
             WCUDA(cudaEventRecord(al->e0, al->st));
             if (phase == 0) {
-                const int ctas = std::max(1, std::min(std::max((W.n + 3) / 4, W.n_long), occ * al->sms));
-                WCUDA(launch_wfa(W, ctas, al->st));
+                WfaArgs B = W;
+                // eight times the tail width: starting a pair over on a cluster late in its scores
+                // costs more than the big CTA takes to finish it (64 pairs of 1-10 kb: 28 ms with
+                // four times, 24 with eight)
+                B.wide_width_tail = (int)std::min<int64_t>(W.wide_width, 8 * (int64_t)W.wide_width_tail);
+                B.order_long = al->d_order.as<int32_t>(), B.n_long = n_big;
+                B.order = B.order_long, B.n = 0;
+                W.order_long = B.order_long + n_big, W.n_long = n_long - n_big;
+                W.order = B.order_long + n_long, W.n = (int32_t)staged.size() - n_long;
+                const bool rest = W.n_long + W.n > 0;
+                if (n_big > 0) {
+                    // its queue counters [4..7] are its own, but the running and started pairs
+                    cudaStream_t s2 = rest ? al->st2 : al->st;
+                    if (rest) {
+                        WCUDA(cudaEventRecord(al->fork, al->st));
+                        WCUDA(cudaStreamWaitEvent(al->st2, al->fork, 0));
+                    }
+                    B.q_long = 4;
+                    WCUDA(launch_wfa(B, WFA_BIG_CTA, std::min(n_big, occ_big * al->sms), s2));
+                    ++launches;
+                    if (rest) WCUDA(cudaEventRecord(al->join, al->st2));
+                }
+                if (rest) {
+                    const int ctas = std::max(1, std::min(std::max((W.n + 3) / 4, W.n_long), occ * al->sms));
+                    W.q_long = 2;
+                    WCUDA(launch_wfa(W, WFA_CTA, ctas, al->st));
+                    ++launches;
+                    if (n_big > 0) WCUDA(cudaStreamWaitEvent(al->st, al->join, 0));
+                }
             } else {
+                W.order = al->d_order.as<int32_t>(), W.n = (int32_t)staged.size();
                 ++al->last_cluster_launches;
                 WCUDA(launch_wfa_wide(W, std::min(W.n, wide_clusters), cl, al->st));
+                ++launches;
             }
             WCUDA(cudaEventRecord(al->e1, al->st));
-            ++launches;
             WCUDA(cudaMemcpyAsync(al->outs.data(), al->d_out.p, sizeof(WfaOutDev) * (size_t)n, cudaMemcpyDeviceToHost,
                                   al->st));
             WCUDA(cudaStreamSynchronize(al->st));
@@ -305,6 +378,9 @@ wavefront_aligner_gpu_t *wavefront_aligner_new_gpu(const wavefront_gpu_attr_t *a
     if (cudaGetDevice(&dev) != cudaSuccess ||
         cudaDeviceGetAttribute(&al->sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
         cudaStreamCreateWithFlags(&al->st, cudaStreamNonBlocking) != cudaSuccess ||
+        cudaStreamCreateWithFlags(&al->st2, cudaStreamNonBlocking) != cudaSuccess ||
+        cudaEventCreateWithFlags(&al->fork, cudaEventDisableTiming) != cudaSuccess ||
+        cudaEventCreateWithFlags(&al->join, cudaEventDisableTiming) != cudaSuccess ||
         cudaEventCreate(&al->e0) != cudaSuccess || cudaEventCreate(&al->e1) != cudaSuccess) {
         set_error("wavefront_aligner_new_gpu: CUDA initialisation failed");
         delete al;

@@ -31,22 +31,34 @@ struct WfaOutDev {
     int64_t mem_bytes;
 };
 
+// Counters of the wavefront pool, zero at the start of a round.
+struct WfaPoolCtl {
+    unsigned long long head;   // bytes taken from the end
+    int32_t avail;             // chunks in the free ring
+    uint32_t pushed, popped;   // ring positions
+    uint32_t pad;
+};
+
 struct WfaArgs {
     const uint8_t *pat, *txt;
     const uint64_t *ppat, *ptxt;  // the same arenas at 2 bits per base (32 bases per word)
     const WfaPairDev *pairs;
     const int32_t *order;
     int32_t n;
-    const int32_t *order_long;  // pairs each run on a whole CTA first (high memory), n_long of them
+    const int32_t *order_long;  // pairs each run on a whole CTA first, n_long of them
     int32_t n_long;
     uint8_t *pool;
     int64_t pool_bytes;
-    unsigned long long *pool_head;
+    WfaPoolCtl *ctl;
+    int32_t *free_ring;   // chunks given back by finished pairs: chunk number + 1, 0 = empty slot
+    uint32_t free_slots;  // at least the chunks of the pool
     int64_t *ctab;
     char *ops;
     WfaOutDev *out;
-    int32_t *queue;       // [0] next position of `order`, [1] pairs running on warps,
-                          // [2] next position of `order_long`
+    int32_t *queue;       // [0] next position of `order`, [1] pairs running, [3] pairs started,
+                          // [q_long] next position of `order_long`
+    int32_t q_long;
+    int32_t n_all;        // pairs of the round, over all launches that share it
     WfaPen pen;
     int singletrack;
     int piggyback;        // medium / low memory: ring of recent scores + packed-CIGAR blocks
@@ -57,18 +69,24 @@ struct WfaArgs {
     int wide_width_cta;   // a pair on a whole CTA whose wavefront grows wider stops with WFA_WIDE
 };
 
-cudaError_t launch_wfa(const WfaArgs &a, int ctas, cudaStream_t st);
+// Pool bytes are taken and given back in chunks of this size.
+constexpr int64_t WFA_CHUNK = 256 << 10;
+// CTA sizes of the kernel: WFA_CTA threads (four fit an SM), or WFA_BIG_CTA (one per SM) for
+// the pairs that would outlast their batch on the small ones.
+constexpr int WFA_CTA = 128, WFA_BIG_CTA = 512;
+
+cudaError_t launch_wfa(const WfaArgs &a, int threads, int ctas, cudaStream_t st);
 // The cluster kernel (high memory: standard and Singletrack): one cluster of `cl` CTAs per
 // pair, the diagonals of a wavefront spread over all of its threads; `clusters` clusters
 // take the pairs of a.order in turn.
 cudaError_t launch_wfa_wide(const WfaArgs &a, int clusters, int cl, cudaStream_t st);
 // Clusters of `cl` CTAs of the cluster kernel that fit on the device at once for a score
 // scope (0 if none, or if the scope is too large for the kernel's header ring).
-int wfa_wide_clusters(int cl, int scope);
+int wfa_wide_clusters(int cl, const WfaPen &pen, int scope);
 // 2-bit copies of the pattern and text arenas (A=0, C=1, G=2, T=3, any other byte 0), and
 // the per-pair flag that the pair's sequences are uppercase ACGT only.
 cudaError_t launch_wfa_pack(const uint8_t *pat, int64_t pbytes, uint64_t *ppat, const uint8_t *txt, int64_t tbytes,
                             uint64_t *ptxt, WfaPairDev *pairs, int n, cudaStream_t st);
-int wfa_occupancy(bool piggyback);
+int wfa_occupancy(bool piggyback, int threads, const WfaPen &pen, int scope);
 
 }  // namespace aw
