@@ -71,7 +71,6 @@ static thread_local int64_t tls_tb_budget = 0;  // per-thread override (serving 
 static std::atomic<bool> g_band_full_pairs{true};
 static int g_large_warps = 8;
 static int g_large_tlen = 4096;
-static int g_band_nc = 0;  // banded kernel columns per lane: 0 = chosen per plan, 4 or 8
 static std::mutex g_cfg_mu;
 
 // ---- pooled buffers ----------------------------------------------------------
@@ -347,27 +346,6 @@ struct aw_ksw_plan {
     ~aw_ksw_plan() { drop_graph(); }
 };
 
-// Columns per lane of the banded kernel for this plan: 4 halves the pipeline lag between
-// strips (the band edge sweeps a strip in 32*nc rows) at a few percent more work per
-// cell; it pays when the plan is bound by the longest pair's chain of strips rather than
-// by total work.  Estimates: ~1 us per strip row-step on the chain, ~300 GCUPS of work.
-static int band_columns(const aw_ksw_plan_t *pl) {
-    int fixed;
-    {
-        std::lock_guard<std::mutex> lk(g_cfg_mu);
-        fixed = g_band_nc;
-    }
-    if (fixed == 4 || fixed == 8) return fixed;
-    double work = 0.0, chain = 0.0;
-    for (int32_t i : pl->band_ids) {
-        const int ql = pl->qlen[i], tl = pl->tlen[i];
-        const int ww = pl->w[i] < 0 ? std::max(ql, tl) : std::min(pl->w[i], std::max(ql, tl));
-        work += 2.0 * std::min<double>(ww, std::max(ql, tl)) * (double)std::max(ql, tl) / 3e11;
-        chain = std::max(chain, (1.25 * tl + 2.0 * ww + 300.0) * 1e-6);
-    }
-    return chain > work ? 4 : 8;
-}
-
 // Seconds that full-matrix pairs take on strips of one width: their cells at the rate of the
 // whole GPU, and half of the longest pair's chain of steps (its rows and the skew of a strip,
 // and a lag of 80 steps per further strip), which the other pairs hide only in part.
@@ -531,7 +509,7 @@ static int plan_build(aw_ksw_plan_t *pl, int n, const int *qlen, const int *tlen
         // ksw_extd2_singletrack_sse works on 16-byte blocks whatever the build's width
         const bool sse_st = (P.flag & AW_EZ_SINGLETRACK) && (P.flag & AW_EZ_SSE_SINGLETRACK);
         if (band_plan_build(pl->band, pl->band_ids, pl->qlen, pl->tlen, pl->w, pl->pairs, P.flag,
-                            sse_st ? 16 : exact_block(), budget, band_columns(pl), &refused)) {
+                            sse_st ? 16 : exact_block(), budget, &refused)) {
             set_error("pair traceback exceeds the HBM traceback budget");
             return AW_E_NOMEM;
         }
@@ -726,7 +704,7 @@ static int plan_launch(aw_ksw_plan_t *pl) {
         D.bnd = B->band_bnd.as<uint2>(), D.tb = B->tb.as<uint8_t>(), D.error = B->error.as<int32_t>();
         D.groups = B->band_groups.as<BandGroupDev>();
         D.deadline = deadline;
-        const int ctas = band_occupancy(P.flag) * B->sms;
+        const int ctas = band_occupancy(P.flag, pl->band.block) * B->sms;
         for (int k = 0; k < nbw; ++k) {
             cudaEvent_t *ev = &B->ev_k[3 * (nw + k)];
             AW_CUDA(record_timing(ev[0], B->st));
@@ -872,10 +850,8 @@ void aw_ksw_set_stop_antidiagonal(int interval, int antidiagonal) { set_exact_st
 
 void aw_set_full_pair_routing(int enabled) { g_band_full_pairs.store(enabled != 0); }
 
-void aw_set_band_columns(int columns) {
-    std::lock_guard<std::mutex> lk(g_cfg_mu);
-    g_band_nc = (columns == 4 || columns == 8) ? columns : 0;
-}
+// One strip width serves every batch (ksw2_band.cu), so there is nothing to choose.
+void aw_set_band_columns(int) {}
 
 void aw_set_tuning(int large_warps, int large_tlen_threshold) {
     std::lock_guard<std::mutex> lk(g_cfg_mu);

@@ -6,48 +6,50 @@
 // so cells just outside the band ("padding") are computed from whatever the arrays
 // held, and the in-band cells and the traceback read them
 // (minimap2/ksw2_extd2_avx.c:255-701, ksw2_extd2_sse.c:136-331).  This kernel
-// computes the same cells in target-column strips swept row by row (the layout of
-// the full-matrix kernel) and restates the array semantics cell by cell:
-//   * a column's registers hold the last value written at its position, so a
-//     column that is not computed on a row keeps its previous values;
-//   * left input of cell (t, j): the cell (t-1, j) if it was computed, else the
-//     array's initial values; at t == st16 the reference's boundary value
-//     (x[st16-1] only on the anti-diagonal where st16 advanced, constants
-//     otherwise, the matrix edge when st16 == 0, ksw2_extd2_avx.c:273-287); at
-//     t == stB < st16 (lane 0 of the first block) the in-register wrap to lane 15,
-//     i.e. cell (stB+15, j-16), kept in a 16-row shared-memory ring;
-//   * up input: the column registers, the top-edge values on row 0;
+// computes the same cells in target-column strips, one warp per strip, which sweeps the
+// anti-diagonals as the reference does: at step r lane L holds the cells of its columns on
+// anti-diagonal r, two per register (ksw2_cell.cuh), and the registers of a column are the
+// reference's arrays at its position:
+//   * the cells of a step do not depend on one another, so a step costs one cell's latency
+//     and a warp alone keeps its scheduler busy (a sweep by rows, each lane's cells a serial
+//     chain, took 0.61 us per 4-column step at the band's edge, one anti-diagonal takes 0.25);
+//   * st0, en0 and the blocks around them are the same for the whole warp, and a lane's columns
+//     lie in one 16-column block, so "computed" is a property of a lane: a lane outside
+//     [stB, en16] skips its cells and its registers keep their last values;
+//   * left input of cell (t, r): the column t-1 at r-1 (the previous lane's last column by a
+//     shuffle); at t == st16 the reference's boundary value (x[st16-1] only on the anti-diagonal
+//     where st16 advanced, constants otherwise, the matrix edge when st16 == 0,
+//     ksw2_extd2_avx.c:273-287); at t == stB < st16 (lane 0 of the first block) the in-register
+//     wrap to lane 15, i.e. column stB+15 at r-1, by another shuffle;
+//   * up input: the column's own registers, the top-edge values on row 0;
 //   * score: the score-fill (ksw2_extd2_avx.c:289-311) refreshes position t on
 //     anti-diagonal r when st0 <= t <= st0+16*ceil((en0-st0+1)/16)-1 (en0 for
-//     generic scoring); otherwise the stale value of the last fill stays;
+//     generic scoring); otherwise the stale value of the last fill stays.  Query codes move
+//     one column per step with the cells (code 0 above the matrix);
 //   * H row: H[t] += v[t] inside the band, H[en0] = H[en0-1] + u[en0] on the right
 //     edge (ksw2_extd2_sse.c:332-367), mqe/mte with ">=" (:369-372), the score
 //     on the last anti-diagonal; the anti-diagonal loop stops at the first empty
 //     band (:151-154, zdropped = 1).
-// Rows above the matrix (j < 0) only refresh the stale score; rows below it and
-// columns right of it never reach a cell of the matrix.
-//
-// Three forms of a step (one row of every lane), chosen for the whole warp:
-//   * interior: every cell strictly inside the band, the full-matrix arithmetic unchanged;
-//     the steps where that holds for all lanes are one range of k, solved once per strip;
-//   * edge: the rules above from closed forms in the distance of a cell to the band's
-//     right edge, e = j + w - t.  The band edge crosses a strip during its first rows and
-//     the strip on the right cannot start before, so these steps are the chain that bounds
-//     long pairs;
-//   * corner (rows 0 and qlen-1, rows above the matrix, and the anti-diagonals where the
-//     rule for st0 changes): the same rules from st0 and en0 of every cell.
-// The stale scores are kept as the last fill of each column in a register of its own, which
-// interior steps refresh for nothing.
+// Cells above the matrix, below it and right of it that a lane computes along with its others
+// never reach a cell of the matrix.  Three ranges of a strip's steps, solved once per strip, run on
+// loops of their own: the steps where the whole strip lies strictly inside the band (no
+// tests), before them those where only the band's right edge is in the strip, and after them
+// those with only its left edge.  Both edges are chains that bound long pairs: every step of
+// a pair has some strip at each of them.  H is kept where a later step needs it: not at all
+// while the right edge is in the strip (it follows from the left column's H and the u and v
+// of an anti-diagonal), for the lane's last column afterwards (the others follow in the same
+// way).
 //
 // Work decomposition: every (pair, strip) is a unit of a device queue, ordered so
-// that a strip is always taken after the strip on its left; a warp takes a unit and
-// sweeps its rows with the one-row lane skew of the full-matrix kernel, reading its left
-// column as the strip on the left writes it.  Many warps, across CTAs, work on one pair at
-// once, so a single long interval fills the GPU.  An entry of a boundary column carries a
-// mark that says it is written (the columns are cleared before the first pass), so a strip
-// reads eight rows ahead and waits (bounded) only for entries that are not there yet: no
-// fence and no counter between the strips.
+// that a strip is always taken after the strip on its left, and reads its left column as that
+// strip writes it.  The band enters a strip SW columns further right 2 SW steps later, so a
+// long pair takes about two steps per target base whatever the strip's width, and its strips
+// run on as many warps, across CTAs, as the band is high.  An entry of a boundary column
+// carries a mark that says it is written (the columns are cleared before the first pass), so
+// a strip reads eight rows ahead and waits (bounded) only for entries that are not there yet:
+// no fence and no counter between the strips.
 #include "ksw2_band.h"
+#include "ksw2_cell.cuh"
 #include "tb_walk.cuh"
 
 #include <algorithm>
@@ -66,66 +68,10 @@ struct Geom {
     __device__ __forceinline__ int en0(int r) const { return min(min(tlen - 1, r), (r + w) >> 1); }
 };
 
-__device__ __forceinline__ int prmt_sx(uint32_t lo, uint32_t hi, uint32_t sel) {
-    uint32_t r;
-    asm("prmt.b32 %0, %1, %2, %3;" : "=r"(r) : "r"(lo), "r"(hi), "r"(sel));
-    return (int)r;
-}
+__device__ __forceinline__ int prmt_sx(uint32_t lo, uint32_t hi, uint32_t sel) { return (int)prmt(lo, hi, sel); }
 __device__ __forceinline__ int sx8(uint32_t w) { return (int)(int8_t)(uint8_t)w; }
-__device__ __forceinline__ uint32_t pack3(int a, int b, int c, uint32_t top) {
-    return (uint32_t)(a & 0xff) | ((uint32_t)(b & 0xff) << 8) | ((uint32_t)(c & 0xff) << 16) | (top << 24);
-}
-__device__ __forceinline__ int edge_diff(int r, const KswScore &S) {
-    return r == 0 ? -S.qe : r < S.long_thres ? -S.e : r == S.long_thres ? S.long_diff : -S.e2;
-}
-
-// One cell of the reference recurrence in 32-bit registers (the host routes only
-// parameter sets whose int8 intermediates cannot wrap).  xs/vs/x2s: left input in,
-// this cell's x/v/x2 out; ut/yt/y2t: up input in, this cell's u/y/y2 out.
-template <bool ARGMAX, bool RIGHT>
-__device__ __forceinline__ void cell(int s, int &xs, int &vs, int &x2s, int &ut, int &yt, int &y2t, int &d,
-                                     const KswScore &S) {
-    const int a = xs + vs, b = yt + ut, a2 = x2s + vs, b2 = y2t + ut;
-    int z = s;
-    if (!ARGMAX) {
-        z = __vimax3_s32(z, a, b);
-        z = __vimax3_s32(z, a2, b2);
-    } else {
-        // arg-max by priority tags in the low 4 bits of 16 * candidate: the larger tag wins a
-        // tie of values, so the max gives z and the state code at once.  Left-aligned: the
-        // first candidate wins a tie (ksw2_extd2_sse.c:244-251), tags s=7 > a=6 > ... > b2=3,
-        // code = tag ^ 7; right-aligned: the last (:291-298), tags = codes 0..4.
-        constexpr int Ts = RIGHT ? 0 : 7, Ta = RIGHT ? 1 : 6, Tb = RIGHT ? 2 : 5, Ta2 = RIGHT ? 3 : 4,
-                      Tb2 = RIGHT ? 4 : 3;
-        int zt = __vimax3_s32(s * 16 + Ts, b * 16 + Tb, b2 * 16 + Tb2);
-        zt = __vimax3_s32(zt, a * 16 + Ta, a2 * 16 + Ta2);
-        d = RIGHT ? (zt & 15) : ((zt & 15) ^ 7);
-        z = zt >> 4;
-    }
-    z = min(z, S.mch);
-    const int un = z - vs, vn = z - ut;
-    if (!(ARGMAX && RIGHT)) {
-        const int nez = -S.e - z, nez2 = -S.e2 - z;
-        xs = __viaddmax_s32(a, nez, -S.qe);
-        yt = __viaddmax_s32(b, nez, -S.qe);
-        x2s = __viaddmax_s32(a2, nez2, -S.qe2);
-        y2t = __viaddmax_s32(b2, nez2, -S.qe2);
-        if (ARGMAX) {
-            d += 0x08 * __viaddmin_s32(xs, S.qe, 1);
-            d += 0x10 * __viaddmin_s32(yt, S.qe, 1);
-            d += 0x20 * __viaddmin_s32(x2s, S.qe2, 1);
-            d += 0x40 * __viaddmin_s32(y2t, S.qe2, 1);
-        }
-    } else {
-        const int aa = a - z + S.q, bb = b - z + S.q, aa2 = a2 - z + S.q2, bb2 = b2 - z + S.q2;
-        xs = max(aa, 0) - S.qe;
-        yt = max(bb, 0) - S.qe;
-        x2s = max(aa2, 0) - S.qe2;
-        y2t = max(bb2, 0) - S.qe2;
-        d |= (aa >= 0 ? 0x08 : 0) | (bb >= 0 ? 0x10 : 0) | (aa2 >= 0 ? 0x20 : 0) | (bb2 >= 0 ? 0x40 : 0);
-    }
-    ut = un;
-    vs = vn;
+__device__ __forceinline__ uint32_t pack3(int a, int b, int c) {
+    return (uint32_t)(a & 0xff) | ((uint32_t)(b & 0xff) << 8) | ((uint32_t)(c & 0xff) << 16);
 }
 
 // The Singletrack tracks (v, u) instead of the state bytes: the Singletrack entries of
@@ -164,12 +110,11 @@ struct BandArgs {
     // recompute rounds: the pairs' walk states; a round's strips stop at the row the walk has
     // reached (it only moves up and left), strips of a finished walk compute nothing
     const BandWalkState *walk;
+    uint32_t one = 1;  // KswFullArgs::one
 };
 
 constexpr uint64_t WAIT_NS = 20ull * 1000 * 1000 * 1000;  // bounded wait on the left strip
-// Rows of the left column read at a time: a strip starts a row once the group it lies in is
-// written (lane 31 finishes row j 31 steps after lane 0), so a hop between strips costs strip
-// width + 31 + PUB lane-steps.
+// Rows of the left column read at a time.
 constexpr int PUB = 8;
 // Mark of a written boundary entry: the byte above its x, v and x2.
 constexpr uint32_t BND_MARK = 0x80000000u;
@@ -183,21 +128,48 @@ __device__ __forceinline__ void bnd_store(uint2 *p, uint32_t x, uint32_t h) {
     asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p), "l"((uint64_t)h << 32 | (x | BND_MARK)) : "memory");
 }
 
-// NC target columns per lane (strips of 32*NC columns): 8 for throughput, 4 for a shorter
-// pipeline lag between strips when few long pairs run.
-template <bool CIGAR, bool RIGHT, bool ST, int NC>
-__global__ void __launch_bounds__(256, 2) ksw_band_kernel(BandArgs A) {
-    constexpr int C = NC;
-    // ARGMAX: the state byte is stored (CIGAR without Singletrack)
-    constexpr bool ARGMAX = CIGAR && !ST;
-    constexpr int CB = ST ? 2 * C : C;  // traceback bytes per lane-step
-    // the block wrap reads column stB+15: lane +D of the stB lane, its last column
-    constexpr int D = 16 / C - 1;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    __shared__ uint32_t ring[8][16][32];
+// Value of a field of 16 * value + FB (+ tag).
+__device__ __forceinline__ int fval(uint32_t w, int f) { return (fld(w, f) - FB) >> 4; }
+// Both fields of a pair from two conditions.
+__device__ __forceinline__ uint32_t mask2(bool lo, bool hi) { return (lo ? 0xffffu : 0u) | (hi ? 0xffff0000u : 0u); }
+
+// The traceback words of a step.  A word holds four columns of one row, whose cells lie on four
+// consecutive anti-diagonals: the bytes of the first three columns wait for the fourth.  put()
+// takes a byte per field (bits 0-7 and 16-23 of d[p]: columns p and p + NP) and returns the
+// word completed at this step, of row r - 3 - (its first column).
+struct RowWords {  // columns 0, 2 in d[0]; 1, 3 in d[1]
+    uint32_t a0 = 0, a1 = 0, a2 = 0;
+    __device__ __forceinline__ uint32_t put(const uint32_t (&d)[2]) {
+        const uint32_t w = prmt(a2, d[1], 0x6210);
+        a2 = prmt(a1, d[0], 0x7610);
+        a1 = prmt(a0, d[1], 0x5540);
+        a0 = d[0];
+        return w;
+    }
+};
+
+// A lane holds C = 4 target columns in NP pairs; a strip is SW = 128 columns.  (Eight columns per
+// lane took 0.45 us a step against 0.25 and were no faster on 512 pairs of 5 kb at w = 50%,
+// which are bound by their work: 15.4 against 14.1 ms.)
+constexpr int NP = 2, C = 2 * NP, SW = 32 * C;
+// Traceback layout: words of 4 columns (state bytes, or v then u bytes), NG words per step.  The
+// word of group g (columns 4g..4g+3 of the strip) and row j is stored (j - jlo) + 4g steps from
+// the strip's start.
+constexpr int NG = SW / 4;
+
+constexpr int BAND_WARPS = 4;  // per CTA: small CTAs spread a pair's strips over the SMs
+
+template <int MODE>
+__global__ void __launch_bounds__(32 * BAND_WARPS, 4) ksw_band_kernel(BandArgs A) {
+    constexpr bool CIGAR = MODE != SCORES;
+    constexpr int WB = MODE == TRACKS ? 8 : 4;
+    using T = Tags<MODE>;
+    const int lane = threadIdx.x & 31;
     const KswScore &S = A.sc;
+    const CellK K = make_cellk<MODE>(S, A.one);
     const int B = A.block;
-    const bool src_lane = B > 16 && lane >= D && (((lane - D) * C) & (B - 1)) == 0;
+    // the block wrap reads the last column of the lane D to the right
+    constexpr int D = 16 / C - 1;
 
     for (;;) {
         int u = 0;
@@ -223,70 +195,124 @@ __global__ void __launch_bounds__(256, 2) ksw_band_kernel(BandArgs A) {
         const int qlen = P.qlen, tlen = P.tlen, qm1 = qlen - 1, tm1 = tlen - 1, w = P.w;
         const int rlim = min(g.nd, g.rb);
         const uint8_t *qs = A.qcodes + P.qoff, *ts = A.tcodes + P.toff;
-        const int col0 = s * 32 * C + lane * C;
+        const int c0 = s * SW, col0 = c0 + lane * C, rs = c0 + jstart;
         const bool last_strip = s + 1 == P.nstrip;
-        // the strip on the left: its stored rows and, after them, its final H (an empty strip
-        // computes nothing, so its column keeps the initial values)
+        // the strip on the left and its stored rows; on other rows (and for an empty strip) the
+        // arrays' initial values, which no cell of the band reads
         int prod_lo = 0, prod_hi = -1;
         const uint2 *bnd_prod = nullptr;
         if (s > 0) {
             const BandStripDev Pr = A.strips[P.strip0 + s - 1];
-            if (min(Pr.jend, wlim) >= Pr.jlo) {
-                prod_lo = Pr.jlo, prod_hi = min(Pr.jend, wlim);
-                bnd_prod = A.bnd + Pr.bnd_off;
-            }
+            prod_lo = Pr.jlo, prod_hi = min(Pr.jend, wlim);
+            bnd_prod = A.bnd + Pr.bnd_off;
         }
         // a recompute round reads the columns of the first pass and writes none
         uint2 *bnd_me = lane == 31 && !last_strip && !A.walk ? A.bnd + St.bnd_off : nullptr;
         const bool store_tb = CIGAR && (!P.ckpt || A.store_ckpt);  // this strip's traceback is kept
-        // this lane's traceback word of step k: tbp + k * 32 * CB
-        uint8_t *tbp = CIGAR ? A.tb + St.tb_off + ((int64_t)(jstart - jlo) * 32 + lane) * CB : nullptr;
+        // this lane's words completed at step 0 (row rs - c0 - 3 of group 0, slot jstart - 3 - jlo)
+        const int slot0 = jstart - 3 - jlo;
+        uint8_t *tbp = CIGAR ? A.tb + St.tb_off + ((int64_t)slot0 * NG + lane) * WB : nullptr;
         BandRes *R = A.res + un.x;
-        // lane constants of the closed-form bounds: floor16 and the block end of the lane's columns
-        const int F16 = col0 & ~15, XB = (col0 & g.bmask) + B - 1;
-        // Score fill right of the band while st0 = (r-w+1)>>1: en0-st0+1 is w+1 where e is even
-        // and w where it is odd, so the fill reaches the columns with e >= -2 pad (even) and
-        // e >= 1 - 2 pad (odd), pad = what rounds that length up to 16.
-        const int fill_even = A.generic ? 0 : 2 * (-(w + 1) & 15), fill_odd = A.generic ? -1 : 2 * (-w & 15) - 1;
-        // rows where the lane's cells all lie strictly inside the band, with natural neighbours
-        const int fa = max(1, col0 + C + 1 - w);
-        const int fb = col0 + C > tm1 ? -1 : min(min(qlen - 2, rlim - col0 - C), col0 > 0 ? col0 + w - 2 : w);
-        // steps where that holds for every lane
-        const int kf0 = (int)__reduce_max_sync(FULL, max(fa, jstart) + lane) - jstart;
-        const int kf1 = (int)__reduce_min_sync(FULL, min(fb, jend) + lane) - jstart + 1;
+        // steps whose cells all lie strictly inside the band
+        const int ri0 = max(c0 + SW, 2 * (c0 + SW) - w);
+        const int ri1 = min(min(rlim - 1, c0 + qm1 - 1), c0 > 0 ? 2 * c0 + w - 2 : w);
+        const int kf0 = ri0 - rs, kf1 = c0 + SW <= tm1 ? ri1 - rs + 1 : 0;
+        // in the last strip, from the step after the last column entered the band
+        const int kz0 = max(tm1, 2 * tm1 - w) + 1 - rs, kz1 = last_strip ? ri1 - rs + 1 : 0;
+        // the steps after kf0 whose left edge may lie in the strip
+        const int kl1 = c0 + SW <= tm1 ? min(rlim, c0 + qm1) - rs : 0;
+        // steps below row 0 with the left edge (st0) left of the strip and the right edge before its
+        // last column, whose H the strip on the right reads from then on
+        const int kr0 = c0 + SW - rs, kr1 = c0 > 0 ? min(kf1, 2 * (c0 + SW - 1) - w - rs) : 0;
+        // the last step: the strip's last word of row jend
+        const int nsteps = c0 + min(SW, ((tlen - c0) + 3) & ~3) - 1 + jend - rs + 1;
 
-        int ut[C], yt[C], y2t[C], H[C], ss[C];
-        uint32_t rlo[C], rhi[C];
+        uint32_t X[NP], V[NP], X2[NP], U[NP], Y[NP], Y2[NP], SS[NP];
+        uint32_t rlo[C], rhi[C], sel[C];
+        int H[C];
+        const uint32_t x_in = K.kxa, v_in = rep2(FB - 16 * S.qe), x2_in = K.kxa2;  // initial values
 #pragma unroll
         for (int c = 0; c < C; ++c) {
             const int t = col0 + c;
             const int tc = t < tlen ? (ts[t] & 7) : 0;
             rlo[c] = S.tab_lo[tc];
             rhi[c] = S.tab_hi[tc];
-            ut[c] = -S.qe, yt[c] = -S.qe, y2t[c] = -S.qe2;
+            sel[c] = 0x8880u;  // query code 0
             H[c] = AW_NEG_INF;
-            ss[c] = 0;
         }
-        const uint32_t init_pack = pack3(-S.qe, -S.qe, -S.qe2, 0);
-        uint32_t carry = 0;
-        int Hcarry = AW_NEG_INF;
+        constexpr int SB = T::s + 2 * FB;
+#pragma unroll
+        for (int p = 0; p < NP; ++p) {
+            X[p] = x_in, V[p] = v_in, X2[p] = x2_in;
+            U[p] = v_in, Y[p] = K.kxb, Y2[p] = K.kxb2;
+            SS[p] = add2(SB);  // score 0
+        }
+        RowWords words, words2;
+        enum { H_NONE, H_LAST, H_ALL };
+        int h_state = H_ALL;             // the columns whose H is up to date
         unsigned long long mte_key = 0;  // last strip: the lane that owns the last column
         const int pm = A.sse_st ? INT_MAX : 0;  // strict end rule: mirrored positions
         // lane 0's left values of row jr: x, v, x2 with the mark, and the H on the left
         auto left_of = [&](int jr) -> uint2 {
-            if (s == 0) return make_uint2(pack3(-S.qe, edge_diff(jr, S), -S.qe2, 0) | BND_MARK, (uint32_t)AW_NEG_INF);
-            if (!bnd_prod || jr < prod_lo) return make_uint2(init_pack | BND_MARK, (uint32_t)AW_NEG_INF);
-            return bnd_load(bnd_prod + (min(jr, prod_hi + 1) - prod_lo));
+            if (s == 0) return make_uint2(pack3(-S.qe, edge_diff(jr, S), -S.qe2) | BND_MARK, (uint32_t)AW_NEG_INF);
+            if (jr < prod_lo || jr > prod_hi) return make_uint2(pack3(-S.qe, -S.qe, -S.qe2) | BND_MARK, (uint32_t)AW_NEG_INF);
+            return bnd_load(bnd_prod + (jr - prod_lo));
         };
-        auto code_of = [&](int jr) -> uint32_t { return jr >= 0 && jr < qlen ? qs[jr] : 0u; };
+        // the score selector of row jr's query code
+        auto code_of = [&](int jr) -> uint32_t { return (jr >= 0 && jr < qlen ? qs[jr] & 7u : 0u) * 0x1111u + 0x8880u; };
         // lane i holds what lane 0 needs for row jstart + (k & ~31) + i: the next group's entries
         // and the next 32 query codes are on their way while the current ones are used
         uint2 ahead = make_uint2(BND_MARK, 0u);
         if (lane < PUB) ahead = left_of(jstart + lane);
-        uint32_t qnext = code_of(jstart + lane), qcur = 0, bx = 0;
+        uint32_t qnext = code_of(jstart + lane), qcur = 0, bx = 0, by = 0;
         int bh = 0;
         bool failed = false, stopped = false;
-        const int nsteps = jend - jstart + 32;
+        // the words of this step into the traceback
+        auto store_words = [&](const uint32_t (&d)[NP], const uint32_t (&d2)[NP], uint8_t *dst) {
+            if constexpr (MODE == TRACKS) {
+                const uint32_t a = words.put(d), b = words2.put(d2);
+                __stcs(reinterpret_cast<uint2 *>(dst), make_uint2(a, b));
+            } else {
+                __stcs(reinterpret_cast<uint32_t *>(dst), words.put(d));
+            }
+        };
+        // the last column's entry: x, v, x2 as bytes (a field's bits 4-11) and H
+        auto store_entry = [&](uint2 *dst) {
+            const uint32_t a = prmt(X[NP - 1], V[NP - 1], 0x7632) >> 4, b = X2[NP - 1] >> 4;
+            bnd_store(dst, prmt(a, b, 0x6620) & 0xffffffu, (uint32_t)H[C - 1]);
+        };
+        auto score_of = [&](int p) -> uint32_t {
+            return (uint32_t)prmt_sx(rlo[p + NP], rhi[p + NP], sel[p + NP]) * (16u << 16) +
+                   ((uint32_t)prmt_sx(rlo[p], rhi[p], sel[p]) * 16u + add2(SB));
+        };
+        // H of every column in the band after step k-1, from the left column's H at that step:
+        // H(t, j) = H(t-1, j) + u(t, j), and along the anti-diagonal H(t+1, j-1) = H(t, j) - v(t, j)
+        // + u(t+1, j-1)
+        auto rebuild_h = [&](int k) {
+            int sum = 0;
+#pragma unroll
+            for (int c = 0; c < C; ++c) sum += fval(U[c % NP], c / NP) - fval(V[c % NP], c / NP);
+            int before = sum;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int t = __shfl_up_sync(FULL, before, o);
+                if (lane >= o) before += t;
+            }
+            int h = __shfl_sync(FULL, bh, (k - 1) & 31) + before - sum;
+#pragma unroll
+            for (int c = 0; c < C; ++c) {
+                h += fval(U[c % NP], c / NP);
+                H[c] = h;
+                h -= fval(V[c % NP], c / NP);
+            }
+        };
+        // The lane's other columns from the last one's: along the anti-diagonal,
+        // H(t, j) = H(t+1, j-1) - u(t+1, j-1) + v(t, j)
+        auto h_from_last = [&]() {
+#pragma unroll
+            for (int c = C - 2; c >= 0; --c)
+                H[c] = H[c + 1] - fval(U[(c + 1) % NP], (c + 1) / NP) + fval(V[c % NP], c / NP);
+        };
         for (int kb = 0; kb < nsteps; kb += PUB) {
             if ((kb & 31) == 0) {
                 if (A.deadline) {
@@ -331,224 +357,239 @@ __global__ void __launch_bounds__(256, 2) ksw_band_kernel(BandArgs A) {
                 if (failed && lane == 0) atomicExch(A.error, 1);
                 if (failed || stopped) break;
             }
-            if (mine) bx = (ahead.x & 0xffffffu) | qcur << 24, bh = (int)ahead.y;
+            if (mine) {
+                bx = (uint32_t)(16 * sx8(ahead.x) + FB + T::a) | (uint32_t)(16 * sx8(ahead.x >> 8) + FB) << 16;
+                by = (uint32_t)(16 * sx8(ahead.x >> 16) + FB + T::a2) | qcur << 16;
+                bh = (int)ahead.y;
+            }
             if ((lane & ~(PUB - 1)) == ((kb + PUB) & 31)) ahead = left_of(jstart + ((kb + PUB) & ~31) + lane);
             const int kend = min(kb + PUB, nsteps);
+            const bool full = kend - kb == PUB;  // the loops below take whole groups, unrolled
             int k = kb;
-            if (k >= kf0 && kend <= kf1) {
+            uint8_t *tb = tbp + (int64_t)kb * (NG * WB);
+            // the last column's entry of the group's first row, and the rows it may be stored for
+            const int je0 = rs + kb - (c0 + SW - 1);
+            uint2 *entry = bnd_me + (je0 - jlo);
+            const bool entries = !last_strip && !A.walk && je0 + PUB > jlo && je0 <= jend;
+            if (full && ((k >= kf0 && kend <= kf1) || (k >= kz0 && kend <= kz1))) {
                 // interior: no tests inside the group
-#pragma unroll 1
-                for (; k < kend; ++k) {
-                    uint32_t in = __shfl_up_sync(FULL, carry, 1);
-                    const uint32_t b = __shfl_sync(FULL, bx, k & 31);
-                    if (lane == 0) in = b;
-                    int xs = sx8(in), vs = sx8(in >> 8), x2s = sx8(in >> 16);
-                    const uint32_t qc = in >> 24, sel = qc * 0x1111u + 0x8880u;
-                    uint32_t w0 = 0, w1 = 0, w2 = 0, w3 = 0;
-                    if (ARGMAX && !store_tb) {
-                        // no traceback is kept for this strip (a recomputed pair's first pass, or a
-                        // pair whose band empties): the cells without their state bytes
+                if (h_state == H_NONE) rebuild_h(k);
+                if (last_strip && h_state == H_LAST) h_from_last();
+                h_state = last_strip ? H_ALL : H_LAST;
+#pragma unroll 4
+                for (int i = 0; i < PUB; ++i) {
+                    uint32_t r0 = __shfl_up_sync(FULL, prmt(X[NP - 1], V[NP - 1], 0x7632), 1);
+                    uint32_t r1 = __shfl_up_sync(FULL, prmt(X2[NP - 1], sel[C - 1], 0x5432), 1);
+                    const uint32_t b0 = __shfl_sync(FULL, bx, (kb & 31) + i), b1 = __shfl_sync(FULL, by, (kb & 31) + i);
+                    if (lane == 0) r0 = b0, r1 = b1;
+                    uint32_t x = prmt(r0, X[NP - 1], 0x5410), v = prmt(r0, V[NP - 1], 0x5432), x2 = prmt(r1, X2[NP - 1], 0x5410);
+#pragma unroll
+                    for (int c = C - 1; c > 0; --c) sel[c] = sel[c - 1];
+                    sel[0] = r1 >> 16;
+                    uint32_t d[NP], d2[NP];
+#pragma unroll
+                    for (int p = NP - 1; p >= 0; --p) {
+                        uint32_t xp = p ? X[p - 1] : x, vp = p ? V[p - 1] : v, x2p = p ? X2[p - 1] : x2;
+                        SS[p] = score_of(p);
+                        cell2<MODE, true>(SS[p], xp, vp, x2p, U[p], Y[p], Y2[p], d[p], K);
+                        X[p] = xp, V[p] = vp, X2[p] = x2p;
+                        if (MODE == TRACKS) d[p] = vp >> 4, d2[p] = U[p] >> 4;
+                    }
+                    if (last_strip) {
+                        // H of the last column (all columns are kept here, for the last row)
 #pragma unroll
                         for (int c = 0; c < C; ++c) {
-                            int d = 0;
-                            ss[c] = prmt_sx(rlo[c], rhi[c], sel);
-                            cell<false, RIGHT>(ss[c], xs, vs, x2s, ut[c], yt[c], y2t[c], d, S);
-                            H[c] += vs;
+                            H[c] += fval(V[c % NP], c / NP);
+                            if (col0 + c == tm1) {
+                                const unsigned long long key = end_key(H[c], pm ^ (rs + kb + i - tm1));
+                                mte_key = key > mte_key ? key : mte_key;
+                            }
                         }
                     } else {
-#pragma unroll
-                        for (int c = 0; c < C; ++c) {
-                            int d = 0;
-                            ss[c] = prmt_sx(rlo[c], rhi[c], sel);
-                            cell<ARGMAX, RIGHT>(ss[c], xs, vs, x2s, ut[c], yt[c], y2t[c], d, S);
-                            H[c] += vs;
-                            if (ARGMAX) {
-                                if (c < 4) w0 |= (uint32_t)d << (8 * c);
-                                else w1 |= (uint32_t)d << (8 * (c - 4));
-                            } else if (ST) {
-                                if (c < 4) w0 |= (uint32_t)(vs & 0xff) << (8 * c), w2 |= (uint32_t)(ut[c] & 0xff) << (8 * c);
-                                else w1 |= (uint32_t)(vs & 0xff) << (8 * (c - 4)), w3 |= (uint32_t)(ut[c] & 0xff) << (8 * (c - 4));
-                            }
-                        }
-                        if (store_tb) {
-                            uint8_t *dst = tbp + (int64_t)k * (32 * CB);
-                            if (C == 8) {
-                                if (ST) __stcs(reinterpret_cast<uint4 *>(dst), make_uint4(w0, w1, w2, w3));
-                                else __stcs(reinterpret_cast<uint2 *>(dst), make_uint2(w0, w1));
-                            } else {
-                                if (ST) __stcs(reinterpret_cast<uint2 *>(dst), make_uint2(w0, w2));
-                                else __stcs(reinterpret_cast<uint32_t *>(dst), w0);
-                            }
-                        }
+                        H[C - 1] += fval(V[NP - 1], 1);
                     }
-                    carry = pack3(xs, vs, x2s, qc);
-                    Hcarry = H[C - 1];
-                    if (src_lane && k >= kf1 - 16) ring[warp][k & 15][lane] = carry;  // the wrap looks 16 rows back
-                    if (bnd_me) bnd_store(bnd_me + (jstart + k - 31 - jlo), carry & 0xffffffu, (uint32_t)Hcarry);
+                    if (CIGAR && store_tb) store_words(d, d2, tb + i * (NG * WB));
+                    if (entries && bnd_me) store_entry(entry + i);
                 }
-                __syncwarp();
                 continue;
             }
+            if (full && k >= kf0 && kend <= kl1) {
+                // the left edge alone: which lanes are computed, the first one's left input, and
+                // where the fill starts
+                if (h_state == H_NONE) rebuild_h(k);
+                h_state = H_LAST;
+#pragma unroll 2
+                for (int i = 0; i < PUB; ++i) {
+                    const int r = rs + kb + i, st0 = max((r - w + 1) >> 1, 0), st16 = st0 & ~15, stB = st0 & g.bmask;
+                    const uint32_t mine0 = prmt(X[NP - 1], V[NP - 1], 0x7632), mine1 = prmt(X2[NP - 1], sel[C - 1], 0x5432);
+                    uint32_t r0 = __shfl_up_sync(FULL, mine0, 1), r1 = __shfl_up_sync(FULL, mine1, 1);
+                    const uint32_t b0 = __shfl_sync(FULL, bx, (kb & 31) + i), b1 = __shfl_sync(FULL, by, (kb & 31) + i);
+                    const uint32_t x0 = __shfl_sync(FULL, mine0, (lane + D) & 31), x1 = __shfl_sync(FULL, mine1, (lane + D) & 31);
+                    if (lane == 0) r0 = b0, r1 = b1;
+#pragma unroll
+                    for (int c = C - 1; c > 0; --c) sel[c] = sel[c - 1];
+                    sel[0] = r1 >> 16;
+                    const bool wrap = col0 == stB && stB != st16;
+                    const bool fix = col0 == st16 && st16 > 0 && ((max((r - w) >> 1, 0)) & ~15) == st16;
+                    r0 = wrap ? x0 : fix ? prmt(x_in, v_in, 0x5410) : r0;
+                    r1 = wrap ? x1 : fix ? x2_in : r1;
+                    const uint32_t x = prmt(r0, X[NP - 1], 0x5410), v = prmt(r0, V[NP - 1], 0x5432), x2 = prmt(r1, X2[NP - 1], 0x5410);
+                    uint32_t d[NP], d2[NP];
+                    const int f0 = st0 - col0;
+#pragma unroll
+                    for (int p = 0; p < NP; ++p) {
+                        const uint32_t m = mask2(p >= f0, p + NP >= f0);
+                        SS[p] = (score_of(p) & m) | (SS[p] & ~m);
+                        d[p] = d2[p] = 0;
+                    }
+                    if (col0 >= stB) {
+#pragma unroll
+                        for (int p = NP - 1; p >= 0; --p) {
+                            uint32_t xp = p ? X[p - 1] : x, vp = p ? V[p - 1] : v, x2p = p ? X2[p - 1] : x2;
+                            cell2<MODE, true>(SS[p], xp, vp, x2p, U[p], Y[p], Y2[p], d[p], K);
+                            X[p] = xp, V[p] = vp, X2[p] = x2p;
+                            if (MODE == TRACKS) d[p] = vp >> 4, d2[p] = U[p] >> 4;
+                        }
+                        if (f0 < C) H[C - 1] += fval(V[NP - 1], 1);
+                    }
+                    if (CIGAR && store_tb) store_words(d, d2, tb + i * (NG * WB));
+                    if (entries && bnd_me && je0 + i <= jend) store_entry(entry + i);
+                }
+                continue;
+            }
+            if (full && k >= kr0 && kend <= kr1 && slot0 + k >= 0) {
+                // the right edge alone: which lanes are computed, and how far the fill reaches
+                h_state = H_NONE;
+#pragma unroll 2
+                for (int i = 0; i < PUB; ++i) {
+                    const int r = rs + kb + i, en0 = (r + w) >> 1, st0 = max(r - qm1, (r - w + 1) >> 1);
+                    const int f1 = (A.generic ? en0 : st0 + ((en0 - st0 + 16) & ~15) - 1) - col0;
+                    uint32_t r0 = __shfl_up_sync(FULL, prmt(X[NP - 1], V[NP - 1], 0x7632), 1);
+                    uint32_t r1 = __shfl_up_sync(FULL, prmt(X2[NP - 1], sel[C - 1], 0x5432), 1);
+                    const uint32_t b0 = __shfl_sync(FULL, bx, (kb & 31) + i), b1 = __shfl_sync(FULL, by, (kb & 31) + i);
+                    if (lane == 0) r0 = b0, r1 = b1;
+                    const uint32_t x = prmt(r0, X[NP - 1], 0x5410), v = prmt(r0, V[NP - 1], 0x5432), x2 = prmt(r1, X2[NP - 1], 0x5410);
+#pragma unroll
+                    for (int c = C - 1; c > 0; --c) sel[c] = sel[c - 1];
+                    sel[0] = r1 >> 16;
+                    uint32_t d[NP], d2[NP];
+#pragma unroll
+                    for (int p = 0; p < NP; ++p) {
+                        const uint32_t m = mask2(p <= f1, p + NP <= f1);
+                        SS[p] = (score_of(p) & m) | (SS[p] & ~m);
+                        d[p] = d2[p] = 0;
+                    }
+                    if (col0 <= (en0 | 15)) {
+#pragma unroll
+                        for (int p = NP - 1; p >= 0; --p) {
+                            uint32_t xp = p ? X[p - 1] : x, vp = p ? V[p - 1] : v, x2p = p ? X2[p - 1] : x2;
+                            cell2<MODE, true>(SS[p], xp, vp, x2p, U[p], Y[p], Y2[p], d[p], K);
+                            X[p] = xp, V[p] = vp, X2[p] = x2p;
+                            if (MODE == TRACKS) d[p] = vp >> 4, d2[p] = U[p] >> 4;
+                        }
+                    }
+                    if (CIGAR && store_tb) store_words(d, d2, tb + i * (NG * WB));
+                    if (entries && bnd_me && je0 + i >= jlo) store_entry(entry + i);
+                }
+                continue;
+            }
+            if (h_state == H_NONE) rebuild_h(k);
+            if (h_state == H_LAST) h_from_last();
+            h_state = H_ALL;
 #pragma unroll 1
             for (; k < kend; ++k) {
-                uint32_t in = __shfl_up_sync(FULL, carry, 1);
-                int Hl = __shfl_up_sync(FULL, Hcarry, 1);
-                const uint32_t b = __shfl_sync(FULL, bx, k & 31);
+                const int r = rs + k;
+                const uint32_t mine0 = prmt(X[NP - 1], V[NP - 1], 0x7632), mine1 = prmt(X2[NP - 1], sel[C - 1], 0x5432);
+                uint32_t r0 = __shfl_up_sync(FULL, mine0, 1), r1 = __shfl_up_sync(FULL, mine1, 1);
+                int Hl = __shfl_up_sync(FULL, H[C - 1], 1);
+                const uint32_t b0 = __shfl_sync(FULL, bx, k & 31), b1 = __shfl_sync(FULL, by, k & 31);
                 const int hb = __shfl_sync(FULL, bh, k & 31);
-                if (lane == 0) in = b, Hl = hb;
-                const int j = jstart + k - lane, r0 = col0 + j;
-                int xs = sx8(in), vs = sx8(in >> 8), x2s = sx8(in >> 16);
-                const uint32_t qc = in >> 24, sel = (j < 0 ? 0u : qc) * 0x1111u + 0x8880u;
-                const bool active = j >= jstart && j <= jend;
-                // Closed forms of the per-cell geometry over this lane-step (cell c: t = col0+c,
-                // r = r0+c, e = e0-c): in band <=> cB <= c <= cE; computed (stB <= t <= en16) <=>
-                // cRlo <= c <= cRhi; score filled <=> cB <= c <= fill0 (even c), fill1 (odd c).
-                const int e0 = j + w - col0, cB = j - w - col0;
-                const int cmax = min(tm1 - col0, rlim - 1 - r0), cE = min(e0, cmax);
-                const int cRlo = 2 * (F16 - col0) - cB - 2 * w;
-                const int cRhi = min(min(XB + qm1, 2 * XB + w) - r0, cmax);
-                // the rule for st0: r-qlen+1 once it is above (r-w+1)>>1, where the fill's length
-                // rounds up with the rows left below
-                const bool tail0 = r0 - qm1 > ((r0 - w + 1) >> 1), tail1 = r0 + C - 1 - qm1 > ((r0 + C - w) >> 1);
-                const bool corner = active && (j < 1 || j >= qm1 || (tail0 != tail1 && cRhi > cE));
-                uint32_t w0 = 0, w1 = 0, w2 = 0, w3 = 0;  // traceback bytes of this lane-step
-                if (!__any_sync(FULL, corner)) {
-                    if (active) {
-                        const int f = tail0 ? (A.generic ? 0 : 2 * ((qm1 - j) & 15)) : 0;
-                        const bool odd = e0 & 1;
-                        const int fill0 = e0 + (tail0 ? f : odd ? fill_odd : fill_even);
-                        const int fill1 = e0 + (tail0 ? f : odd ? fill_even : fill_odd);
-                        // the band-edge lane st16 and the block wrap stB can only be column col0 (c = 0)
-                        if (r0 < rlim) {
-                            const int st0 = g.st0(r0), st16 = st0 & ~15, stB = st0 & g.bmask;
-                            if (col0 == st16) {
-                                if (st16 == 0) xs = -S.qe, vs = edge_diff(j, S), x2s = -S.qe2;
-                                else if ((g.st0(r0 - 1) & ~15) == st16) xs = -S.qe, vs = -S.qe, x2s = -S.qe2;
-                            } else if (col0 == stB) {
-                                const uint32_t wv = ring[warp][(k + D) & 15][lane + D];
-                                xs = sx8(wv), vs = sx8(wv >> 8), x2s = sx8(wv >> 16);
+                if (lane == 0) r0 = b0, r1 = b1, Hl = hb;
+#pragma unroll
+                for (int c = C - 1; c > 0; --c) sel[c] = sel[c - 1];
+                sel[0] = r1 >> 16;
+                uint32_t d[NP], d2[NP];
+#pragma unroll
+                for (int p = 0; p < NP; ++p) d[p] = 0, d2[p] = 0;
+                if (r < rlim) {
+                    const int st0 = g.st0(r), en0 = g.en0(r);
+                    const int st16 = st0 & ~15, stB = st0 & g.bmask, en16 = en0 | 15;
+                    const int fe = A.generic ? en0 : st0 + ((en0 - st0 + 16) & ~15) - 1;
+                    if (stB != st16) {
+                        const uint32_t x0 = __shfl_sync(FULL, mine0, (lane + D) & 31), x1 = __shfl_sync(FULL, mine1, (lane + D) & 31);
+                        if (col0 == stB) r0 = x0, r1 = x1;
+                    }
+                    if (col0 == st16 && st16 > 0 && (g.st0(r - 1) & ~15) == st16)
+                        r0 = prmt(x_in, v_in, 0x5410), r1 = x2_in;
+                    uint32_t x = prmt(r0, X[NP - 1], 0x5410), v = prmt(r0, V[NP - 1], 0x5432), x2 = prmt(r1, X2[NP - 1], 0x5410);
+                    // score fill
+                    const int f0 = st0 - col0, f1 = fe - col0;
+                    if (f0 < C && f1 >= 0) {
+#pragma unroll
+                        for (int p = 0; p < NP; ++p) {
+                            const uint32_t m = mask2(p >= f0 && p <= f1, p + NP >= f0 && p + NP <= f1);
+                            SS[p] = (score_of(p) & m) | (SS[p] & ~m);
+                        }
+                    }
+                    if (col0 >= stB && col0 <= en16) {
+                        if (r < c0 + SW) {
+                            // row 0: the top edge above column r
+                            const uint32_t eu = rep2(16 * edge_diff(r, S) + FB);
+#pragma unroll
+                            for (int p = 0; p < NP; ++p) {
+                                const uint32_t m = mask2(col0 + p == r, col0 + p + NP == r);
+                                U[p] = (eu & m) | (U[p] & ~m);
+                                Y[p] = (K.kxb & m) | (Y[p] & ~m), Y2[p] = (K.kxb2 & m) | (Y2[p] & ~m);
                             }
                         }
-                        const int ctm = tm1 - col0;
+#pragma unroll
+                        for (int p = NP - 1; p >= 0; --p) {
+                            uint32_t xp = p ? X[p - 1] : x, vp = p ? V[p - 1] : v, x2p = p ? X2[p - 1] : x2;
+                            cell2<MODE, true>(SS[p], xp, vp, x2p, U[p], Y[p], Y2[p], d[p], K);
+                            X[p] = xp, V[p] = vp, X2[p] = x2p;
+                            if (MODE == TRACKS) d[p] = vp >> 4, d2[p] = U[p] >> 4;
+                        }
+                        // H inside the band: on its right edge from the left neighbour, else down
+                        const int b0c = st0 - col0, ce = en0 - col0;
+                        int hn[C];
 #pragma unroll
                         for (int c = 0; c < C; ++c) {
-                            const bool inBand = c >= cB && c <= cE;
-                            const bool inR = c >= cRlo && c <= cRhi;
-                            const bool fresh = c >= cB && c <= ((c & 1) ? fill1 : fill0);
-                            const int sc = prmt_sx(rlo[c], rhi[c], sel);
-                            ss[c] = fresh ? sc : ss[c];
-                            int uu = ut[c], yy = yt[c], yy2 = y2t[c], d = 0;
-                            cell<ARGMAX, RIGHT>(ss[c], xs, vs, x2s, uu, yy, yy2, d, S);
-                            // H[en0] = H[en0-1] + u on the right edge of the band, else H += v
-                            const bool re = (c >= e0 - 1 || c == ctm) && (c > 0 || col0 > 0);
-                            const int hn = re ? Hl + uu : H[c] + vs;
-                            H[c] = inBand ? hn : H[c];
-                            Hl = H[c];
-                            ut[c] = inR ? uu : ut[c], yt[c] = inR ? yy : yt[c], y2t[c] = inR ? yy2 : y2t[c];
-                            if (ARGMAX) {
-                                const uint32_t dd = inR ? (uint32_t)d : 0u;
-                                if (c < 4) w0 |= dd << (8 * c);
-                                else w1 |= dd << (8 * (c - 4));
-                            } else if (ST) {
-                                const uint32_t bv = inR ? (uint32_t)(vs & 0xff) : 0u, bu = inR ? (uint32_t)(uu & 0xff) : 0u;
-                                if (c < 4) w0 |= bv << (8 * c), w2 |= bu << (8 * c);
-                                else w1 |= bv << (8 * (c - 4)), w3 |= bu << (8 * (c - 4));
-                            }
-                            xs = inR ? xs : -S.qe, vs = inR ? vs : -S.qe, x2s = inR ? x2s : -S.qe2;
+                            const int down = H[c] + fval(V[c % NP], c / NP);
+                            const int across = (c ? H[c - 1] : Hl) + fval(U[c % NP], c / NP);
+                            hn[c] = c == ce ? across : down;
+                            hn[c] = c >= b0c && c <= ce ? hn[c] : H[c];
                         }
-                        if (last_strip) {
-                            // H of the last column in band: the largest, later rows on a tie
+                        if (en0 == 0 && col0 == 0) hn[0] = r ? H[0] + fval(V[0], 0) : fval(V[0], 0) - S.qe_pre;
 #pragma unroll
-                            for (int c = 0; c < C; ++c)
-                                if (c == ctm && c >= cB && c <= cE) {
-                                    const unsigned long long key = end_key(H[c], pm ^ j);
+                        for (int c = 0; c < C; ++c) H[c] = hn[c];
+                        if (r >= qm1 || (last_strip && en0 == tm1)) {
+                            // end tracking straight into the pair's record (rare cells; the packed
+                            // keys make the ">=" later-wins rule an unsigned max, and the strict
+                            // earlier-wins rule one on the mirrored position)
+                            const int cq = r - qm1 - col0, ctm = tm1 - col0;
+#pragma unroll
+                            for (int c = 0; c < C; ++c) {
+                                if (c < b0c || c > ce) continue;
+                                if (c == cq) {
+                                    atomicMax(&R->mqe_key, end_key(H[c], pm ^ (col0 + c)));
+                                    if (c == ctm) R->score = H[c], R->has_score = 1;
+                                }
+                                if (c == ctm) {
+                                    const unsigned long long key = end_key(H[c], pm ^ (r - tm1));
                                     mte_key = key > mte_key ? key : mte_key;
                                 }
-                        }
-                        carry = pack3(xs, vs, x2s, qc);
-                        Hcarry = Hl;
-                    }
-                } else if (active) {
-                    int fx = xs, fv = vs, fx2 = x2s, Hf = Hl;
-                    if (r0 < rlim && j >= 0) {
-                        const int st0 = g.st0(r0), st16 = st0 & ~15, stB = st0 & g.bmask;
-                        if (col0 == st16) {
-                            if (st16 == 0) fx = -S.qe, fv = edge_diff(j, S), fx2 = -S.qe2;
-                            else if ((g.st0(r0 - 1) & ~15) == st16) fx = -S.qe, fv = -S.qe, fx2 = -S.qe2;
-                        } else if (col0 == stB) {
-                            const uint32_t wv = ring[warp][(k + D) & 15][lane + D];
-                            fx = sx8(wv), fv = sx8(wv >> 8), fx2 = sx8(wv >> 16);
-                        }
-                    }
-                    const bool top = j == 0;
-#pragma unroll
-                    for (int c = 0; c < C; ++c) {
-                        const int t = col0 + c, r = r0 + c;
-                        if (t <= tm1 && r >= 0 && r < rlim) {
-                            const int st0 = g.st0(r), en0 = g.en0(r);
-                            const int fe = A.generic ? en0 : st0 + ((en0 - st0 + 16) & ~15) - 1;
-                            if (st0 <= t && t <= fe) ss[c] = prmt_sx(rlo[c], rhi[c], sel);
-                        }
-                        if (j < 0) continue;  // above the matrix: only the score fill of the reference runs here
-                        const bool inBand = c >= cB && c <= cE;
-                        const bool inR = c >= cRlo && c <= cRhi;
-                        int lx = fx, lv = fv, lx2 = fx2;
-                        int uu = top ? edge_diff(t, S) : ut[c];
-                        int yy = top ? -S.qe : yt[c], yy2 = top ? -S.qe2 : y2t[c];
-                        int d = 0;
-                        cell<ARGMAX, RIGHT>(ss[c], lx, lv, lx2, uu, yy, yy2, d, S);
-                        if (inR) ut[c] = uu, yt[c] = yy, y2t[c] = yy2;
-                        fx = inR ? lx : -S.qe, fv = inR ? lv : -S.qe, fx2 = inR ? lx2 : -S.qe2;
-                        const bool re = t == tm1 || top || c >= e0 - 1;
-                        const int hn = r == 0 ? lv - S.qe_pre : (re && t > 0) ? Hf + uu : H[c] + lv;
-                        if (inBand) {
-                            H[c] = hn;
-                            // end tracking straight into the pair's record (rare cells; the
-                            // packed keys make the ">=" later-wins rule an unsigned max, and
-                            // the strict earlier-wins rule one on the mirrored position)
-                            if (re && t == tm1) atomicMax(&R->mte_key, end_key(hn, pm ^ j));
-                            if (j == qm1) atomicMax(&R->mqe_key, end_key(hn, pm ^ t));
-                            if (j == qm1 && t == tm1) R->score = hn, R->has_score = 1;
-                        }
-                        if (ARGMAX) {
-                            const uint32_t dd = inR ? (uint32_t)d : 0u;
-                            if (c < 4) w0 |= dd << (8 * c);
-                            else w1 |= dd << (8 * (c - 4));
-                        } else if (ST) {
-                            const uint32_t bv = inR ? (uint32_t)(lv & 0xff) : 0u, bu = inR ? (uint32_t)(uu & 0xff) : 0u;
-                            if (c < 4) w0 |= bv << (8 * c), w2 |= bu << (8 * c);
-                            else w1 |= bv << (8 * (c - 4)), w3 |= bu << (8 * (c - 4));
-                        }
-                        Hf = H[c];
-                    }
-                    if (j < 0) fx = -S.qe, fv = -S.qe, fx2 = -S.qe2, Hf = H[C - 1];
-                    carry = pack3(fx, fv, fx2, qc);
-                    Hcarry = Hf;
-                }
-                if (active) {
-                    if (src_lane) ring[warp][k & 15][lane] = carry;
-                    if (j >= jlo) {
-                        if (store_tb) {
-                            uint8_t *dst = tbp + (int64_t)k * (32 * CB);
-                            if (C == 8) {
-                                if (ST) __stcs(reinterpret_cast<uint4 *>(dst), make_uint4(w0, w1, w2, w3));
-                                else __stcs(reinterpret_cast<uint2 *>(dst), make_uint2(w0, w1));
-                            } else {
-                                if (ST) __stcs(reinterpret_cast<uint2 *>(dst), make_uint2(w0, w2));
-                                else __stcs(reinterpret_cast<uint32_t *>(dst), w0);
                             }
                         }
-                        if (bnd_me) bnd_store(bnd_me + (j - jlo), carry & 0xffffffu, (uint32_t)Hcarry);
                     }
                 }
-                if (B > 16) __syncwarp();
+                if (CIGAR && store_tb && slot0 + k >= 0) store_words(d, d2, tb + (k - kb) * (NG * WB));
+                else if (CIGAR && store_tb) words.put(d), words2.put(d2);
+                const int je = r - (c0 + SW - 1);
+                if (bnd_me && je >= jlo && je <= jend) store_entry(bnd_me + (je - jlo));
             }
         }
         if (failed) break;
-        if (stopped) continue;
-        // the strip's final H, for the rows below its last one
-        if (bnd_me) bnd_store(bnd_me + (jend - jlo + 1), init_pack, (uint32_t)Hcarry);
-        if (mte_key) atomicMax(&R->mte_key, mte_key);
+        if (mte_key && !stopped) atomicMax(&R->mte_key, mte_key);
     }
 }
 
@@ -576,14 +617,14 @@ __device__ __forceinline__ int band_force(const Geom &g, int i, int j) {
     return i > (g.en0(r) | 15) ? 1 : i < (g.st0(r) & g.bmask) ? 2 : -1;
 }
 
-// The stored rows of a column group of a pair's strips (words of WB bytes).
-template <int WB, int NC>
+// The stored rows of a column group (4 columns) of a pair's strips (words of WB bytes).
+template <int WB>
 __device__ __forceinline__ TbGroup band_group(const BandStripDev *strips, const uint8_t *tb, int tlen, int col_lo,
                                               int gg) {
-    if (gg < 0 || gg * NC >= tlen || gg * NC < col_lo) return TbGroup{tb, 0, -1};
-    const BandStripDev St = strips[gg >> 5];
-    const int L = gg & 31;
-    return TbGroup{tb + St.tb_off + ((int64_t)L * 32 + L) * WB, St.jlo, St.jend};
+    if (gg < 0 || gg * 4 >= tlen || gg * 4 < col_lo) return TbGroup{tb, 0, -1};
+    const BandStripDev St = strips[gg / NG];
+    const int g = gg % NG;
+    return TbGroup{tb + St.tb_off + ((int64_t)4 * g * NG + g) * WB, St.jlo, St.jend};
 }
 
 // Warps per block of the finishing kernel: the Singletrack words are twice as large, and its
@@ -594,11 +635,11 @@ constexpr int fin_warps() { return ST ? 1 : 4; }
 // Result record of one pair, then ksw_backtrack (minimap2/ksw2.h:160-192) with the
 // off/off_end forcing of the band, or the Singletrack reconstruction
 // (minimap2/ksw2_singletrack.cpp:63-176); one warp per pair walks in runs (tb_walk.cuh).
-template <bool ST, int NC>
+template <bool ST>
 __global__ void __launch_bounds__(32 * fin_warps<ST>()) ksw_band_finish_kernel(BtArgs A) {
-    constexpr int WB = ST ? 2 * NC : NC;  // bytes per lane-word: NC columns (v then u for Singletrack)
-    using Window = TbWindow<WB, NC, ST ? 1 : 0, true>;
-    using Probe = TbWindow<WB, NC, 0, false>;  // the rows and columns of a Singletrack gap search
+    constexpr int WB = ST ? 8 : 4;
+    using Window = TbWindow<WB, 4, ST ? 1 : 0, true>;
+    using Probe = TbWindow<WB, 4, 0, false>;  // the rows and columns of a Singletrack gap search
     __shared__ __align__(16) uint8_t tiles[fin_warps<ST>()][Window::BYTES + (ST ? Probe::BYTES : 0)];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int pi = blockIdx.x * fin_warps<ST>() + warp;
@@ -632,8 +673,8 @@ __global__ void __launch_bounds__(32 * fin_warps<ST>()) ksw_band_finish_kernel(B
     const BandStripDev *strips = A.strips + P.strip0;
     const uint8_t *tb = A.tb;
     Window win;
-    win.init(tiles[warp], 32 * WB);
-    auto grp = [&](int gg) -> TbGroup { return band_group<WB, NC>(strips, tb, tlen, 0, gg); };
+    win.init(tiles[warp], NG * WB);
+    auto grp = [&](int gg) -> TbGroup { return band_group<WB>(strips, tb, tlen, 0, gg); };
     WarpCigar cg{A.cig + P.cig_off, 0, 0, 0};
     if (cigar && ST) {
         // ksw_extd2_singletrack_sse reconstructs whatever the EXTZ/SEMIGLOBAL flags
@@ -641,7 +682,7 @@ __global__ void __launch_bounds__(32 * fin_warps<ST>()) ksw_band_finish_kernel(B
         if (!o.zdropped && (sse_st || !(flag & (AW_EZ_EXTZ_ONLY | AW_EZ_SEMIGLOBAL_END)))) {
             const uint8_t *qs = A.qcodes + P.qoff, *ts = A.tcodes + P.toff;
             Probe probe;
-            probe.init(tiles[warp] + Window::BYTES, 32 * WB);
+            probe.init(tiles[warp] + Window::BYTES, NG * WB);
             int i = tlen - 1, j = qlen - 1;
             if (tb_singletrack(i, j, cg, win, probe, grp, [&](int a, int c) { return band_force(g, a, c); }, A.sc, A.mat,
                                A.m, qs, ts)) {
@@ -684,9 +725,8 @@ __global__ void __launch_bounds__(32 * fin_warps<ST>()) ksw_band_finish_kernel(B
 // walk through the group's freshly stored traceback until it leaves the group on the left
 // (or ends); in the pair's first group, close the walk (the leading gap, the reversal, the
 // CIGAR length).
-template <int NC>
 __global__ void __launch_bounds__(32) ksw_band_round_walk_kernel(BtArgs A, const BandGroupDev *groups) {
-    using Window = TbWindow<NC, NC, 0, true>;
+    using Window = TbWindow<4, 4, 0, true>;
     __shared__ __align__(16) uint8_t tiles[Window::BYTES];
     const BandGroupDev G = groups[blockIdx.x];
     const int slot = G.slot, col_lo = G.col_lo;
@@ -706,8 +746,8 @@ __global__ void __launch_bounds__(32) ksw_band_round_walk_kernel(BtArgs A, const
     const BandStripDev *strips = A.strips + P.strip0;
     const uint8_t *tb = A.tb;
     Window win;
-    win.init(tiles, 32 * NC);
-    auto grp = [&](int gg) -> TbGroup { return band_group<NC, NC>(strips, tb, tlen, col_lo, gg); };
+    win.init(tiles, NG * 4);
+    auto grp = [&](int gg) -> TbGroup { return band_group<4>(strips, tb, tlen, col_lo, gg); };
     WarpCigar cg{A.cig + P.cig_off, w.n, (uint32_t)w.op, w.len};
     int i = w.i, j = w.j, state = w.state;
     tb_walk(i, j, state, col_lo, cg, win, grp, [&](int a, int b) { return band_force(g, a, b); });
@@ -727,18 +767,11 @@ __global__ void __launch_bounds__(32) ksw_band_round_walk_kernel(BtArgs A, const
     }
 }
 
-template <bool CIGAR, bool RIGHT, bool ST>
-void *kernel_ptr() {
-    return (void *)ksw_band_kernel<CIGAR, RIGHT, ST, 8>;
-}
-
-void *band_kernel_for(int flag, int block) {
-    const bool cigar = !(flag & AW_EZ_SCORE_ONLY), right = !!(flag & AW_EZ_RIGHT);
-    const bool st = cigar && singletrack_tracks(flag, block);
-    if (st) return kernel_ptr<true, false, true>();
-    if (cigar && right) return kernel_ptr<true, true, false>();
-    if (cigar) return kernel_ptr<true, false, false>();
-    return kernel_ptr<false, false, false>();
+typedef void (*BandKernel)(BandArgs);
+BandKernel band_kernel_for(int flag, int block) {
+    if (flag & AW_EZ_SCORE_ONLY) return ksw_band_kernel<SCORES>;
+    if (singletrack_tracks(flag, block)) return ksw_band_kernel<TRACKS>;
+    return (flag & AW_EZ_RIGHT) ? ksw_band_kernel<RIGHTMOST> : ksw_band_kernel<LEFT>;
 }
 
 int64_t ceil_div(int64_t a, int64_t b) { return (a + b - 1) / b; }
@@ -783,14 +816,12 @@ int64_t band_cells(int qlen, int tlen, int w) {
 
 int band_plan_build(BandPlan &bp, const std::vector<int32_t> &ids, const std::vector<int> &qlen,
                     const std::vector<int> &tlen, const std::vector<int> &w, const std::vector<KswPair> &pairs,
-                    int flag, int block, int64_t tb_budget, int nc, std::vector<int32_t> *refused) {
+                    int flag, int block, int64_t tb_budget, std::vector<int32_t> *refused) {
     bp = BandPlan();
     bp.block = block;
-    bp.nc = nc == 4 ? 4 : 8;
-    const int SW = 32 * bp.nc;  // strip width
     const bool cigar = !(flag & AW_EZ_SCORE_ONLY);
     const bool st = cigar && singletrack_tracks(flag, block);
-    const int CB = st ? 2 * bp.nc : bp.nc;  // traceback bytes per lane-step
+    const int WB = st ? 8 : 4;  // bytes of a traceback word
     const int B = block;
     struct PairGeo {
         int32_t id, ww, rb;
@@ -809,16 +840,15 @@ int band_plan_build(BandPlan &bp, const std::vector<int32_t> &ids, const std::ve
         const int nd = ql + tl - 1;
         const int nstrip = (int)ceil_div(tl, SW);
         G.tb = 0, G.bnd = 0;
-        int64_t T = 0;
-        int prev_js = 0;
         for (int s = 0; s < nstrip; ++s) {
             const int c0 = s * SW;
             BandStripDev sd;
-            // rows the strip sweeps: from the first score-fill row of any of its columns
-            // (fills reach 15 past en0, so no earlier than c0-w-31, and no row above -15)
-            // to the last row where one of its columns is computed (stB <= t)
-            sd.jstart = (int)std::max<int64_t>(-15, (int64_t)c0 - ww - 32);
-            sd.jlo = std::max(0, sd.jstart);
+            // the strip's first anti-diagonal: the score fill reaches its first column (15 past
+            // en0 at most); jstart is the row of that column there
+            sd.jstart = (int)(std::max<int64_t>(std::max<int64_t>(0, c0 - 15), 2 * ((int64_t)c0 - 15) - ww) - c0);
+            // stored rows: from the first row of any of its columns that may be computed (no
+            // earlier than c0-w-32) to the last one that is (stB <= t)
+            sd.jlo = (int)std::max<int64_t>(0, (int64_t)c0 - ww - 32);
             int64_t jend = -1;
             for (int tg = c0; tg < std::min(c0 + SW, tl); tg += B) {
                 const int64_t X = (int64_t)tg + B - 1;
@@ -832,16 +862,13 @@ int band_plan_build(BandPlan &bp, const std::vector<int32_t> &ids, const std::ve
             sd.bnd_off = G.bnd;
             int64_t stb = 0;
             if (rows > 0) {
-                if (cigar) stb = (rows + 31) * 32 * CB;
+                if (cigar) stb = (rows + 4 * (NG - 1)) * NG * WB;
                 G.tb += stb;
-                G.bnd += rows + 1;
+                G.bnd += rows;
             }
             G.stb.push_back(stb);
-            // estimated start: the left strip must have swept this strip's first rows
-            T += (s == 0 ? 0 : std::max(0, sd.jstart - prev_js) + 64);
-            prev_js = sd.jstart;
             G.strips.push_back(sd);
-            G.start.push_back(T);
+            G.start.push_back((int64_t)sd.jstart + c0);  // its first step
         }
         G.tb = (G.tb + 255) / 256 * 256;
         if (G.rb < nd) {
@@ -1030,9 +1057,10 @@ int band_plan_build(BandPlan &bp, const std::vector<int32_t> &ids, const std::ve
     return 0;
 }
 
-int band_occupancy(int flag) {
+int band_occupancy(int flag, int block) {
     int nb = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, band_kernel_for(flag, 64), 256, 0) != cudaSuccess) return 1;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, band_kernel_for(flag, block), 32 * BAND_WARPS, 0) != cudaSuccess)
+        return 1;
     return std::max(nb, 1);
 }
 
@@ -1064,20 +1092,8 @@ cudaError_t band_launch_dp(const BandPlan &bp, int k, const BandDev &D, const ui
 }
 
 cudaError_t band_launch_units(const BandPlan &bp, const BandArgs &a, int flag, int ctas, cudaStream_t st) {
-    const bool cigar = !(flag & AW_EZ_SCORE_ONLY), right = !!(flag & AW_EZ_RIGHT);
-    const bool stk = cigar && singletrack_tracks(flag, bp.block);
-    const int grid = std::max(1, std::min(ctas, (a.n_units + 7) / 8));
-#define AW_BAND_LAUNCH(NCV)                                                                   \
-    if (stk) ksw_band_kernel<true, false, true, NCV><<<grid, 256, 0, st>>>(a);               \
-    else if (cigar && right) ksw_band_kernel<true, true, false, NCV><<<grid, 256, 0, st>>>(a); \
-    else if (cigar) ksw_band_kernel<true, false, false, NCV><<<grid, 256, 0, st>>>(a);        \
-    else ksw_band_kernel<false, false, false, NCV><<<grid, 256, 0, st>>>(a);
-    if (bp.nc == 4) {
-        AW_BAND_LAUNCH(4)
-    } else {
-        AW_BAND_LAUNCH(8)
-    }
-#undef AW_BAND_LAUNCH
+    const int grid = std::max(1, std::min(ctas, (a.n_units + BAND_WARPS - 1) / BAND_WARPS));
+    band_kernel_for(flag, bp.block)<<<grid, 32 * BAND_WARPS, 0, st>>>(a);
     return cudaGetLastError();
 }
 
@@ -1095,13 +1111,8 @@ cudaError_t band_launch_finish(const BandPlan &bp, int k, const BandDev &D, cons
     const bool stk = singletrack_tracks(flag, b.block) && !(flag & AW_EZ_SCORE_ONLY);
     const int fw = stk ? fin_warps<true>() : fin_warps<false>();
     const int grid = (W.npair + fw - 1) / fw;
-    if (bp.nc == 4) {
-        if (stk) ksw_band_finish_kernel<true, 4><<<grid, 32 * fw, 0, st>>>(b);
-        else ksw_band_finish_kernel<false, 4><<<grid, 32 * fw, 0, st>>>(b);
-    } else {
-        if (stk) ksw_band_finish_kernel<true, 8><<<grid, 32 * fw, 0, st>>>(b);
-        else ksw_band_finish_kernel<false, 8><<<grid, 32 * fw, 0, st>>>(b);
-    }
+    if (stk) ksw_band_finish_kernel<true><<<grid, 32 * fw, 0, st>>>(b);
+    else ksw_band_finish_kernel<false><<<grid, 32 * fw, 0, st>>>(b);
     return cudaGetLastError();
 }
 
@@ -1138,8 +1149,7 @@ cudaError_t band_launch_groups(const BandPlan &bp, int k, const BandDev &D, cons
         a.deadline = D.deadline;
         a.walk = D.walk;
         if ((e = band_launch_units(bp, a, flag, ctas, st)) != cudaSuccess) return e;
-        if (bp.nc == 4) ksw_band_round_walk_kernel<4><<<R.ngroup, 32, 0, st>>>(b, gd);
-        else ksw_band_round_walk_kernel<8><<<R.ngroup, 32, 0, st>>>(b, gd);
+        ksw_band_round_walk_kernel<<<R.ngroup, 32, 0, st>>>(b, gd);
         if ((e = cudaGetLastError()) != cudaSuccess) return e;
     }
     return cudaSuccess;

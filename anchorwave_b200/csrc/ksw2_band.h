@@ -18,14 +18,14 @@ struct BandPairDev {
     int32_t ckpt;           // 1: traceback too large for the budget; recomputed strip group by group
 };
 
-// One 256-column strip: the rows it sweeps and where its traceback and its right-edge
+// One strip: the anti-diagonals it sweeps and where its traceback and its right-edge
 // column (read by the next strip) live.
 struct BandStripDev {
     int64_t tb_off;   // bytes into the traceback arena (CIGAR modes)
     int64_t bnd_off;  // uint2 entries into the boundary arena
-    int32_t jstart;   // first row swept (may be negative: score-fill rows above the matrix)
-    int32_t jlo;      // first stored row, max(0, jstart)
-    int32_t jend;     // last row swept (< jlo: empty strip)
+    int32_t jstart;   // row of the strip's first column on its first anti-diagonal (may be negative)
+    int32_t jlo;      // first stored row
+    int32_t jend;     // last stored row (< jlo: empty strip)
     int32_t pad;
 };
 
@@ -83,7 +83,6 @@ struct BandPlan {
     std::vector<BandWave> waves;
     int64_t tb_cap = 0, bnd_cap = 0, tb_total = 0, cells = 0;
     int block = 64;
-    int nc = 8;  // target columns per lane: strips of 32*nc columns
 };
 
 // Geometry of the reference's band (ksw2_extd2_sse.c:147-154): the first anti-diagonal
@@ -100,7 +99,7 @@ int64_t band_cells(int qlen, int tlen, int w);
 // nullptr the build fails with AW_E_NOMEM_INTERNAL instead.
 int band_plan_build(BandPlan &bp, const std::vector<int32_t> &ids, const std::vector<int> &qlen,
                     const std::vector<int> &tlen, const std::vector<int> &w, const std::vector<KswPair> &pairs,
-                    int flag, int block, int64_t tb_budget, int nc, std::vector<int32_t> *refused);
+                    int flag, int block, int64_t tb_budget, std::vector<int32_t> *refused);
 
 struct BandDev {
     BandPairDev *pairs;
@@ -116,7 +115,7 @@ struct BandDev {
     const BandGroupDev *groups = nullptr;          // the group table of the recompute rounds
 };
 
-int band_occupancy(int flag);
+int band_occupancy(int flag, int block);
 
 // Enqueues wave k's counter resets and DP kernel.
 cudaError_t band_launch_dp(const BandPlan &bp, int k, const BandDev &D, const uint8_t *qcodes,

@@ -284,7 +284,7 @@ class deadline:
 
 
 def set_band_columns(columns: int = 0):
-    """Target columns per lane of the banded kernel: 4, 8, or 0 to choose per batch."""
+    """Formerly the banded kernel's target columns per lane; accepted without effect."""
     lib.aw_set_band_columns(int(columns))
 
 

@@ -419,8 +419,8 @@ void aw_set_traceback_budget(int64_t bytes);
  * unless large_warps is 1, and small batches always run on narrow strips, one warp each
  * (autotuner knobs; 0 keeps the current value).  Results are identical. */
 void aw_set_tuning(int large_warps, int large_tlen_threshold);
-/* Target columns per lane of the banded kernel (4 or 8; 0 = chosen per batch from
- * its work and its longest pair).  No counterpart in the reference (tuning knob). */
+/* Formerly the target columns per lane of the banded kernel (4, 8, or 0 to choose per batch): one
+ * width is now the faster one for every batch, and the setting is accepted without effect. */
 void aw_set_band_columns(int columns);
 /* 1 (default): a full-matrix pair that would be its batch's critical path (a long interval
  * alone or among short ones) and whose traceback exceeds the HBM traceback budget runs on the
