@@ -91,6 +91,19 @@ __device__ __forceinline__ int64_t pool_grab(const Pool &A, int64_t bytes) {
     return (int64_t)b;
 }
 
+// The same, but `bytes` becomes what is left of the pool if that is less, down to `least`.
+__device__ __noinline__ int64_t pool_grab_rest(Pool A, int64_t &bytes, int64_t least) {
+    for (int i = 0; i < 64; ++i) {
+        const int64_t h = *(volatile int64_t *)&A.ctl->head;
+        const int64_t len = min(bytes, (A.bytes - h) & ~(int64_t)255);
+        if (len < least) return -1;
+        if (atomicCAS(&A.ctl->head, (unsigned long long)h, (unsigned long long)(h + len)) != (unsigned long long)h) continue;
+        bytes = len;
+        return h;
+    }
+    return pool_grab(A, bytes);
+}
+
 // A chunk of a finished pair, or -1.  The ring holds `avail` complete entries; the entry at the
 // taken position may still be on its way from the thread that reserved it, hence the wait.
 __device__ __forceinline__ int64_t free_pop(const Pool &A) {
@@ -179,6 +192,7 @@ struct HdrRing {
     __device__ __forceinline__ void put(int c, int sc, const CompHdr &h) const {
         if (sh.mm >= 0) *at(c, sc) = h;
     }
+    __device__ __forceinline__ int mask(int c) const { return c == CM ? sh.mm : c <= CD1 ? sh.m1 : sh.m2; }
 };
 
 __device__ __forceinline__ int32_t getv(const WfaArgs &A, const CompHdr &h, int k) {
@@ -198,8 +212,14 @@ __device__ __forceinline__ InHdr in_hdr(const WfaArgs &A, const CompHdr &h) {
 __device__ __forceinline__ int32_t getv(const InHdr &h, int k) {
     return (k < h.lo || k > h.hi) ? WF_NULL : h.p[k];
 }
-__device__ __forceinline__ int32_t getv_l2(const InHdr &h, int k) {
-    return (k < h.lo || k > h.hi) ? WF_NULL : __ldcg(h.p + k);
+// The same as a predicated load, so that a lane's loads from several inputs are in flight together.
+__device__ __forceinline__ int32_t getv_pred(const InHdr &h, int k) {
+    int32_t r;
+    const int ok = k >= h.lo && k <= h.hi;
+    asm volatile("{ .reg .pred q; setp.ne.s32 q, %2, 0; mov.b32 %0, %3; @q ld.global.b32 %0, [%1]; }"
+                 : "=r"(r)
+                 : "l"(h.p + k), "r"(ok), "n"(WF_NULL));
+    return r;
 }
 
 // A piggyback cell: offset, packed CIGAR, link.  In a ring slot the three arrays of a
@@ -224,13 +244,27 @@ __device__ __forceinline__ uint64_t load8(const uint8_t *base, int64_t pos) {
 }
 
 // 32 bases from base g of a 2-bit arena (base i at bits 2*(i%32) of word i/32); the arena
-// ends with a spare word.
-__device__ __forceinline__ uint64_t load32b(const uint64_t *p, int64_t g) {
-    const int64_t w = g >> 5;
-    const int sh = (int)(g & 31) * 2;
-    const uint64_t lo = __ldg(p + w);
-    if (!sh) return lo;
-    return (lo >> sh) | (__ldg(p + w + 1) << (64 - sh));
+// ends with a spare word.  SH: the words lie in shared memory.
+template <bool SH = false>
+__device__ __forceinline__ uint64_t load32b(const uint64_t *p, int g) {
+    const int w = g >> 5, sh = (g & 31) * 2;
+    const uint64_t lo = SH ? p[w] : __ldg(p + w), hi = SH ? p[w + 1] : __ldg(p + w + 1);
+    return (lo >> sh) | ((hi << 1) << (63 - sh));
+}
+// 16 bases from base g, read as 32-bit words.
+template <bool SH>
+__device__ __forceinline__ uint32_t load16b(const uint32_t *p, int g) {
+    const int w = g >> 4;
+    return __funnelshift_r(SH ? p[w] : __ldg(p + w), SH ? p[w + 1] : __ldg(p + w + 1), 2 * g);
+}
+// A pair's sequences at 2 bits a base: the words that hold their first bases, and the places
+// of those bases in them.
+struct Bases {
+    const uint64_t *p, *t;
+    int po, to;
+};
+__device__ __forceinline__ Bases bases_of(const WfaArgs &A, const WfaPairDev &PR) {
+    return Bases{A.ppat + (PR.poff >> 5), A.ptxt + (PR.toff >> 5), (int)(PR.poff & 31), (int)(PR.toff & 31)};
 }
 
 __device__ __forceinline__ bool in_matrix(int32_t o, int k, int plen, int tlen) {
@@ -245,8 +279,9 @@ __device__ int64_t lcp1(const WfaArgs &A, const WfaPairDev &PR, const uint8_t *p
     if (rem <= 0) return 0;
     int64_t n = 0;
     if (PR.packed) {
+        const Bases B = bases_of(A, PR);
         for (;;) {
-            const uint64_t x = load32b(A.ppat, PR.poff + v + n) ^ load32b(A.ptxt, PR.toff + h + n);
+            const uint64_t x = load32b(B.p, B.po + (int)(v + n)) ^ load32b(B.t, B.to + (int)(h + n));
             n += x ? (int64_t)((__ffsll((long long)x) - 1) >> 1) : 32;
             if (x || n >= rem) return min(n, rem);
         }
@@ -286,43 +321,46 @@ __device__ __forceinline__ bool any_of(const bool (&r)[N]) {
     return a;
 }
 
-template <int N>
-__device__ __forceinline__ void extend_n(const WfaArgs &A, const WfaPairDev &PR, const uint8_t *pat,
-                                         const uint8_t *txt, int k0, int stride, int32_t (&o)[N]) {
+template <int N, bool SH = false>
+__device__ __forceinline__ void extend_n(const WfaPairDev &PR, const Bases &B, const uint8_t *pat, const uint8_t *txt,
+                                         int k0, int stride, int32_t (&o)[N]) {
     // o[u] is the text position h; the pattern position is h - k
     const int plen = PR.plen, tlen = PR.tlen;
     bool run[N];
 #pragma unroll
     for (int u = 0; u < N; ++u) run[u] = o[u] != WF_NULL;
-    bool any = any_of(run);
     if (PR.packed) {
-        // 32 bases per XOR; the run ends at the first differing base or at the end of either
-        // sequence (the sentinels of the byte path)
+        // the run ends at the first differing base or at the end of either sequence (the
+        // sentinels of the byte path).  The first round compares 16 bases, in 32-bit words: most
+        // runs are shorter; the others compare 32
+        int rem[N];
+        const uint32_t *wp = (const uint32_t *)B.p, *wt = (const uint32_t *)B.t;
 #pragma unroll
-        for (int u = 0; u < N; ++u)
-            if (run[u] && min(plen - (o[u] - (k0 + stride * u)), tlen - o[u]) <= 0) run[u] = false;
-        any = any_of(run);
-        while (any) {
+        for (int u = 0; u < N; ++u) {
+            rem[u] = min(plen + (k0 + stride * u), tlen) - o[u];
+            run[u] = run[u] && rem[u] > 0;
+            uint32_t x = 1;
+            if (run[u])
+                x = load16b<SH>(wp, B.po + (o[u] - (k0 + stride * u))) ^ load16b<SH>(wt, B.to + o[u]);
+            const int nb = run[u] ? min(__clz((int)__brev(x)) >> 1, rem[u]) : 0;
+            o[u] += nb, rem[u] -= nb;
+            run[u] = nb == 16 && rem[u] > 0;
+        }
+        while (any_of(run)) {
             uint64_t x[N];
 #pragma unroll
             for (int u = 0; u < N; ++u)
-                x[u] = run[u] ? (load32b(A.ppat, PR.poff + (o[u] - (k0 + stride * u))) ^ load32b(A.ptxt, PR.toff + o[u]))
-                              : 0;
-            any = false;
+                x[u] = run[u] ? load32b<SH>(B.p, B.po + (o[u] - (k0 + stride * u))) ^ load32b<SH>(B.t, B.to + o[u]) : 1;
 #pragma unroll
             for (int u = 0; u < N; ++u) {
-                if (!run[u]) continue;
-                const int rem = min(plen - (o[u] - (k0 + stride * u)), tlen - o[u]);
-                int nb = x[u] ? (__ffsll((long long)x[u]) - 1) >> 1 : 32;
-                const bool stop = x[u] != 0 || nb >= rem;
-                if (nb > rem) nb = rem;
-                o[u] += nb;
-                if (stop || rem == nb) run[u] = false;
-                else any = true;
+                const int nb = run[u] ? min(__clzll((long long)__brevll(x[u])) >> 1, rem[u]) : 0;
+                o[u] += nb, rem[u] -= nb;
+                run[u] = nb == 32 && rem[u] > 0;
             }
         }
         return;
     }
+    bool any = any_of(run);
     while (any) {
         uint64_t x[N];
 #pragma unroll
@@ -592,7 +630,7 @@ __device__ __forceinline__ bool pig_trip(const WfaArgs &A, const WfaPairDev &PR,
         int32_t mo[PIG_U];
 #pragma unroll
         for (int u = 0; u < PIG_U; ++u) mo[u] = k0 + G * u <= hi ? C[u][CM].o : WF_NULL;
-        extend_n<PIG_U>(A, PR, pat, txt, k0, G, mo);
+        extend_n<PIG_U>(PR, bases_of(A, PR), pat, txt, k0, G, mo);
 #pragma unroll
         for (int u = 0; u < PIG_U; ++u) {
             const int k = k0 + G * u;
@@ -654,6 +692,8 @@ enum { WOP_COMPUTE = 0, WOP_DONE = 1, WOP_EXIT = 2 };
 
 struct WidePlan {
     int op, lo, hi, mask;  // mask: components allocated at the planned score (bit c)
+    int ilo, ihi;          // the diagonals that every input has; ilo > ihi unless mask is full
+    int s;                 // the planned score (cluster kernel)
     CompHdr in[7];         // M[s-x], M[s-o1-e1], I1[s-e1], D1[s-e1], M[s-o2-e2], I2[s-e2], D2[s-e2]
     CompHdr out[5];
     InHdr view[7];         // the same inputs as the compute step of the high memory modes reads them
@@ -708,6 +748,13 @@ __device__ __forceinline__ void plan_limits(const PlanLane &L, int lane, const C
     if (some & (1u << 4 | 1u << 6)) mask |= 1 << CD2;
 }
 
+// The diagonals that all seven inputs have, if every component is an output.
+__device__ __forceinline__ void plan_inner(WidePlan &q, int mask, int lane, const CompHdr &h) {
+    const int ilo = __reduce_max_sync(0xffffffffu, lane < 7 ? h.lo : INT_MIN);
+    const int ihi = __reduce_min_sync(0xffffffffu, lane < 7 ? h.hi : INT_MAX);
+    if (lane == 0) q.ilo = ilo, q.ihi = mask == 31 ? ihi : ilo - 1;
+}
+
 // A warp's trimmed ends and end check, folded into its CTA's partials.
 __device__ __forceinline__ void fold_partials(const int (&kmin)[5], const int (&kmax)[5], bool reached, WidePart &pp) {
     const int lane = threadIdx.x & 31;
@@ -735,69 +782,156 @@ __device__ __forceinline__ int64_t pig_slot(int c, int sc, int SR, int R1, int R
 #define AW_WFA_CTA_U 2
 #endif
 
-// One thread's diagonals lo + g0 + G*u of a planned score (high memory): the compute step,
-// the fused extension of M, the stores, and this thread's trimmed ends and end check, folded
-// per warp into the CTA's partials.  `ld_l2` reads the inputs through L2 (other CTAs wrote them).
-template <bool L2>
-__device__ __forceinline__ void plan_compute(const WfaArgs &A, const WfaPairDev &PR, const uint8_t *pat,
-                                             const uint8_t *txt, const WidePlan &Q, int g0, int G, WidePart &pp) {
-    const int plen = PR.plen, tlen = PR.tlen, k_end = tlen - plen;
-    const int lo = Q.lo, hi = Q.hi;
-    if (lo + (g0 & ~31) > hi) return;  // no diagonal for this warp
-    const InHdr m_misms = Q.view[0], m_open1 = Q.view[1], i1 = Q.view[2], d1 = Q.view[3], m_open2 = Q.view[4],
-                i2 = Q.view[5], d2 = Q.view[6];
-    int32_t *oM = Q.dst[CM], *oI1 = Q.dst[CI1], *oD1 = Q.dst[CD1], *oI2 = Q.dst[CI2], *oD2 = Q.dst[CD2];
+// U diagonals k0 + G*u <= hi of one thread (high memory): the compute step, the fused extension
+// of M, the stores, this thread's trimmed ends (TRIM), and whether it met the end cell or an
+// offset beyond the end of a sequence.  v: the inputs; dst[c]: where component c's diagonal lo
+// goes (null: nowhere).  INNER: every input has the diagonals k-1 .. k+1, and all components are
+// stored; without GUARD no k is beyond hi either.  A trip is bound by its instructions and
+// their latencies (few warps per SM): G is known at build time so that a trip's diagonals
+// differ by an immediate, and as a real offset is never negative, nor before the start of a
+// sequence, one compare with the diagonal's length puts an offset inside the matrix.
+template <int U, int G, bool INNER, bool GUARD, bool TRIM, bool SH>
+__device__ __forceinline__ void wf_trip(const WfaPairDev &PR, const Bases &B, const uint8_t *pat, const uint8_t *txt,
+                                        const InHdr (&v)[7], int32_t *const (&dst)[5], int lo, int hi, int k0,
+                                        int (&kmin)[5], int (&kmax)[5], bool &reached, bool &beyond) {
+    int32_t g[U][4], misms[U], mo[U];  // I1, D1, I2, D2
+    int32_t *to[5];
+#pragma unroll
+    for (int c = 0; c < 5; ++c) to[c] = INNER || dst[c] ? dst[c] + (k0 - lo) : nullptr;
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+        const int k = k0 + G * u;
+        auto in = [&](int j, int d) -> int32_t {
+            if constexpr (!INNER) return getv_pred(v[j], k + d);
+            else return !GUARD || k <= hi ? (v[j].p + k0)[G * u + d] : WF_NULL;
+        };
+        g[u][0] = max(in(1, -1), in(2, -1)) + 1;
+        g[u][1] = max(in(1, 1), in(3, 1));
+        g[u][2] = max(in(4, -1), in(5, -1)) + 1;
+        g[u][3] = max(in(4, 1), in(6, 1));
+        misms[u] = in(0, 0) + 1;
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+        const int k = k0 + G * u;
+        const bool here = !GUARD || k <= hi;
+        // offsets 0 .. lim - 1 lie in the matrix
+        const uint32_t lim = here ? (uint32_t)max(min(PR.tlen, k + PR.plen) + 1, 0) : 0u;
+        const int32_t gap = max(max(g[u][0], g[u][1]), max(g[u][2], g[u][3]));
+        const int32_t best = max(gap, misms[u]);
+        mo[u] = (uint32_t)best < lim ? best : WF_NULL;
+        if (here && gap >= (int32_t)lim) beyond = true;
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+            if (here && (INNER || to[c + 1])) to[c + 1][G * u] = g[u][c];
+            if (TRIM && (uint32_t)g[u][c] < lim) kmin[c + 1] = min(kmin[c + 1], k), kmax[c + 1] = max(kmax[c + 1], k);
+        }
+        if (TRIM && (uint32_t)best < lim) kmin[CM] = min(kmin[CM], k), kmax[CM] = max(kmax[CM], k);
+    }
+    extend_n<U, SH>(PR, B, pat, txt, k0, G, mo);
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+        const int k = k0 + G * u;
+        if (GUARD && k > hi) break;
+        if (k == PR.tlen - PR.plen && mo[u] >= PR.tlen) reached = true;
+        to[CM][G * u] = mo[u];
+    }
+}
+
+// The trip whose first lane has diagonal kw, with or without checks.
+template <int U, int G, bool SH>
+__device__ __forceinline__ void plan_trip(const WfaPairDev &PR, const Bases &B, const uint8_t *pat, const uint8_t *txt,
+                                          const WidePlan &Q, int kw, int lane, int (&kmin)[5], int (&kmax)[5],
+                                          bool &reached, bool &beyond) {
+    if (kw > Q.ilo && kw + 31 + G * (U - 1) < Q.ihi)
+        wf_trip<U, G, true, false, true, SH>(PR, B, pat, txt, Q.view, Q.dst, Q.lo, Q.hi, kw + lane, kmin, kmax, reached, beyond);
+    else if (kw <= Q.hi)
+        wf_trip<U, G, false, true, true, SH>(PR, B, pat, txt, Q.view, Q.dst, Q.lo, Q.hi, kw + lane, kmin, kmax, reached, beyond);
+}
+
+// The diagonals of a planned score (high memory) of one warp of CTA `rank` of CL, each CTA with G
+// computing threads, folded into the CTA's partials.  The wavefront is taken in rounds of
+// CL*G*U diagonals, with the fewest diagonals per thread that end it: narrow ones are spread over
+// all threads.  Returns, for the warp, 1 when the end cell was reached, plus 2 when a gap
+// component got an offset beyond the end of a sequence.
+template <int UMAX, int G, bool SH>
+__device__ __forceinline__ int plan_compute(const WfaPairDev &PR, const Bases &B, const uint8_t *pat,
+                                            const uint8_t *txt, const WidePlan &Q, int rank, int CL, WidePart &pp) {
+    const int lane = threadIdx.x & 31, w0 = threadIdx.x & ~31;
     int kmin[5], kmax[5];
-    bool reached = false;
+    bool reached = false, beyond = false, any = false;
 #pragma unroll
     for (int c = 0; c < 5; ++c) kmin[c] = INT_MAX, kmax[c] = INT_MIN;
-    constexpr int U = L2 ? 4 : AW_WFA_CTA_U;
-    for (int k0 = lo + g0; k0 <= hi; k0 += G * U) {
-        int32_t ins1[U], ins2[U], del1[U], del2[U], misms[U];
-#pragma unroll
-        for (int u = 0; u < U; ++u) {
-            const int k = k0 + G * u;
-            if constexpr (L2) {
-                ins1[u] = max(getv_l2(m_open1, k - 1), getv_l2(i1, k - 1)) + 1;
-                ins2[u] = max(getv_l2(m_open2, k - 1), getv_l2(i2, k - 1)) + 1;
-                del1[u] = max(getv_l2(m_open1, k + 1), getv_l2(d1, k + 1));
-                del2[u] = max(getv_l2(m_open2, k + 1), getv_l2(d2, k + 1));
-                misms[u] = getv_l2(m_misms, k) + 1;
-            } else {
-                ins1[u] = max(getv(m_open1, k - 1), getv(i1, k - 1)) + 1;
-                ins2[u] = max(getv(m_open2, k - 1), getv(i2, k - 1)) + 1;
-                del1[u] = max(getv(m_open1, k + 1), getv(d1, k + 1));
-                del2[u] = max(getv(m_open2, k + 1), getv(d2, k + 1));
-                misms[u] = getv(m_misms, k) + 1;
-            }
+    for (int kb = Q.lo; kb <= Q.hi;) {
+        const int left = Q.hi - kb + 1, round = CL * G;
+        const int U = UMAX >= 4 && left > 2 * round ? 4 : UMAX >= 2 && left > round ? 2 : 1;
+        const int kw = kb + rank * G * U + w0;
+        any |= kw <= Q.hi;
+        if (UMAX >= 4 && U == 4) plan_trip<4, G, SH>(PR, B, pat, txt, Q, kw, lane, kmin, kmax, reached, beyond);
+        else if (UMAX >= 2 && U == 2) plan_trip<2, G, SH>(PR, B, pat, txt, Q, kw, lane, kmin, kmax, reached, beyond);
+        else plan_trip<1, G, SH>(PR, B, pat, txt, Q, kw, lane, kmin, kmax, reached, beyond);
+        kb += round * U;
+    }
+    if (!any) return 0;  // no diagonal for this warp
+    fold_partials(kmin, kmax, reached, pp);
+    return (__any_sync(0xffffffffu, reached) ? 1 : 0) | (__any_sync(0xffffffffu, beyond) ? 2 : 0);
+}
+
+// The same without trimmed ends, for the cluster kernel's CTAs of G + 32 computing threads: G of
+// them take the diagonals that every input has; the few on either side, with their checks, are
+// the work of the last warp of the first and of the last CTA.
+template <int G, bool SH>
+__device__ __forceinline__ int plan_open(const WfaPairDev &PR, const Bases &B, const uint8_t *pat, const uint8_t *txt,
+                                         const WidePlan &Q, int rank, int CL) {
+    const int lane = threadIdx.x & 31, w0 = threadIdx.x & ~31;
+    int kmin[5], kmax[5];  // not used
+    bool reached = false, beyond = false;
+    const int first = Q.ilo + 1, last = Q.ihi - 1;
+    if (last - first < 64) {
+        for (int kw = Q.lo + rank * (G + 32) + w0; kw <= Q.hi; kw += CL * (G + 32))
+            wf_trip<1, G, false, true, false, SH>(PR, B, pat, txt, Q.view, Q.dst, Q.lo, Q.hi, kw + lane, kmin, kmax,
+                                                  reached, beyond);
+    } else if (w0 == G) {
+        for (int side = 0; side < 2; ++side) {
+            if (rank != (side ? CL - 1 : 0)) continue;
+            const int end = side ? Q.hi : first - 1;
+            for (int kw = side ? last + 1 : Q.lo; kw <= end; kw += 32)
+                wf_trip<1, G, false, true, false, SH>(PR, B, pat, txt, Q.view, Q.dst, Q.lo, end, kw + lane, kmin, kmax,
+                                                      reached, beyond);
         }
-        int32_t mo[U];
-#pragma unroll
-        for (int u = 0; u < U; ++u) {
-            const int k = k0 + G * u;
-            const int32_t best = max(max(del1[u], del2[u]), max(misms[u], max(ins1[u], ins2[u])));
-            mo[u] = (k <= hi && in_matrix(best, k, plen, tlen)) ? best : WF_NULL;
-            if (k > hi) continue;
-            if (oI1) oI1[k - lo] = ins1[u];
-            if (oD1) oD1[k - lo] = del1[u];
-            if (oI2) oI2[k - lo] = ins2[u];
-            if (oD2) oD2[k - lo] = del2[u];
-            const int32_t vals[4] = {ins1[u], del1[u], ins2[u], del2[u]};
-#pragma unroll
-            for (int c = 0; c < 4; ++c)
-                if (in_matrix(vals[c], k, plen, tlen)) kmin[c + 1] = min(kmin[c + 1], k), kmax[c + 1] = max(kmax[c + 1], k);
-            if (mo[u] != WF_NULL) kmin[CM] = min(kmin[CM], k), kmax[CM] = max(kmax[CM], k);
-        }
-        extend_n<U>(A, PR, pat, txt, k0, G, mo);
-#pragma unroll
-        for (int u = 0; u < U; ++u) {
-            const int k = k0 + G * u;
-            if (k > hi) break;
-            if (k == k_end && mo[u] != WF_NULL && mo[u] >= tlen) reached = true;
-            oM[k - lo] = mo[u];
+    } else {
+        for (int kb = first; kb <= last;) {
+            const int left = last - kb + 1, round = CL * G;
+            const int U = left > 2 * round ? 4 : left > round ? 2 : 1;
+            const int kw = kb + rank * G * U + w0;
+            if (kw > last) break;
+            if (U == 4)
+                wf_trip<4, G, true, true, false, SH>(PR, B, pat, txt, Q.view, Q.dst, Q.lo, last, kw + lane, kmin, kmax,
+                                                     reached, beyond);
+            else if (U == 2)
+                wf_trip<2, G, true, true, false, SH>(PR, B, pat, txt, Q.view, Q.dst, Q.lo, last, kw + lane, kmin, kmax,
+                                                     reached, beyond);
+            else
+                wf_trip<1, G, true, true, false, SH>(PR, B, pat, txt, Q.view, Q.dst, Q.lo, last, kw + lane, kmin, kmax,
+                                                     reached, beyond);
+            kb += round * U;
         }
     }
-    fold_partials(kmin, kmax, reached, pp);
+    return (__any_sync(0xffffffffu, reached) ? 1 : 0) | (__any_sync(0xffffffffu, beyond) ? 2 : 0);
+}
+
+// The trimmed ends of a computed score, from its stored offsets, folded into the CTA's partials.
+__device__ __noinline__ void plan_trim(const WfaPairDev &PR, const WidePlan &Q, int g0, int G, WidePart &pp) {
+    int kmin[5], kmax[5];
+#pragma unroll
+    for (int c = 0; c < 5; ++c) kmin[c] = INT_MAX, kmax[c] = INT_MIN;
+    for (int k = Q.lo + g0; k <= Q.hi; k += G) {
+#pragma unroll
+        for (int c = 0; c < 5; ++c)
+            if (Q.dst[c] && in_matrix(Q.dst[c][k - Q.lo], k, PR.plen, PR.tlen)) kmin[c] = min(kmin[c], k), kmax[c] = max(kmax[c], k);
+    }
+    __syncwarp();
+    fold_partials(kmin, kmax, false, pp);
 }
 
 // CTA-cooperative mode: one long pair on all threads of a CTA.  Warp 0 plans every score, a
@@ -814,10 +948,10 @@ struct CtaPlanner {  // warp 0's state (shared memory)
     int rcap, pad;
     Alloc al;
 };
-template <bool PIG>
+template <bool PIG, int NT>
 __device__ void cta_pair(const WfaArgs &A, int idx, const HdrRing &HR, WidePlan &plan, WidePart &part, CtaPlanner &Q,
                          Alloc &wal) {
-    const int tid = threadIdx.x, NT = blockDim.x, lane = tid & 31;
+    const int tid = threadIdx.x, lane = tid & 31;
     const WfaPen P = A.pen;
     const WfaPairDev PR = A.pairs[idx];
     const int plen = PR.plen, tlen = PR.tlen;
@@ -921,6 +1055,7 @@ __device__ void cta_pair(const WfaArgs &A, int idx, const HdrRing &HR, WidePlan 
                 if (lane < 7) plan.in[lane] = in;
             } else {
                 if (lane < 7) plan.view[lane] = in_hdr(A, in);
+                plan_inner(plan, mask, lane, in);
                 if (lane < 5) plan.dst[lane] = mine ? (int32_t *)(A.pool + out.off) : nullptr;
             }
             if (lane < 5) plan.out[lane] = out;
@@ -989,7 +1124,7 @@ __device__ void cta_pair(const WfaArgs &A, int idx, const HdrRing &HR, WidePlan 
             fold_partials(kmin, kmax, reached, part);
             if (!ok && lane == 0) part.retry = 1;
         } else {
-            plan_compute<false>(A, PR, pat, txt, plan, tid, NT, part);
+            plan_compute<AW_WFA_CTA_U, NT, false>(PR, bases_of(A, PR), pat, txt, plan, 0, 1, part);
         }
         __syncthreads();
         if (tid < 32) {
@@ -1056,7 +1191,7 @@ __global__ void __launch_bounds__(NT, AW_WFA_MINB * WFA_CTA / NT) wfa_kernel(Wfa
             const int pi = cpi;
             __syncthreads();
             if (pi >= A.n_long) break;
-            cta_pair<PIG>(A, A.order_long[pi], HdrRing{hring_all, rs}, cplan, cpart, cstate, al);
+            cta_pair<PIG, NT>(A, A.order_long[pi], HdrRing{hring_all, rs}, cplan, cpart, cstate, al);
         }
     }
     const HdrRing HR{hring_all + (threadIdx.x >> 5) * rs.entries(), rs};
@@ -1139,7 +1274,7 @@ __global__ void __launch_bounds__(NT, AW_WFA_MINB * WFA_CTA / NT) wfa_kernel(Wfa
                                 const int k = k0 + 32 * u;
                                 o[u] = k <= m.hi ? d[k - m.base] : WF_NULL;
                             }
-                            extend_n<4>(A, PR, pat, txt, k0, 32, o);
+                            extend_n<4>(PR, bases_of(A, PR), pat, txt, k0, 32, o);
 #pragma unroll
                             for (int u = 0; u < 4; ++u) {
                                 const int k = k0 + 32 * u;
@@ -1323,7 +1458,7 @@ __global__ void __launch_bounds__(NT, AW_WFA_MINB * WFA_CTA / NT) wfa_kernel(Wfa
                     }
                     // then M[s], extended (the extend step of the next iteration, fused: the
                     // offsets never round-trip through memory unextended)
-                    extend_n<WU>(A, PR, pat, txt, k0, 32, mo);
+                    extend_n<WU>(PR, bases_of(A, PR), pat, txt, k0, 32, mo);
     #pragma unroll
                     for (int u = 0; u < WU; ++u) {
                         const int k = k0 + 32 * u;
@@ -1359,26 +1494,38 @@ __global__ void __launch_bounds__(NT, AW_WFA_MINB * WFA_CTA / NT) wfa_kernel(Wfa
 
 // ---------------------------------------------------------------------------------------
 // Cluster kernel for pairs whose wavefronts outgrow a warp (high memory: standard and
-// Singletrack).  One cluster of CL CTAs (WIDE_NT threads each) per pair, one cluster barrier
-// per score:
-//   1. every thread of the cluster computes and extends the diagonals lo + gtid + GT*u of the
-//      plan (gtid = rank * WIDE_NT + thread, GT = CL * WIDE_NT), and each warp folds its
-//      trimmed ends per component, and whether the end cell was reached, into its CTA's
-//      partials;
-//   2. cluster barrier;
-//   3. warp 0 of every CTA (the CTA's planner) gathers all CTAs' partials through
-//      distributed shared memory, four lanes per CTA, finishes the score's headers and plans the
-//      next score, a lane per input and per component.  Every planner holds the same state
-//      (the headers of the last scores in shared-memory rings, the pool position), so all
-//      plans agree without being exchanged.
-// Pool space is carved deterministically out of reserve chunks that thread 0 of the first
-// CTA (the leader) takes from the pool one score ahead of need and announces to every CTA
-// through distributed shared memory before the barrier; the leader alone writes the pool
-// copy of the headers and the chunk table that the backtrace reads.  The cell arithmetic,
-// the limits, the trimming and the backtrace are the warp kernel's; only the split of the
-// diagonals differs, so the results are identical.  Offsets written by other CTAs are read
-// through L2 (ld.global.cg), after the barrier's release/acquire.
-constexpr int WIDE_NT = 384;
+// Singletrack).  One cluster of CL CTAs per pair; in each, WIDE_CW warps compute and one plans.
+// A pair is a chain of scores, each as long as one pass over the wavefront and a barrier of the
+// cluster take, so nothing else may stand in it.
+//
+// Trimming a wavefront to the diagonals inside the matrix needs the ends of all CTAs.  But the
+// cells that it cuts off are null, which reads the same stored or not, or offsets beyond the end
+// of a sequence; until there is one of those, the ranges depend on nothing but the score (they come
+// out a few diagonals wider than trimmed ones), and the planners go ahead of the warps:
+//   1. the computing warps of all CTAs compute and extend the diagonals of the planned score
+//      (plan_open);
+//   2. meanwhile the planning warps plan the next one, a lane per input and per component.
+//      Every planner holds the same state (the headers of the last scores in shared-memory
+//      rings, the pool position), so all plans agree without being exchanged;
+//   3. cluster barrier.
+// A warp that computes an offset beyond the end says so in every CTA's shared memory before the
+// barrier, and from that score on wavefronts are trimmed: its own is, from what is stored, and
+// the next score is planned again; after that the warps fold their trimmed ends into their CTA's
+// partials (plan_compute), and after the barrier the planners gather all CTAs' partials through
+// distributed shared memory, finish the score's headers and plan the next one.  The end is
+// announced in the same way.
+// Measured on one pair at 12% in us per score, with trimmed ends gathered and the next score planned
+// by the first warp after each barrier, and now: 10 kb 5.4 -> 2.8, 24 kb 7.7 -> 3.5.
+//
+// Pool space is carved deterministically out of reserve chunks that the first CTA's planner
+// (the leader) takes from the pool one score ahead of need and announces to every CTA
+// through distributed shared memory before the barrier; the first CTA's planner alone writes the
+// pool copy of the headers and the chunk table that the backtrace reads.  The cell arithmetic and
+// the backtrace are the warp kernel's, so the results are identical.  Offsets written by other
+// CTAs are ordered by the barrier's release/acquire.
+constexpr int WIDE_SEQ_WORDS = 12 * 1024;  // 2-bit words of a pair kept in shared memory
+constexpr int WIDE_CW = 12, WIDE_NT = 32 * (WIDE_CW + 1);
+constexpr int WIDE_MAX_CL = 16;  // CTAs of a cluster, at most
 constexpr int WIDE_CHUNKS = 8;  // reserve chunks a planner keeps track of (a ring)
 
 // A reserve chunk announced by the leader: for pair `tag`, the planners' chunk number `seq`
@@ -1388,12 +1535,15 @@ struct WideAnn {
     int64_t off, len;
 };
 
-// The planner's state (the same in all lanes of warp 0 of every CTA).
+// The planner's state (the same in all lanes of every CTA's planning warp).
 struct WidePlanner {
     int pi, idx;  // queue position and pair
     int s, num_null, status, end_score, smax, R, ring_cap;
     int lo_all, hi_all;  // the union of the planned diagonal ranges so far
     int64_t ring, hdr_off, ctab_off;
+    int s_hdr, committed;  // the first score of the header chunk hdr_off, the last score with headers
+    int plen, tlen;
+    int slot;            // s mod R
     int64_t cur, end;    // carving position in the current chunk
     int nchunks, cidx;   // chunks received, chunk being carved
     bool exhausted;
@@ -1411,29 +1561,36 @@ __global__ void __launch_bounds__(WIDE_NT, 1) wfa_wide_kernel(WfaArgs A, RingSha
     const int CL = (int)cl.num_blocks();
     const int rank = (int)cl.block_rank();
     const int tid = threadIdx.x, lane = tid & 31;
-    const int GT = CL * WIDE_NT, gtid = rank * WIDE_NT + tid;
-    const bool planner = tid < 32;
-    const bool leader = rank == 0 && tid == 0;
+    const bool planner = tid >= 32 * WIDE_CW;
+    const bool leader = rank == 0 && planner && lane == 0;
     const WfaPen P = A.pen;
-    __shared__ WidePlan plan;
-    __shared__ WidePart part[2];
+    // plan of step it in plan[it & 1], its partials in part[it & 1] (part[2]: of the first trimmed
+    // score), its end and beyond flags at it % 3 (cleared at step it + 2)
+    __shared__ WidePlan plan[2];
+    __shared__ WidePart part[3];
+    __shared__ int at_end[3], beyond[3];
     __shared__ WideAnn ann[2];     // reserve chunks announced before the barrier of step it (it & 1)
     __shared__ WideAnn pstart[2];  // the pair of the np-th pair start (np & 1): tag = queue position,
                                    // seq = pair, off/len = its first chunk
     __shared__ int64_t qoff[WIDE_CHUNKS], qlen[WIDE_CHUNKS];  // the planner's chunks
+    // the header ring, then the pair's packed sequences if they fit (the barrier of a score drops
+    // the L1 lines, so that from global memory the extension would wait for the L2 each time)
     extern __shared__ CompHdr wring[];
     const HdrRing HR{wring, rs};
+    uint64_t *const seqs = (uint64_t *)(wring + rs.entries());
     const PlanLane L = plan_lane(P, lane);
-    if (planner) {
-        part_reset(part[0], lane), part_reset(part[1], lane);
-        if (lane < 2) ann[lane] = WideAnn{-1, -1, -1, 0};
-    }
+    // where this lane of a planner reads its input and writes its component
+    const CompHdr *const rd = HR.at(L.comp, 0);
+    CompHdr *const wr = HR.at(min(lane, 4), 0);
+    const int rd_mask = HR.mask(L.comp), wr_mask = HR.mask(min(lane, 4));
+    if (planner && lane < 2) ann[lane] = WideAnn{-1, -1, -1, 0};
     const CompHdr NUL{1, -1, 0, 0, 0};
     WidePlanner W{};
+    CompHdr mine = NUL;  // a planner's lane c < 5: component c's header of the planned score
     int64_t used = 0;  // the leader's pool bytes for the pair
     int it = 0, np = 0;
 
-    // ---- planner helpers (all lanes of warp 0)
+    // ---- planner helpers (all lanes of the planning warp)
     auto carve = [&](int64_t bytes) -> int64_t {
         bytes = (bytes + 15) & ~(int64_t)15;
         while (W.cur + bytes > W.end) {
@@ -1458,21 +1615,61 @@ __global__ void __launch_bounds__(WIDE_NT, 1) wfa_wide_kernel(WfaArgs A, RingSha
     auto reserve_ok = [&]() -> bool {
         const int64_t need = need_next();
         bool ok = W.end - W.cur >= need;
+        if (ok) return true;
         for (int j = W.cidx + 1; j < W.nchunks; ++j) ok |= qlen[j % WIDE_CHUNKS] >= need;
         return ok;
     };
     // lane c < 5: component c's header of score sc (the first CTA's planner writes the pool copy)
     auto set_hdr = [&](int sc, const CompHdr &o) {
         if (lane < 5) {
-            if (rank == 0) ((ScoreHdr *)(A.pool + W.hdr_off))[sc % HDR_CHUNK].c[lane] = o;
-            HR.put(lane, sc, o);
+            if (rank == 0) {
+                const int64_t off = sc >= W.s_hdr ? W.hdr_off : A.ctab[W.ctab_off + sc / HDR_CHUNK];
+                ((ScoreHdr *)(A.pool + off))[sc % HDR_CHUNK].c[lane] = o;
+            }
+            wr[sc & wr_mask] = o;
         }
         __syncwarp();
     };
-    // plans the next score with a non-null input; op = DONE with W.status set if the pair stops
-    auto plan_next = [&]() {
+    // the headers of score sc, and of the null scores before it
+    auto commit = [&](int sc, const CompHdr &o) {
+        for (int z = W.committed + 1; z < sc; ++z) set_hdr(z, NUL);
+        set_hdr(sc, o);
+        W.committed = sc;
+    };
+    // a reserve chunk announced at step k
+    auto take_ann = [&](int k) {
+        const WideAnn &a = ann[k & 1];
+        if (a.tag == W.pi && a.seq == W.nchunks) {
+            if (lane == 0) qoff[W.nchunks % WIDE_CHUNKS] = a.off, qlen[W.nchunks % WIDE_CHUNKS] = a.len;
+            __syncwarp();
+            ++W.nchunks;
+            if (a.off < 0) W.exhausted = true;
+        }
+    };
+    // the headers of plan q's score with the trimmed ends of all CTAs (partials b)
+    auto finish_score = [&](const WidePlan &q, int b) {
+        // lane i < 10: value i of every CTA's partials
+        int v = INT_MIN;
+        if (lane < 10) {
+#pragma unroll
+            for (int r = 0; r < WIDE_MAX_CL; ++r)
+                if (r < CL) v = max(v, *cl.map_shared_rank(&part[b].k[lane], r));
+        }
+        const int top = v, bottom = __shfl_down_sync(0xffffffffu, v, 5);
+        CompHdr out = lane < 5 ? q.out[lane] : NUL;
+        if (lane < 5 && (q.mask >> lane & 1)) {
+            // no diagonal in the matrix: the empty range [lo, lo-1] of the scan
+            if (top == INT_MIN) out.hi = out.lo - 1;
+            else out.lo = -bottom, out.hi = top;
+        }
+        commit(q.s, out);
+    };
+    // plans the next score with a non-null input into `q`; op = DONE with W.status set if the
+    // pair stops
+    auto plan_next = [&](WidePlan &q) {
         for (;;) {
             ++W.s;
+            W.slot = W.slot + 1 == W.R ? 0 : W.slot + 1;
             const int s = W.s;
             if (s > W.smax) {
                 W.status = WFA_OVERFLOW;
@@ -1484,14 +1681,15 @@ __global__ void __launch_bounds__(WIDE_NT, 1) wfa_wide_kernel(WfaArgs A, RingSha
                     W.status = WFA_RETRY;
                     break;
                 }
-                W.hdr_off = hb;
+                W.hdr_off = hb, W.s_hdr = s;
                 if (leader) A.ctab[W.ctab_off + s / HDR_CHUNK] = hb;
                 __syncwarp();
             }
-            CompHdr in;
-            const unsigned some = plan_input(A, A.ctab + W.ctab_off, HR, L, s, lane, in);
+            // the scores since the last committed one are null
+            CompHdr in = NUL;
+            if (lane < 7 && s - L.dist >= 0 && s - L.dist <= W.committed) in = rd[(s - L.dist) & rd_mask];
+            const unsigned some = __ballot_sync(0xffffffffu, lane < 7 && in.lo <= in.hi);
             if (!some) {
-                set_hdr(s, NUL);
                 // the top of the next step: M[s] is empty
                 if (++W.num_null > A.max_score_scope) {
                     W.status = -3;
@@ -1502,6 +1700,8 @@ __global__ void __launch_bounds__(WIDE_NT, 1) wfa_wide_kernel(WfaArgs A, RingSha
             W.num_null = 0;
             int lo, hi, mask;
             plan_limits(L, lane, in, some, lo, hi, mask);
+            // no diagonal beyond these has a cell
+            lo = max(lo, -W.plen), hi = min(hi, W.tlen);
             W.lo_all = min(W.lo_all, lo), W.hi_all = max(W.hi_all, hi);
             const int width = hi - lo + 1;
             const int64_t wb = (((int64_t)width * 4) + 15) & ~(int64_t)15;
@@ -1519,15 +1719,30 @@ __global__ void __launch_bounds__(WIDE_NT, 1) wfa_wide_kernel(WfaArgs A, RingSha
                 if (mask >> lane & 1)
                     out = CompHdr{lo, hi, lo, 0,
                                   lane == CM || !A.singletrack ? blk + wb * __popc(mask & ((1 << lane) - 1))
-                                                               : W.ring + ((int64_t)((s % W.R) * 4 + (lane - 1)) * W.ring_cap) * 4};
-                plan.out[lane] = out;
-                plan.dst[lane] = mask >> lane & 1 ? (int32_t *)(A.pool + out.off) : nullptr;
+                                                               : W.ring + ((int64_t)(W.slot * 4 + (lane - 1)) * W.ring_cap) * 4};
+                mine = out;
+                q.out[lane] = out;
+                q.dst[lane] = mask >> lane & 1 ? (int32_t *)(A.pool + out.off) : nullptr;
             }
-            if (lane < 7) plan.view[lane] = in_hdr(A, in);
-            if (lane == 0) plan.op = WOP_COMPUTE, plan.lo = lo, plan.hi = hi, plan.mask = mask;
+            if (lane < 7) q.view[lane] = in_hdr(A, in);
+            plan_inner(q, mask, lane, in);
+            if (lane == 0) q.op = WOP_COMPUTE, q.lo = lo, q.hi = hi, q.mask = mask, q.s = s;
+            __syncwarp();
             return;
         }
-        if (lane == 0) plan.op = WOP_DONE;
+        if (lane == 0) q.op = WOP_DONE;
+        __syncwarp();
+    };
+    // the leader reserves the next plan's space ahead of need
+    auto reserve = [&](int k) {
+        if (leader && !W.exhausted && W.nchunks - W.cidx < WIDE_CHUNKS - 1 && !reserve_ok()) {
+            int64_t len = wide_chunk(A, need_next());
+            const int64_t off = pool_grab_rest(pool_of(A), len, need_next());
+            if (off >= 0) used += len;
+            const WideAnn a{W.pi, W.nchunks, off, off >= 0 ? len : 0};
+            for (int c = 0; c < CL; ++c) *cl.map_shared_rank(&ann[k & 1], c) = a;
+        }
+        __syncwarp();
     };
 
     for (;;) {
@@ -1547,10 +1762,13 @@ __global__ void __launch_bounds__(WIDE_NT, 1) wfa_wide_kernel(WfaArgs A, RingSha
             for (int c = 0; c < CL; ++c) *cl.map_shared_rank(&pstart[np & 1], c) = a;
         }
         cl.sync();
+        it = 0;
         if (planner) {
+            for (int b = 0; b < 3; ++b) part_reset(part[b], lane);
+            if (lane < 3) at_end[lane] = 0, beyond[lane] = 0;
             const WideAnn a = pstart[np & 1];
             if (a.tag >= A.n) {
-                if (lane == 0) plan.op = WOP_EXIT;
+                if (lane == 0) plan[0].op = WOP_EXIT;
             } else {
                 const WfaPairDev PR = A.pairs[a.seq];
                 W = WidePlanner{};
@@ -1558,6 +1776,7 @@ __global__ void __launch_bounds__(WIDE_NT, 1) wfa_wide_kernel(WfaArgs A, RingSha
                 W.smax = PR.ctab_cap * HDR_CHUNK - 1;
                 W.R = (P.e1 > P.e2 ? P.e1 : P.e2) + 1;
                 W.ring_cap = PR.plen + PR.tlen + 8;
+                W.plen = PR.plen, W.tlen = PR.tlen;
                 W.end_score = -1, W.lo_all = 0, W.hi_all = 0;
                 W.ring = -1;
                 if (lane == 0) qoff[0] = a.off, qlen[0] = a.len;
@@ -1583,80 +1802,83 @@ __global__ void __launch_bounds__(WIDE_NT, 1) wfa_wide_kernel(WfaArgs A, RingSha
                     if (PR.tlen - PR.plen == 0 && o0 >= PR.tlen) W.end_score = 0;
                 }
                 if (W.status != 0 || W.end_score == 0) {
-                    if (lane == 0) plan.op = WOP_DONE;
+                    if (lane == 0) plan[0].op = WOP_DONE;
                 } else {
-                    plan_next();
+                    plan_next(plan[0]);
+                    reserve(1);  // announced in ann[1], read at step 0's planning
                 }
             }
         }
-        __syncthreads();
+        // flags and partials are clear in every CTA before another one's first step
+        cl.sync();
         ++np;
-        int op = plan.op;
+        int op = plan[0].op;
         if (op == WOP_EXIT) break;
         const int pidx = pstart[(np - 1) & 1].seq;
         const WfaPairDev PR = A.pairs[pidx];
         const uint8_t *pat = A.pat + PR.poff, *txt = A.txt + PR.toff;
-        while (op == WOP_COMPUTE) {
-            // ---- 1. this thread's diagonals of the planned score
-            plan_compute<true>(A, PR, pat, txt, plan, gtid, GT, part[it & 1]);
-            // the leader reserves the next plan's space ahead of need
-            if (leader && !W.exhausted && W.nchunks - W.cidx < WIDE_CHUNKS - 1 && !reserve_ok()) {
-                const int64_t len = wide_chunk(A, need_next());
-                const int64_t off = pool_grab(pool_of(A), len);
-                if (off >= 0) used += len;
-                const WideAnn a{W.pi, W.nchunks, off, off >= 0 ? len : 0};
-                for (int c = 0; c < CL; ++c) *cl.map_shared_rank(&ann[it & 1], c) = a;
-            }
-            cl.sync();
-            // ---- 3. gather, finish the score, plan the next one (warp 0 of every CTA)
-            if (planner) {
-                // lane 4r + q: the q-th quadruple of CTA r's partials, then the maxima over the CTAs
-                int4 v = make_int4(INT_MIN, INT_MIN, INT_MIN, INT_MIN);
-                if ((lane >> 2) < CL && (lane & 3) < 3)
-                    v = *reinterpret_cast<const int4 *>(cl.map_shared_rank(part[it & 1].k, lane >> 2) + 4 * (lane & 3));
-#pragma unroll
-                for (int o = 4; o < 32; o <<= 1) {
-                    v.x = max(v.x, __shfl_xor_sync(0xffffffffu, v.x, o)), v.y = max(v.y, __shfl_xor_sync(0xffffffffu, v.y, o));
-                    v.z = max(v.z, __shfl_xor_sync(0xffffffffu, v.z, o)), v.w = max(v.w, __shfl_xor_sync(0xffffffffu, v.w, o));
-                }
-                // value i of the quadruples: field i & 3 of lane i >> 2
-                auto value = [&](int i) {
-                    const int x = __shfl_sync(0xffffffffu, v.x, i >> 2), y = __shfl_sync(0xffffffffu, v.y, i >> 2);
-                    const int z = __shfl_sync(0xffffffffu, v.z, i >> 2), w = __shfl_sync(0xffffffffu, v.w, i >> 2);
-                    return (i & 3) == 0 ? x : (i & 3) == 1 ? y : (i & 3) == 2 ? z : w;
-                };
-                const int c5 = min(lane, 4), top = value(c5), bottom = value(5 + c5);
-                const bool reached = __shfl_sync(0xffffffffu, v.z, 2) == 1;
-                part_reset(part[(it + 1) & 1], lane);
-                const WideAnn a = ann[it & 1];
-                if (a.tag == W.pi && a.seq == W.nchunks) {
-                    if (lane == 0) qoff[W.nchunks % WIDE_CHUNKS] = a.off, qlen[W.nchunks % WIDE_CHUNKS] = a.len;
-                    __syncwarp();
-                    ++W.nchunks;
-                    if (a.off < 0) W.exhausted = true;
-                }
-                CompHdr out = lane < 5 ? plan.out[lane] : NUL;
-                if (lane < 5 && (plan.mask >> lane & 1)) {
-                    // no diagonal in the matrix: the empty range [lo, lo-1] of the scan
-                    if (top == INT_MIN) out.hi = out.lo - 1;
-                    else out.lo = -bottom, out.hi = top;
-                }
-                __syncwarp();
-                set_hdr(W.s, out);
-                if (reached) {
-                    W.end_score = W.s;
-                    if (lane == 0) plan.op = WOP_DONE;
-                } else {
-                    plan_next();
-                }
-            }
+        Bases B = bases_of(A, PR);
+        const int pw = (B.po + PR.plen) / 32 + 2, tw = (B.to + PR.tlen) / 32 + 2;
+        const bool staged = PR.packed && op == WOP_COMPUTE && pw + tw <= WIDE_SEQ_WORDS;
+        if (staged) {
+            for (int i = tid; i < pw; i += WIDE_NT) seqs[i] = __ldg(B.p + i);
+            for (int i = tid; i < tw; i += WIDE_NT) seqs[pw + i] = __ldg(B.t + i);
+            B.p = seqs, B.t = seqs + pw;
             __syncthreads();
+        }
+        bool trimmed = false;
+        while (op == WOP_COMPUTE) {
+            const WidePlan &now = plan[it & 1];
+            if (!planner) {
+                // ---- 1. this warp's diagonals of the planned score
+                int told;
+                if (trimmed) told = plan_compute<2, 32 * WIDE_CW, false>(PR, bases_of(A, PR), pat, txt, now, rank, CL, part[it & 1]);
+                else if (staged) told = plan_open<32 * (WIDE_CW - 1), true>(PR, B, pat, txt, now, rank, CL);
+                else told = plan_open<32 * (WIDE_CW - 1), false>(PR, B, pat, txt, now, rank, CL);
+                if (told && lane < CL) {
+                    if (told & 1) *cl.map_shared_rank(&at_end[it % 3], lane) = 1;
+                    if (told & 2) *cl.map_shared_rank(&beyond[it % 3], lane) = 1;
+                }
+            } else {
+                // ---- 2. its headers, and the plan of the next one
+                if (lane == 0) at_end[(it + 1) % 3] = 0, beyond[(it + 1) % 3] = 0;
+                if (!trimmed) {
+                    take_ann(it - 1);
+                    commit(W.s, mine);
+                    plan_next(plan[(it + 1) & 1]);
+                }
+                reserve(it);
+            }
+            // ---- 3.
+            cl.sync();
+            const bool end = at_end[it % 3] != 0;
+            if (!end && (trimmed || beyond[it % 3])) {
+                if (!trimmed) {
+                    if (!planner) plan_trim(PR, now, rank * 32 * WIDE_CW + tid, CL * 32 * WIDE_CW, part[2]);
+                    cl.sync();
+                }
+                if (planner) {
+                    if (trimmed) part_reset(part[(it + 1) & 1], lane);
+                    else W.s = now.s, W.slot = now.s % W.R, W.num_null = 0, W.status = 0;  // drop the plan made meanwhile
+                    take_ann(it);
+                    finish_score(now, trimmed ? it & 1 : 2);
+                    plan_next(plan[(it + 1) & 1]);
+                }
+                trimmed = true;
+                __syncthreads();
+            }
+            if (planner && end) {
+                W.end_score = now.s, W.status = 0;
+                if (trimmed) finish_score(now, it & 1);
+            }
             ++it;
-            op = plan.op;
+            op = end ? WOP_DONE : plan[it & 1].op;
         }
         // ---- backtrace (leader)
         if (leader)
-            finish_pair<false>(A, PR, W.idx, pat, txt, A.ctab + PR.ctab_off, HR, W.status, W.end_score, W.s, used);
+            finish_pair<false>(A, PR, W.idx, pat, txt, A.ctab + PR.ctab_off, HR, W.status, W.end_score, W.end_score >= 0 ? W.end_score : W.s,
+                               used);
+        cl.sync();
     }
 }
 
@@ -1710,31 +1932,41 @@ static cudaLaunchConfig_t wide_config(int ctas, int cl, size_t smem, cudaStream_
     return cfg;
 }
 
+// Dynamic shared memory of the cluster kernel, and what its launches need set; an
+// error if the header ring of this score scope does not fit.
+static cudaError_t wide_setup(const WfaPen &pen, int scope, int cl, RingShape &rs, size_t &smem) {
+    rs = ring_shape(pen, scope, WIDE_RING_BYTES);
+    if (rs.mm < 0 || cl > WIDE_MAX_CL) return cudaErrorInvalidValue;
+    smem = (size_t)rs.entries() * sizeof(CompHdr) + WIDE_SEQ_WORDS * sizeof(uint64_t);
+    cudaError_t e = cudaFuncSetAttribute(wfa_wide_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e == cudaSuccess && cl > 8) e = cudaFuncSetAttribute(wfa_wide_kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    return e;
+}
+
 cudaError_t launch_wfa_wide(const WfaArgs &a, int clusters, int cl, cudaStream_t st) {
-    const RingShape rs = ring_shape(a.pen, a.max_score_scope, WIDE_RING_BYTES);
-    if (rs.mm < 0) return cudaErrorInvalidValue;
-    const size_t smem = (size_t)rs.entries() * sizeof(CompHdr);
-    if (smem > 48 * 1024) {
-        const cudaError_t e = cudaFuncSetAttribute(wfa_wide_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e != cudaSuccess) return e;
-    }
+    RingShape rs;
+    size_t smem;
+    cudaError_t e = wide_setup(a.pen, a.max_score_scope, cl, rs, smem);
+    if (e != cudaSuccess) return e;
     cudaLaunchAttribute at[1];
     const cudaLaunchConfig_t cfg = wide_config(clusters * cl, cl, smem, st, at);
-    const cudaError_t e = cudaLaunchKernelEx(&cfg, wfa_wide_kernel, a, rs);
+    e = cudaLaunchKernelEx(&cfg, wfa_wide_kernel, a, rs);
     return e != cudaSuccess ? e : cudaGetLastError();
 }
 
 int wfa_wide_clusters(int cl, const WfaPen &pen, int scope) {
-    const RingShape rs = ring_shape(pen, scope, WIDE_RING_BYTES);
-    if (rs.mm < 0) return 0;
-    const size_t smem = (size_t)rs.entries() * sizeof(CompHdr);
-    if (smem > 48 * 1024 &&
-        cudaFuncSetAttribute(wfa_wide_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
+    RingShape rs;
+    size_t smem;
+    if (wide_setup(pen, scope, cl, rs, smem) != cudaSuccess) {
+        cudaGetLastError();
         return 0;
+    }
     cudaLaunchAttribute at[1];
     const cudaLaunchConfig_t cfg = wide_config(cl, cl, smem, 0, at);
     int n = 0;
-    return cudaOccupancyMaxActiveClusters(&n, (void *)wfa_wide_kernel, &cfg) == cudaSuccess ? n : 0;
+    if (cudaOccupancyMaxActiveClusters(&n, (void *)wfa_wide_kernel, &cfg) == cudaSuccess) return n;
+    cudaGetLastError();
+    return 0;
 }
 
 namespace {

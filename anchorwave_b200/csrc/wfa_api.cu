@@ -297,7 +297,11 @@ static int run_batch(wavefront_aligner_gpu *al, int n, const char *const *patter
             } else {
                 W.order = al->d_order.as<int32_t>(), W.n = (int32_t)staged.size();
                 ++al->last_cluster_launches;
-                WCUDA(launch_wfa_wide(W, std::min(W.n, wide_clusters), cl, al->st));
+                // few pairs: clusters of twice the size, as long as each pair has one (one pair of
+                // 24 kb at 12%: 5.1 us a score on 8 CTAs, 3.9 on 16; below 10 kb no difference)
+                const int pairs_wide = cl == 8 && W.n <= wide_clusters / 2 ? wfa_wide_clusters(16, W.pen, W.max_score_scope) : 0;
+                if (W.n <= pairs_wide) WCUDA(launch_wfa_wide(W, W.n, 16, al->st));
+                else WCUDA(launch_wfa_wide(W, std::min(W.n, wide_clusters), cl, al->st));
                 ++launches;
             }
             WCUDA(cudaEventRecord(al->e1, al->st));

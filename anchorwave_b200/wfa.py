@@ -32,7 +32,7 @@ WAVEFRONT_MEMORY_LOW = 2
 def set_wide(width: int = -1, tail_width: int = -1, cluster_ctas: int = 0) -> None:
     """aw_set_wfa_wide: wavefront width from which a high-memory pair leaves its warp for a
     cluster of CTAs (0 = never), the lower width that applies once every pair of the call has
-    started, and the CTAs of a cluster (1..8).  Negative widths and cluster_ctas 0 keep the
+    started, and the CTAs of a cluster (1..8; with 8, few pairs get 16).  Negative widths and cluster_ctas 0 keep the
     setting.  Results are identical under every setting."""
     lib.aw_set_wfa_wide(int(width), int(tail_width), int(cluster_ctas))
 

@@ -245,7 +245,8 @@ int wavefront_gpu_memory(const wavefront_aligner_gpu_t *aligner, int64_t *pair_m
  * warp and runs again from score 0 on a cluster of `cluster_ctas` CTAs (1..8) that spreads
  * each wavefront over all of their threads; results are identical.  width 0: every pair
  * stays on one warp; a negative value or cluster_ctas <= 0 keeps that setting.  Defaults:
- * 8192, 1024 and 8.  Process-wide.  No counterpart in the reference (tuning knob). */
+ * 8192, 1024 and 8.  With 8, pairs so few that each can have a cluster of 16 get one.
+ * Process-wide.  No counterpart in the reference (tuning knob). */
 void aw_set_wfa_wide(int width, int tail_width, int cluster_ctas);
 /* Pairs whose pattern and text lengths sum to at least `min_length_sum` run first, each on a
  * whole CTA (the longest pairs of a batch otherwise set its duration, one warp each): four
