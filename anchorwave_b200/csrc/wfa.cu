@@ -229,9 +229,15 @@ struct Cell {
     uint32_t pc, pv;
 };
 __device__ __forceinline__ Cell getc(const WfaArgs &A, const CompHdr &h, int k) {
-    if (k < h.lo || k > h.hi) return Cell{WF_NULL, 0u, BT_NULL};
-    const int32_t *d = (const int32_t *)(A.pool + h.off) + (k - h.base);
-    return Cell{d[0], (uint32_t)d[h.pad], (uint32_t)d[2 * h.pad]};
+    // three predicated loads: branches would put the cells of a lane one after the other
+    Cell c;
+    const int ok = k >= h.lo && k <= h.hi;
+    const int32_t *p = (const int32_t *)(A.pool + h.off) + (k - h.base);
+    asm volatile("{ .reg .pred q; setp.ne.s32 q, %6, 0; mov.b32 %0, %7; mov.b32 %1, 0; mov.b32 %2, %8;"
+                 " @q ld.global.b32 %0, [%3]; @q ld.global.b32 %1, [%4]; @q ld.global.b32 %2, [%5]; }"
+                 : "=r"(c.o), "=r"(c.pc), "=r"(c.pv)
+                 : "l"(p), "l"(p + h.pad), "l"(p + 2 * h.pad), "r"(ok), "n"(WF_NULL), "n"(BT_NULL));
+    return c;
 }
 
 __device__ __forceinline__ uint64_t load8(const uint8_t *base, int64_t pos) {
@@ -1430,11 +1436,11 @@ __global__ void __launch_bounds__(NT, AW_WFA_MINB * WFA_CTA / NT) wfa_kernel(Wfa
     #pragma unroll
                     for (int u = 0; u < WU; ++u) {
                         const int k = k0 + 32 * u;
-                        ins1[u] = max(getv(h_o1, k - 1), getv(h_i1, k - 1)) + 1;
-                        ins2[u] = max(getv(h_o2, k - 1), getv(h_i2, k - 1)) + 1;
-                        del1[u] = max(getv(h_o1, k + 1), getv(h_d1, k + 1));
-                        del2[u] = max(getv(h_o2, k + 1), getv(h_d2, k + 1));
-                        misms[u] = getv(h_mm, k) + 1;
+                        ins1[u] = max(getv_pred(h_o1, k - 1), getv_pred(h_i1, k - 1)) + 1;
+                        ins2[u] = max(getv_pred(h_o2, k - 1), getv_pred(h_i2, k - 1)) + 1;
+                        del1[u] = max(getv_pred(h_o1, k + 1), getv_pred(h_d1, k + 1));
+                        del2[u] = max(getv_pred(h_o2, k + 1), getv_pred(h_d2, k + 1));
+                        misms[u] = getv_pred(h_mm, k) + 1;
                     }
                     // the gap components are final: store them (and their trimmed ends) first, so
                     // that only M stays live across its extension
