@@ -209,11 +209,9 @@ struct InHdr {
 __device__ __forceinline__ InHdr in_hdr(const WfaArgs &A, const CompHdr &h) {
     return InHdr{h.lo, h.hi, (const int32_t *)(A.pool + h.off) - h.base};
 }
+// As a predicated load, so that a lane's loads from several inputs are in flight together (the
+// compiler made a branch of each check).
 __device__ __forceinline__ int32_t getv(const InHdr &h, int k) {
-    return (k < h.lo || k > h.hi) ? WF_NULL : h.p[k];
-}
-// The same as a predicated load, so that a lane's loads from several inputs are in flight together.
-__device__ __forceinline__ int32_t getv_pred(const InHdr &h, int k) {
     int32_t r;
     const int ok = k >= h.lo && k <= h.hi;
     asm volatile("{ .reg .pred q; setp.ne.s32 q, %2, 0; mov.b32 %0, %3; @q ld.global.b32 %0, [%1]; }"
@@ -808,7 +806,7 @@ __device__ __forceinline__ void wf_trip(const WfaPairDev &PR, const Bases &B, co
     for (int u = 0; u < U; ++u) {
         const int k = k0 + G * u;
         auto in = [&](int j, int d) -> int32_t {
-            if constexpr (!INNER) return getv_pred(v[j], k + d);
+            if constexpr (!INNER) return getv(v[j], k + d);
             else return !GUARD || k <= hi ? (v[j].p + k0)[G * u + d] : WF_NULL;
         };
         g[u][0] = max(in(1, -1), in(2, -1)) + 1;
@@ -845,14 +843,14 @@ __device__ __forceinline__ void wf_trip(const WfaPairDev &PR, const Bases &B, co
 }
 
 // The trip whose first lane has diagonal kw, with or without checks.
-template <int U, int G, bool SH>
+template <int U, int G, bool SH, bool TRIM>
 __device__ __forceinline__ void plan_trip(const WfaPairDev &PR, const Bases &B, const uint8_t *pat, const uint8_t *txt,
                                           const WidePlan &Q, int kw, int lane, int (&kmin)[5], int (&kmax)[5],
                                           bool &reached, bool &beyond) {
     if (kw > Q.ilo && kw + 31 + G * (U - 1) < Q.ihi)
-        wf_trip<U, G, true, false, true, SH>(PR, B, pat, txt, Q.view, Q.dst, Q.lo, Q.hi, kw + lane, kmin, kmax, reached, beyond);
+        wf_trip<U, G, true, false, TRIM, SH>(PR, B, pat, txt, Q.view, Q.dst, Q.lo, Q.hi, kw + lane, kmin, kmax, reached, beyond);
     else if (kw <= Q.hi)
-        wf_trip<U, G, false, true, true, SH>(PR, B, pat, txt, Q.view, Q.dst, Q.lo, Q.hi, kw + lane, kmin, kmax, reached, beyond);
+        wf_trip<U, G, false, true, TRIM, SH>(PR, B, pat, txt, Q.view, Q.dst, Q.lo, Q.hi, kw + lane, kmin, kmax, reached, beyond);
 }
 
 // The diagonals of a planned score (high memory) of one warp of CTA `rank` of CL, each CTA with G
@@ -860,7 +858,7 @@ __device__ __forceinline__ void plan_trip(const WfaPairDev &PR, const Bases &B, 
 // CL*G*U diagonals, with the fewest diagonals per thread that end it: narrow ones are spread over
 // all threads.  Returns, for the warp, 1 when the end cell was reached, plus 2 when a gap
 // component got an offset beyond the end of a sequence.
-template <int UMAX, int G, bool SH>
+template <int UMAX, int G, bool SH, bool TRIM = true>
 __device__ __forceinline__ int plan_compute(const WfaPairDev &PR, const Bases &B, const uint8_t *pat,
                                             const uint8_t *txt, const WidePlan &Q, int rank, int CL, WidePart &pp) {
     const int lane = threadIdx.x & 31, w0 = threadIdx.x & ~31;
@@ -873,13 +871,13 @@ __device__ __forceinline__ int plan_compute(const WfaPairDev &PR, const Bases &B
         const int U = UMAX >= 4 && left > 2 * round ? 4 : UMAX >= 2 && left > round ? 2 : 1;
         const int kw = kb + rank * G * U + w0;
         any |= kw <= Q.hi;
-        if (UMAX >= 4 && U == 4) plan_trip<4, G, SH>(PR, B, pat, txt, Q, kw, lane, kmin, kmax, reached, beyond);
-        else if (UMAX >= 2 && U == 2) plan_trip<2, G, SH>(PR, B, pat, txt, Q, kw, lane, kmin, kmax, reached, beyond);
-        else plan_trip<1, G, SH>(PR, B, pat, txt, Q, kw, lane, kmin, kmax, reached, beyond);
+        if (UMAX >= 4 && U == 4) plan_trip<4, G, SH, TRIM>(PR, B, pat, txt, Q, kw, lane, kmin, kmax, reached, beyond);
+        else if (UMAX >= 2 && U == 2) plan_trip<2, G, SH, TRIM>(PR, B, pat, txt, Q, kw, lane, kmin, kmax, reached, beyond);
+        else plan_trip<1, G, SH, TRIM>(PR, B, pat, txt, Q, kw, lane, kmin, kmax, reached, beyond);
         kb += round * U;
     }
     if (!any) return 0;  // no diagonal for this warp
-    fold_partials(kmin, kmax, reached, pp);
+    if (TRIM) fold_partials(kmin, kmax, reached, pp);
     return (__any_sync(0xffffffffu, reached) ? 1 : 0) | (__any_sync(0xffffffffu, beyond) ? 2 : 0);
 }
 
@@ -940,21 +938,20 @@ __device__ __noinline__ void plan_trim(const WfaPairDev &PR, const WidePlan &Q, 
     fold_partials(kmin, kmax, false, pp);
 }
 
-// CTA-cooperative mode: one long pair on all threads of a CTA.  Warp 0 plans every score, a
-// lane per input and per output component (the headers in the CTA's header ring and the pool,
-// the allocations), and all threads compute and extend the diagonals lo + tid + NT*u; two
-// CTA barriers per score.  A pair whose wavefront grows too wide stops with WFA_WIDE for
-// the cluster kernel.  The cell arithmetic, the limits, the trimming and the backtrace are the
-// warp's.  In the piggyback modes every warp reserves its own block runs; no pair moves to
-// the cluster kernel.
+// CTA-cooperative mode, piggyback memory modes: one long pair on all threads of a CTA.  Warp 0
+// plans every score, a lane per input and per output component (the headers in the CTA's header
+// ring and the pool, the allocations), and all threads compute and extend the diagonals
+// lo + tid + NT*u; two CTA barriers per score.  The cell arithmetic, the limits, the trimming and
+// the backtrace are the warp's.  Every warp reserves its own block runs; no pair moves to the
+// cluster kernel.
 struct CtaPlanner {  // warp 0's state (shared memory)
     int s, num_null, status, end_score;
-    int64_t ring, hdr_off;
-    int64_t rbase;  // piggyback rings: their place and the elements of a slot's array
+    int64_t hdr_off;
+    int64_t rbase;  // the rings' place and the elements of a slot's array
     int rcap, pad;
     Alloc al;
 };
-template <bool PIG, int NT>
+template <int NT>
 __device__ void cta_pair(const WfaArgs &A, int idx, const HdrRing &HR, WidePlan &plan, WidePart &part, CtaPlanner &Q,
                          Alloc &wal) {
     const int tid = threadIdx.x, lane = tid & 31;
@@ -965,8 +962,7 @@ __device__ void cta_pair(const WfaArgs &A, int idx, const HdrRing &HR, WidePlan 
     int64_t *ctab = A.ctab + PR.ctab_off;
     const CompHdr NUL{1, -1, 0, 0, 0};
     const int smax = PR.ctab_cap * HDR_CHUNK - 1;
-    const int R = (P.e1 > P.e2 ? P.e1 : P.e2) + 1, ring_cap = plen + tlen + 8;
-    // piggyback rings, and every warp's block reservations
+    // rings, and every warp's block reservations
     const int SR = A.max_score_scope, R1 = P.e1 + 1, R2 = P.e2 + 1;
     const int64_t ring_arrays = 3 * (int64_t)(SR + 2 * R1 + 2 * R2);
     uint32_t bnext = 0, bend = 0;
@@ -1013,57 +1009,19 @@ __device__ void cta_pair(const WfaArgs &A, int idx, const HdrRing &HR, WidePlan 
             const int width = hi - lo + 1;
             const bool mine = lane < 5 && (mask >> lane & 1);
             CompHdr out = NUL;
-            if constexpr (PIG) {
-                if (width > Q.rcap) {
-                    const int nc = max(2 * Q.rcap, (width + 3) & ~3);
-                    const int64_t nb = warp_alloc(A, Q.al, ring_arrays * nc * 4, lane);
-                    if (nb < 0) {
-                        status = WFA_RETRY;
-                        break;
-                    }
-                    __syncwarp();
-                    if (lane == 0) Q.rcap = nc, Q.rbase = nb;
-                    __syncwarp();
-                }
-                if (mine) out = CompHdr{lo, hi, lo, Q.rcap, Q.rbase + pig_slot(lane, s, SR, R1, R2) * Q.rcap * 4};
-            } else {
-                // a wavefront too wide for the CTA: the cluster kernel re-runs the pair (past
-                // wide_width_cta always; past wide_width_tail in the call's tail, checked every 32
-                // scores: every pair started and few still running)
-                if (A.wide_width_cta > 0 && width > A.wide_width_tail) {
-                    bool wide = width > A.wide_width_cta;
-                    if (!wide && (s & 31) == 0)
-                        wide = __all_sync(0xffffffffu, *(volatile int32_t *)(A.queue + 3) >= A.n_all &&
-                                                           *(volatile int32_t *)(A.queue + 1) <= A.wide_tail_pairs);
-                    if (wide) {
-                        status = WFA_WIDE;
-                        break;
-                    }
-                }
-                if (A.singletrack && width > ring_cap) {
-                    status = WFA_OVERFLOW;
-                    break;
-                }
-                const int64_t wb = (((int64_t)width * 4) + 15) & ~(int64_t)15;
-                const int64_t blk = warp_alloc(A, Q.al, wb * (A.singletrack ? 1 : __popc(mask)), lane);
-                if (blk < 0) {
+            if (width > Q.rcap) {
+                const int nc = max(2 * Q.rcap, (width + 3) & ~3);
+                const int64_t nb = warp_alloc(A, Q.al, ring_arrays * nc * 4, lane);
+                if (nb < 0) {
                     status = WFA_RETRY;
                     break;
                 }
-                if (mine) {
-                    const int64_t place = lane == CM || !A.singletrack
-                                              ? blk + wb * __popc(mask & ((1 << lane) - 1))
-                                              : Q.ring + ((int64_t)((s % R) * 4 + (lane - 1)) * ring_cap) * 4;
-                    out = CompHdr{lo, hi, lo, 0, place};
-                }
+                __syncwarp();
+                if (lane == 0) Q.rcap = nc, Q.rbase = nb;
+                __syncwarp();
             }
-            if constexpr (PIG) {
-                if (lane < 7) plan.in[lane] = in;
-            } else {
-                if (lane < 7) plan.view[lane] = in_hdr(A, in);
-                plan_inner(plan, mask, lane, in);
-                if (lane < 5) plan.dst[lane] = mine ? (int32_t *)(A.pool + out.off) : nullptr;
-            }
+            if (mine) out = CompHdr{lo, hi, lo, Q.rcap, Q.rbase + pig_slot(lane, s, SR, R1, R2) * Q.rcap * 4};
+            if (lane < 7) plan.in[lane] = in;
             if (lane < 5) plan.out[lane] = out;
             if (lane == 0) {
                 plan.op = WOP_COMPUTE, plan.lo = lo, plan.hi = hi, plan.mask = mask;
@@ -1075,38 +1033,29 @@ __device__ void cta_pair(const WfaArgs &A, int idx, const HdrRing &HR, WidePlan 
     };
     if (tid < 32) {
         int status = 0, end_score = -1;
-        int64_t ring = -1, rbase = -1;
         constexpr int rcap = 32;
         if (lane == 0) Q.al.init(), Q.s = Q.num_null = 0, Q.rcap = rcap;
         __syncwarp();
         if (lane == 0) atomicAdd(A.queue + 1, 1), atomicAdd(A.queue + 3, 1);  // pairs running, started
         part_reset(part, lane);
         if (lane == 0) part.retry = 0, part.used = 0;
-        if (!PIG && A.singletrack) {
-            ring = warp_alloc(A, Q.al, (int64_t)R * 4 * ring_cap * 4, lane);
-            if (ring < 0) status = WFA_RETRY;
-        }
-        if (PIG) {
-            rbase = warp_alloc(A, Q.al, ring_arrays * rcap * 4, lane);
-            if (rbase < 0) status = WFA_RETRY;
-        }
+        const int64_t rbase = warp_alloc(A, Q.al, ring_arrays * rcap * 4, lane);
+        if (rbase < 0) status = WFA_RETRY;
         const int64_t h0 = status == 0 ? warp_alloc(A, Q.al, (int64_t)sizeof(ScoreHdr) * HDR_CHUNK, lane) : -1;
-        const int64_t d0 = h0 < 0 ? -1 : PIG ? rbase : warp_alloc(A, Q.al, 16, lane);  // piggyback: slot 0 of M
+        const int64_t d0 = h0 < 0 ? -1 : rbase;  // slot 0 of M
         if (status == 0 && d0 < 0) status = WFA_RETRY;
         if (status == 0) {
             // M[0] = {0} on diagonal 0, extended
             const int32_t o0 = (int32_t)lcp1(A, PR, pat, txt, 0, 0);
             if (lane == 0) {
-                Q.hdr_off = h0, Q.ring = ring, Q.rbase = rbase;
+                Q.hdr_off = h0, Q.rbase = rbase;
                 ctab[0] = h0;
                 *(int32_t *)(A.pool + d0) = o0;
-                if (PIG) {
-                    ((uint32_t *)(A.pool + d0))[rcap] = 0u;
-                    ((uint32_t *)(A.pool + d0))[2 * rcap] = BT_NULL;  // the start (0, 0)
-                }
+                ((uint32_t *)(A.pool + d0))[rcap] = 0u;
+                ((uint32_t *)(A.pool + d0))[2 * rcap] = BT_NULL;  // the start (0, 0)
             }
             __syncwarp();
-            set_hdr(0, lane == 0 ? CompHdr{0, 0, 0, PIG ? rcap : 0, d0} : NUL);
+            set_hdr(0, lane == 0 ? CompHdr{0, 0, 0, rcap, d0} : NUL);
             if (tlen - plen == 0 && o0 >= tlen) end_score = 0;
         }
         if (lane == 0) Q.status = status, Q.end_score = end_score;
@@ -1118,20 +1067,16 @@ __device__ void cta_pair(const WfaArgs &A, int idx, const HdrRing &HR, WidePlan 
     }
     __syncthreads();
     while (plan.op == WOP_COMPUTE) {
-        if constexpr (PIG) {
-            int kmin[5], kmax[5];
-            bool reached = false, ok = true;
+        int kmin[5], kmax[5];
+        bool reached = false, ok = true;
 #pragma unroll
-            for (int c = 0; c < 5; ++c) kmin[c] = INT_MAX, kmax[c] = INT_MIN;
-            // a warp whose first diagonal lies beyond the wavefront has none in the trip
-            for (int kb = plan.lo; kb + (tid & ~31) <= plan.hi && ok; kb += NT * PIG_U)
-                ok = pig_trip(A, PR, pat, txt, kb, tid, NT, plan.lo, plan.hi, plan.in, plan.out, plan.mask,
-                              plan.out[CM].pad, wal, bnext, bend, kmin, kmax, reached);
-            fold_partials(kmin, kmax, reached, part);
-            if (!ok && lane == 0) part.retry = 1;
-        } else {
-            plan_compute<AW_WFA_CTA_U, NT, false>(PR, bases_of(A, PR), pat, txt, plan, 0, 1, part);
-        }
+        for (int c = 0; c < 5; ++c) kmin[c] = INT_MAX, kmax[c] = INT_MIN;
+        // a warp whose first diagonal lies beyond the wavefront has none in the trip
+        for (int kb = plan.lo; kb + (tid & ~31) <= plan.hi && ok; kb += NT * PIG_U)
+            ok = pig_trip(A, PR, pat, txt, kb, tid, NT, plan.lo, plan.hi, plan.in, plan.out, plan.mask,
+                          plan.out[CM].pad, wal, bnext, bend, kmin, kmax, reached);
+        fold_partials(kmin, kmax, reached, part);
+        if (!ok && lane == 0) part.retry = 1;
         __syncthreads();
         if (tid < 32) {
             if (part.retry) {
@@ -1156,15 +1101,215 @@ __device__ void cta_pair(const WfaArgs &A, int idx, const HdrRing &HR, WidePlan 
         }
         __syncthreads();
     }
-    if (PIG && lane == 0) atomicAdd(&part.used, (unsigned long long)wal.used);
+    if (lane == 0) atomicAdd(&part.used, (unsigned long long)wal.used);
     __syncthreads();
     if (tid == 0) {
-        finish_pair<PIG>(A, PR, idx, pat, txt, ctab, HR, Q.status, Q.end_score, Q.s, Q.al.used + (int64_t)part.used);
+        finish_pair<true>(A, PR, idx, pat, txt, ctab, HR, Q.status, Q.end_score, Q.s, Q.al.used + (int64_t)part.used);
         atomicSub(A.queue + 1, 1);
     }
     __syncthreads();
     if (tid == 0) give_back(pool_of(A), Q.al);
-    if (PIG && lane == 0) give_back(pool_of(A), wal);
+    if (lane == 0) give_back(pool_of(A), wal);
+}
+
+// CTA-cooperative mode, high memory: one long pair on a CTA of NT computing threads and one
+// planning warp.  As in the cluster kernel (below), wavefronts are not trimmed before the first
+// offset beyond the end of a sequence, so that the planner works a score ahead of the others and one
+// CTA barrier per score is left (two, with the plan between them, took 3.8 us a score at 2 kb,
+// half of it waiting for the plan; now 2.3).  A pair whose wavefront grows too wide stops with
+// WFA_WIDE for the cluster kernel.
+struct CtaShared {
+    WidePlan plan[2];
+    WidePart part;
+    int at_end[3], beyond[3];
+    int next;  // position of the pair
+};
+template <int NT>
+__device__ void cta_open(const WfaArgs &A, int idx, const HdrRing &HR, CtaShared &S, Alloc &al) {
+    const int tid = threadIdx.x, lane = tid & 31;
+    const bool planner = tid >= NT;
+    const WfaPen P = A.pen;
+    const WfaPairDev PR = A.pairs[idx];
+    const int plen = PR.plen, tlen = PR.tlen;
+    const uint8_t *pat = A.pat + PR.poff, *txt = A.txt + PR.toff;
+    const Bases B = bases_of(A, PR);
+    int64_t *ctab = A.ctab + PR.ctab_off;
+    const CompHdr NUL{1, -1, 0, 0, 0};
+    const int smax = PR.ctab_cap * HDR_CHUNK - 1;
+    const int R = (P.e1 > P.e2 ? P.e1 : P.e2) + 1, ring_cap = plen + tlen + 8;
+    const PlanLane L = plan_lane(P, lane);
+    // the planner's state: the planned score, the last one with headers, the header chunk of the
+    // scores from s_hdr on, the planned score's header of component `lane`
+    int s = 0, committed = 0, num_null = 0, status = 0, end_score = -1, s_hdr = 0, slot = 0;
+    int64_t ring = -1, hdr_off = 0;
+    CompHdr mine = NUL;
+    auto set_hdr = [&](int sc, const CompHdr &o) {
+        if (lane < 5) {
+            const int64_t off = sc >= s_hdr ? hdr_off : ctab[sc / HDR_CHUNK];
+            ((ScoreHdr *)(A.pool + off))[sc % HDR_CHUNK].c[lane] = o;
+            HR.put(lane, sc, o);
+        }
+        __syncwarp();
+    };
+    // the headers of score sc, and of the null scores before it
+    auto commit = [&](int sc, const CompHdr &o) {
+        for (int z = committed + 1; z < sc; ++z) set_hdr(z, NUL);
+        set_hdr(sc, o);
+        committed = sc;
+    };
+    auto plan_next = [&](WidePlan &q) {
+        for (;;) {
+            ++s;
+            slot = slot + 1 == R ? 0 : slot + 1;
+            if (s > smax) {
+                status = WFA_OVERFLOW;
+                break;
+            }
+            if (s % HDR_CHUNK == 0) {
+                const int64_t hb = warp_alloc(A, al, (int64_t)sizeof(ScoreHdr) * HDR_CHUNK, lane);
+                if (hb < 0) {
+                    status = WFA_RETRY;
+                    break;
+                }
+                hdr_off = hb, s_hdr = s;
+                if (lane == 0) ctab[s / HDR_CHUNK] = hb;
+                __syncwarp();
+            }
+            // the scores since the last committed one are null
+            CompHdr in = NUL;
+            if (lane < 7 && s - L.dist >= 0 && s - L.dist <= committed) in = HR.get(A, ctab, L.comp, s - L.dist);
+            const unsigned some = __ballot_sync(0xffffffffu, lane < 7 && in.lo <= in.hi);
+            if (!some) {
+                if (++num_null > A.max_score_scope) {  // the top of the next step: M[s] is empty
+                    status = -3;
+                    break;
+                }
+                continue;
+            }
+            num_null = 0;
+            int lo, hi, mask;
+            plan_limits(L, lane, in, some, lo, hi, mask);
+            // no diagonal beyond these has a cell
+            lo = max(lo, -plen), hi = min(hi, tlen);
+            const int width = hi - lo + 1;
+            // a wavefront too wide for the CTA: the cluster kernel re-runs the pair (past
+            // wide_width_cta always; past wide_tail_cta in the call's tail, checked every 32
+            // scores: every pair started and few still running)
+            if (A.wide_width_cta > 0 && width > A.wide_tail_cta) {
+                bool wide = width > A.wide_width_cta;
+                if (!wide && (s & 31) == 0)
+                    wide = __all_sync(0xffffffffu, *(volatile int32_t *)(A.queue + 3) >= A.n_all &&
+                                                       *(volatile int32_t *)(A.queue + 1) <= A.wide_tail_pairs);
+                if (wide) {
+                    status = WFA_WIDE;
+                    break;
+                }
+            }
+            if (A.singletrack && width > ring_cap) {
+                status = WFA_OVERFLOW;
+                break;
+            }
+            const int64_t wb = (((int64_t)width * 4) + 15) & ~(int64_t)15;
+            const int64_t blk = warp_alloc(A, al, wb * (A.singletrack ? 1 : __popc(mask)), lane);
+            if (blk < 0) {
+                status = WFA_RETRY;
+                break;
+            }
+            if (lane < 5) {
+                mine = NUL;
+                if (mask >> lane & 1)
+                    mine = CompHdr{lo, hi, lo, 0,
+                                   lane == CM || !A.singletrack ? blk + wb * __popc(mask & ((1 << lane) - 1))
+                                                                : ring + ((int64_t)(slot * 4 + (lane - 1)) * ring_cap) * 4};
+                q.out[lane] = mine;
+                q.dst[lane] = mask >> lane & 1 ? (int32_t *)(A.pool + mine.off) : nullptr;
+            }
+            if (lane < 7) q.view[lane] = in_hdr(A, in);
+            plan_inner(q, mask, lane, in);
+            if (lane == 0) q.op = WOP_COMPUTE, q.lo = lo, q.hi = hi, q.mask = mask, q.s = s;
+            __syncwarp();
+            return;
+        }
+        if (lane == 0) q.op = WOP_DONE;
+        __syncwarp();
+    };
+    if (planner) {
+        if (lane == 0) {
+            al.init();
+            atomicAdd(A.queue + 1, 1), atomicAdd(A.queue + 3, 1);  // pairs running, started
+            for (int b = 0; b < 3; ++b) S.at_end[b] = S.beyond[b] = 0;
+        }
+        __syncwarp();
+        part_reset(S.part, lane);
+        if (A.singletrack) {
+            ring = warp_alloc(A, al, (int64_t)R * 4 * ring_cap * 4, lane);
+            if (ring < 0) status = WFA_RETRY;
+        }
+        hdr_off = status == 0 ? warp_alloc(A, al, (int64_t)sizeof(ScoreHdr) * HDR_CHUNK, lane) : -1;
+        const int64_t d0 = hdr_off >= 0 ? warp_alloc(A, al, 16, lane) : -1;
+        if (status == 0 && d0 < 0) status = WFA_RETRY;
+        if (status == 0) {
+            // M[0] = {0} on diagonal 0, extended
+            const int32_t o0 = (int32_t)lcp1(A, PR, pat, txt, 0, 0);
+            if (lane == 0) ctab[0] = hdr_off, *(int32_t *)(A.pool + d0) = o0;
+            __syncwarp();
+            set_hdr(0, lane == 0 ? CompHdr{0, 0, 0, 0, d0} : NUL);
+            if (tlen - plen == 0 && o0 >= tlen) end_score = 0;
+        }
+        if (status != 0 || end_score == 0) {
+            if (lane == 0) S.plan[0].op = WOP_DONE;
+        } else {
+            plan_next(S.plan[0]);
+        }
+    }
+    __syncthreads();
+    bool trimmed = false;
+    int op = S.plan[0].op;
+    for (int it = 0; op == WOP_COMPUTE; ++it) {
+        const WidePlan &now = S.plan[it & 1];
+        WidePlan &next = S.plan[(it + 1) & 1];
+        if (!planner) {
+            const int told = trimmed ? plan_compute<AW_WFA_CTA_U, NT, false>(PR, B, pat, txt, now, 0, 1, S.part)
+                                     : plan_compute<AW_WFA_CTA_U, NT, false, false>(PR, B, pat, txt, now, 0, 1, S.part);
+            if (lane == 0 && (told & 1)) S.at_end[it % 3] = 1;
+            if (lane == 0 && (told & 2)) S.beyond[it % 3] = 1;
+        } else {
+            if (lane == 0) S.at_end[(it + 1) % 3] = 0, S.beyond[(it + 1) % 3] = 0;
+            if (!trimmed) commit(s, mine), plan_next(next);
+        }
+        __syncthreads();
+        const bool end = S.at_end[it % 3] != 0;
+        if (!end && (trimmed || S.beyond[it % 3])) {
+            if (!trimmed) {
+                // from here on the trimmed ends count, and the plan made meanwhile is dropped
+                if (!planner) plan_trim(PR, now, tid, NT, S.part);
+                else s = now.s, slot = s % R, num_null = 0, status = 0;
+                trimmed = true;
+                __syncthreads();
+            }
+            if (planner) {
+                CompHdr out = lane < 5 ? now.out[lane] : NUL;
+                if (lane < 5 && (now.mask >> lane & 1)) {
+                    // no diagonal in the matrix: the empty range [lo, lo-1] of the scan
+                    if (S.part.k[lane] == INT_MIN) out.hi = out.lo - 1;
+                    else out.lo = -S.part.k[5 + lane], out.hi = S.part.k[lane];
+                }
+                __syncwarp();
+                part_reset(S.part, lane);
+                commit(now.s, out);
+                plan_next(next);
+            }
+            __syncthreads();
+        }
+        if (planner && end) end_score = now.s, status = 0;
+        op = end ? WOP_DONE : next.op;
+    }
+    if (planner && lane == 0) {
+        finish_pair<false>(A, PR, idx, pat, txt, ctab, HR, status, end_score, end_score >= 0 ? end_score : s, al.used);
+        atomicSub(A.queue + 1, 1);
+        give_back(pool_of(A), al);
+    }
+    __syncthreads();
 }
 
 // Build-time tuning of the warp kernel: CTAs per SM the registers are sized for (4 warps
@@ -1173,20 +1318,23 @@ __device__ void cta_pair(const WfaArgs &A, int idx, const HdrRing &HR, WidePlan 
 #define AW_WFA_MINB 4
 #endif
 #ifndef AW_WFA_WARP_U
-#define AW_WFA_WARP_U 4
+#define AW_WFA_WARP_U 2
 #endif
 constexpr int WU = AW_WFA_WARP_U;
 
+// Threads of a CTA: in high memory, the long pairs' planning warp comes on top.
+constexpr int wfa_threads(bool pig, int nt) { return nt + (pig ? 0 : 32); }
+
 template <bool PIG, int NT>
-__global__ void __launch_bounds__(NT, AW_WFA_MINB * WFA_CTA / NT) wfa_kernel(WfaArgs A, RingShape rs) {
+__global__ void __launch_bounds__(wfa_threads(PIG, NT), AW_WFA_MINB * WFA_CTA / NT) wfa_kernel(WfaArgs A, RingShape rs) {
     const int lane = threadIdx.x & 31;
     const WfaPen P = A.pen;
     extern __shared__ CompHdr hring_all[];
-    __shared__ Alloc allocs[NT / 32];
+    __shared__ Alloc allocs[wfa_threads(PIG, NT) / 32];
     Alloc &al = allocs[threadIdx.x >> 5];
-    {
-        // the long pairs first, each on the whole CTA (warp 0's header ring serves the
-        // planner; the warps take their own rings afterwards)
+    // the long pairs first, each on the whole CTA (the first warp's header ring serves the
+    // planner; the warps take their own rings afterwards)
+    if constexpr (PIG) {
         __shared__ WidePlan cplan;
         __shared__ WidePart cpart;
         __shared__ CtaPlanner cstate;
@@ -1197,7 +1345,17 @@ __global__ void __launch_bounds__(NT, AW_WFA_MINB * WFA_CTA / NT) wfa_kernel(Wfa
             const int pi = cpi;
             __syncthreads();
             if (pi >= A.n_long) break;
-            cta_pair<PIG, NT>(A, A.order_long[pi], HdrRing{hring_all, rs}, cplan, cpart, cstate, al);
+            cta_pair<NT>(A, A.order_long[pi], HdrRing{hring_all, rs}, cplan, cpart, cstate, al);
+        }
+    } else {
+        __shared__ CtaShared S;
+        for (;;) {
+            if (threadIdx.x == 0) S.next = A.n_long > 0 ? atomicAdd(A.queue + A.q_long, 1) : A.n_long;
+            __syncthreads();
+            const int pi = S.next;
+            __syncthreads();
+            if (pi >= A.n_long) break;
+            cta_open<NT>(A, A.order_long[pi], HdrRing{hring_all, rs}, S, allocs[NT / 32]);
         }
     }
     const HdrRing HR{hring_all + (threadIdx.x >> 5) * rs.entries(), rs};
@@ -1211,6 +1369,7 @@ __global__ void __launch_bounds__(NT, AW_WFA_MINB * WFA_CTA / NT) wfa_kernel(Wfa
         const WfaPairDev PR = A.pairs[idx];
         const int plen = PR.plen, tlen = PR.tlen;
         const uint8_t *pat = A.pat + PR.poff, *txt = A.txt + PR.toff;
+        const Bases bases = bases_of(A, PR);
         int64_t *ctab = A.ctab + PR.ctab_off;
         if (lane == 0) al.init();
         uint32_t bnext = 0, bend = 0;  // this lane's reserved piggyback blocks
@@ -1402,11 +1561,6 @@ __global__ void __launch_bounds__(NT, AW_WFA_MINB * WFA_CTA / NT) wfa_kernel(Wfa
                     out[c] = CompHdr{lo, hi, lo, 0, place};
                 }
             }
-            int32_t *oM = (int32_t *)(A.pool + out[CM].off);
-            int32_t *oI1 = a_i1 ? (int32_t *)(A.pool + out[CI1].off) : nullptr;
-            int32_t *oD1 = a_d1 ? (int32_t *)(A.pool + out[CD1].off) : nullptr;
-            int32_t *oI2 = a_i2 ? (int32_t *)(A.pool + out[CI2].off) : nullptr;
-            int32_t *oD2 = a_d2 ? (int32_t *)(A.pool + out[CD2].off) : nullptr;
             // trimmed ends (wavefront/wavefront_compute.c:654-690): the lowest and highest
             // diagonal whose offset lies in the matrix, per component, from the lanes' values
             int kmin[5], kmax[5];
@@ -1427,51 +1581,28 @@ __global__ void __launch_bounds__(NT, AW_WFA_MINB * WFA_CTA / NT) wfa_kernel(Wfa
                 }
                 if (status != 0) break;
             } else {
-                // WU diagonals per lane at a time: all input loads before any output store
-                const InHdr h_mm = in_hdr(A, m_misms), h_o1 = in_hdr(A, m_open1), h_i1 = in_hdr(A, i1),
-                            h_d1 = in_hdr(A, d1), h_o2 = in_hdr(A, m_open2), h_i2 = in_hdr(A, i2),
-                            h_d2 = in_hdr(A, d2);
-                for (int k0 = lo + lane; k0 <= hi; k0 += 32 * WU) {
-                    int32_t ins1[WU], ins2[WU], del1[WU], del2[WU], misms[WU];
-    #pragma unroll
-                    for (int u = 0; u < WU; ++u) {
-                        const int k = k0 + 32 * u;
-                        ins1[u] = max(getv_pred(h_o1, k - 1), getv_pred(h_i1, k - 1)) + 1;
-                        ins2[u] = max(getv_pred(h_o2, k - 1), getv_pred(h_i2, k - 1)) + 1;
-                        del1[u] = max(getv_pred(h_o1, k + 1), getv_pred(h_d1, k + 1));
-                        del2[u] = max(getv_pred(h_o2, k + 1), getv_pred(h_d2, k + 1));
-                        misms[u] = getv_pred(h_mm, k) + 1;
-                    }
-                    // the gap components are final: store them (and their trimmed ends) first, so
-                    // that only M stays live across its extension
-                    int32_t mo[WU];
-    #pragma unroll
-                    for (int u = 0; u < WU; ++u) {
-                        const int k = k0 + 32 * u;
-                        const int32_t best = max(max(del1[u], del2[u]), max(misms[u], max(ins1[u], ins2[u])));
-                        mo[u] = (k <= hi && in_matrix(best, k, plen, tlen)) ? best : WF_NULL;
-                        if (k > hi) continue;
-                        if (oI1) oI1[k - lo] = ins1[u];
-                        if (oD1) oD1[k - lo] = del1[u];
-                        if (oI2) oI2[k - lo] = ins2[u];
-                        if (oD2) oD2[k - lo] = del2[u];
-                        const int32_t vals[4] = {ins1[u], del1[u], ins2[u], del2[u]};
-    #pragma unroll
-                        for (int c = 0; c < 4; ++c)
-                            if (in_matrix(vals[c], k, plen, tlen))
-                                kmin[c + 1] = min(kmin[c + 1], k), kmax[c + 1] = max(kmax[c + 1], k);
-                        if (mo[u] != WF_NULL) kmin[CM] = min(kmin[CM], k), kmax[CM] = max(kmax[CM], k);
-                    }
-                    // then M[s], extended (the extend step of the next iteration, fused: the
-                    // offsets never round-trip through memory unextended)
-                    extend_n<WU>(PR, bases_of(A, PR), pat, txt, k0, 32, mo);
-    #pragma unroll
-                    for (int u = 0; u < WU; ++u) {
-                        const int k = k0 + 32 * u;
-                        if (k > hi) break;
-                        if (k == k_end && mo[u] != WF_NULL && mo[u] >= tlen) fused_reached = true;
-                        oM[k - lo] = mo[u];
-                    }
+                const InHdr h[7] = {in_hdr(A, m_misms), in_hdr(A, m_open1), in_hdr(A, i1), in_hdr(A, d1),
+                                    in_hdr(A, m_open2), in_hdr(A, i2),      in_hdr(A, d2)};
+                int32_t *dst[5];
+                int ilo = INT_MIN, ihi = INT_MAX;  // the diagonals that every input has
+#pragma unroll
+                for (int c = 0; c < 5; ++c) {
+                    dst[c] = alloc_c[c] ? (int32_t *)(A.pool + out[c].off) : nullptr;
+                    if (!alloc_c[c]) ihi = INT_MIN;
+                }
+#pragma unroll
+                for (int j = 0; j < 7; ++j) ilo = max(ilo, h[j].lo), ihi = min(ihi, h[j].hi);
+                bool beyond;  // not used
+                for (int kw = lo; kw <= hi; kw += 32 * WU) {
+                    if (kw > ilo && kw + 32 * WU <= ihi)
+                        wf_trip<WU, 32, true, false, true, false>(PR, bases, pat, txt, h, dst, lo, hi, kw + lane, kmin,
+                                                                  kmax, fused_reached, beyond);
+                    else if (hi - kw >= 32)
+                        wf_trip<WU, 32, false, true, true, false>(PR, bases, pat, txt, h, dst, lo, hi, kw + lane, kmin,
+                                                                  kmax, fused_reached, beyond);
+                    else
+                        wf_trip<1, 32, false, true, true, false>(PR, bases, pat, txt, h, dst, lo, hi, kw + lane, kmin,
+                                                                 kmax, fused_reached, beyond);
                 }
             }
             __syncwarp();
@@ -1907,13 +2038,13 @@ constexpr int WARP_RING_BYTES = 8 * 1024, WIDE_RING_BYTES = 96 * 1024;
 template <bool PIG, int NT>
 static cudaError_t launch_wfa_t(const WfaArgs &a, int ctas, cudaStream_t st) {
     const RingShape rs = ring_shape(a.pen, a.max_score_scope, WARP_RING_BYTES);
-    const size_t smem = (size_t)(NT / 32) * rs.entries() * sizeof(CompHdr);
+    const size_t smem = (size_t)(wfa_threads(PIG, NT) / 32) * rs.entries() * sizeof(CompHdr);
     if (smem > 48 * 1024) {
         const cudaError_t e =
             cudaFuncSetAttribute(wfa_kernel<PIG, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return e;
     }
-    wfa_kernel<PIG, NT><<<ctas, NT, smem, st>>>(a, rs);
+    wfa_kernel<PIG, NT><<<ctas, wfa_threads(PIG, NT), smem, st>>>(a, rs);
     return cudaGetLastError();
 }
 
@@ -2029,13 +2160,14 @@ cudaError_t launch_wfa_pack(const uint8_t *pat, int64_t pbytes, uint64_t *ppat, 
 }
 
 int wfa_occupancy(bool piggyback, int threads, const WfaPen &pen, int scope) {
-    const size_t smem = (size_t)(threads / 32) * ring_shape(pen, scope, WARP_RING_BYTES).entries() * sizeof(CompHdr);
+    const int nt = wfa_threads(piggyback, threads);
+    const size_t smem = (size_t)(nt / 32) * ring_shape(pen, scope, WARP_RING_BYTES).entries() * sizeof(CompHdr);
     const void *k = threads == WFA_BIG_CTA
                         ? (piggyback ? (const void *)wfa_kernel<true, WFA_BIG_CTA> : (const void *)wfa_kernel<false, WFA_BIG_CTA>)
                         : (piggyback ? (const void *)wfa_kernel<true, WFA_CTA> : (const void *)wfa_kernel<false, WFA_CTA>);
     if (smem > 48 * 1024) cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     int nb = 0;
-    const cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k, threads, smem);
+    const cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k, nt, smem);
     return e == cudaSuccess ? nb : 1;
 }
 

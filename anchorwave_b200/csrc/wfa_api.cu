@@ -49,7 +49,7 @@ std::atomic<int> g_wide_width{8192};
 std::atomic<int> g_wide_tail{1024};
 std::atomic<int> g_wide_cluster{8};
 // Pairs with pattern + text length from which a pair runs on a whole CTA (aw_set_wfa_long).
-std::atomic<int> g_long_sum{1536};
+std::atomic<int> g_long_sum{800};
 
 }  // namespace
 
@@ -94,29 +94,32 @@ struct wavefront_aligner_gpu {
 
 constexpr int64_t kClusterSum = 8000;  // pattern + text of a pair that starts on the cluster kernel
 
-// How many of the long pairs (largest first) run on big CTAs.  A pair's work grows with the
-// square of its length; a batch takes as long as its longest pair or as its work over all CTA
-// slots, and big CTAs shorten the first at the cost of the second.  Measured (small CTAs
-// only / this rule): 2,048 pairs of 0.1-10 kb in medium memory 97 / 45 ms, 4,096 in high
-// memory 66 / 43 ms; 8,192 and 16,384 pairs choose no or few big CTAs.  A speedup of 1.5 in its
-// place gave 72 / 45 ms, 2.5 54 / 45 ms.
+// How many of the long pairs (largest first) run on big CTAs.  A batch takes as long as its
+// longest pair or as its work over all CTA slots; big CTAs shorten the first at the cost of the
+// second.  A score costs a latency plus a share of the wavefront, so a pair's work grows with
+// length * (4000 + length) (lengths: pattern + text), and a big CTA speeds a pair up the more the
+// longer it is (against a small CTA that shares its SM with three others, pairs of 1, 4, 7 and
+// 10 kb at 3% by 1.3, 2.3, 2.9 and 3.5; the rule's factors are larger, as the longest pairs of a batch
+// may also be its most divergent ones).  Measured with a constant factor of 4 / with this rule:
+// pairs of 0.1-10 kb, high memory 4,096 44 / 33 ms, 8,192 79 / 60 ms, medium memory 2,048
+// 37 / 37 ms; 592 of 4 kb 15 / 11 ms.
 static int big_pairs(const std::vector<int32_t> &longest, const int *plen, const int *tlen, int sms) {
-    const double kSpeedup = 4.0;       // a pair on a big CTA against one on a small CTA
-    std::vector<double> cost(longest.size());
+    std::vector<double> cost(longest.size()), big_cost(longest.size());
     double rest = 0.0;
     for (size_t k = 0; k < longest.size(); ++k) {
         const double len = (double)plen[longest[k]] + tlen[longest[k]];
-        rest += cost[k] = len * len;
+        rest += cost[k] = len * (4000.0 + len);
+        big_cost[k] = cost[k] / std::min(8.0, 1.0 + len / 4000.0);
     }
     double best = 0.0, big = 0.0;
     int n_big = 0;
     for (size_t k = 0; k <= longest.size(); ++k) {
-        // k pairs on big CTAs; the small ones have the SMs' other slots
-        const double t_big = k ? std::max(cost[0] / kSpeedup, big / kSpeedup / sms) : 0.0;
-        const double t_small = k < longest.size() ? std::max(cost[k], (rest + big * 4 / kSpeedup) / (4.0 * sms)) : 0.0;
+        // k pairs on big CTAs, each in the place of four small ones
+        const double t_big = k ? std::max(big_cost[0], big / sms) : 0.0;
+        const double t_small = k < longest.size() ? std::max(cost[k], (rest + 4.0 * big) / (4.0 * sms)) : 0.0;
         const double t = std::max(t_big, t_small);
         if (k == 0 || t < 0.98 * best) best = t, n_big = (int)k;
-        if (k < longest.size()) big += cost[k], rest -= cost[k];
+        if (k < longest.size()) big += big_cost[k], rest -= cost[k];
     }
     return n_big;
 }
@@ -215,7 +218,10 @@ static int run_batch(wavefront_aligner_gpu *al, int n, const char *const *patter
     W.wide_width = wide_clusters > 0 ? std::max(0, g_wide_width.load()) : 0;
     W.wide_width_tail = std::min(W.wide_width, std::max(0, g_wide_tail.load()));
     W.wide_tail_pairs = std::max(1, wide_clusters);
+    // a CTA's pair: eight times the tail width, as starting it over on a cluster late in its scores costs
+    // more than the CTA takes to finish it (64 pairs of 1-10 kb: 28 ms with four times, 24 with eight)
     W.wide_width_cta = W.wide_width;
+    W.wide_tail_cta = (int)std::min<int64_t>(W.wide_width, 8 * (int64_t)W.wide_width_tail);
     const int64_t long_sum = g_long_sum.load();
     std::vector<int32_t> staged;
     // Rounds: every round restarts the pool and runs up to `chunk` pending pairs, largest
@@ -266,10 +272,6 @@ static int run_batch(wavefront_aligner_gpu *al, int n, const char *const *patter
             WCUDA(cudaEventRecord(al->e0, al->st));
             if (phase == 0) {
                 WfaArgs B = W;
-                // eight times the tail width: starting a pair over on a cluster late in its scores
-                // costs more than the big CTA takes to finish it (64 pairs of 1-10 kb: 28 ms with
-                // four times, 24 with eight)
-                B.wide_width_tail = (int)std::min<int64_t>(W.wide_width, 8 * (int64_t)W.wide_width_tail);
                 B.order_long = al->d_order.as<int32_t>(), B.n_long = n_big;
                 B.order = B.order_long, B.n = 0;
                 W.order_long = B.order_long + n_big, W.n_long = n_long - n_big;

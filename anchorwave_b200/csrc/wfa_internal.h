@@ -66,7 +66,8 @@ struct WfaArgs {
     int wide_width;       // warp kernel: a pair whose wavefront grows wider stops with WFA_WIDE (0 = never)
     int wide_width_tail;  // the same once every pair has started and at most wide_tail_pairs
     int wide_tail_pairs;  // still run on warps (<= wide_width)
-    int wide_width_cta;   // a pair on a whole CTA whose wavefront grows wider stops with WFA_WIDE
+    int wide_width_cta;   // the same for a pair on a whole CTA: the width that always stops it,
+    int wide_tail_cta;    // and the one of the tail
 };
 
 // Pool bytes are taken and given back in chunks of this size.

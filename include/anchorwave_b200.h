@@ -250,9 +250,11 @@ int wavefront_gpu_memory(const wavefront_aligner_gpu_t *aligner, int64_t *pair_m
 void aw_set_wfa_wide(int width, int tail_width, int cluster_ctas);
 /* Pairs whose pattern and text lengths sum to at least `min_length_sum` run first, each on a
  * whole CTA (the longest pairs of a batch otherwise set its duration, one warp each): four
- * warps, or sixteen for those that would outlast the batch; the others then run one per warp.  0: every pair starts on one
- * warp.  Default 1536.  A CTA's pair moves to the cluster kernel by the widths of
- * aw_set_wfa_wide, as a warp's does.  Results are identical.  Process-wide. */
+ * warps, or sixteen for those that would outlast the batch, and in high memory a warp that plans
+ * ahead of them; the others then run one per warp.  0: every pair starts on one warp.  Default
+ * 800.  A CTA's pair moves to the cluster kernel by the width of aw_set_wfa_wide, as a warp's
+ * does, and in the call's tail by eight times the tail width.  Results are identical.
+ * Process-wide. */
 void aw_set_wfa_long(int min_length_sum);
 /* Kernel launches of the last call (every round and phase) and, of them, the cluster
  * kernel's, with the number of pairs that moved to it. */

@@ -49,3 +49,24 @@ def test_cluster_scores(gpu, restatement, singletrack, pen):
     finally:
         wfa.set_wide(8192, 1024, 8)
         al.close()
+
+
+@pytest.mark.parametrize("pen", [(4, 4, 2, 24, 1), (4, 6, 2, 24, 2), (6, 8, 2, 75, 1)])
+@pytest.mark.parametrize("singletrack", [False, True])
+def test_cta_scores(gpu, restatement, singletrack, pen):
+    """The same pairs on CTAs of both sizes (few pairs, then many) and on warps."""
+    ps, ts = _pairs(12)
+    want = [restatement.wfa_align(p, t, *pen, singletrack, memory_mode=0) for p, t in zip(ps, ts)]
+    al = wfa.WfaAligner(*pen, singletrack=singletrack, memory_mode=0, max_memory_abort=2 << 30)
+    try:
+        wfa.set_wide(0, 0, 8)
+        for long_sum in (1, 1536, 0):
+            wfa.set_long(long_sum)
+            for times in (1, 80):
+                got, _ = al.align_batch(ps * times, ts * times)
+                for i, r in enumerate(got):
+                    assert r == want[i % len(want)], (long_sum, times, i)
+    finally:
+        wfa.set_wide(8192, 1024, 8)
+        wfa.set_long(800)
+        al.close()
