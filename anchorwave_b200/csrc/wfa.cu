@@ -595,11 +595,12 @@ __device__ void finish_pair(const WfaArgs &A, const WfaPairDev &PR, int idx, con
 // block from the lane's reserved run; lanes whose run is short reserve LANE_BLOCKS more in one
 // allocation of the warp (`wal`).  Every lane of the warp must call it.  Returns false when
 // the pool is exhausted.
+template <bool TRIM = true>
 __device__ __forceinline__ bool pig_trip(const WfaArgs &A, const WfaPairDev &PR, const uint8_t *pat,
                                          const uint8_t *txt, int kb, int g0, int G, int lo, int hi,
                                          const CompHdr (&in)[7], const CompHdr (&out)[5], int mask, int rcap,
                                          Alloc &wal, uint32_t &bnext, uint32_t &bend, int (&kmin)[5], int (&kmax)[5],
-                                         bool &reached) {
+                                         bool &reached, bool &beyond) {
     const int plen = PR.plen, tlen = PR.tlen, k_end = tlen - plen, lane = threadIdx.x & 31;
     const CompHdr &m_misms = in[0], &m_open1 = in[1], &i1 = in[2], &d1 = in[3], &m_open2 = in[4], &i2 = in[5],
                   &d2 = in[6];
@@ -629,6 +630,8 @@ __device__ __forceinline__ bool pig_trip(const WfaArgs &A, const WfaPairDev &PR,
                           : best == C[u][CI2].o ? C[u][CI2]
                                                 : C[u][CI1];
         C[u][CM] = Cell{in_matrix(best, k, plen, tlen) ? best : WF_NULL, (src.pc << 2) | 2u, src.pv};
+        const int32_t gap = max(max(C[u][CD1].o, C[u][CD2].o), max(C[u][CI1].o, C[u][CI2].o));
+        if (k <= hi && gap >= 0 && gap > min(tlen, k + plen)) beyond = true;
     }
     {
         int32_t mo[PIG_U];
@@ -682,7 +685,7 @@ __device__ __forceinline__ bool pig_trip(const WfaArgs &A, const WfaPairDev &PR,
             if (!(mask & (1 << c))) continue;
             int32_t *d = (int32_t *)(A.pool + out[c].off) + (k - lo);
             d[0] = C[u][c].o, d[rcap] = (int32_t)C[u][c].pc, d[2 * rcap] = (int32_t)C[u][c].pv;
-            if (in_matrix(C[u][c].o, k, plen, tlen)) kmin[c] = min(kmin[c], k), kmax[c] = max(kmax[c], k);
+            if (TRIM && in_matrix(C[u][c].o, k, plen, tlen)) kmin[c] = min(kmin[c], k), kmax[c] = max(kmax[c], k);
         }
     }
     return true;
@@ -707,8 +710,8 @@ struct WidePlan {
 // c in the matrix, k[5 + c] minus the lowest, k[10] 1 when the end cell was reached.
 struct __align__(16) WidePart {
     int k[12];
-    int retry, pad;           // a warp found the pool exhausted (CTA-cooperative piggyback mode)
-    unsigned long long used;  // pool bytes of the warps' block reservations (the same)
+    int pad[2];
+    unsigned long long used;  // pool bytes of the warps' block reservations (CTA-cooperative piggyback mode)
 };
 
 __device__ __forceinline__ void part_reset(WidePart &p, int lane) {
@@ -732,13 +735,6 @@ __device__ __forceinline__ PlanLane plan_lane(const WfaPen &P, int lane) {
     case 6: return PlanLane{CD2, P.e2, -1, -1};
     default: return PlanLane{CM, 0, 0, 0};
     }
-}
-// Lane j's input header of score s; returns the lanes whose input is not null.
-__device__ __forceinline__ unsigned plan_input(const WfaArgs &A, const int64_t *ctab, const HdrRing &HR, const PlanLane &L,
-                                               int s, int lane, CompHdr &h) {
-    h = CompHdr{1, -1, 0, 0, 0};
-    if (lane < 7 && s - L.dist >= 0) h = HR.get(A, ctab, L.comp, s - L.dist);
-    return __ballot_sync(0xffffffffu, lane < 7 && h.lo <= h.hi);
 }
 // The limits of the compute step and which I/D outputs exist (one of their inputs exists).
 __device__ __forceinline__ void plan_limits(const PlanLane &L, int lane, const CompHdr &h, unsigned some, int &lo, int &hi,
@@ -938,193 +934,19 @@ __device__ __noinline__ void plan_trim(const WfaPairDev &PR, const WidePlan &Q, 
     fold_partials(kmin, kmax, false, pp);
 }
 
-// CTA-cooperative mode, piggyback memory modes: one long pair on all threads of a CTA.  Warp 0
-// plans every score, a lane per input and per output component (the headers in the CTA's header
-// ring and the pool, the allocations), and all threads compute and extend the diagonals
-// lo + tid + NT*u; two CTA barriers per score.  The cell arithmetic, the limits, the trimming and
-// the backtrace are the warp's.  Every warp reserves its own block runs; no pair moves to the
-// cluster kernel.
-struct CtaPlanner {  // warp 0's state (shared memory)
-    int s, num_null, status, end_score;
-    int64_t hdr_off;
-    int64_t rbase;  // the rings' place and the elements of a slot's array
-    int rcap, pad;
-    Alloc al;
-};
-template <int NT>
-__device__ void cta_pair(const WfaArgs &A, int idx, const HdrRing &HR, WidePlan &plan, WidePart &part, CtaPlanner &Q,
-                         Alloc &wal) {
-    const int tid = threadIdx.x, lane = tid & 31;
-    const WfaPen P = A.pen;
-    const WfaPairDev PR = A.pairs[idx];
-    const int plen = PR.plen, tlen = PR.tlen;
-    const uint8_t *pat = A.pat + PR.poff, *txt = A.txt + PR.toff;
-    int64_t *ctab = A.ctab + PR.ctab_off;
-    const CompHdr NUL{1, -1, 0, 0, 0};
-    const int smax = PR.ctab_cap * HDR_CHUNK - 1;
-    // rings, and every warp's block reservations
-    const int SR = A.max_score_scope, R1 = P.e1 + 1, R2 = P.e2 + 1;
-    const int64_t ring_arrays = 3 * (int64_t)(SR + 2 * R1 + 2 * R2);
-    uint32_t bnext = 0, bend = 0;
-    if (lane == 0) wal.init();
-    // lane c < 5: component c's header of score sc
-    auto set_hdr = [&](int sc, const CompHdr &o) {
-        if (lane < 5) {
-            ((ScoreHdr *)(A.pool + Q.hdr_off))[sc % HDR_CHUNK].c[lane] = o;
-            HR.put(lane, sc, o);
-        }
-        __syncwarp();
-    };
-    auto plan_next = [&]() {
-        const PlanLane L = plan_lane(P, lane);
-        int s = Q.s, num_null = Q.num_null, status = 0;
-        for (;;) {
-            ++s;
-            if (s > smax) {
-                status = WFA_OVERFLOW;
-                break;
-            }
-            if (s % HDR_CHUNK == 0) {
-                const int64_t hb = warp_alloc(A, Q.al, (int64_t)sizeof(ScoreHdr) * HDR_CHUNK, lane);
-                if (hb < 0) {
-                    status = WFA_RETRY;
-                    break;
-                }
-                if (lane == 0) Q.hdr_off = hb, ctab[s / HDR_CHUNK] = hb;
-                __syncwarp();
-            }
-            CompHdr in;
-            const unsigned some = plan_input(A, ctab, HR, L, s, lane, in);
-            if (!some) {
-                set_hdr(s, NUL);
-                if (++num_null > A.max_score_scope) {  // the top of the next step: M[s] is empty
-                    status = -3;
-                    break;
-                }
-                continue;
-            }
-            num_null = 0;
-            int lo, hi, mask;
-            plan_limits(L, lane, in, some, lo, hi, mask);
-            const int width = hi - lo + 1;
-            const bool mine = lane < 5 && (mask >> lane & 1);
-            CompHdr out = NUL;
-            if (width > Q.rcap) {
-                const int nc = max(2 * Q.rcap, (width + 3) & ~3);
-                const int64_t nb = warp_alloc(A, Q.al, ring_arrays * nc * 4, lane);
-                if (nb < 0) {
-                    status = WFA_RETRY;
-                    break;
-                }
-                __syncwarp();
-                if (lane == 0) Q.rcap = nc, Q.rbase = nb;
-                __syncwarp();
-            }
-            if (mine) out = CompHdr{lo, hi, lo, Q.rcap, Q.rbase + pig_slot(lane, s, SR, R1, R2) * Q.rcap * 4};
-            if (lane < 7) plan.in[lane] = in;
-            if (lane < 5) plan.out[lane] = out;
-            if (lane == 0) {
-                plan.op = WOP_COMPUTE, plan.lo = lo, plan.hi = hi, plan.mask = mask;
-                Q.s = s, Q.num_null = 0;
-            }
-            return;
-        }
-        if (lane == 0) plan.op = WOP_DONE, Q.s = s, Q.status = status;
-    };
-    if (tid < 32) {
-        int status = 0, end_score = -1;
-        constexpr int rcap = 32;
-        if (lane == 0) Q.al.init(), Q.s = Q.num_null = 0, Q.rcap = rcap;
-        __syncwarp();
-        if (lane == 0) atomicAdd(A.queue + 1, 1), atomicAdd(A.queue + 3, 1);  // pairs running, started
-        part_reset(part, lane);
-        if (lane == 0) part.retry = 0, part.used = 0;
-        const int64_t rbase = warp_alloc(A, Q.al, ring_arrays * rcap * 4, lane);
-        if (rbase < 0) status = WFA_RETRY;
-        const int64_t h0 = status == 0 ? warp_alloc(A, Q.al, (int64_t)sizeof(ScoreHdr) * HDR_CHUNK, lane) : -1;
-        const int64_t d0 = h0 < 0 ? -1 : rbase;  // slot 0 of M
-        if (status == 0 && d0 < 0) status = WFA_RETRY;
-        if (status == 0) {
-            // M[0] = {0} on diagonal 0, extended
-            const int32_t o0 = (int32_t)lcp1(A, PR, pat, txt, 0, 0);
-            if (lane == 0) {
-                Q.hdr_off = h0, Q.rbase = rbase;
-                ctab[0] = h0;
-                *(int32_t *)(A.pool + d0) = o0;
-                ((uint32_t *)(A.pool + d0))[rcap] = 0u;
-                ((uint32_t *)(A.pool + d0))[2 * rcap] = BT_NULL;  // the start (0, 0)
-            }
-            __syncwarp();
-            set_hdr(0, lane == 0 ? CompHdr{0, 0, 0, rcap, d0} : NUL);
-            if (tlen - plen == 0 && o0 >= tlen) end_score = 0;
-        }
-        if (lane == 0) Q.status = status, Q.end_score = end_score;
-        if (status != 0 || end_score == 0) {
-            if (lane == 0) plan.op = WOP_DONE;
-        } else {
-            plan_next();
-        }
-    }
-    __syncthreads();
-    while (plan.op == WOP_COMPUTE) {
-        int kmin[5], kmax[5];
-        bool reached = false, ok = true;
-#pragma unroll
-        for (int c = 0; c < 5; ++c) kmin[c] = INT_MAX, kmax[c] = INT_MIN;
-        // a warp whose first diagonal lies beyond the wavefront has none in the trip
-        for (int kb = plan.lo; kb + (tid & ~31) <= plan.hi && ok; kb += NT * PIG_U)
-            ok = pig_trip(A, PR, pat, txt, kb, tid, NT, plan.lo, plan.hi, plan.in, plan.out, plan.mask,
-                          plan.out[CM].pad, wal, bnext, bend, kmin, kmax, reached);
-        fold_partials(kmin, kmax, reached, part);
-        if (!ok && lane == 0) part.retry = 1;
-        __syncthreads();
-        if (tid < 32) {
-            if (part.retry) {
-                if (lane == 0) plan.op = WOP_DONE, Q.status = WFA_RETRY;
-            } else {
-                CompHdr out = lane < 5 ? plan.out[lane] : NUL;
-                if (lane < 5 && (plan.mask >> lane & 1)) {
-                    // no diagonal in the matrix: the empty range [lo, lo-1] of the scan
-                    if (part.k[lane] == INT_MIN) out.hi = out.lo - 1;
-                    else out.lo = -part.k[5 + lane], out.hi = part.k[lane];
-                }
-                const bool reached = part.k[10] == 1;
-                __syncwarp();
-                part_reset(part, lane);
-                set_hdr(Q.s, out);
-                if (reached) {
-                    if (lane == 0) plan.op = WOP_DONE, Q.end_score = Q.s;
-                } else {
-                    plan_next();
-                }
-            }
-        }
-        __syncthreads();
-    }
-    if (lane == 0) atomicAdd(&part.used, (unsigned long long)wal.used);
-    __syncthreads();
-    if (tid == 0) {
-        finish_pair<true>(A, PR, idx, pat, txt, ctab, HR, Q.status, Q.end_score, Q.s, Q.al.used + (int64_t)part.used);
-        atomicSub(A.queue + 1, 1);
-    }
-    __syncthreads();
-    if (tid == 0) give_back(pool_of(A), Q.al);
-    if (lane == 0) give_back(pool_of(A), wal);
-}
-
-// CTA-cooperative mode, high memory: one long pair on a CTA of NT computing threads and one
-// planning warp.  As in the cluster kernel (below), wavefronts are not trimmed before the first
+// CTA-cooperative mode: one long pair on a CTA of NT computing threads and one planning warp.  As in the cluster kernel (below), wavefronts are not trimmed before the first
 // offset beyond the end of a sequence, so that the planner works a score ahead of the others and one
 // CTA barrier per score is left (two, with the plan between them, took 3.8 us a score at 2 kb,
 // half of it waiting for the plan; now 2.3).  A pair whose wavefront grows too wide stops with
-// WFA_WIDE for the cluster kernel.
+// WFA_WIDE for the cluster kernel; in the piggyback modes none does, and every warp reserves its own
+// block runs.
 struct CtaShared {
     WidePlan plan[2];
     WidePart part;
-    int at_end[3], beyond[3];
-    int next;  // position of the pair
+    int at_end[3], beyond[3], retry;  // retry: a warp found the pool exhausted
+    int next;                         // position of the pair
 };
-template <int NT>
+template <bool PIG, int NT>
 __device__ void cta_open(const WfaArgs &A, int idx, const HdrRing &HR, CtaShared &S, Alloc &al) {
     const int tid = threadIdx.x, lane = tid & 31;
     const bool planner = tid >= NT;
@@ -1143,6 +965,12 @@ __device__ void cta_open(const WfaArgs &A, int idx, const HdrRing &HR, CtaShared
     int s = 0, committed = 0, num_null = 0, status = 0, end_score = -1, s_hdr = 0, slot = 0;
     int64_t ring = -1, hdr_off = 0;
     CompHdr mine = NUL;
+    // piggyback: the rings' place and the elements of a slot's array, every warp's block run
+    const int SR = A.max_score_scope, R1 = P.e1 + 1, R2 = P.e2 + 1;
+    const int64_t ring_arrays = 3 * (int64_t)(SR + 2 * R1 + 2 * R2);
+    int rcap = 32;
+    uint32_t bnext = 0, bend = 0;
+    if (PIG && !planner && lane == 0) al.init();
     auto set_hdr = [&](int sc, const CompHdr &o) {
         if (lane < 5) {
             const int64_t off = sc >= s_hdr ? hdr_off : ctab[sc / HDR_CHUNK];
@@ -1192,6 +1020,28 @@ __device__ void cta_open(const WfaArgs &A, int idx, const HdrRing &HR, CtaShared
             // no diagonal beyond these has a cell
             lo = max(lo, -plen), hi = min(hi, tlen);
             const int width = hi - lo + 1;
+            if constexpr (PIG) {
+                if (width > rcap) {
+                    const int nc = max(2 * rcap, (width + 3) & ~3);
+                    const int64_t nb = warp_alloc(A, al, ring_arrays * nc * 4, lane);
+                    if (nb < 0) {
+                        status = WFA_RETRY;
+                        break;
+                    }
+                    rcap = nc, ring = nb;
+                }
+                if (lane < 5) {
+                    mine = mask >> lane & 1
+                               ? CompHdr{lo, hi, lo, rcap, ring + pig_slot(lane, s, SR, R1, R2) * rcap * 4}
+                               : NUL;
+                    q.out[lane] = mine;
+                    q.dst[lane] = mask >> lane & 1 ? (int32_t *)(A.pool + mine.off) : nullptr;
+                }
+                if (lane < 7) q.in[lane] = in;
+                if (lane == 0) q.op = WOP_COMPUTE, q.lo = lo, q.hi = hi, q.mask = mask, q.s = s;
+                __syncwarp();
+                return;
+            }
             // a wavefront too wide for the CTA: the cluster kernel re-runs the pair (past
             // wide_width_cta always; past wide_tail_cta in the call's tail, checked every 32
             // scores: every pair started and few still running)
@@ -1238,22 +1088,29 @@ __device__ void cta_open(const WfaArgs &A, int idx, const HdrRing &HR, CtaShared
             al.init();
             atomicAdd(A.queue + 1, 1), atomicAdd(A.queue + 3, 1);  // pairs running, started
             for (int b = 0; b < 3; ++b) S.at_end[b] = S.beyond[b] = 0;
+            S.retry = 0, S.part.used = 0;
         }
         __syncwarp();
         part_reset(S.part, lane);
-        if (A.singletrack) {
-            ring = warp_alloc(A, al, (int64_t)R * 4 * ring_cap * 4, lane);
+        if (PIG || A.singletrack) {
+            ring = warp_alloc(A, al, PIG ? ring_arrays * rcap * 4 : (int64_t)R * 4 * ring_cap * 4, lane);
             if (ring < 0) status = WFA_RETRY;
         }
         hdr_off = status == 0 ? warp_alloc(A, al, (int64_t)sizeof(ScoreHdr) * HDR_CHUNK, lane) : -1;
-        const int64_t d0 = hdr_off >= 0 ? warp_alloc(A, al, 16, lane) : -1;
+        const int64_t d0 = hdr_off < 0 ? -1 : PIG ? ring : warp_alloc(A, al, 16, lane);  // piggyback: M's slot 0
         if (status == 0 && d0 < 0) status = WFA_RETRY;
         if (status == 0) {
             // M[0] = {0} on diagonal 0, extended
             const int32_t o0 = (int32_t)lcp1(A, PR, pat, txt, 0, 0);
-            if (lane == 0) ctab[0] = hdr_off, *(int32_t *)(A.pool + d0) = o0;
+            if (lane == 0) {
+                ctab[0] = hdr_off, *(int32_t *)(A.pool + d0) = o0;
+                if (PIG) {
+                    ((uint32_t *)(A.pool + d0))[rcap] = 0u;
+                    ((uint32_t *)(A.pool + d0))[2 * rcap] = BT_NULL;  // the start (0, 0)
+                }
+            }
             __syncwarp();
-            set_hdr(0, lane == 0 ? CompHdr{0, 0, 0, 0, d0} : NUL);
+            set_hdr(0, lane == 0 ? CompHdr{0, 0, 0, PIG ? rcap : 0, d0} : NUL);
             if (tlen - plen == 0 && o0 >= tlen) end_score = 0;
         }
         if (status != 0 || end_score == 0) {
@@ -1269,8 +1126,23 @@ __device__ void cta_open(const WfaArgs &A, int idx, const HdrRing &HR, CtaShared
         const WidePlan &now = S.plan[it & 1];
         WidePlan &next = S.plan[(it + 1) & 1];
         if (!planner) {
-            const int told = trimmed ? plan_compute<AW_WFA_CTA_U, NT, false>(PR, B, pat, txt, now, 0, 1, S.part)
-                                     : plan_compute<AW_WFA_CTA_U, NT, false, false>(PR, B, pat, txt, now, 0, 1, S.part);
+            int told = 0;
+            if constexpr (PIG) {
+                int kmin[5], kmax[5];
+                bool reached = false, past = false, ok = true;
+#pragma unroll
+                for (int c = 0; c < 5; ++c) kmin[c] = INT_MAX, kmax[c] = INT_MIN;
+                // a warp whose first diagonal lies beyond the wavefront has none in the trip
+                for (int kb = now.lo; kb + (tid & ~31) <= now.hi && ok; kb += NT * PIG_U)
+                    ok = pig_trip(A, PR, pat, txt, kb, tid, NT, now.lo, now.hi, now.in, now.out, now.mask, now.out[CM].pad,
+                                  al, bnext, bend, kmin, kmax, reached, past);
+                if (trimmed) fold_partials(kmin, kmax, reached, S.part);
+                if (!ok && lane == 0) S.retry = 1;
+                told = (__any_sync(0xffffffffu, reached) ? 1 : 0) | (__any_sync(0xffffffffu, past) ? 2 : 0);
+            } else {
+                told = trimmed ? plan_compute<AW_WFA_CTA_U, NT, false>(PR, B, pat, txt, now, 0, 1, S.part)
+                               : plan_compute<AW_WFA_CTA_U, NT, false, false>(PR, B, pat, txt, now, 0, 1, S.part);
+            }
             if (lane == 0 && (told & 1)) S.at_end[it % 3] = 1;
             if (lane == 0 && (told & 2)) S.beyond[it % 3] = 1;
         } else {
@@ -1278,8 +1150,8 @@ __device__ void cta_open(const WfaArgs &A, int idx, const HdrRing &HR, CtaShared
             if (!trimmed) commit(s, mine), plan_next(next);
         }
         __syncthreads();
-        const bool end = S.at_end[it % 3] != 0;
-        if (!end && (trimmed || S.beyond[it % 3])) {
+        const bool stop = PIG && S.retry, end = S.at_end[it % 3] != 0 && !stop;
+        if (!end && !stop && (trimmed || S.beyond[it % 3])) {
             if (!trimmed) {
                 // from here on the trimmed ends count, and the plan made meanwhile is dropped
                 if (!planner) plan_trim(PR, now, tid, NT, S.part);
@@ -1301,15 +1173,23 @@ __device__ void cta_open(const WfaArgs &A, int idx, const HdrRing &HR, CtaShared
             }
             __syncthreads();
         }
-        if (planner && end) end_score = now.s, status = 0;
-        op = end ? WOP_DONE : next.op;
+        if (planner && end) {
+            end_score = now.s, status = 0;
+            if (PIG && trimmed) commit(now.s, lane < 5 ? now.out[lane] : NUL);  // read by the backtrace
+        }
+        if (planner && stop) status = WFA_RETRY;
+        op = end || stop ? WOP_DONE : next.op;
     }
+    if (PIG && !planner && lane == 0) atomicAdd(&S.part.used, (unsigned long long)al.used);
+    if (PIG) __syncthreads();
     if (planner && lane == 0) {
-        finish_pair<false>(A, PR, idx, pat, txt, ctab, HR, status, end_score, end_score >= 0 ? end_score : s, al.used);
+        finish_pair<PIG>(A, PR, idx, pat, txt, ctab, HR, status, end_score, end_score >= 0 ? end_score : s,
+                         al.used + (PIG ? (int64_t)S.part.used : 0));
         atomicSub(A.queue + 1, 1);
         give_back(pool_of(A), al);
     }
     __syncthreads();
+    if (PIG && !planner && lane == 0) give_back(pool_of(A), al);
 }
 
 // Build-time tuning of the warp kernel: CTAs per SM the registers are sized for (4 warps
@@ -1322,41 +1202,26 @@ __device__ void cta_open(const WfaArgs &A, int idx, const HdrRing &HR, CtaShared
 #endif
 constexpr int WU = AW_WFA_WARP_U;
 
-// Threads of a CTA: in high memory, the long pairs' planning warp comes on top.
-constexpr int wfa_threads(bool pig, int nt) { return nt + (pig ? 0 : 32); }
+// Threads of a CTA: the long pairs' planning warp comes on top.
+constexpr int wfa_threads(int nt) { return nt + 32; }
 
 template <bool PIG, int NT>
-__global__ void __launch_bounds__(wfa_threads(PIG, NT), AW_WFA_MINB * WFA_CTA / NT) wfa_kernel(WfaArgs A, RingShape rs) {
+__global__ void __launch_bounds__(wfa_threads(NT), NT > WFA_CTA ? 1 : PIG ? 3 : AW_WFA_MINB) wfa_kernel(WfaArgs A, RingShape rs) {
     const int lane = threadIdx.x & 31;
     const WfaPen P = A.pen;
     extern __shared__ CompHdr hring_all[];
-    __shared__ Alloc allocs[wfa_threads(PIG, NT) / 32];
+    __shared__ Alloc allocs[wfa_threads(NT) / 32];
     Alloc &al = allocs[threadIdx.x >> 5];
     // the long pairs first, each on the whole CTA (the first warp's header ring serves the
     // planner; the warps take their own rings afterwards)
-    if constexpr (PIG) {
-        __shared__ WidePlan cplan;
-        __shared__ WidePart cpart;
-        __shared__ CtaPlanner cstate;
-        __shared__ int cpi;
-        for (;;) {
-            if (threadIdx.x == 0) cpi = A.n_long > 0 ? atomicAdd(A.queue + A.q_long, 1) : A.n_long;
-            __syncthreads();
-            const int pi = cpi;
-            __syncthreads();
-            if (pi >= A.n_long) break;
-            cta_pair<NT>(A, A.order_long[pi], HdrRing{hring_all, rs}, cplan, cpart, cstate, al);
-        }
-    } else {
-        __shared__ CtaShared S;
-        for (;;) {
-            if (threadIdx.x == 0) S.next = A.n_long > 0 ? atomicAdd(A.queue + A.q_long, 1) : A.n_long;
-            __syncthreads();
-            const int pi = S.next;
-            __syncthreads();
-            if (pi >= A.n_long) break;
-            cta_open<NT>(A, A.order_long[pi], HdrRing{hring_all, rs}, S, allocs[NT / 32]);
-        }
+    __shared__ CtaShared S;
+    for (;;) {
+        if (threadIdx.x == 0) S.next = A.n_long > 0 ? atomicAdd(A.queue + A.q_long, 1) : A.n_long;
+        __syncthreads();
+        const int pi = S.next;
+        __syncthreads();
+        if (pi >= A.n_long) break;
+        cta_open<PIG, NT>(A, A.order_long[pi], HdrRing{hring_all, rs}, S, PIG ? al : allocs[NT / 32]);
     }
     const HdrRing HR{hring_all + (threadIdx.x >> 5) * rs.entries(), rs};
     for (; A.n > 0;) {
@@ -1573,8 +1438,9 @@ __global__ void __launch_bounds__(wfa_threads(PIG, NT), AW_WFA_MINB * WFA_CTA / 
                 int mask = 0;
                 for (int c = 0; c < 5; ++c) mask |= alloc_c[c] ? 1 << c : 0;
                 for (int kb = lo; kb <= hi; kb += 32 * PIG_U) {
+                    bool beyond;  // not used
                     if (!pig_trip(A, PR, pat, txt, kb, lane, 32, lo, hi, in7, out, mask, rcap, al, bnext, bend, kmin, kmax,
-                                  fused_reached)) {
+                                  fused_reached, beyond)) {
                         status = WFA_RETRY;
                         break;
                     }
@@ -2004,10 +1870,7 @@ __global__ void __launch_bounds__(WIDE_NT, 1) wfa_wide_kernel(WfaArgs A, RingSha
                 trimmed = true;
                 __syncthreads();
             }
-            if (planner && end) {
-                W.end_score = now.s, W.status = 0;
-                if (trimmed) finish_score(now, it & 1);
-            }
+            if (planner && end) W.end_score = now.s, W.status = 0;
             ++it;
             op = end ? WOP_DONE : plan[it & 1].op;
         }
@@ -2038,13 +1901,13 @@ constexpr int WARP_RING_BYTES = 8 * 1024, WIDE_RING_BYTES = 96 * 1024;
 template <bool PIG, int NT>
 static cudaError_t launch_wfa_t(const WfaArgs &a, int ctas, cudaStream_t st) {
     const RingShape rs = ring_shape(a.pen, a.max_score_scope, WARP_RING_BYTES);
-    const size_t smem = (size_t)(wfa_threads(PIG, NT) / 32) * rs.entries() * sizeof(CompHdr);
+    const size_t smem = (size_t)(wfa_threads(NT) / 32) * rs.entries() * sizeof(CompHdr);
     if (smem > 48 * 1024) {
         const cudaError_t e =
             cudaFuncSetAttribute(wfa_kernel<PIG, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return e;
     }
-    wfa_kernel<PIG, NT><<<ctas, wfa_threads(PIG, NT), smem, st>>>(a, rs);
+    wfa_kernel<PIG, NT><<<ctas, wfa_threads(NT), smem, st>>>(a, rs);
     return cudaGetLastError();
 }
 
@@ -2160,7 +2023,7 @@ cudaError_t launch_wfa_pack(const uint8_t *pat, int64_t pbytes, uint64_t *ppat, 
 }
 
 int wfa_occupancy(bool piggyback, int threads, const WfaPen &pen, int scope) {
-    const int nt = wfa_threads(piggyback, threads);
+    const int nt = wfa_threads(threads);
     const size_t smem = (size_t)(nt / 32) * ring_shape(pen, scope, WARP_RING_BYTES).entries() * sizeof(CompHdr);
     const void *k = threads == WFA_BIG_CTA
                         ? (piggyback ? (const void *)wfa_kernel<true, WFA_BIG_CTA> : (const void *)wfa_kernel<false, WFA_BIG_CTA>)

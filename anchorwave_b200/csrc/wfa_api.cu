@@ -98,25 +98,24 @@ constexpr int64_t kClusterSum = 8000;  // pattern + text of a pair that starts o
 // longest pair or as its work over all CTA slots; big CTAs shorten the first at the cost of the
 // second.  A score costs a latency plus a share of the wavefront, so a pair's work grows with
 // length * (4000 + length) (lengths: pattern + text), and a big CTA speeds a pair up the more the
-// longer it is (against a small CTA that shares its SM with three others, pairs of 1, 4, 7 and
-// 10 kb at 3% by 1.3, 2.3, 2.9 and 3.5; the rule's factors are larger, as the longest pairs of a batch
-// may also be its most divergent ones).  Measured with a constant factor of 4 / with this rule:
-// pairs of 0.1-10 kb, high memory 4,096 44 / 33 ms, 8,192 79 / 60 ms, medium memory 2,048
-// 37 / 37 ms; 592 of 4 kb 15 / 11 ms.
+// longer it is: against a small CTA that shares its SM with three others, pairs of 1, 4, 7 and
+// 10 kb at 3% by 1.3, 2.3, 2.9 and 3.5.  Lengths do not show how divergent a pair is, so the
+// longest one counts twice.  Measured with a constant speedup of 4 / with this rule: pairs of
+// 0.1-10 kb, high memory 4,096 44 / 34 ms, 8,192 79 / 59 ms, medium memory 2,048 37 / 36 ms.
 static int big_pairs(const std::vector<int32_t> &longest, const int *plen, const int *tlen, int sms) {
     std::vector<double> cost(longest.size()), big_cost(longest.size());
     double rest = 0.0;
     for (size_t k = 0; k < longest.size(); ++k) {
         const double len = (double)plen[longest[k]] + tlen[longest[k]];
         rest += cost[k] = len * (4000.0 + len);
-        big_cost[k] = cost[k] / std::min(8.0, 1.0 + len / 4000.0);
+        big_cost[k] = cost[k] / std::min(4.0, 1.0 + len / 8000.0);
     }
     double best = 0.0, big = 0.0;
     int n_big = 0;
     for (size_t k = 0; k <= longest.size(); ++k) {
         // k pairs on big CTAs, each in the place of four small ones
-        const double t_big = k ? std::max(big_cost[0], big / sms) : 0.0;
-        const double t_small = k < longest.size() ? std::max(cost[k], (rest + 4.0 * big) / (4.0 * sms)) : 0.0;
+        const double t_big = k ? std::max(2.0 * big_cost[0], big / sms) : 0.0;
+        const double t_small = k < longest.size() ? std::max(2.0 * cost[k], (rest + 4.0 * big) / (4.0 * sms)) : 0.0;
         const double t = std::max(t_big, t_small);
         if (k == 0 || t < 0.98 * best) best = t, n_big = (int)k;
         if (k < longest.size()) big += big_cost[k], rest -= cost[k];

@@ -72,9 +72,11 @@ struct WfaArgs {
 
 // Pool bytes are taken and given back in chunks of this size.
 constexpr int64_t WFA_CHUNK = 256 << 10;
-// CTA sizes of the kernel: WFA_CTA threads (four fit an SM), or WFA_BIG_CTA (one per SM) for
-// the pairs that would outlast their batch on the small ones.
-constexpr int WFA_CTA = 128, WFA_BIG_CTA = 512;
+// Computing threads of the kernel's CTAs, beside a planning warp: WFA_CTA (four CTAs fit an SM,
+// three in the piggyback modes, whose trips need the registers: 2,048 pairs 36.7 against 39.3 ms
+// with four), or WFA_BIG_CTA (one per SM; sixteen warps with the planner's) for the pairs that
+// would outlast their batch on the small ones.
+constexpr int WFA_CTA = 128, WFA_BIG_CTA = 480;
 
 cudaError_t launch_wfa(const WfaArgs &a, int threads, int ctas, cudaStream_t st);
 // The cluster kernel (high memory: standard and Singletrack): one cluster of `cl` CTAs per
