@@ -954,8 +954,8 @@ def main():
         "tuning": tuning,
         "latency_ms": {"batch_step_p50": float(np.percentile(step_ms, 50)),
                        "batch_step_p99": float(np.percentile(step_ms, 99)),
-                       "serving_p50": serving["latency_ms_p50"] if serving else None,
-                       "serving_p99": serving["latency_ms_p99"] if serving else None,
+                       "serving_p50": (serving or {}).get("latency_ms_p50"),
+                       "serving_p99": (serving or {}).get("latency_ms_p99"),
                        "plain_per_call_p50": plain["latency_ms_p50"], "plain_per_call_p99": plain["latency_ms_p99"]},
         "plain_per_call": plain,
         "plain_5kb": plain5,
