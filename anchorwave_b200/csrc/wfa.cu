@@ -1,13 +1,14 @@
 // Gap-affine-2p end-to-end WFA (WFA2-lib as AnchorWave configures it:
 // src/myImportandFunction/WfaAlignment.cpp:143-170) on sm_100a.
 //
-// One warp per pair; the lanes cover the diagonals of a wavefront.  Per score s:
+// A warp, a CTA or a cluster of CTAs per pair, by length; its threads cover the diagonals of a
+// wavefront.  Per score s:
 //   * extend M[s] (wavefront/wavefront_extend.c:86-121): each lane advances its
-//     diagonal by comparing 32 bases of pattern and text at a time in 2-bit copies of
-//     the sequences (one XOR and __ffsll per 32 bases; the run also ends at the end of
-//     either sequence); pairs with any byte other than A, C, G, T (the reference compares
-//     raw characters) compare 8 bytes at a time instead, where the sentinels after each
-//     sequence ('!' pattern, '?' text, wavefront/wavefront_sequences.c:37-39) stop the run;
+//     diagonal by comparing 16, then 32 bases of pattern and text at a time in 2-bit copies
+//     of the sequences (the run also ends at the end of either sequence); pairs with any byte
+//     other than A, C, G, T (the reference compares raw characters) compare 8 bytes at a time
+//     instead, where the sentinels after each sequence ('!' pattern, '?' text,
+//     wavefront/wavefront_sequences.c:37-39) stop the run;
 //   * end-to-end check on diagonal tlen-plen (wavefront/wavefront_termination.c:37-60);
 //   * compute s+1 from M[s-x], M[s-o1-e1], I1/D1[s-e1], M[s-o2-e2], I2/D2[s-e2]
 //     (wavefront/wavefront_compute_affine2p.c:45-106) over the limits of
@@ -960,6 +961,29 @@ __device__ void cta_open(const WfaArgs &A, int idx, const HdrRing &HR, CtaShared
     const int smax = PR.ctab_cap * HDR_CHUNK - 1;
     const int R = (P.e1 > P.e2 ? P.e1 : P.e2) + 1, ring_cap = plen + tlen + 8;
     const PlanLane L = plan_lane(P, lane);
+    // where this lane of the planner reads its input and writes its component (no rings: the
+    // pool).  Kept for the high-memory planner only, which bounds a score of short wavefronts (4,096
+    // pairs 33.3 -> 32.4 ms, 16,384 103 -> 96); the piggyback trips need the registers.
+    const bool rings = !PIG && HR.sh.mm >= 0;
+    const CompHdr *const rd = rings ? HR.at(L.comp, 0) : nullptr;
+    CompHdr *const wr = rings ? HR.at(min(lane, 4), 0) : nullptr;
+    const int rd_mask = HR.mask(L.comp), wr_mask = HR.mask(min(lane, 4));
+    // the planner's place in its chunk, the same in all lanes
+    int64_t cur = 0, chunk_end = 0;
+    auto alloc = [&](int64_t bytes) -> int64_t {
+        if constexpr (PIG) return warp_alloc(A, al, bytes, lane);
+        bytes = (bytes + 15) & ~(int64_t)15;
+        if (cur + bytes > chunk_end) {
+            int ok = lane == 0 ? take_chunk(pool_of(A), al, bytes) : 0;
+            ok = __shfl_sync(0xffffffffu, ok, 0);
+            if (!ok) return -1;
+            __syncwarp();
+            cur = al.cur, chunk_end = al.end;
+        }
+        const int64_t r = cur;
+        cur += bytes;
+        return r;
+    };
     // the planner's state: the planned score, the last one with headers, the header chunk of the
     // scores from s_hdr on, the planned score's header of component `lane`
     int s = 0, committed = 0, num_null = 0, status = 0, end_score = -1, s_hdr = 0, slot = 0;
@@ -975,7 +999,8 @@ __device__ void cta_open(const WfaArgs &A, int idx, const HdrRing &HR, CtaShared
         if (lane < 5) {
             const int64_t off = sc >= s_hdr ? hdr_off : ctab[sc / HDR_CHUNK];
             ((ScoreHdr *)(A.pool + off))[sc % HDR_CHUNK].c[lane] = o;
-            HR.put(lane, sc, o);
+            if (rings) wr[sc & wr_mask] = o;
+            else HR.put(lane, sc, o);
         }
         __syncwarp();
     };
@@ -994,7 +1019,7 @@ __device__ void cta_open(const WfaArgs &A, int idx, const HdrRing &HR, CtaShared
                 break;
             }
             if (s % HDR_CHUNK == 0) {
-                const int64_t hb = warp_alloc(A, al, (int64_t)sizeof(ScoreHdr) * HDR_CHUNK, lane);
+                const int64_t hb = alloc((int64_t)sizeof(ScoreHdr) * HDR_CHUNK);
                 if (hb < 0) {
                     status = WFA_RETRY;
                     break;
@@ -1005,7 +1030,7 @@ __device__ void cta_open(const WfaArgs &A, int idx, const HdrRing &HR, CtaShared
             }
             // the scores since the last committed one are null
             CompHdr in = NUL;
-            if (lane < 7 && s - L.dist >= 0 && s - L.dist <= committed) in = HR.get(A, ctab, L.comp, s - L.dist);
+            if (lane < 7 && s - L.dist >= 0 && s - L.dist <= committed) in = rings ? rd[(s - L.dist) & rd_mask] : HR.get(A, ctab, L.comp, s - L.dist);
             const unsigned some = __ballot_sync(0xffffffffu, lane < 7 && in.lo <= in.hi);
             if (!some) {
                 if (++num_null > A.max_score_scope) {  // the top of the next step: M[s] is empty
@@ -1023,7 +1048,7 @@ __device__ void cta_open(const WfaArgs &A, int idx, const HdrRing &HR, CtaShared
             if constexpr (PIG) {
                 if (width > rcap) {
                     const int nc = max(2 * rcap, (width + 3) & ~3);
-                    const int64_t nb = warp_alloc(A, al, ring_arrays * nc * 4, lane);
+                    const int64_t nb = alloc(ring_arrays * nc * 4);
                     if (nb < 0) {
                         status = WFA_RETRY;
                         break;
@@ -1060,7 +1085,7 @@ __device__ void cta_open(const WfaArgs &A, int idx, const HdrRing &HR, CtaShared
                 break;
             }
             const int64_t wb = (((int64_t)width * 4) + 15) & ~(int64_t)15;
-            const int64_t blk = warp_alloc(A, al, wb * (A.singletrack ? 1 : __popc(mask)), lane);
+            const int64_t blk = alloc(wb * (A.singletrack ? 1 : __popc(mask)));
             if (blk < 0) {
                 status = WFA_RETRY;
                 break;
@@ -1093,11 +1118,11 @@ __device__ void cta_open(const WfaArgs &A, int idx, const HdrRing &HR, CtaShared
         __syncwarp();
         part_reset(S.part, lane);
         if (PIG || A.singletrack) {
-            ring = warp_alloc(A, al, PIG ? ring_arrays * rcap * 4 : (int64_t)R * 4 * ring_cap * 4, lane);
+            ring = alloc(PIG ? ring_arrays * rcap * 4 : (int64_t)R * 4 * ring_cap * 4);
             if (ring < 0) status = WFA_RETRY;
         }
-        hdr_off = status == 0 ? warp_alloc(A, al, (int64_t)sizeof(ScoreHdr) * HDR_CHUNK, lane) : -1;
-        const int64_t d0 = hdr_off < 0 ? -1 : PIG ? ring : warp_alloc(A, al, 16, lane);  // piggyback: M's slot 0
+        hdr_off = status == 0 ? alloc((int64_t)sizeof(ScoreHdr) * HDR_CHUNK) : -1;
+        const int64_t d0 = hdr_off < 0 ? -1 : PIG ? ring : alloc(16);  // piggyback: M's slot 0
         if (status == 0 && d0 < 0) status = WFA_RETRY;
         if (status == 0) {
             // M[0] = {0} on diagonal 0, extended
