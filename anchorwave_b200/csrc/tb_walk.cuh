@@ -15,7 +15,7 @@
 // larger drift is a miss: the tile at the walk's position is fetched and the tiles ahead of
 // it again.  Bound by the tiles' latency; measured against byte-by-byte walks over tiles
 // fetched on a miss: one 5 kb pair 1.25 -> 0.14 ms, 768 pairs of 0.2-20 kb 6.8 -> 0.8 ms, four
-// banded pairs of 60-160 kb 85 -> 6.8 ms, 128 Singletrack pairs of 2-8 kb 6.6 -> 0.65 ms.
+// banded pairs of 60-160 kb 85 -> 10 ms, 128 Singletrack pairs of 2-8 kb 6.6 -> 0.6 ms.
 #pragma once
 #include <stdint.h>
 #include <climits>

@@ -510,7 +510,7 @@ WFA_LONG_PAIRS = ((12_000, 0.15), (24_000, 0.12), (40_000, 0.08))
 def wfa_long_measurement(npairs: int, rank: int, cpu: bool):
     """Single long divergent intervals through the Singletrack WFA (high memory, penalties
     x=4, o1=4, e1=2, o2=24, e2=1), one call each: the device time of the call (a pair whose
-    wavefronts outgrow a warp or a CTA moves to the 8-CTA cluster kernel) and, for the first,
+    wavefronts outgrow a warp or a CTA moves to the cluster kernel) and, for the first,
     the same call with every pair kept on one warp; beside them the reference's WFA2 code on
     one host thread on the same interval (status, score and operation string compared)."""
     import time
@@ -657,11 +657,8 @@ def long_banded_measurement(rank: int, cpu: bool, npairs: int = 64, lmin: int = 
     warm.upload()
     warm.execute()
     warm.close()
-    # the autotuner picks the banded kernel's columns per lane (4, 8, or the per-batch rule) on the
-    # four pairs with the most band cells, score-only: the batch's largest pairs hold most of its
-    # cells and run first, together, in its first wave.  Samples of small or random pairs (alone,
-    # or with a traceback budget scaled to them) are chain-bound where the whole workload is
-    # work-bound, and picked 4 columns, which made the whole workload 20-25% slower than 8.
+    # the autotuner's trials of the banded kernel, on the four pairs with the most band cells,
+    # score-only (the kernel has one lane width, so they differ by noise only)
     from anchorwave_b200 import autotune
     t_tune = time.perf_counter()
     pick = sorted(sorted(range(len(ps)), key=lambda i: -pair_cells[i])[:4])
