@@ -233,8 +233,8 @@ static int run_batch(wavefront_aligner_gpu *al, int n, const char *const *patter
     float total_ms = 0.f;
     int launches = 0;
     // A call of a few pairs: its long ones start on the cluster kernel, where they would end up
-    // (10 kb at 5%: 15.8 ms against 17.5 by way of a CTA and 23 on a CTA to the end; at small
-    // scores the two cost about the same per score).
+    // (one pair at 5%: 10 kb 8.3 ms against 13.6 on a CTA to the end, 5 kb 4.1 against 5.4, 2 kb
+    // 1.7 against 1.5).
     std::vector<int32_t> first = order;
     if (W.wide_width > 0 && n <= wide_clusters) {
         auto is_long = [&](int32_t i) { return (int64_t)plen[i] + tlen[i] >= kClusterSum; };
