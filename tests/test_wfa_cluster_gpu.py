@@ -70,3 +70,22 @@ def test_cta_scores(gpu, restatement, singletrack, pen):
         wfa.set_wide(8192, 1024, 8)
         wfa.set_long(800)
         al.close()
+
+
+def test_cluster_beyond_shared_memory(gpu, restatement):
+    """Sequences too long for the cluster kernel's shared memory: extended from global memory."""
+    rng = np.random.default_rng(5)
+    t = rng.integers(0, 4, 210_000).astype(np.uint8)
+    q = np.delete(t, rng.integers(0, len(t), 12))
+    at = rng.integers(0, len(q), 30)
+    q[at] = (q[at] + 1) & 3
+    p, x = W.to_ascii(t), W.to_ascii(q)
+    al = wfa.WfaAligner(4, 4, 2, 24, 1, singletrack=True, max_memory_abort=2 << 30)
+    try:
+        wfa.set_wide(1, 1, 8)
+        (got,), _ = al.align_batch([p], [x])
+        assert al.launches()[1] == 1
+    finally:
+        wfa.set_wide(8192, 1024, 8)
+        al.close()
+    assert got == restatement.wfa_align(p, x, 4, 4, 2, 24, 1, True, memory_mode=0)
