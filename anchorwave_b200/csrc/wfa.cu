@@ -944,8 +944,10 @@ __device__ __noinline__ void plan_trim(const WfaPairDev &PR, const WidePlan &Q, 
 struct CtaShared {
     WidePlan plan[2];
     WidePart part;
-    int at_end[3], beyond[3], retry;  // retry: a warp found the pool exhausted
-    int next;                         // position of the pair
+    // flags of step it at it % 3 (a fast warp may set those of step it + 1 before a slow one has
+    // read step it's); retry: a warp found the pool exhausted
+    int at_end[3], beyond[3], retry[3];
+    int next;  // position of the pair
 };
 template <bool PIG, int NT>
 __device__ void cta_open(const WfaArgs &A, int idx, const HdrRing &HR, CtaShared &S, Alloc &al) {
@@ -1112,8 +1114,8 @@ __device__ void cta_open(const WfaArgs &A, int idx, const HdrRing &HR, CtaShared
         if (lane == 0) {
             al.init();
             atomicAdd(A.queue + 1, 1), atomicAdd(A.queue + 3, 1);  // pairs running, started
-            for (int b = 0; b < 3; ++b) S.at_end[b] = S.beyond[b] = 0;
-            S.retry = 0, S.part.used = 0;
+            for (int b = 0; b < 3; ++b) S.at_end[b] = S.beyond[b] = S.retry[b] = 0;
+            S.part.used = 0;
         }
         __syncwarp();
         part_reset(S.part, lane);
@@ -1162,7 +1164,7 @@ __device__ void cta_open(const WfaArgs &A, int idx, const HdrRing &HR, CtaShared
                     ok = pig_trip(A, PR, pat, txt, kb, tid, NT, now.lo, now.hi, now.in, now.out, now.mask, now.out[CM].pad,
                                   al, bnext, bend, kmin, kmax, reached, past);
                 if (trimmed) fold_partials(kmin, kmax, reached, S.part);
-                if (!ok && lane == 0) S.retry = 1;
+                if (!ok && lane == 0) S.retry[it % 3] = 1;
                 told = (__any_sync(0xffffffffu, reached) ? 1 : 0) | (__any_sync(0xffffffffu, past) ? 2 : 0);
             } else {
                 told = trimmed ? plan_compute<AW_WFA_CTA_U, NT, false>(PR, B, pat, txt, now, 0, 1, S.part)
@@ -1171,11 +1173,11 @@ __device__ void cta_open(const WfaArgs &A, int idx, const HdrRing &HR, CtaShared
             if (lane == 0 && (told & 1)) S.at_end[it % 3] = 1;
             if (lane == 0 && (told & 2)) S.beyond[it % 3] = 1;
         } else {
-            if (lane == 0) S.at_end[(it + 1) % 3] = 0, S.beyond[(it + 1) % 3] = 0;
+            if (lane == 0) S.at_end[(it + 1) % 3] = 0, S.beyond[(it + 1) % 3] = 0, S.retry[(it + 1) % 3] = 0;
             if (!trimmed) commit(s, mine), plan_next(next);
         }
         __syncthreads();
-        const bool stop = PIG && S.retry, end = S.at_end[it % 3] != 0 && !stop;
+        const bool stop = PIG && S.retry[it % 3] != 0, end = S.at_end[it % 3] != 0 && !stop;
         if (!end && !stop && (trimmed || S.beyond[it % 3])) {
             if (!trimmed) {
                 // from here on the trimmed ends count, and the plan made meanwhile is dropped
