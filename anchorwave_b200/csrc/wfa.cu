@@ -1619,6 +1619,8 @@ __global__ void __launch_bounds__(WIDE_NT, 1) wfa_wide_kernel(WfaArgs A, RingSha
     CompHdr mine = NUL;  // a planner's lane c < 5: component c's header of the planned score
     int64_t used = 0;  // the leader's pool bytes for the pair
     int it = 0, np = 0;
+    // every CTA of the cluster has started (and cleared ann) before one writes another's shared memory
+    cl.sync();
 
     // ---- planner helpers (all lanes of the planning warp)
     auto carve = [&](int64_t bytes) -> int64_t {
