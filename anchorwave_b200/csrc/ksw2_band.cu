@@ -152,9 +152,10 @@ struct RowWords {  // columns 0, 2 in d[0]; 1, 3 in d[1]
 // lane took 0.45 us a step against 0.25 and were no faster on 512 pairs of 5 kb at w = 50%,
 // which are bound by their work: 15.4 against 14.1 ms.)
 constexpr int NP = 2, C = 2 * NP, SW = 32 * C;
-// Traceback layout: words of 4 columns (state bytes, or v then u bytes), NG words per step.  The
-// word of group g (columns 4g..4g+3 of the strip) and row j is stored (j - jlo) + 4g steps from
-// the strip's start.
+// Traceback layout: words of 4 columns (state bytes, or v then u bytes), NG words per slot.  The
+// word of group g (columns 4g..4g+3 of the strip) and row j lies in slot (j - jlo) + 4g from the
+// strip's start.  The next strip of the pair starts after as many slots as this one has rows: the
+// corner that the skew leaves free at its start is where this one's last rows end.
 constexpr int NG = SW / 4;
 
 constexpr int BAND_WARPS = 4;  // per CTA: small CTAs spread a pair's strips over the SMs
@@ -209,8 +210,10 @@ __global__ void __launch_bounds__(32 * BAND_WARPS, 4) ksw_band_kernel(BandArgs A
         // a recompute round reads the columns of the first pass and writes none
         uint2 *bnd_me = lane == 31 && !last_strip && !A.walk ? A.bnd + St.bnd_off : nullptr;
         const bool store_tb = CIGAR && (!P.ckpt || A.store_ckpt);  // this strip's traceback is kept
-        // this lane's words completed at step 0 (row rs - c0 - 3 of group 0, slot jstart - 3 - jlo)
-        const int slot0 = jstart - 3 - jlo;
+        // this lane's word completed at step 0 (row rs - c0 - 3 of group 0, slot jstart - 3 - jlo), and
+        // its stored row; only words of stored rows are written, the slots are shared with others
+        const int slot0 = jstart - 3 - jlo, row0 = slot0 - 4 * lane;
+        const unsigned nrows = col0 < tlen ? (unsigned)(St.jend - jlo + 1) : 0u;
         uint8_t *tbp = CIGAR ? A.tb + St.tb_off + ((int64_t)slot0 * NG + lane) * WB : nullptr;
         BandRes *R = A.res + un.x;
         // steps whose cells all lie strictly inside the band
@@ -267,13 +270,14 @@ __global__ void __launch_bounds__(32 * BAND_WARPS, 4) ksw_band_kernel(BandArgs A
         uint32_t qnext = code_of(jstart + lane), qcur = 0, bx = 0, by = 0;
         int bh = 0;
         bool failed = false, stopped = false;
-        // the words of this step into the traceback
-        auto store_words = [&](const uint32_t (&d)[NP], const uint32_t (&d2)[NP], uint8_t *dst) {
+        // the words of step k into the traceback
+        auto store_words = [&](const uint32_t (&d)[NP], const uint32_t (&d2)[NP], uint8_t *dst, int k) {
+            const uint32_t a = words.put(d);
             if constexpr (MODE == TRACKS) {
-                const uint32_t a = words.put(d), b = words2.put(d2);
-                __stcs(reinterpret_cast<uint2 *>(dst), make_uint2(a, b));
+                const uint32_t b = words2.put(d2);
+                if ((unsigned)(row0 + k) < nrows) __stcs(reinterpret_cast<uint2 *>(dst), make_uint2(a, b));
             } else {
-                __stcs(reinterpret_cast<uint32_t *>(dst), words.put(d));
+                if ((unsigned)(row0 + k) < nrows) __stcs(reinterpret_cast<uint32_t *>(dst), a);
             }
         };
         // the last column's entry: x, v, x2 as bytes (a field's bits 4-11) and H
@@ -408,7 +412,7 @@ __global__ void __launch_bounds__(32 * BAND_WARPS, 4) ksw_band_kernel(BandArgs A
                     } else {
                         H[C - 1] += fval(V[NP - 1], 1);
                     }
-                    if (CIGAR && store_tb) store_words(d, d2, tb + i * (NG * WB));
+                    if (CIGAR && store_tb) store_words(d, d2, tb + i * (NG * WB), kb + i);
                     if (entries && bnd_me) store_entry(entry + i);
                 }
                 continue;
@@ -452,12 +456,12 @@ __global__ void __launch_bounds__(32 * BAND_WARPS, 4) ksw_band_kernel(BandArgs A
                         }
                         if (f0 < C) H[C - 1] += fval(V[NP - 1], 1);
                     }
-                    if (CIGAR && store_tb) store_words(d, d2, tb + i * (NG * WB));
+                    if (CIGAR && store_tb) store_words(d, d2, tb + i * (NG * WB), kb + i);
                     if (entries && bnd_me && je0 + i <= jend) store_entry(entry + i);
                 }
                 continue;
             }
-            if (full && k >= kr0 && kend <= kr1 && slot0 + k >= 0) {
+            if (full && k >= kr0 && kend <= kr1) {
                 // the right edge alone: which lanes are computed, and how far the fill reaches
                 h_state = H_NONE;
 #pragma unroll 2
@@ -488,7 +492,7 @@ __global__ void __launch_bounds__(32 * BAND_WARPS, 4) ksw_band_kernel(BandArgs A
                             if (MODE == TRACKS) d[p] = vp >> 4, d2[p] = U[p] >> 4;
                         }
                     }
-                    if (CIGAR && store_tb) store_words(d, d2, tb + i * (NG * WB));
+                    if (CIGAR && store_tb) store_words(d, d2, tb + i * (NG * WB), kb + i);
                     if (entries && bnd_me && je0 + i >= jlo) store_entry(entry + i);
                 }
                 continue;
@@ -582,8 +586,7 @@ __global__ void __launch_bounds__(32 * BAND_WARPS, 4) ksw_band_kernel(BandArgs A
                         }
                     }
                 }
-                if (CIGAR && store_tb && slot0 + k >= 0) store_words(d, d2, tb + (k - kb) * (NG * WB));
-                else if (CIGAR && store_tb) words.put(d), words2.put(d2);
+                if (CIGAR && store_tb) store_words(d, d2, tb + (k - kb) * (NG * WB), k);
                 const int je = r - (c0 + SW - 1);
                 if (bnd_me && je >= jlo && je <= jend) store_entry(bnd_me + (je - jlo));
             }
@@ -826,6 +829,7 @@ int band_plan_build(BandPlan &bp, const std::vector<int32_t> &ids, const std::ve
     struct PairGeo {
         int32_t id, ww, rb;
         int64_t tb, bnd;
+        int64_t tail;  // bytes by which the skew of its strips reaches beyond their rows (<= 32 KB)
         bool ckpt = false, refused = false, notb = false;
         std::vector<BandStripDev> strips;
         std::vector<int64_t> start;  // estimated start step of each strip
@@ -839,7 +843,8 @@ int band_plan_build(BandPlan &bp, const std::vector<int32_t> &ids, const std::ve
         G.id = i, G.ww = ww, G.rb = band_break(ql, tl, ww);
         const int nd = ql + tl - 1;
         const int nstrip = (int)ceil_div(tl, SW);
-        G.tb = 0, G.bnd = 0;
+        G.tb = 0, G.bnd = 0, G.tail = 0;
+        int64_t reach = 0;
         for (int s = 0; s < nstrip; ++s) {
             const int c0 = s * SW;
             BandStripDev sd;
@@ -862,21 +867,25 @@ int band_plan_build(BandPlan &bp, const std::vector<int32_t> &ids, const std::ve
             sd.bnd_off = G.bnd;
             int64_t stb = 0;
             if (rows > 0) {
-                if (cigar) stb = (rows + 4 * (NG - 1)) * NG * WB;
+                if (cigar) {
+                    stb = rows * NG * WB;
+                    reach = std::max(reach, G.tb + stb + 4 * (ceil_div(std::min(SW, tl - c0), 4) - 1) * NG * WB);
+                }
                 G.tb += stb;
-                G.bnd += rows;
+                if (s + 1 < nstrip) G.bnd += rows;  // the last strip's column is not read
             }
             G.stb.push_back(stb);
             G.strips.push_back(sd);
             G.start.push_back((int64_t)sd.jstart + c0);  // its first step
         }
+        G.tail = (std::max(reach, G.tb) - G.tb + 255) / 256 * 256;
         G.tb = (G.tb + 255) / 256 * 256;
         if (G.rb < nd) {
             // the band becomes empty before the end: the reference stops there with
             // zdropped = 1 and no traceback (ksw2_extd2_sse.c:151-154), so the DP runs without
             // storing one (the first pass of a recomputed pair, with nothing to recompute)
             G.ckpt = G.notb = true;
-            G.tb = 0;
+            G.tb = G.tail = 0;
         }
     }
     // The budget is split once between the boundary-column arena and the traceback arena
@@ -889,22 +898,26 @@ int band_plan_build(BandPlan &bp, const std::vector<int32_t> &ids, const std::ve
     const int64_t cap_bnd = std::min(bnd_all, tb_budget / 3);
     const int64_t cap_tb = std::max<int64_t>(tb_budget - cap_bnd, 1);
     const int64_t gres = cap_tb;
+    // What a pair alone may take: the tail is not charged, and of the boundary columns only as many
+    // as strips of twice the width would have, so that the narrow strips refuse nothing that wider
+    // ones would run (the two arenas then exceed the budget by 1/64 of the traceback at most).
+    const int64_t cap_one = std::max<int64_t>(tb_budget - std::min(bnd_all / 2, tb_budget / 3), 1);
     for (PairGeo &G : geo) {
         if (G.notb) continue;
         // Singletrack pairs keep their whole two-track traceback: the reconstruction probes
         // arbitrarily far left in one gap search, so it cannot be split into strip groups.  A
         // pair whose traceback does not fit is refused like an allocation failure of the
         // reference (ksw2_extd2_avx.c:206-210: reset result, zdropped = 1).
-        bool refuse = st && G.tb > cap_tb;
-        if (!st && G.tb > cap_tb) {
+        bool refuse = st && G.tb > cap_one;
+        if (!st && G.tb + G.tail > cap_tb) {
             // Traceback beyond the budget: the first pass stores only the strips' boundary
             // columns; then the traceback is recomputed in groups of strips, from the last group
             // to the first, each from the stored column on its left, and the walk continues
             // through each group as it is recomputed.  The groups are cut per wave (below).
-            for (int s = 0; s < (int)G.strips.size(); ++s) refuse |= G.stb[s] > cap_tb;
+            for (int s = 0; s < (int)G.strips.size(); ++s) refuse |= G.stb[s] > cap_one;
             if (!refuse) {
                 G.ckpt = true;
-                G.tb = 0;  // the first pass stores no traceback
+                G.tb = G.tail = 0;  // the first pass stores no traceback
             }
         }
         if (refuse) {
@@ -915,7 +928,7 @@ int band_plan_build(BandPlan &bp, const std::vector<int32_t> &ids, const std::ve
     }
     for (const PairGeo &G : geo) {
         if (G.refused) continue;
-        bp.tb_total += G.tb;
+        bp.tb_total += G.tb + G.tail;
         bp.cells += band_cells(qlen[G.id], tlen[G.id], G.ww);
     }
     // Pairs largest first into the fewest waves whose boundary columns and tracebacks stored in
@@ -931,10 +944,10 @@ int band_plan_build(BandPlan &bp, const std::vector<int32_t> &ids, const std::ve
     std::vector<int64_t> wtb, wbnd;
     for (size_t a : ord) {
         const PairGeo &G = geo[a];
-        const int64_t pb = band_bnd_bytes(G.bnd);
+        const int64_t pb = band_bnd_bytes(G.bnd), ptb = G.tb + G.tail;
         int best = -1;
         for (size_t k = 0; k < wv.size(); ++k) {
-            if (wtb[k] + G.tb <= cap_tb && wbnd[k] + pb <= cap_bnd &&
+            if (wtb[k] + ptb <= cap_tb && wbnd[k] + pb <= cap_bnd &&
                 (best < 0 || wbnd[k] * cap_tb + wtb[k] * cap_bnd < wbnd[best] * cap_tb + wtb[best] * cap_bnd))
                 best = (int)k;
         }
@@ -943,7 +956,7 @@ int band_plan_build(BandPlan &bp, const std::vector<int32_t> &ids, const std::ve
             wtb.push_back(0), wbnd.push_back(0);
             best = (int)wv.size() - 1;
         }
-        wtb[best] += G.tb, wbnd[best] += pb;
+        wtb[best] += ptb, wbnd[best] += pb;
         wv[best].push_back(a);
     }
     struct U {
@@ -979,7 +992,7 @@ int band_plan_build(BandPlan &bp, const std::vector<int32_t> &ids, const std::ve
                 us.push_back(U{G.start[s], slot, (int)s});
             }
             if (G.ckpt && !G.notb) ck.push_back({slot, a});
-            tb += G.tb;
+            tb += G.tb + G.tail;
             bnd += (G.bnd + 31) / 32 * 32;
         }
         // strips in estimated start order; a pair's strips keep their left-to-right order
@@ -1005,14 +1018,15 @@ int band_plan_build(BandPlan &bp, const std::vector<int32_t> &ids, const std::ve
             const PairGeo &G = geo[ck[c].second];
             double tb_pair = 0;
             for (int64_t x : G.stb) tb_pair += (double)x;
-            const int64_t share = std::max<int64_t>((int64_t)((double)gres * tb_pair / std::max(tb_all, 1.0)), 1);
+            const int64_t tail = 4 * (NG - 1) * NG * WB;
+            const int64_t share = std::max<int64_t>((int64_t)((double)gres * tb_pair / std::max(tb_all, 1.0)) - tail, 1);
             int s1 = (int)G.strips.size();
             while (s1 > 0) {
                 int s0 = s1 - 1;
                 int64_t acc = G.stb[s0];
                 while (s0 > 0 && acc + G.stb[s0 - 1] <= share) acc += G.stb[--s0];
                 groups[c].push_back({s0, s1});
-                gtb[c].push_back(acc);
+                gtb[c].push_back(acc + tail);
                 s1 = s0;
             }
             nround = std::max(nround, groups[c].size());
