@@ -737,14 +737,38 @@ static int plan_launch(aw_ksw_plan_t *pl) {
     return AW_OK;
 }
 
-// Waits for plan_launch's work, checks the device error flag, collects timings.
+// Banded pairs with a value beyond the sweep's 16-bit fields (BandRes::wide; first gaps that cost 40
+// and more to open, junk cells only) again, on the anti-diagonal kernel.
+static int plan_rerun_wide(aw_ksw_plan_t *pl) {
+    Buffers *B = pl->B;
+    const Params &P = pl->P;
+    std::vector<BandRes> res(pl->band.pairs.size());
+    AW_CUDA(cudaMemcpy(res.data(), B->band_res.p, sizeof(BandRes) * res.size(), cudaMemcpyDeviceToHost));
+    std::vector<int32_t> ids;
+    for (size_t k = 0; k < res.size(); ++k)
+        if (res[k].wide && !res[k].stopped) ids.push_back(pl->band.pairs[k].idx);
+    if (getenv("AW_VERBOSE")) fprintf(stderr, "[aw_b200] %zu banded pairs again in int8\n", ids.size());
+    const int rc = run_exact_ksw(ids.size(), nullptr, B->qcodes.as<uint8_t>(), B->tcodes.as<uint8_t>(),
+                                 B->pairs.as<KswPair>(), pl->pairs, ids, pl->w, P.m, P.mat, pl->S, P.zdrop, P.end_bonus,
+                                 P.flag, B->out.as<KswOut>(), B->cig.as<uint32_t>(), B->exact_ws, B->st, &pl->launches,
+                                 tls_has_deadline ? B->deadline.as<unsigned long long>() : nullptr);
+    if (rc) return rc;
+    AW_CUDA(cudaStreamSynchronize(B->st));
+    return AW_OK;
+}
+
+// Waits for plan_launch's work, checks the device error flags, collects timings.
 static int plan_finish(aw_ksw_plan_t *pl, float *ms) {
     Buffers *B = pl->B;
     const int nw = (int)(pl->waves.size() + (pl->band_ids.empty() ? 0 : pl->band.waves.size()));
     AW_CUDA(cudaStreamSynchronize(B->st));
-    int32_t err = 0;
-    AW_CUDA(cudaMemcpy(&err, B->error.p, 4, cudaMemcpyDeviceToHost));
-    if (err) { set_error("a bounded device wait gave up (pipeline stall)"); return AW_E_TIMEOUT; }
+    int32_t err[2] = {0, 0};
+    AW_CUDA(cudaMemcpy(err, B->error.p, sizeof(err), cudaMemcpyDeviceToHost));
+    if (err[0]) { set_error("a bounded device wait gave up (pipeline stall)"); return AW_E_TIMEOUT; }
+    if (err[1]) {
+        const int rc = plan_rerun_wide(pl);
+        if (rc) return rc;
+    }
     if (ms) AW_CUDA(cudaEventElapsedTime(ms, B->ev_t0, B->ev_t1));
     float dp = 0.f, bt = 0.f;
     for (int k = 0; k < nw; ++k) {

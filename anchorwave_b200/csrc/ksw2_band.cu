@@ -15,12 +15,11 @@
 //     chain, took 0.61 us per 4-column step at the band's edge, one anti-diagonal takes 0.25);
 //   * st0, en0 and the blocks around them are the same for the whole warp, and a lane's columns
 //     lie in one 16-column block, so "computed" is a property of a lane: a lane outside
-//     [stB, en16] skips its cells and its registers keep their last values;
+//     [st16, en16] skips its cells and its registers keep their last values;
 //   * left input of cell (t, r): the column t-1 at r-1 (the previous lane's last column by a
 //     shuffle); at t == st16 the reference's boundary value (x[st16-1] only on the anti-diagonal
 //     where st16 advanced, constants otherwise, the matrix edge when st16 == 0,
-//     ksw2_extd2_avx.c:273-287); at t == stB < st16 (lane 0 of the first block) the in-register
-//     wrap to lane 15, i.e. column stB+15 at r-1, by another shuffle;
+//     ksw2_extd2_avx.c:273-287);
 //   * up input: the column's own registers, the top-edge values on row 0;
 //   * score: the score-fill (ksw2_extd2_avx.c:289-311) refreshes position t on
 //     anti-diagonal r when st0 <= t <= st0+16*ceil((en0-st0+1)/16)-1 (en0 for
@@ -31,7 +30,17 @@
 //     on the last anti-diagonal; the anti-diagonal loop stops at the first empty
 //     band (:151-154, zdropped = 1).
 // Cells above the matrix, below it and right of it that a lane computes along with its others
-// never reach a cell of the matrix.  Three ranges of a strip's steps, solved once per strip, run on
+// never reach a cell of the matrix.
+//
+// The blocks left of st16 that the reference computes as well (blocks of 32 or 64 bytes) feed no
+// cell from st16 on, and only a traceback that leaves the band by more than its last 16-column
+// block reads them (89 of 420,000 walks in bands of 1 to 24 around random, shifted and gapped
+// pairs), while their y and y2 grow without a bound of use (by q + e - e2 a step: 629 under (4, 2,
+// 24, 1), 4,150 under (30, 4, 40, 1), beyond a 16-bit field).  So the sweep leaves them out: when
+// st16 passes a block its columns' state is stored (DeepRows), and a walk that gets there
+// computes the cells from it in 32 bits (deep_fill).
+//
+// Three ranges of a strip's steps, solved once per strip, run on
 // loops of their own: the steps where the whole strip lies strictly inside the band (no
 // tests), before them those where only the band's right edge is in the strip, and after them
 // those with only its left edge.  Both edges are chains that bound long pairs: every step of
@@ -111,6 +120,7 @@ struct BandArgs {
     // reached (it only moves up and left), strips of a finished walk compute nothing
     const BandWalkState *walk;
     uint32_t one = 1;  // KswFullArgs::one
+    int peak_max;      // largest field of x, y, x2, y2 (as often as they are checked) that keeps the cells exact
 };
 
 constexpr uint64_t WAIT_NS = 20ull * 1000 * 1000 * 1000;  // bounded wait on the left strip
@@ -158,9 +168,25 @@ constexpr int NP = 2, C = 2 * NP, SW = 32 * C;
 // corner that the skew leaves free at its start is where this one's last rows end.
 constexpr int NG = SW / 4;
 
+// The state of the columns that st16 passes (this comment's "deep" cells: columns below st16 of its
+// block), stored as further rows of the strip's traceback: 14 words of a lane's registers, then
+// a word that is 1 once the block's bytes are computed (in the block's first lane).
+template <int WB>
+struct DeepRows {
+    static constexpr int WORDS = 14;
+    // word w of lane l of a strip
+    static __device__ __forceinline__ uint32_t *word(uint8_t *tb, const BandStripDev &St, int l, int w) {
+        const int row = St.jend - St.jlo + 1 + w * 4 / WB;
+        return reinterpret_cast<uint32_t *>(tb + St.tb_off + ((int64_t)(row + 4 * l) * NG + l) * WB + w * 4 % WB);
+    }
+};
+// Whether a pair's walk can meet one: not in 16-byte blocks, nor in bands that no column leaves.
+__host__ __device__ inline bool deep_cells(int block, int w, int qlen) { return block > 16 && w < qlen; }
+
 constexpr int BAND_WARPS = 4;  // per CTA: small CTAs spread a pair's strips over the SMs
 
-template <int MODE>
+// STRICT: every step's values are checked, not those of every PUB-th step (band_strict).
+template <int MODE, bool STRICT>
 __global__ void __launch_bounds__(32 * BAND_WARPS, 4) ksw_band_kernel(BandArgs A) {
     constexpr bool CIGAR = MODE != SCORES;
     constexpr int WB = MODE == TRACKS ? 8 : 4;
@@ -169,8 +195,6 @@ __global__ void __launch_bounds__(32 * BAND_WARPS, 4) ksw_band_kernel(BandArgs A
     const KswScore &S = A.sc;
     const CellK K = make_cellk<MODE>(S, A.one);
     const int B = A.block;
-    // the block wrap reads the last column of the lane D to the right
-    constexpr int D = 16 / C - 1;
 
     for (;;) {
         int u = 0;
@@ -215,6 +239,7 @@ __global__ void __launch_bounds__(32 * BAND_WARPS, 4) ksw_band_kernel(BandArgs A
         const int slot0 = jstart - 3 - jlo, row0 = slot0 - 4 * lane;
         const unsigned nrows = col0 < tlen ? (unsigned)(St.jend - jlo + 1) : 0u;
         uint8_t *tbp = CIGAR ? A.tb + St.tb_off + ((int64_t)slot0 * NG + lane) * WB : nullptr;
+        const bool deep = CIGAR && store_tb && deep_cells(B, w, qlen);
         BandRes *R = A.res + un.x;
         // steps whose cells all lie strictly inside the band
         const int ri0 = max(c0 + SW, 2 * (c0 + SW) - w);
@@ -250,6 +275,7 @@ __global__ void __launch_bounds__(32 * BAND_WARPS, 4) ksw_band_kernel(BandArgs A
             U[p] = v_in, Y[p] = K.kxb, Y2[p] = K.kxb2;
             SS[p] = add2(SB);  // score 0
         }
+        uint32_t peak = 0;  // the largest x, y, x2, y2 field so far
         RowWords words, words2;
         enum { H_NONE, H_LAST, H_ALL };
         int h_state = H_ALL;             // the columns whose H is up to date
@@ -279,6 +305,23 @@ __global__ void __launch_bounds__(32 * BAND_WARPS, 4) ksw_band_kernel(BandArgs A
             } else {
                 if ((unsigned)(row0 + k) < nrows) __stcs(reinterpret_cast<uint32_t *>(dst), a);
             }
+        };
+        // no candidate before the next call can leave its field while these stay below peak_max
+        auto grown = [&]() {
+#pragma unroll
+            for (int p = 0; p < NP; ++p)
+                peak = __vimax3_s16x2(peak, X[p], X2[p]), peak = __vimax3_s16x2(peak, Y[p], Y2[p]);
+        };
+        // the columns of the 16 that st16 has just passed, before the first step without them
+        auto store_deep = [&](int st16) {
+            if ((st16 & (B - 1)) == 0 || (col0 & ~15) != st16 - 16) return;
+            // DeepRows::word by what the warp has in registers
+            uint8_t *at = tbp + (int64_t)((int)nrows - row0) * (NG * WB);
+            const uint32_t st[DeepRows<WB>::WORDS + 1] = {X[0],  X[1], V[0],  V[1],  X2[0], X2[1], U[0], U[1],
+                                                          Y[0],  Y[1], Y2[0], Y2[1], SS[0], SS[1], 0u};
+#pragma unroll
+            for (int i = 0; i <= DeepRows<WB>::WORDS; ++i)
+                *reinterpret_cast<uint32_t *>(at + i * 4 / WB * (NG * WB) + i * 4 % WB) = st[i];
         };
         // the last column's entry: x, v, x2 as bytes (a field's bits 4-11) and H
         auto store_entry = [&](uint2 *dst) {
@@ -367,6 +410,7 @@ __global__ void __launch_bounds__(32 * BAND_WARPS, 4) ksw_band_kernel(BandArgs A
                 bh = (int)ahead.y;
             }
             if ((lane & ~(PUB - 1)) == ((kb + PUB) & 31)) ahead = left_of(jstart + ((kb + PUB) & ~31) + lane);
+            if (!STRICT) grown();
             const int kend = min(kb + PUB, nsteps);
             const bool full = kend - kb == PUB;  // the loops below take whole groups, unrolled
             int k = kb;
@@ -412,6 +456,7 @@ __global__ void __launch_bounds__(32 * BAND_WARPS, 4) ksw_band_kernel(BandArgs A
                     } else {
                         H[C - 1] += fval(V[NP - 1], 1);
                     }
+                    if (STRICT) grown();
                     if (CIGAR && store_tb) store_words(d, d2, tb + i * (NG * WB), kb + i);
                     if (entries && bnd_me) store_entry(entry + i);
                 }
@@ -422,42 +467,48 @@ __global__ void __launch_bounds__(32 * BAND_WARPS, 4) ksw_band_kernel(BandArgs A
                 // where the fill starts
                 if (h_state == H_NONE) rebuild_h(k);
                 h_state = H_LAST;
+                // the group in two parts when st16 advances in it (with a test and the stores in
+                // each step one 100 kb pair at w = 10 kb took 69.7 ms of sweep, like this 61.7)
+                const int adv = -(rs + kb - w + 1) & 31;
+                int i = 0;
+                for (int to = deep && adv < PUB ? adv : PUB;; to = PUB) {
 #pragma unroll 2
-                for (int i = 0; i < PUB; ++i) {
-                    const int r = rs + kb + i, st0 = max((r - w + 1) >> 1, 0), st16 = st0 & ~15, stB = st0 & g.bmask;
-                    const uint32_t mine0 = prmt(X[NP - 1], V[NP - 1], 0x7632), mine1 = prmt(X2[NP - 1], sel[C - 1], 0x5432);
-                    uint32_t r0 = __shfl_up_sync(FULL, mine0, 1), r1 = __shfl_up_sync(FULL, mine1, 1);
-                    const uint32_t b0 = __shfl_sync(FULL, bx, (kb & 31) + i), b1 = __shfl_sync(FULL, by, (kb & 31) + i);
-                    const uint32_t x0 = __shfl_sync(FULL, mine0, (lane + D) & 31), x1 = __shfl_sync(FULL, mine1, (lane + D) & 31);
-                    if (lane == 0) r0 = b0, r1 = b1;
+                    for (; i < to; ++i) {
+                        const int r = rs + kb + i, st0 = max((r - w + 1) >> 1, 0), st16 = st0 & ~15;
+                        uint32_t r0 = __shfl_up_sync(FULL, prmt(X[NP - 1], V[NP - 1], 0x7632), 1);
+                        uint32_t r1 = __shfl_up_sync(FULL, prmt(X2[NP - 1], sel[C - 1], 0x5432), 1);
+                        const uint32_t b0 = __shfl_sync(FULL, bx, (kb & 31) + i), b1 = __shfl_sync(FULL, by, (kb & 31) + i);
+                        if (lane == 0) r0 = b0, r1 = b1;
 #pragma unroll
-                    for (int c = C - 1; c > 0; --c) sel[c] = sel[c - 1];
-                    sel[0] = r1 >> 16;
-                    const bool wrap = col0 == stB && stB != st16;
-                    const bool fix = col0 == st16 && st16 > 0 && ((max((r - w) >> 1, 0)) & ~15) == st16;
-                    r0 = wrap ? x0 : fix ? prmt(x_in, v_in, 0x5410) : r0;
-                    r1 = wrap ? x1 : fix ? x2_in : r1;
-                    const uint32_t x = prmt(r0, X[NP - 1], 0x5410), v = prmt(r0, V[NP - 1], 0x5432), x2 = prmt(r1, X2[NP - 1], 0x5410);
-                    uint32_t d[NP], d2[NP];
-                    const int f0 = st0 - col0;
+                        for (int c = C - 1; c > 0; --c) sel[c] = sel[c - 1];
+                        sel[0] = r1 >> 16;
+                        const bool fix = col0 == st16 && st16 > 0 && ((max((r - w) >> 1, 0)) & ~15) == st16;
+                        if (fix) r0 = prmt(x_in, v_in, 0x5410), r1 = x2_in;
+                        const uint32_t x = prmt(r0, X[NP - 1], 0x5410), v = prmt(r0, V[NP - 1], 0x5432), x2 = prmt(r1, X2[NP - 1], 0x5410);
+                        uint32_t d[NP], d2[NP];
+                        const int f0 = st0 - col0;
 #pragma unroll
-                    for (int p = 0; p < NP; ++p) {
-                        const uint32_t m = mask2(p >= f0, p + NP >= f0);
-                        SS[p] = (score_of(p) & m) | (SS[p] & ~m);
-                        d[p] = d2[p] = 0;
-                    }
-                    if (col0 >= stB) {
-#pragma unroll
-                        for (int p = NP - 1; p >= 0; --p) {
-                            uint32_t xp = p ? X[p - 1] : x, vp = p ? V[p - 1] : v, x2p = p ? X2[p - 1] : x2;
-                            cell2<MODE, true>(SS[p], xp, vp, x2p, U[p], Y[p], Y2[p], d[p], K);
-                            X[p] = xp, V[p] = vp, X2[p] = x2p;
-                            if (MODE == TRACKS) d[p] = vp >> 4, d2[p] = U[p] >> 4;
+                        for (int p = 0; p < NP; ++p) {
+                            const uint32_t m = mask2(p >= f0, p + NP >= f0);
+                            SS[p] = (score_of(p) & m) | (SS[p] & ~m);
+                            d[p] = d2[p] = 0;
                         }
-                        if (f0 < C) H[C - 1] += fval(V[NP - 1], 1);
+                        if (col0 >= st16) {
+#pragma unroll
+                            for (int p = NP - 1; p >= 0; --p) {
+                                uint32_t xp = p ? X[p - 1] : x, vp = p ? V[p - 1] : v, x2p = p ? X2[p - 1] : x2;
+                                cell2<MODE, true>(SS[p], xp, vp, x2p, U[p], Y[p], Y2[p], d[p], K);
+                                X[p] = xp, V[p] = vp, X2[p] = x2p;
+                                if (MODE == TRACKS) d[p] = vp >> 4, d2[p] = U[p] >> 4;
+                            }
+                            if (f0 < C) H[C - 1] += fval(V[NP - 1], 1);
+                        }
+                        if (STRICT) grown();
+                        if (CIGAR && store_tb) store_words(d, d2, tb + i * (NG * WB), kb + i);
+                        if (entries && bnd_me && je0 + i <= jend) store_entry(entry + i);
                     }
-                    if (CIGAR && store_tb) store_words(d, d2, tb + i * (NG * WB), kb + i);
-                    if (entries && bnd_me && je0 + i <= jend) store_entry(entry + i);
+                    if (to == PUB) break;
+                    store_deep(max((rs + kb + i - w + 1) >> 1, 0) & ~15);
                 }
                 continue;
             }
@@ -492,6 +543,7 @@ __global__ void __launch_bounds__(32 * BAND_WARPS, 4) ksw_band_kernel(BandArgs A
                             if (MODE == TRACKS) d[p] = vp >> 4, d2[p] = U[p] >> 4;
                         }
                     }
+                    if (STRICT) grown();
                     if (CIGAR && store_tb) store_words(d, d2, tb + i * (NG * WB), kb + i);
                     if (entries && bnd_me && je0 + i >= jlo) store_entry(entry + i);
                 }
@@ -503,8 +555,8 @@ __global__ void __launch_bounds__(32 * BAND_WARPS, 4) ksw_band_kernel(BandArgs A
 #pragma unroll 1
             for (; k < kend; ++k) {
                 const int r = rs + k;
-                const uint32_t mine0 = prmt(X[NP - 1], V[NP - 1], 0x7632), mine1 = prmt(X2[NP - 1], sel[C - 1], 0x5432);
-                uint32_t r0 = __shfl_up_sync(FULL, mine0, 1), r1 = __shfl_up_sync(FULL, mine1, 1);
+                uint32_t r0 = __shfl_up_sync(FULL, prmt(X[NP - 1], V[NP - 1], 0x7632), 1);
+                uint32_t r1 = __shfl_up_sync(FULL, prmt(X2[NP - 1], sel[C - 1], 0x5432), 1);
                 int Hl = __shfl_up_sync(FULL, H[C - 1], 1);
                 const uint32_t b0 = __shfl_sync(FULL, bx, k & 31), b1 = __shfl_sync(FULL, by, k & 31);
                 const int hb = __shfl_sync(FULL, bh, k & 31);
@@ -517,14 +569,11 @@ __global__ void __launch_bounds__(32 * BAND_WARPS, 4) ksw_band_kernel(BandArgs A
                 for (int p = 0; p < NP; ++p) d[p] = 0, d2[p] = 0;
                 if (r < rlim) {
                     const int st0 = g.st0(r), en0 = g.en0(r);
-                    const int st16 = st0 & ~15, stB = st0 & g.bmask, en16 = en0 | 15;
+                    const int st16 = st0 & ~15, en16 = en0 | 15;
                     const int fe = A.generic ? en0 : st0 + ((en0 - st0 + 16) & ~15) - 1;
-                    if (stB != st16) {
-                        const uint32_t x0 = __shfl_sync(FULL, mine0, (lane + D) & 31), x1 = __shfl_sync(FULL, mine1, (lane + D) & 31);
-                        if (col0 == stB) r0 = x0, r1 = x1;
-                    }
-                    if (col0 == st16 && st16 > 0 && (g.st0(r - 1) & ~15) == st16)
-                        r0 = prmt(x_in, v_in, 0x5410), r1 = x2_in;
+                    const int before16 = st16 > 0 ? g.st0(r - 1) & ~15 : 0;
+                    if (deep && st16 != before16) store_deep(st16);
+                    if (col0 == st16 && st16 > 0 && before16 == st16) r0 = prmt(x_in, v_in, 0x5410), r1 = x2_in;
                     uint32_t x = prmt(r0, X[NP - 1], 0x5410), v = prmt(r0, V[NP - 1], 0x5432), x2 = prmt(r1, X2[NP - 1], 0x5410);
                     // score fill
                     const int f0 = st0 - col0, f1 = fe - col0;
@@ -535,7 +584,7 @@ __global__ void __launch_bounds__(32 * BAND_WARPS, 4) ksw_band_kernel(BandArgs A
                             SS[p] = (score_of(p) & m) | (SS[p] & ~m);
                         }
                     }
-                    if (col0 >= stB && col0 <= en16) {
+                    if (col0 >= st16 && col0 <= en16) {
                         if (r < c0 + SW) {
                             // row 0: the top edge above column r
                             const uint32_t eu = rep2(16 * edge_diff(r, S) + FB);
@@ -586,12 +635,17 @@ __global__ void __launch_bounds__(32 * BAND_WARPS, 4) ksw_band_kernel(BandArgs A
                         }
                     }
                 }
+                if (STRICT) grown();
                 if (CIGAR && store_tb) store_words(d, d2, tb + (k - kb) * (NG * WB), k);
                 const int je = r - (c0 + SW - 1);
                 if (bnd_me && je >= jlo && je <= jend) store_entry(bnd_me + (je - jlo));
             }
         }
         if (failed) break;
+        if (__any_sync(FULL, (int)(peak & 0xffffu) > A.peak_max || (int)(peak >> 16) > A.peak_max) && lane == 0) {
+            R->wide = 1;
+            atomicExch(A.error + 1, 1);
+        }
         if (mte_key && !stopped) atomicMax(&R->mte_key, mte_key);
     }
 }
@@ -602,7 +656,7 @@ struct BtArgs {
     const BandPairDev *pairs;
     int npair;
     const BandStripDev *strips;
-    const uint8_t *tb;
+    uint8_t *tb;
     const BandRes *res;
     BandWalkState *walk;
     const uint8_t *qcodes, *tcodes;
@@ -614,10 +668,82 @@ struct BtArgs {
 };
 
 // The move that ksw_backtrack's off/off_end forcing takes outside the computed blocks of the
-// cell's anti-diagonal (1: deletion, 2: insertion), or -1.
-__device__ __forceinline__ int band_force(const Geom &g, int i, int j) {
-    const int r = i + j;
-    return i > (g.en0(r) | 15) ? 1 : i < (g.st0(r) & g.bmask) ? 2 : -1;
+// cell's anti-diagonal (1: deletion, 2: insertion), -1, or -2 for a deep cell whose bytes are not
+// computed yet.
+template <int WB>
+__device__ __forceinline__ int band_force(const Geom &g, const BandStripDev *strips, uint8_t *tb, int i, int j) {
+    const int r = i + j, st0 = g.st0(r);
+    if (i > (g.en0(r) | 15)) return 1;
+    if (i >= (st0 & ~15)) return -1;
+    if (i < (st0 & g.bmask)) return 2;
+    const int cb = i & g.bmask;
+    return *(volatile uint32_t *)DeepRows<WB>::word(tb, strips[cb / SW], cb % SW / C, DeepRows<WB>::WORDS) == 1 ? -1 : -2;
+}
+
+// Computes the deep cells of the block that starts at column cb (a warp): the columns below st16
+// of its anti-diagonals, from the state each had when st16 passed it, two columns a lane.  Their
+// scores stay those of the last fill; column cb takes its left input from column cb + 15 (the
+// in-register wrap of the reference's blocks, ksw2_extd2_avx.c:313-330).
+template <int WB>
+__device__ __noinline__ void deep_fill(const BandPairDev &P, const Geom &g, const BandStripDev &St, uint8_t *tb, int cb,
+                                       const KswScore &S, bool right) {
+    const int lane = threadIdx.x & 31, B = -g.bmask, lim = min(g.nd, g.rb);
+    // the first anti-diagonal whose st0 has reached column X (> 0)
+    auto reached = [&](int X) { return min(X + P.qlen - 1, 2 * X + P.w - 1); };
+    const int end = min(reached(cb + B), lim);
+    int x[2], v[2], x2[2], u[2], y[2], y2[2], s[2];
+#pragma unroll
+    for (int c = 0; c < 2; ++c) x[c] = v[c] = x2[c] = u[c] = y[c] = y2[c] = s[c] = 0;
+    int n = 0;  // columns passed
+    for (int r = reached(cb + 16); r < end; ++r) {
+        if (n + 16 < B && r == reached(cb + n + 16)) {
+            if (2 * lane >= n && 2 * lane < n + 16) {
+                // columns 2*lane and 2*lane + 1 of the block: fields of the words of their strip's lane
+                const int l = cb % SW / C + lane / 2, f = lane & 1;
+                auto at = [&](int w) { return fld(*DeepRows<WB>::word(tb, St, l, w), f); };
+#pragma unroll
+                for (int c = 0; c < 2; ++c) {
+                    x[c] = (at(c) - FB) >> 4, v[c] = (at(2 + c) - FB) >> 4, x2[c] = (at(4 + c) - FB) >> 4;
+                    u[c] = (at(6 + c) - FB) >> 4, y[c] = (at(8 + c) - FB) >> 4, y2[c] = (at(10 + c) - FB) >> 4;
+                    s[c] = (at(12 + c) - 2 * FB) >> 4;
+                }
+            }
+            n += 16;
+        }
+        int xl = __shfl_up_sync(FULL, x[1], 1), vl = __shfl_up_sync(FULL, v[1], 1), x2l = __shfl_up_sync(FULL, x2[1], 1);
+        const int xw = __shfl_sync(FULL, x[1], 7), vw = __shfl_sync(FULL, v[1], 7), x2w = __shfl_sync(FULL, x2[1], 7);
+        if (lane == 0) xl = xw, vl = vw, x2l = x2w;
+        if (2 * lane >= n) continue;
+#pragma unroll
+        for (int c = 1; c >= 0; --c) {
+            const int xi = c ? x[0] : xl, vi = c ? v[0] : vl, x2i = c ? x2[0] : x2l;
+            const int cand[4] = {xi + vi, y[c] + u[c], x2i + vi, y2[c] + u[c]};
+            int z = s[c], d = 0;
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                // left-aligned: the first candidate wins a tie, right-aligned: the last
+                if (right ? cand[k] >= z : cand[k] > z) d = k + 1;
+                z = max(z, cand[k]);
+            }
+            z = min(z, S.mch);
+            const int un = z - vi, vn = z - u[c];
+            const int open[4] = {cand[0] - z + S.q, cand[1] - z + S.q, cand[2] - z + S.q2, cand[3] - z + S.q2};
+#pragma unroll
+            for (int k = 0; k < 4; ++k) d |= (right ? open[k] >= 0 : open[k] > 0) ? 8 << k : 0;
+            x[c] = max(open[0], 0) - S.qe, y[c] = max(open[1], 0) - S.qe;
+            x2[c] = max(open[2], 0) - S.qe2, y2[c] = max(open[3], 0) - S.qe2;
+            u[c] = un, v[c] = vn;
+            const int t = cb + 2 * lane + c, j = r - t, gr = t % SW / 4;
+            if (j < St.jlo || j > St.jend) continue;
+            uint8_t *p = tb + St.tb_off + ((int64_t)(j - St.jlo + 4 * gr) * NG + gr) * WB + t % 4;
+            if (WB == 8) p[0] = (uint8_t)vn, p[4] = (uint8_t)un;
+            else p[0] = (uint8_t)d;
+        }
+    }
+    __syncwarp();
+    if (lane == 0) *DeepRows<WB>::word(tb, St, cb % SW / C, DeepRows<WB>::WORDS) = 1;
+    __threadfence_block();
+    __syncwarp();
 }
 
 // The stored rows of a column group (4 columns) of a pair's strips (words of WB bytes).
@@ -674,7 +800,11 @@ __global__ void __launch_bounds__(32 * fin_warps<ST>()) ksw_band_finish_kernel(B
     }
     const bool cigar = !(flag & AW_EZ_SCORE_ONLY);
     const BandStripDev *strips = A.strips + P.strip0;
-    const uint8_t *tb = A.tb;
+    uint8_t *tb = A.tb;
+    auto force = [&](int a, int b) { return band_force<WB>(g, strips, tb, a, b); };
+    auto fill = [&](int a, int) {
+        deep_fill<WB>(P, g, strips[a / SW], tb, a & g.bmask, A.sc, (flag & AW_EZ_RIGHT) != 0);
+    };
     Window win;
     win.init(tiles[warp], NG * WB);
     auto grp = [&](int gg) -> TbGroup { return band_group<WB>(strips, tb, tlen, 0, gg); };
@@ -687,8 +817,7 @@ __global__ void __launch_bounds__(32 * fin_warps<ST>()) ksw_band_finish_kernel(B
             Probe probe;
             probe.init(tiles[warp] + Window::BYTES, NG * WB);
             int i = tlen - 1, j = qlen - 1;
-            if (tb_singletrack(i, j, cg, win, probe, grp, [&](int a, int c) { return band_force(g, a, c); }, A.sc, A.mat,
-                               A.m, qs, ts)) {
+            if (tb_singletrack(i, j, cg, win, probe, grp, force, fill, A.sc, A.mat, A.m, qs, ts)) {
                 if (i >= 0) cg.push(2, i + 1);
                 if (j >= 0) cg.push(1, j + 1);
                 o.n_cigar = cg.finish(true);
@@ -715,7 +844,7 @@ __global__ void __launch_bounds__(32 * fin_warps<ST>()) ksw_band_finish_kernel(B
             }
         } else if (i0 >= 0 || j0 >= 0) {
             int i = i0, j = j0, state = 0;
-            tb_walk(i, j, state, 0, cg, win, grp, [&](int a, int b) { return band_force(g, a, b); });
+            tb_walk(i, j, state, 0, cg, win, grp, force, fill);
             if (i >= 0) cg.push(2, i + 1);
             if (j >= 0) cg.push(1, j + 1);
             o.n_cigar = cg.finish(!(flag & AW_EZ_REV_CIGAR));
@@ -747,13 +876,14 @@ __global__ void __launch_bounds__(32) ksw_band_round_walk_kernel(BtArgs A, const
     const Geom g{P.qlen, P.tlen, P.w, P.qlen + P.tlen - 1, P.rb, ~(A.block - 1)};
     const int tlen = P.tlen;
     const BandStripDev *strips = A.strips + P.strip0;
-    const uint8_t *tb = A.tb;
+    uint8_t *tb = A.tb;
     Window win;
     win.init(tiles, NG * 4);
     auto grp = [&](int gg) -> TbGroup { return band_group<4>(strips, tb, tlen, col_lo, gg); };
     WarpCigar cg{A.cig + P.cig_off, w.n, (uint32_t)w.op, w.len};
     int i = w.i, j = w.j, state = w.state;
-    tb_walk(i, j, state, col_lo, cg, win, grp, [&](int a, int b) { return band_force(g, a, b); });
+    tb_walk(i, j, state, col_lo, cg, win, grp, [&](int a, int b) { return band_force<4>(g, strips, tb, a, b); },
+            [&](int a, int) { deep_fill<4>(P, g, strips[a / SW], tb, a & g.bmask, A.sc, (A.flag & AW_EZ_RIGHT) != 0); });
     if (G.last) {
         if (i >= 0) cg.push(2, i + 1);
         if (j >= 0) cg.push(1, j + 1);
@@ -771,13 +901,28 @@ __global__ void __launch_bounds__(32) ksw_band_round_walk_kernel(BtArgs A, const
 }
 
 typedef void (*BandKernel)(BandArgs);
-BandKernel band_kernel_for(int flag, int block) {
-    if (flag & AW_EZ_SCORE_ONLY) return ksw_band_kernel<SCORES>;
-    if (singletrack_tracks(flag, block)) return ksw_band_kernel<TRACKS>;
-    return (flag & AW_EZ_RIGHT) ? ksw_band_kernel<RIGHTMOST> : ksw_band_kernel<LEFT>;
+template <bool STRICT>
+BandKernel band_kernel_of(int flag, int block) {
+    if (flag & AW_EZ_SCORE_ONLY) return ksw_band_kernel<SCORES, STRICT>;
+    if (singletrack_tracks(flag, block)) return ksw_band_kernel<TRACKS, STRICT>;
+    return (flag & AW_EZ_RIGHT) ? ksw_band_kernel<RIGHTMOST, STRICT> : ksw_band_kernel<LEFT, STRICT>;
+}
+BandKernel band_kernel_for(int flag, int block, bool strict) {
+    return strict ? band_kernel_of<true>(flag, block) : band_kernel_of<false>(flag, block);
 }
 
 int64_t ceil_div(int64_t a, int64_t b) { return (a + b - 1) / b; }
+
+// x, y, x2 and y2 grow by grow = qe - min(e, e2) a step at most, and a candidate adds a u or v of at
+// most qe.  Within 30 steps at the band's left edge (16 columns) they reach 30 * grow: 149 under (4, 2,
+// 24, 1), 989 under (30, 4, 40, 1); in the band and above it 57 was the largest value met.  A look
+// every PUB steps has room for that while grow is below 39; above, every step is checked (and a gap
+// that costs 49 to open still sends some pairs to the anti-diagonal kernel).
+int band_grow(const KswScore &S) { return S.qe - std::min(S.e, S.e2); }
+bool band_strict(const KswScore &S) { return 30 * band_grow(S) + 57 > CAND_MAX - S.qe - PUB * band_grow(S); }
+int band_peak_max(const KswScore &S) {
+    return 16 * std::max(CAND_MAX - S.qe - (band_strict(S) ? 1 : PUB) * band_grow(S), 0) + FB;
+}
 
 // Device bytes of a pair's boundary columns (entries rounded as the wave packs them).
 int64_t band_bnd_bytes(int64_t entries) { return (entries + 31) / 32 * 32 * (int64_t)sizeof(uint2); }
@@ -842,7 +987,7 @@ int band_plan_build(BandPlan &bp, const std::vector<int32_t> &ids, const std::ve
         const int ww = w[i] < 0 ? std::max(ql, tl) : std::min(w[i], std::max(ql, tl));
         G.id = i, G.ww = ww, G.rb = band_break(ql, tl, ww);
         const int nd = ql + tl - 1;
-        const int nstrip = (int)ceil_div(tl, SW);
+        const int nstrip = (int)ceil_div(tl, SW), deep_rows = deep_cells(B, ww, ql) ? 64 / WB : 0;
         G.tb = 0, G.bnd = 0, G.tail = 0;
         int64_t reach = 0;
         for (int s = 0; s < nstrip; ++s) {
@@ -868,7 +1013,7 @@ int band_plan_build(BandPlan &bp, const std::vector<int32_t> &ids, const std::ve
             int64_t stb = 0;
             if (rows > 0) {
                 if (cigar) {
-                    stb = rows * NG * WB;
+                    stb = (rows + deep_rows) * NG * WB;
                     reach = std::max(reach, G.tb + stb + 4 * (ceil_div(std::min(SW, tl - c0), 4) - 1) * NG * WB);
                 }
                 G.tb += stb;
@@ -1073,7 +1218,7 @@ int band_plan_build(BandPlan &bp, const std::vector<int32_t> &ids, const std::ve
 
 int band_occupancy(int flag, int block) {
     int nb = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, band_kernel_for(flag, block), 32 * BAND_WARPS, 0) != cudaSuccess)
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, band_kernel_for(flag, block, false), 32 * BAND_WARPS, 0) != cudaSuccess)
         return 1;
     return std::max(nb, 1);
 }
@@ -1102,12 +1247,13 @@ cudaError_t band_launch_dp(const BandPlan &bp, int k, const BandDev &D, const ui
     a.store_ckpt = 0;
     a.deadline = D.deadline;
     a.walk = nullptr;
+    a.peak_max = band_peak_max(S);
     return band_launch_units(bp, a, flag, ctas, st);
 }
 
 cudaError_t band_launch_units(const BandPlan &bp, const BandArgs &a, int flag, int ctas, cudaStream_t st) {
     const int grid = std::max(1, std::min(ctas, (a.n_units + BAND_WARPS - 1) / BAND_WARPS));
-    band_kernel_for(flag, bp.block)<<<grid, 32 * BAND_WARPS, 0, st>>>(a);
+    band_kernel_for(flag, bp.block, band_strict(a.sc))<<<grid, 32 * BAND_WARPS, 0, st>>>(a);
     return cudaGetLastError();
 }
 
@@ -1162,6 +1308,7 @@ cudaError_t band_launch_groups(const BandPlan &bp, int k, const BandDev &D, cons
         a.store_ckpt = 1;
         a.deadline = D.deadline;
         a.walk = D.walk;
+        a.peak_max = band_peak_max(S);
         if ((e = band_launch_units(bp, a, flag, ctas, st)) != cudaSuccess) return e;
         ksw_band_round_walk_kernel<<<R.ngroup, 32, 0, st>>>(b, gd);
         if ((e = cudaGetLastError()) != cudaSuccess) return e;

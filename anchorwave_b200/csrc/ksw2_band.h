@@ -35,7 +35,7 @@ struct BandRes {
     unsigned long long mqe_key, mte_key;
     int32_t score, has_score;
     int32_t stopped;  // a strip of the pair saw the calling thread's deadline pass
-    int32_t pad;
+    int32_t wide;     // a value outgrew the sweep's 16-bit fields: the pair's results do not count
 };
 
 struct BandWave {
@@ -110,7 +110,7 @@ struct BandDev {
     int32_t *queue;     // one counter per wave, 64 ints apart
     uint2 *bnd;
     uint8_t *tb;
-    int32_t *error;
+    int32_t *error;     // [0] a bounded wait gave up, [1] some pair's BandRes::wide is set
     const unsigned long long *deadline = nullptr;  // the calling thread's deadline word, or null
     const BandGroupDev *groups = nullptr;          // the group table of the recompute rounds
 };

@@ -19,12 +19,21 @@ __device__ __forceinline__ int edge_diff(int r, const KswScore &S) {
 // ---- packed cell fields ------------------------------------------------------------
 // Every field holds 16*value + FB; x, y, x2, y2 carry their candidate's priority tag on
 // top (so x + v is already the tagged candidate a), and the score carries 2*FB + its tag.
-// With the magnitude bound of full_path_ok (|u|, |v|, |x|, ... <= 300, and the bounded
-// excursions of masked-off fields within one step) every 32-bit add below keeps each field
-// inside [0, 65536) and every value a DPX op compares for a live field inside [0, 32768).
+// Every 32-bit add below keeps each field inside [0, 65536), and every value a DPX op compares
+// inside [0, 32768), while no candidate is above CAND_MAX.  The other bounds hold for any cell,
+// also the ones outside a band that have no consistent neighbours, whatever x and y are: with
+// u, v in [-qe, mch + qe] before a step (qe = q + e; the initial and the boundary values are, and
+// mch < 0 moves the bounds by -mch at most),
+// z = min(max(s, a, ...), mch) is either mch, and then z - v >= -qe, or at least a = x + v >= v - qe,
+// as x >= -qe, and then z - v >= -qe as well; z - v <= mch + qe since v >= -qe; the same for
+// z - u.  x, y >= -qe and x2, y2 >= -(q2 + e2) by their max, and mch <= 0.  So by the magnitude
+// bound of full_path_ok (all of these together at most 100) no field falls below -256 * 16.
+// In a full matrix x <= q and so on; above a cell of a band they may grow by at most qe a step
+// (max(a - z - e, ..) with a = x + v, where z is clipped to mch), which the banded kernel checks.
 // The adds are 2-input multiply-adds by a runtime one (or minus one), so they issue on the
 // FMA pipe and leave the ALU pipe to the max/min/permute work.
-constexpr int FB = 12288;
+constexpr int FB = 4096;  // a multiple of 16 * 256: the byte above a field's tag is the value
+constexpr int CAND_MAX = (32768 - 2 * FB) / 16 - 1;
 // A constant in both fields: for 32-bit adds (c * 65537, so that a negative c borrows
 // exactly what the field sum carries back) and for SIMD operands (each field = c).
 __host__ __device__ constexpr uint32_t add2(int c) { return (uint32_t)c * 0x10001u; }

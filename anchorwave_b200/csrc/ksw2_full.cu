@@ -539,18 +539,19 @@ __global__ void __launch_bounds__(32 * BtShape<NP, TRK>::WARPS) ksw_backtrack_fu
         return TbGroup{tb + (((int64_t)s * steps + k) * (32 * WPL) + g) * Sh::WB, 0, qlen - 1};
     };
     auto inside = [](int, int) { return -1; };
+    auto no_fill = [](int, int) {};
     WarpCigar w{A.cig + P.cig_off, 0, 0, 0};
     if constexpr (TRK) {
         typename Sh::Probe probe;
         probe.init(tiles[warp] + Sh::Window::BYTES, 32 * WPL * Sh::WB);
-        if (tb_singletrack(i, j, w, win, probe, grp, inside, A.sc, A.mat, A.m, A.qcodes + P.qoff, A.tcodes + P.toff)) {
+        if (tb_singletrack(i, j, w, win, probe, grp, inside, no_fill, A.sc, A.mat, A.m, A.qcodes + P.qoff, A.tcodes + P.toff)) {
             if (i >= 0) w.push(2, i + 1);
             if (j >= 0) w.push(1, j + 1);
             o.n_cigar = w.finish(true);
         }
         if (o.n_cigar == 0) o.zdropped = 1;
     } else {
-        tb_walk(i, j, state, 0, w, win, grp, inside);
+        tb_walk(i, j, state, 0, w, win, grp, inside, no_fill);
         if (i >= 0) w.push(2, i + 1);
         if (j >= 0) w.push(1, j + 1);
         o.n_cigar = w.finish(!(flag & AW_EZ_REV_CIGAR));

@@ -60,8 +60,10 @@ struct TbWindow {
 
     __device__ void init(uint8_t *smem, int64_t row_stride) {
         sm = smem, sa = (uint32_t)__cvta_generic_to_shared(smem), stride = row_stride;
-        cur = 0, cg = cj = INT_MIN / 2, og = oj = INT_MIN / 2, oseq = -1, issued = 0;
+        reset();
     }
+    // Forgets every tile (no copy may be under way).
+    __device__ void reset() { cur = 0, cg = cj = INT_MIN / 2, og = oj = INT_MIN / 2, oseq = -1, issued = 0; }
 
     // Starts the copy of the tile whose last cell is (group g, row j); GRP(gg) describes group gg.
     template <class GRP>
@@ -177,9 +179,10 @@ struct WarpCigar {
 
 // ksw_backtrack (minimap2/ksw2.h:160-192) from (i, j) until the walk leaves the matrix or the
 // columns >= col_lo, in runs.  FORCE(i, j): the move forced outside the computed band (1:
-// deletion, 2: insertion) or -1.
-template <class Window, class GRP, class FORCE, class Cig>
-__device__ void tb_walk(int &i, int &j, int &state, int col_lo, Cig &cg, Window &win, GRP &&grp, FORCE &&force) {
+// deletion, 2: insertion), -1, or -2 for a cell whose bytes FILL(i, j) has to compute first.
+template <class Window, class GRP, class FORCE, class FILL, class Cig>
+__device__ void tb_walk(int &i, int &j, int &state, int col_lo, Cig &cg, Window &win, GRP &&grp, FORCE &&force,
+                        FILL &&fill) {
     const int lane = threadIdx.x & 31;
     while (i >= 0 && j >= 0 && i >= col_lo) {
         win.ensure(i, j, grp);
@@ -187,9 +190,9 @@ __device__ void tb_walk(int &i, int &j, int &state, int col_lo, Cig &cg, Window 
         const int li = i - (di ? lane : 0), lj = j - (dj ? lane : 0);
         const bool in = li >= 0 && lj >= 0 && li >= col_lo && win.has(li, lj);
         const int fc = in ? force(li, lj) : -1;
-        const uint32_t c = in && fc < 0 ? win.at(li, lj) : 0u;
+        const uint32_t c = in && fc == -1 ? win.at(li, lj) : 0u;
         // the cell takes the walk's state on: an M cell in state 0, a continued gap otherwise
-        const bool on = in && fc < 0 && (state == 0 ? (c & 7u) == 0 : ((c >> (state + 2)) & 1u) != 0);
+        const bool on = in && fc == -1 && (state == 0 ? (c & 7u) == 0 : ((c >> (state + 2)) & 1u) != 0);
         const unsigned off = __ballot_sync(TB_ALL, !on);
         const int run = off ? __ffs(off) - 1 : 32;
         if (run > 0) {
@@ -199,6 +202,14 @@ __device__ void tb_walk(int &i, int &j, int &state, int col_lo, Cig &cg, Window 
         // the cell that ends the run, if it is there: a forced move, or its own state
         if (run == 32 || !__shfl_sync(TB_ALL, in ? 1 : 0, run)) continue;
         const int f = __shfl_sync(TB_ALL, fc, run);
+        if (f == -2) {
+            if (run == 0) {
+                tb_wait(0);
+                fill(i, j);
+                win.reset();
+            }
+            continue;
+        }
         state = f >= 0 ? f : (int)(__shfl_sync(TB_ALL, c, run) & 7u);
         if (state == 0) continue;  // an M cell after a gap: the next round takes its run
         if (state == 1 || state == 3) cg.push(2, 1), --i;
@@ -215,23 +226,34 @@ __device__ __forceinline__ int tb_st_gap(int l, int o1, int e1, int o2, int e2) 
 
 // The Singletrack reconstruction (minimap2/ksw2_singletrack.cpp:63-176) from (i, j) to a matrix
 // edge.  FORCE as above (insertions above the computed blocks of an anti-diagonal, deletions
-// below).  Returns false when no gap explains a cell.  `probe` holds the tiles of a gap search.
-template <class Window, class Probe, class GRP, class FORCE>
+// below), FILL too.  Returns false when no gap explains a cell.  `probe` holds the tiles of a gap
+// search.
+template <class Window, class Probe, class GRP, class FORCE, class FILL>
 __device__ bool tb_singletrack(int &i, int &j, WarpCigar &cg, Window &win, Probe &probe, GRP &&grp, FORCE &&force,
-                               const KswScore &S, const int8_t *mat, int m, const uint8_t *qs, const uint8_t *ts) {
+                               FILL &&fill, const KswScore &S, const int8_t *mat, int m, const uint8_t *qs, const uint8_t *ts) {
     const int lane = threadIdx.x & 31;
     auto stored = [&](int a, int b) { return force(a, b) < 0; };
     const int o1 = -S.q, g1 = -S.e, o2 = -S.q2, g2 = -S.e2;
+    auto fill_at = [&](int a, int b) {
+        tb_wait(0);
+        fill(a, b);
+        win.reset(), probe.reset();
+    };
     // the difference along the matrix edge for edge cell c
     auto edge = [&](int c) { return tb_st_gap(c + 1, o1, g1, o2, g2) - tb_st_gap(c, o1, g1, o2, g2); };
     while (i >= 0 && j >= 0) {
         const int f = force(i, j);
         if (f == 2) { cg.push(1, 1); --j; continue; }
         if (f == 1) { cg.push(2, 1); --i; continue; }
+        if (f == -2 || (j > 0 && force(i, j - 1) == -2)) {
+            fill_at(i, f == -2 ? j : j - 1);
+            continue;
+        }
         // the run of diagonal moves: v(i, j) + u(i, j-1) is the cell's substitution score
         win.ensure(i, j, grp);
         const int li = i - lane, lj = j - lane;
-        const bool in = li >= 0 && lj >= 0 && win.has(li, lj) && stored(li, lj);
+        const bool in = li >= 0 && lj >= 0 && win.has(li, lj) && stored(li, lj) &&
+                        force(li, lj) != -2 && (lj == 0 || force(li, lj - 1) != -2);
         bool on = in;
         if (in) {
             const int h = tb_sx8(win.at(li, lj, 0));
@@ -254,6 +276,10 @@ __device__ bool tb_singletrack(int &i, int &j, WarpCigar &cg, Window &win, Probe
         bool d_ok = true, i_ok = true;
         for (;;) {
             const int l = base + lane + 1, id = i - l, jn = j - l;
+            // lengths from the first cell on that is not computed yet do not count (the cells above
+            // (i, j) were computed with it)
+            const unsigned nb = __ballot_sync(TB_ALL, d_ok && id + 1 >= 0 && force(id + 1, j) == -2);
+            const unsigned known = nb ? (nb & (0u - nb)) - 1u : TB_ALL;
             // differences of the l-th cell: u(i-l+1, j) and v(i, j-l+1)
             int du = 0, dv = 0;
             bool uf = true, vf = true;
@@ -279,8 +305,8 @@ __device__ bool tb_singletrack(int &i, int &j, WarpCigar &cg, Window &win, Probe
             const int a1 = o1 + l * g1, a2 = o2 + l * g2, dd = dsum + du, di = isum + dv;
             const bool dhit = d_ok && !(ub & upto) && id >= -1 && (dd == a1 || dd == a2);
             const bool ihit = i_ok && !(vb & upto) && jn >= -1 && (di == a1 || di == a2);
-            const unsigned end = __ballot_sync(TB_ALL, l > i + 1 && l > j + 1);
-            const unsigned db = __ballot_sync(TB_ALL, dhit), hit = db | __ballot_sync(TB_ALL, ihit);
+            const unsigned end = __ballot_sync(TB_ALL, l > i + 1 && l > j + 1) & known;
+            const unsigned db = __ballot_sync(TB_ALL, dhit), hit = (db | __ballot_sync(TB_ALL, ihit)) & known;
             if (hit && (!end || __ffs(hit) <= __ffs(end))) {
                 const int k = __ffs(hit) - 1, len = base + k + 1;
                 if (db >> k & 1u) cg.push(2, len), i -= len;
@@ -288,6 +314,10 @@ __device__ bool tb_singletrack(int &i, int &j, WarpCigar &cg, Window &win, Probe
                 break;
             }
             if (end) return false;
+            if (nb) {
+                fill_at(i - base - (__ffs(nb) - 1), j);
+                continue;
+            }
             dsum += __shfl_sync(TB_ALL, du, 31), isum += __shfl_sync(TB_ALL, dv, 31);
             d_ok = d_ok && !ub, i_ok = i_ok && !vb;
             base += 32;
