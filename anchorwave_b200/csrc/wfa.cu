@@ -61,9 +61,12 @@ enum { CM = 0, CI1 = 1, CD1 = 2, CI2 = 3, CD2 = 4 };
 // one lane of a warp uses it, and every lane would pay for its registers.
 struct Alloc {
     int64_t cur, end;
-    int64_t used;   // bytes taken from the pool
+    int64_t from;   // the current chunk's first byte
+    int64_t used;   // bytes allocated in the chunks before it
     int64_t list;
-    __device__ void init() { cur = end = used = 0, list = -1; }
+    __device__ void init() { cur = end = from = used = 0, list = -1; }
+    // Bytes allocated: what a pair holds, whatever the chunks that they lie in.
+    __device__ int64_t total() const { return used + (cur - from); }
 };
 
 // Packed CIGAR of the piggyback modes (wavefront/wavefront_pcigar.h:44-71): 2 bits per
@@ -138,8 +141,8 @@ __device__ __noinline__ bool take_chunk(Pool A, Alloc &al, int64_t bytes) {
     if (b < 0) return false;
     int64_t *h = (int64_t *)(A.base + b);
     h[0] = al.list, h[1] = sz;
-    al.list = b, al.cur = b + 16, al.end = b + sz;
-    al.used += bytes > WFA_CHUNK ? bytes : WFA_CHUNK;
+    al.used = al.total();
+    al.list = b, al.cur = al.from = b + 16, al.end = b + sz;
     return true;
 }
 
@@ -712,7 +715,7 @@ struct WidePlan {
 struct __align__(16) WidePart {
     int k[12];
     int pad[2];
-    unsigned long long used;  // pool bytes of the warps' block reservations (CTA-cooperative piggyback mode)
+    unsigned long long used;  // bytes of the warps' block reservations (CTA-cooperative piggyback mode)
 };
 
 __device__ __forceinline__ void part_reset(WidePart &p, int lane) {
@@ -976,6 +979,7 @@ __device__ void cta_open(const WfaArgs &A, int idx, const HdrRing &HR, CtaShared
         if constexpr (PIG) return warp_alloc(A, al, bytes, lane);
         bytes = (bytes + 15) & ~(int64_t)15;
         if (cur + bytes > chunk_end) {
+            if (lane == 0) al.cur = cur;
             int ok = lane == 0 ? take_chunk(pool_of(A), al, bytes) : 0;
             ok = __shfl_sync(0xffffffffu, ok, 0);
             if (!ok) return -1;
@@ -1207,11 +1211,12 @@ __device__ void cta_open(const WfaArgs &A, int idx, const HdrRing &HR, CtaShared
         if (planner && stop) status = WFA_RETRY;
         op = end || stop ? WOP_DONE : next.op;
     }
-    if (PIG && !planner && lane == 0) atomicAdd(&S.part.used, (unsigned long long)al.used);
+    if (PIG && !planner && lane == 0) atomicAdd(&S.part.used, (unsigned long long)al.total());
     if (PIG) __syncthreads();
     if (planner && lane == 0) {
+        if (!PIG) al.cur = cur;
         finish_pair<PIG>(A, PR, idx, pat, txt, ctab, HR, status, end_score, end_score >= 0 ? end_score : s,
-                         al.used + (PIG ? (int64_t)S.part.used : 0));
+                         al.total() + (PIG ? (int64_t)S.part.used : 0));
         atomicSub(A.queue + 1, 1);
         give_back(pool_of(A), al);
     }
@@ -1514,7 +1519,7 @@ __global__ void __launch_bounds__(wfa_threads(NT), NT > WFA_CTA ? 1 : PIG ? 3 : 
         }
         // ---- backtrace (lane 0)
         if (lane == 0) {
-            finish_pair<PIG>(A, PR, idx, pat, txt, ctab, HR, status, end_score, s, al.used);
+            finish_pair<PIG>(A, PR, idx, pat, txt, ctab, HR, status, end_score, s, al.total());
             atomicSub(A.queue + 1, 1);
         }
         __syncwarp();
@@ -1575,6 +1580,7 @@ struct WidePlanner {
     int plen, tlen;
     int slot;            // s mod R
     int64_t cur, end;    // carving position in the current chunk
+    int64_t used;        // bytes carved
     int nchunks, cidx;   // chunks received, chunk being carved
     bool exhausted;
 };
@@ -1617,7 +1623,6 @@ __global__ void __launch_bounds__(WIDE_NT, 1) wfa_wide_kernel(WfaArgs A, RingSha
     const CompHdr NUL{1, -1, 0, 0, 0};
     WidePlanner W{};
     CompHdr mine = NUL;  // a planner's lane c < 5: component c's header of the planned score
-    int64_t used = 0;  // the leader's pool bytes for the pair
     int it = 0, np = 0;
     // every CTA of the cluster has started (and cleared ann) before one writes another's shared memory
     cl.sync();
@@ -1633,7 +1638,7 @@ __global__ void __launch_bounds__(WIDE_NT, 1) wfa_wide_kernel(WfaArgs A, RingSha
             if (W.cur < 0) return -1;
         }
         const int64_t r = W.cur;
-        W.cur += bytes;
+        W.cur += bytes, W.used += bytes;
         return r;
     };
     // bytes the next plan may carve: one header chunk and the stored components over the
@@ -1770,7 +1775,6 @@ __global__ void __launch_bounds__(WIDE_NT, 1) wfa_wide_kernel(WfaArgs A, RingSha
         if (leader && !W.exhausted && W.nchunks - W.cidx < WIDE_CHUNKS - 1 && !reserve_ok()) {
             int64_t len = wide_chunk(A, need_next());
             const int64_t off = pool_grab_rest(pool_of(A), len, need_next());
-            if (off >= 0) used += len;
             const WideAnn a{W.pi, W.nchunks, off, off >= 0 ? len : 0};
             for (int c = 0; c < CL; ++c) *cl.map_shared_rank(&ann[k & 1], c) = a;
         }
@@ -1789,7 +1793,6 @@ __global__ void __launch_bounds__(WIDE_NT, 1) wfa_wide_kernel(WfaArgs A, RingSha
                 const int64_t ring_b = A.singletrack ? (int64_t)R * 4 * (PR.plen + PR.tlen + 8) * 4 + 16 : 0;
                 const int64_t len = wide_chunk(A, ring_b + (int64_t)sizeof(ScoreHdr) * HDR_CHUNK + 4096);
                 a = WideAnn{pi, idx, pool_grab(pool_of(A), len), len};
-                used = a.off >= 0 ? len : 0;
             }
             for (int c = 0; c < CL; ++c) *cl.map_shared_rank(&pstart[np & 1], c) = a;
         }
@@ -1906,7 +1909,7 @@ __global__ void __launch_bounds__(WIDE_NT, 1) wfa_wide_kernel(WfaArgs A, RingSha
         // ---- backtrace (leader)
         if (leader)
             finish_pair<false>(A, PR, W.idx, pat, txt, A.ctab + PR.ctab_off, HR, W.status, W.end_score, W.end_score >= 0 ? W.end_score : W.s,
-                               used);
+                               W.used);
         cl.sync();
     }
 }

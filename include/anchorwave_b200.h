@@ -235,7 +235,7 @@ int wavefront_align_batch_gpu(wavefront_aligner_gpu_t *aligner, int n, const cha
                               const int *text_length, int *status, int *score,
                               int64_t *ops_offset, int *n_ops, char *ops, int64_t ops_capacity,
                               float *device_ms);
-/* Device memory the last call's alignments took from the wavefront pool (headers,
+/* Bytes the last call's alignments allocated in the wavefront pool (headers,
  * wavefronts and packed-CIGAR blocks; the reference's align_status.memory_used,
  * WfaAlignment.cpp:353-354): the largest single alignment and the sum over the call. */
 int wavefront_gpu_memory(const wavefront_aligner_gpu_t *aligner, int64_t *pair_max, int64_t *total);
