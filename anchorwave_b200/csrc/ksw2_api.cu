@@ -326,7 +326,7 @@ struct aw_ksw_plan {
     std::vector<int32_t> band_ids;   // pairs for the banded kernel
     BandPlan band;
     int refused = 0;                 // banded pairs refused for the budget (reported zdropped)
-    int64_t tb_cap = 0, bnd_cap = 0;
+    int64_t tb_cap = 0, bnd_cap = 0, budget = 0;
     int64_t cells = 0, tb_total = 0;
     int launches = 0;
     bool uploaded = false, executed = false;
@@ -417,7 +417,7 @@ static int plan_build(aw_ksw_plan_t *pl, int n, const int *qlen, const int *tlen
         work += (double)pl->qlen[i] * pl->tlen[i];
         for (int c = 0; c < 2; ++c) chain[c] = std::max(chain[c], chain_steps(pl->qlen[i], pl->tlen[i], c));
     }
-    pl->narrow = strip_seconds(work, chain[1], true) < strip_seconds(work, chain[0], false);
+    const bool narrow_faster = strip_seconds(work, chain[1], true) < strip_seconds(work, chain[0], false);
     const double batch_s = work / 1e12;
     for (int i = 0; i < n; ++i) {
         if (pl->route[i] != 1) continue;
@@ -446,33 +446,50 @@ static int plan_build(aw_ksw_plan_t *pl, int n, const int *qlen, const int *tlen
         const int64_t ca = (int64_t)pl->qlen[a] * pl->tlen[a], cb = (int64_t)pl->qlen[b] * pl->tlen[b];
         return ca != cb ? ca > cb : a < b;
     });
-    // LPT multiway partition of traceback bytes into the fewest waves that fit
-    std::vector<std::vector<int32_t>> wv;
-    std::vector<int64_t> wload, wbnd;
-    for (int32_t i : strip) {
-        const int64_t tbb = cigar ? ksw_full_tb_bytes(pl->qlen[i], pl->tlen[i], pl->narrow, tracks) : 0;
-        const int64_t bw = ksw_full_bnd_words(pl->qlen[i], pl->tlen[i], pl->narrow);
-        pl->tb_total += tbb;
+    for (int32_t i : strip)
         if (cigar && ksw_full_tb_bytes(pl->qlen[i], pl->tlen[i], false, tracks) > budget) {
             set_error("pair traceback exceeds the HBM traceback budget");
             return AW_E_NOMEM;
         }
-        int best = -1;
-        for (size_t k = 0; k < wv.size(); ++k)
-            if (wload[k] + tbb <= budget && (best < 0 || wload[k] < wload[best])) best = (int)k;
-        if (best < 0) {
-            wv.emplace_back();
-            wload.push_back(0);
-            wbnd.push_back(0);
-            best = (int)wv.size() - 1;
+    // LPT multiway partition into the fewest waves whose tracebacks fit the budget, and with narrow
+    // strips their boundary columns as well (a 16th of a traceback; a 64th with wide ones, which
+    // come on top of it).  False: a pair alone does not fit.
+    std::vector<std::vector<int32_t>> wv;
+    std::vector<int64_t> wload, wbnd;
+    auto pack = [&](bool narrow) {
+        wv.clear(), wload.clear(), wbnd.clear(), pl->tb_total = 0;
+        for (int32_t i : strip) {
+            const int64_t tbb = cigar ? ksw_full_tb_bytes(pl->qlen[i], pl->tlen[i], narrow, tracks) : 0;
+            const int64_t bw = ksw_full_bnd_words(pl->qlen[i], pl->tlen[i], narrow);
+            auto fits = [&](size_t k) {
+                return wload[k] + tbb + (narrow ? 4 * (wbnd[k] + bw) : 0) <= budget;
+            };
+            int best = -1;
+            for (size_t k = 0; k < wv.size(); ++k)
+                if (fits(k) && (best < 0 || wload[k] < wload[best])) best = (int)k;
+            if (best < 0) {
+                wv.emplace_back();
+                wload.push_back(0);
+                wbnd.push_back(0);
+                best = (int)wv.size() - 1;
+                if (narrow && !fits(best)) return false;
+            }
+            KswPair &kp = pl->pairs[i];
+            kp.tb_off = wload[best];
+            kp.bnd_off = wbnd[best];
+            wload[best] += (tbb + 255) / 256 * 256;
+            wbnd[best] += (bw + 63) / 64 * 64;
+            wv[best].push_back(i);
+            pl->tb_total += tbb;
         }
-        KswPair &kp = pl->pairs[i];
-        kp.tb_off = wload[best];
-        kp.bnd_off = wbnd[best];
-        wload[best] += (tbb + 255) / 256 * 256;
-        wbnd[best] += (bw + 63) / 64 * 64;
-        wv[best].push_back(i);
-    }
+        return true;
+    };
+    // narrow strips where they are faster and need no further wave
+    pack(false);
+    const size_t wide_waves = wv.size();
+    pl->narrow = narrow_faster && pack(true) && wv.size() <= wide_waves;
+    if (narrow_faster && !pl->narrow) pack(false);
+    pl->budget = budget;
     // Work units: the strips of a pair on as many warps, or the whole pair on one warp (no
     // waiting between strips, which is the better use of a warp while there are pairs enough).
     // A pair is split when its strips are narrow, when its target is long (aw_set_tuning), when
@@ -548,8 +565,12 @@ static int plan_alloc(aw_ksw_plan_t *pl) {
     AW_CUDA(B->cig.ensure(4 * (size_t)(pl->cig_words + 1)));
     AW_CUDA(B->packed.ensure(4 * (size_t)(pl->cig_words + 1)));
     AW_CUDA(B->packed_off.ensure(8 * (size_t)std::max(n, 1)));
+    // boundary columns that an earlier plan's narrow strips left larger than this plan's: given back
+    // when they and this plan's traceback would exceed its budget together
+    const int64_t bnd_bytes = 4 * pl->bnd_cap + 256;
+    if ((int64_t)B->bnd.cap > bnd_bytes && pl->tb_cap + (int64_t)B->bnd.cap > pl->budget) B->bnd.release();
     AW_CUDA(B->tb.ensure((size_t)pl->tb_cap + 256));
-    AW_CUDA(B->bnd.ensure(4 * (size_t)pl->bnd_cap + 256));
+    AW_CUDA(B->bnd.ensure((size_t)bnd_bytes));
     AW_CUDA(B->queue.ensure(sizeof(int32_t) * 64 * (pl->waves.size() + 1)));  // a counter per wave
     AW_CUDA(B->error.ensure(sizeof(int32_t) * 4));
     if (!pl->band_ids.empty()) {

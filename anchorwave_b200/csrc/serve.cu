@@ -77,7 +77,8 @@ int64_t predict_bytes(const Req &rq) {
     if (rq.method == AW_ROUTE_SLIDING_WINDOW) {
         // one window's full traceback at a time
         const int64_t w = std::max<int64_t>(1, std::min<int64_t>(rq.window + 1, std::max(ql, tl)));
-        return ksw_full_tb_bytes((int)std::min<int64_t>(w, ql), (int)std::min<int64_t>(w, tl));
+        const int wq = (int)std::min<int64_t>(w, ql), wt = (int)std::min<int64_t>(w, tl);
+        return ksw_full_tb_bytes(wq, wt) + 4 * ksw_full_bnd_words(wq, wt, true);
     }
     if (rq.method >= AW_ROUTE_WFA) {
         // wavefront retention grows with the alignment score; a length-based proxy (the
@@ -89,7 +90,8 @@ int64_t predict_bytes(const Req &rq) {
         const int64_t n = std::min(std::min(ql, tl), (int64_t)rq.band + 1);
         return (ql + tl) * ((n + 63) / 64 + 1) * 64 * (rq.method == AW_ROUTE_KSW2_SINGLETRACK ? 2 : 1);
     }
-    return ksw_full_tb_bytes((int)ql, (int)tl) * (rq.method == AW_ROUTE_KSW2_SINGLETRACK ? 2 : 1);
+    return ksw_full_tb_bytes((int)ql, (int)tl) * (rq.method == AW_ROUTE_KSW2_SINGLETRACK ? 2 : 1) +
+           4 * ksw_full_bnd_words((int)ql, (int)tl, true);
 }
 
 // encodeKswSequence (src/myImportandFunction/alignSlidingWindow.cpp:645-660)
@@ -132,8 +134,9 @@ struct aw_server {
 
 namespace {
 
-// Device memory of one worker: its share of the budget, split between the KSW2 traceback
-// arena (50%, reserved when the worker starts) and the wavefront pools of the four WFA
+// Device memory of one worker: its share of the budget, split between KSW2 (50%: 16/17 of it the
+// traceback arena, reserved when the worker starts, 1/17 left to the boundary columns of narrow
+// strips, which a plan counts with its traceback) and the wavefront pools of the four WFA
 // engines (allocated when an engine first runs; high memory 16%, Singletrack 26% -- the
 // engine AnchorWave's selector picks most, for intervals up to tens of kb -- medium and low
 // 4% each as they keep a ring and packed-CIGAR blocks), so that the pooled allocations of
@@ -310,7 +313,7 @@ void worker_main(aw_server *S, int slot) {
     // each worker's batches get an equal share of the device budget
     const int64_t tb = std::max<int64_t>(ksw_tb_share(S), (int64_t)1 << 26);
     set_thread_tb_budget(tb);
-    reserve_thread_tb(tb);
+    reserve_thread_tb(tb / 17 * 16);
     std::vector<Req> batch;
     std::vector<Res> res;
     wavefront_aligner_gpu_t *al[4] = {nullptr, nullptr, nullptr, nullptr};
