@@ -75,6 +75,7 @@ constexpr uint32_t PC_ALMOST_FULL = 0x10000000u;  // 15 operations or more
 constexpr uint32_t BT_NULL = 0xFFFFFFFFu;          // no earlier block
 constexpr int PIG_U = 2;                           // diagonals per lane in flight
 constexpr uint32_t LANE_BLOCKS = 32;               // blocks a lane reserves at a time
+constexpr int64_t TIGHT_PIECE = 64 << 10;          // bytes taken at a time by a pair alone (WfaArgs::free_slots)
 
 // The pool as the allocating functions (out of line, so no reference to the kernel's arguments)
 // take it.
@@ -134,6 +135,18 @@ __device__ __forceinline__ void free_push(const Pool &A, int64_t off) {
 
 // One thread: a chunk that holds `bytes`, linked to the allocation's list; false if there is none.
 __device__ __noinline__ bool take_chunk(Pool A, Alloc &al, int64_t bytes) {
+    if (A.slots == 0) {  // a pair alone
+        const int64_t len = *(volatile int64_t *)&A.ctl->head + TIGHT_PIECE <= A.bytes ? max(bytes, TIGHT_PIECE) : bytes;
+        const int64_t b = pool_grab(A, len);
+        if (b < 0) return false;
+        if (b == al.end) {  // the current piece grows
+            al.end += len;
+            return true;
+        }
+        al.used = al.total();
+        al.cur = al.from = b, al.end = b + len;
+        return true;
+    }
     const int64_t sz = (bytes + 16 + WFA_CHUNK - 1) / WFA_CHUNK * WFA_CHUNK;
     int64_t b = sz == WFA_CHUNK ? free_pop(A) : -1;
     if (b < 0) b = pool_grab(A, sz);
@@ -943,7 +956,7 @@ __device__ __noinline__ void plan_trim(const WfaPairDev &PR, const WidePlan &Q, 
 // CTA barrier per score is left (two, with the plan between them, took 3.8 us a score at 2 kb,
 // half of it waiting for the plan; now 2.3).  A pair whose wavefront grows too wide stops with
 // WFA_WIDE for the cluster kernel; in the piggyback modes none does, and every warp reserves its own
-// block runs.
+// block runs.  A pair that takes the last of the pool (WfaArgs::free_slots) is trimmed from the start.
 struct CtaShared {
     WidePlan plan[2];
     WidePart part;
@@ -1120,6 +1133,7 @@ __device__ void cta_open(const WfaArgs &A, int idx, const HdrRing &HR, CtaShared
             atomicAdd(A.queue + 1, 1), atomicAdd(A.queue + 3, 1);  // pairs running, started
             for (int b = 0; b < 3; ++b) S.at_end[b] = S.beyond[b] = S.retry[b] = 0;
             S.part.used = 0;
+            if (A.free_slots == 0) S.beyond[0] = 1;  // trimmed from the first score on
         }
         __syncwarp();
         part_reset(S.part, lane);

@@ -223,11 +223,32 @@ static int run_batch(wavefront_aligner_gpu *al, int n, const char *const *patter
     W.wide_tail_cta = (int)std::min<int64_t>(W.wide_width, 8 * (int64_t)W.wide_width_tail);
     const int64_t long_sum = g_long_sum.load();
     std::vector<int32_t> staged;
+    // One pair on the pool to itself, in the least memory: what a batch that stores wavefronts
+    // untrimmed and in chunks of 256 KiB, or in a cluster's reserve chunks, has refused (in a pool of
+    // 64 MB pairs of up to 1,494 against 1,369 bases at 25%, 8,681 against 8,292 at 4%).
+    auto run_tight = [&](int32_t i, float &ms) -> int {
+        WCUDA(cudaMemcpyAsync(al->d_order.p, &i, sizeof(i), cudaMemcpyHostToDevice, al->st));
+        WCUDA(cudaMemsetAsync(al->d_queue.p, 0, 32, al->st));
+        WCUDA(cudaMemsetAsync(al->d_ctl.p, 0, sizeof(WfaPoolCtl), al->st));
+        WfaArgs T = W;
+        T.free_slots = 0, T.n_all = 1, T.q_long = 2;
+        T.wide_width = T.wide_width_tail = T.wide_width_cta = T.wide_tail_cta = 0;
+        T.order = T.order_long = al->d_order.as<int32_t>();
+        T.n_long = long_sum > 0 ? 1 : 0, T.n = 1 - T.n_long;
+        WCUDA(cudaEventRecord(al->e0, al->st));
+        WCUDA(launch_wfa(T, WFA_CTA, 1, al->st));
+        WCUDA(cudaEventRecord(al->e1, al->st));
+        WCUDA(cudaMemcpyAsync(&al->outs[i], al->d_out.as<WfaOutDev>() + i, sizeof(WfaOutDev), cudaMemcpyDeviceToHost,
+                              al->st));
+        WCUDA(cudaStreamSynchronize(al->st));
+        WCUDA(cudaEventElapsedTime(&ms, al->e0, al->e1));
+        return AW_OK;
+    };
     // Rounds: every round restarts the pool and runs up to `chunk` pending pairs, largest
     // first; pairs that found the pool exhausted stay pending.  A round that completes
     // nothing halves the chunk (the pairs in flight together share the pool), one that
     // completes all of its pairs doubles it again; a pair that cannot finish with the whole
-    // pool to itself reports WF_STATUS_OOM (the reference's max-memory abort).
+    // pool to itself, in the least memory, reports WF_STATUS_OOM (the reference's max-memory abort).
     std::vector<int32_t> wide;
     al->last_cluster_launches = 0;
     float total_ms = 0.f;
@@ -323,7 +344,10 @@ static int run_batch(wavefront_aligner_gpu *al, int n, const char *const *patter
                         launches, phase ? "cluster" : "warp", batch.size(), again.size(), handed, ms);
             const size_t done = batch.size() - again.size();
             if (done == 0 && take == 1) {
-                al->outs[batch[0]].status = WFA_OOM;
+                const int rc = run_tight(batch[0], ms);
+                if (rc) return rc;
+                total_ms += ms, ++launches;
+                if (al->outs[batch[0]].status == WFA_RETRY) al->outs[batch[0]].status = WFA_OOM;
                 again.clear();
             } else if (done == 0) {
                 chunk = std::max<size_t>(1, take / 2);

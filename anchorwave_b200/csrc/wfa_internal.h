@@ -51,7 +51,9 @@ struct WfaArgs {
     int64_t pool_bytes;
     WfaPoolCtl *ctl;
     int32_t *free_ring;   // chunks given back by finished pairs: chunk number + 1, 0 = empty slot
-    uint32_t free_slots;  // at least the chunks of the pool
+    // at least the chunks of the pool; 0: one pair alone, in as little of the pool as it can do with
+    // (wavefronts trimmed from the start, memory taken in exact pieces that are not given back)
+    uint32_t free_slots;
     int64_t *ctab;
     char *ops;
     WfaOutDev *out;

@@ -28,3 +28,26 @@ def test_pool_exhausted_inside_cta_pairs(gpu, restatement, mode):
     assert launches > 2  # one round takes two launches at most
     for i, (p, t, r) in enumerate(zip(ps, ts, res)):
         assert r == restatement.wfa_align(p, t, *PEN, False, memory_mode=mode), i
+
+
+@pytest.mark.parametrize("length,d,singletrack,mode", [(8681, 0.04, False, 0), (1494, 0.25, False, 0),
+                                                       (3336, 0.25, True, 0), (3774, 0.25, False, 1)])
+def test_pair_that_takes_the_last_of_the_pool(gpu, restatement, length, d, singletrack, mode):
+    """A pair alone in a pool that holds its trimmed wavefronts and little more, among pairs that
+    share the same pool before and after it."""
+    rng = np.random.default_rng(1)
+    q, t = W.divergent_pair(rng, length, d, d, 4.0)
+    p, x = W.to_ascii(t), W.to_ascii(q)
+    few, fex = _pairs(3, [900] * 12, 0.05)
+    al = wfa.WfaAligner(*PEN, singletrack=singletrack, memory_mode=mode, max_memory_abort=64 << 20)
+    try:
+        alone, _ = al.align_batch([p], [x])
+        batch, _ = al.align_batch(few[:6] + [p] + few[6:], fex[:6] + [x] + fex[6:])
+    finally:
+        al.close()
+    want = restatement.wfa_align(p, x, *PEN, singletrack, memory_mode=mode)
+    assert want[0] == 0
+    same = [alone[0] == want, batch[6] == want]
+    same += [r == restatement.wfa_align(few[i], fex[i], *PEN, singletrack, memory_mode=mode)
+             for i, r in enumerate(batch[:6] + batch[7:])]
+    assert all(same), (same, alone[0][:2], batch[6][:2])
