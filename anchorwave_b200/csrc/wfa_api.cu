@@ -257,7 +257,7 @@ static int run_batch(wavefront_aligner_gpu *al, int n, const char *const *patter
     // (one pair at 5%: 10 kb 8.3 ms against 13.6 on a CTA to the end, 5 kb 4.1 against 5.4, 2 kb
     // 1.7 against 1.5).
     std::vector<int32_t> first = order;
-    if (W.wide_width > 0 && n <= wide_clusters) {
+    if (W.wide_width > 0 && long_sum > 0 && n <= wide_clusters) {
         auto is_long = [&](int32_t i) { return (int64_t)plen[i] + tlen[i] >= kClusterSum; };
         std::copy_if(order.begin(), order.end(), std::back_inserter(wide), is_long);
         first.erase(std::remove_if(first.begin(), first.end(), is_long), first.end());
