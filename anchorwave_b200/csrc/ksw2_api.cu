@@ -316,7 +316,8 @@ struct aw_ksw_plan {
     int64_t qbytes = 0, tbytes = 0, cig_words = 0;
     // waves of strip-kernel pairs: their ranges in order[] and units[]
     struct Wave {
-        int begin, n, unit0, nunit;
+        int begin, n;
+        int unit0[2], nunit[2];  // by large_warps: 1, more
         int64_t tb_bytes, bnd_words;
     };
     std::vector<Wave> waves;
@@ -335,7 +336,7 @@ struct aw_ksw_plan {
     // eagerly (lazy set-up of the kernels), the second captures the launch sequence, later
     // ones replay it
     int eager_runs = 0;
-    bool graph_off = false, graph_used = false;
+    bool graph_off = false, graph_used = false, graph_split = false;
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t gexec = nullptr;
     void drop_graph() {
@@ -396,11 +397,11 @@ static int plan_build(aw_ksw_plan_t *pl, int n, const int *qlen, const int *tlen
     pl->qbytes = qb, pl->tbytes = tbt, pl->cig_words = cw;
     const bool cigar = !(P.flag & AW_EZ_SCORE_ONLY), tracks = cigar && (P.flag & AW_EZ_SINGLETRACK);
     int64_t budget = tls_tb_budget;
-    int large_tlen, large_warps;
+    int large_tlen;
     {
         std::lock_guard<std::mutex> lk(g_cfg_mu);
         if (budget <= 0) budget = g_tb_budget;
-        large_tlen = g_large_tlen, large_warps = g_large_warps;
+        large_tlen = g_large_tlen;
     }
     if (budget <= 0) {
         size_t fr = 0, tot = 0;
@@ -494,7 +495,8 @@ static int plan_build(aw_ksw_plan_t *pl, int n, const int *qlen, const int *tlen
     // waiting between strips, which is the better use of a warp while there are pairs enough).
     // A pair is split when its strips are narrow, when its target is long (aw_set_tuning), when
     // all strips of the wave are on warps at once anyway, or when one warp would take longer for
-    // it (0.65 us a step on a full SM) than half the wave's work.
+    // it (0.65 us a step on a full SM) than half the wave's work.  Both forms of aw_set_tuning's
+    // large_warps are kept, as a plan follows the setting at each execution.
     for (size_t k = 0; k < wv.size(); ++k) {
         aw_ksw_plan::Wave W;
         int64_t strips = 0;
@@ -503,18 +505,24 @@ static int plan_build(aw_ksw_plan_t *pl, int n, const int *qlen, const int *tlen
             strips += ksw_full_strips(pl->tlen[i], pl->narrow);
             cells += (double)pl->qlen[i] * pl->tlen[i];
         }
-        W.begin = (int)pl->order.size(), W.unit0 = (int)pl->units.size();
-        for (int32_t i : wv[k]) {
-            pl->order.push_back(i);
-            const int ns = (int)ksw_full_strips(pl->tlen[i], pl->narrow);
-            const bool split = pl->narrow || (large_warps > 1 && (pl->tlen[i] >= large_tlen || strips <= kResidentWarps ||
-                                                                  ns * (pl->qlen[i] + 64.0) * 0.65e-6 > 0.5 * cells / 1e12));
-            if (!split || ns == 1) pl->units.push_back(make_int2(i, -1));
-            else
-                for (int u = 0; u < ns; ++u) pl->units.push_back(make_int2(i, u));
+        W.begin = (int)pl->order.size(), W.n = (int)wv[k].size();
+        pl->order.insert(pl->order.end(), wv[k].begin(), wv[k].end());
+        for (int more = 0; more < 2; ++more) {
+            W.unit0[more] = (int)pl->units.size();
+            for (int32_t i : wv[k]) {
+                const int ns = (int)ksw_full_strips(pl->tlen[i], pl->narrow);
+                const bool split = pl->narrow || (more && (pl->tlen[i] >= large_tlen || strips <= kResidentWarps ||
+                                                           ns * (pl->qlen[i] + 64.0) * 0.65e-6 > 0.5 * cells / 1e12));
+                if (!split || ns == 1) pl->units.push_back(make_int2(i, -1));
+                else
+                    for (int u = 0; u < ns; ++u) pl->units.push_back(make_int2(i, u));
+            }
+            W.nunit[more] = (int)pl->units.size() - W.unit0[more];
+            if (pl->narrow) {
+                W.unit0[1] = W.unit0[0], W.nunit[1] = W.nunit[0];
+                break;
+            }
         }
-        W.n = (int)pl->order.size() - W.begin;
-        W.nunit = (int)pl->units.size() - W.unit0;
         W.tb_bytes = wload[k];
         W.bnd_words = wbnd[k];
         pl->tb_cap = std::max(pl->tb_cap, W.tb_bytes);
@@ -655,6 +663,11 @@ static int plan_upload(aw_ksw_plan_t *pl, const uint8_t *const *query, const uin
     return AW_OK;
 }
 
+static bool large_split() {
+    std::lock_guard<std::mutex> lk(g_cfg_mu);
+    return g_large_warps > 1;
+}
+
 // Enqueues every wave of the plan on its stream (no host synchronisation).
 static int plan_launch(aw_ksw_plan_t *pl) {
     Buffers *B = pl->B;
@@ -685,7 +698,7 @@ static int plan_launch(aw_ksw_plan_t *pl) {
         AW_CUDA(cudaEventCreate(&e));
         B->ev_k.push_back(e);
     }
-    const int nw = (int)pl->waves.size();
+    const int nw = (int)pl->waves.size(), more = large_split() ? 1 : 0;
     for (int k = 0; k < nw; ++k) {
         const auto &W = pl->waves[k];
         KswFullArgs a;
@@ -698,8 +711,8 @@ static int plan_launch(aw_ksw_plan_t *pl) {
         a.deadline = deadline;
         AW_CUDA(record_timing(B->ev_k[3 * k], B->st));
         AW_CUDA(cudaMemsetAsync(B->bnd.p, 0, 4 * (size_t)W.bnd_words, B->st));
-        a.units = B->units.as<int2>() + W.unit0;
-        a.n = W.nunit;
+        a.units = B->units.as<int2>() + W.unit0[more];
+        a.n = W.nunit[more];
         a.queue = B->queue.as<int32_t>() + 64 * k;
         const int per = ksw_full_warps_per_cta(pl->narrow);
         const int occ = std::max(1, ksw_full_occupancy(P.flag, pl->narrow));
@@ -937,6 +950,8 @@ int aw_ksw_plan_execute(aw_ksw_plan_t *pl, float *ms) {
     if (pl->graph_off || !pl->uploaded || !pl->exact_ids.empty() || tls_has_deadline ||
         pl->cells > kGraphMaxCells)
         return plan_execute(pl, ms);
+    const bool split = large_split();
+    if (pl->gexec && pl->graph_split != split) pl->drop_graph();  // tuning changed: capture again
     if (!pl->gexec) {
         if (pl->eager_runs < 1) {
             ++pl->eager_runs;
@@ -957,7 +972,7 @@ int aw_ksw_plan_execute(aw_ksw_plan_t *pl, float *ms) {
             pl->graph_off = true;
             return plan_execute(pl, ms);
         }
-        pl->graph = g, pl->gexec = ge;
+        pl->graph = g, pl->gexec = ge, pl->graph_split = split;
     }
     AW_CUDA(cudaGraphLaunch(pl->gexec, pl->B->st));
     pl->graph_used = true;
