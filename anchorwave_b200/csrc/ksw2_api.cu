@@ -361,9 +361,10 @@ static double strip_seconds(double cells, double longest_chain, bool narrow) {
 static double chain_steps(double qlen, int tlen, bool narrow) {
     return qlen + KSW_LAG + 80.0 * (double)(ksw_full_strips(tlen, narrow) - 1);
 }
-static constexpr int64_t kResidentWarps = 2368;  // 148 SMs x 16 warps of wide strips
+static constexpr int64_t kWarpsPerSM = 16;  // of wide strips
 
 static int plan_build(aw_ksw_plan_t *pl, int n, const int *qlen, const int *tlen, const int *w) {
+    if (const int rc = pl->B->init()) return rc;
     pl->n = n;
     pl->qlen.assign(qlen, qlen + n);
     pl->tlen.assign(tlen, tlen + n);
@@ -511,7 +512,7 @@ static int plan_build(aw_ksw_plan_t *pl, int n, const int *qlen, const int *tlen
             W.unit0[more] = (int)pl->units.size();
             for (int32_t i : wv[k]) {
                 const int ns = (int)ksw_full_strips(pl->tlen[i], pl->narrow);
-                const bool split = pl->narrow || (more && (pl->tlen[i] >= large_tlen || strips <= kResidentWarps ||
+                const bool split = pl->narrow || (more && (pl->tlen[i] >= large_tlen || strips <= kWarpsPerSM * pl->B->sms ||
                                                            ns * (pl->qlen[i] + 64.0) * 0.65e-6 > 0.5 * cells / 1e12));
                 if (!split || ns == 1) pl->units.push_back(make_int2(i, -1));
                 else
@@ -559,8 +560,6 @@ static int plan_build(aw_ksw_plan_t *pl, int n, const int *qlen, const int *tlen
 
 static int plan_alloc(aw_ksw_plan_t *pl) {
     Buffers *B = pl->B;
-    int rc = B->init();
-    if (rc) return rc;
     const int n = pl->n;
     AW_CUDA(B->qcodes.ensure(pl->qbytes + 16));
     AW_CUDA(B->tcodes.ensure(pl->tbytes + 16));

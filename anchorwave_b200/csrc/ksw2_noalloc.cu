@@ -189,7 +189,10 @@ extern "C" int aw_ksw_extd2_device_noalloc(int qlen, const uint8_t *d_query, int
     // one strip per warp; no boundary entry is written yet.  A strip only waits for units taken
     // before it, so the grid need not be resident as a whole.
     const int per = ksw_full_warps_per_cta(narrow);
-    const int ctas = (int)std::min<int64_t>((a.n + (int64_t)per - 1) / per, 148);
+    int dev = 0, sms = 1;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    const int ctas = (int)std::min<int64_t>((a.n + (int64_t)per - 1) / per, sms);
     if (cudaMemsetAsync(bnd, 0, (size_t)bnd_bytes, st) != cudaSuccess ||
         launch_ksw_full(a, flag, narrow, ctas, st) != cudaSuccess) {
         set_error("aw_ksw_extd2_device_noalloc: DP launch failed");
