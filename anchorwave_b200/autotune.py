@@ -5,8 +5,8 @@ distribution), the fastest installed or returned:
   * full-matrix strip kernel (aw_set_tuning): large_warps (above 1: the strips of a large pair
     run on a warp each), and large_tlen_threshold, the target length from which a pair counts
     as large;
-  * banded strip kernel (aw_set_band_columns): formerly its target columns per lane; the kernel
-    has one width now, so the trials differ by noise only;
+  * banded strip kernel (aw_set_band_columns): formerly its target columns per lane; nothing to
+    choose any more;
   * serving loop: worker slots and the micro-batch size, chosen for the lowest p99 latency at
     a fixed offered request rate among the settings that finish the trace within 15% of the
     fastest one.  The trials should run the whole trace: a sample's tail is made of other
@@ -27,7 +27,7 @@ import numpy as np
 
 from . import ksw2
 
-WARPS = (2, 4, 8)
+WARPS = (1, 8)  # 2 and 4 are the same setting as 8
 THRESHOLDS = (1024, 2048, 4096, 8192)
 BAND_COLUMNS = (4, 8)
 SERVE_SLOTS = (2,)
@@ -66,8 +66,9 @@ def tune(queries: Sequence[np.ndarray], targets: Sequence[np.ndarray], mat, q, e
 def tune_band(queries: Sequence[np.ndarray], targets: Sequence[np.ndarray], bands: Sequence[int], mat, q, e, q2,
               e2, flag: int = 0, sample: int = 8, reps: int = 1, seed: int = 0,
               budget: int = 0) -> Tuple[int, List[Dict]]:
-    """Banded kernel: times the sample under each setting of aw_set_band_columns (without effect
-    since the kernel has one width); returns (columns, trials) and installs the winner.  `budget` > 0: the traceback
+    """Banded kernel: times the sample under each setting of aw_set_band_columns, which has no effect
+    since the kernel has one width, so that the trials show the noise of a timing and nothing else;
+    returns (columns, trials) as it did when there was a choice.  `budget` > 0: the traceback
     budget of the trials (a share of the whole batch's, so that the sample's pairs recompute
     their tracebacks in rounds as the batch's do)."""
     idx = _sample(len(queries), sample, seed)

@@ -631,7 +631,7 @@ def cigar_check(res, q, t, mis=4, o1=4, e1=2, o2=24, e2=1):
 
 
 def long_banded_measurement(rank: int, cpu: bool, npairs: int = 64, lmin: int = 100_000, lmax: int = 1_000_000,
-                            long_max: int = 50_000, budget_gb: float = 0.0, tuning=None):
+                            long_max: int = 50_000, budget_gb: float = 0.0):
     """The long-interval banded and Singletrack workload (target length U(lmin, lmax), 30% of
     the query replaced by repeat structure, 3% substitutions, 5-20 long indels of U(1,
     long_max), w = 10% of the shorter length): one execution of the whole set per traceback,
@@ -657,17 +657,6 @@ def long_banded_measurement(rank: int, cpu: bool, npairs: int = 64, lmin: int = 
     warm.upload()
     warm.execute()
     warm.close()
-    # the autotuner's trials of the banded kernel, on the four pairs with the most band cells,
-    # score-only (the kernel has one lane width, so they differ by noise only)
-    from anchorwave_b200 import autotune
-    t_tune = time.perf_counter()
-    pick = sorted(sorted(range(len(ps)), key=lambda i: -pair_cells[i])[:4])
-    cols, trials = autotune.tune_band([ps.queries[i] for i in pick], [ps.targets[i] for i in pick],
-                                      [ps.band[i] for i in pick], mat, 4, 2, 24, 1, flag=0x01, sample=len(pick),
-                                      reps=1)
-    if tuning is not None:
-        tuning["band_kernel"] = {"columns_per_lane": cols, "trials_ms": {str(t["columns"]): t["ms"] for t in trials},
-                                 "seconds": time.perf_counter() - t_tune, "sample_pairs": len(pick)}
     results = {}
     if budget_gb > 0:
         ksw2.set_traceback_budget(int(budget_gb * 1e9))
@@ -699,7 +688,6 @@ def long_banded_measurement(rank: int, cpu: bool, npairs: int = 64, lmin: int = 
                      # score (the reference re-scores for that reason, alignSlidingWindow.cpp:872-876)
                      "cigars_rescoring_to_score": rescored}
         ksw2.release_thread_buffers()
-    ksw2.set_band_columns(0)
     if budget_gb > 0:
         ksw2.set_traceback_budget(0)
     if cpu:
@@ -924,8 +912,7 @@ def main():
     serving = serving_measurement(args.serve_requests, rank, tuning) if args.serve_requests > 0 else None
     long_banded = None if args.no_long_banded else long_banded_measurement(
         rank, cpu_on, args.long_banded_pairs, args.long_banded_min, args.long_banded_max, args.long_banded_indel,
-        args.long_banded_budget_gb,
-        tuning)
+        args.long_banded_budget_gb)
     wfa_res = (wfa_measurement(args.wfa_pairs, rank, cpu_on, args.wfa_pool_gb) if args.wfa_pairs > 0 else None)
     wfa_long = wfa_long_measurement(args.wfa_long_pairs, rank, cpu_on) if args.wfa_long_pairs > 0 else None
     summary_res = (None if args.no_selector_summary else selector_summary_measurement(ps, rank, cpu_on))
@@ -1062,7 +1049,6 @@ def compact_summary(line):
         par["selector_pass"] = get(ss, "cpu_reference", "summaries_identical")
     tn = line.get("tuning") or {}
     out["tuning"] = {"full": [get(tn, "full_kernel", "large_warps"), get(tn, "full_kernel", "large_tlen_threshold")],
-                     "band_columns": get(tn, "band_kernel", "columns_per_lane"),
                      "serve": [get(tn, "serving", "slots"), get(tn, "serving", "max_batch")]}
     out["parity"] = par
     return sig(out)
