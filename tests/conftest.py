@@ -42,3 +42,12 @@ def gpu():
         pytest.fail("no CUDA device visible to libaw_b200.so (gpu tests must run on a GPU box)")
     from anchorwave_b200 import ksw2
     return ksw2
+
+
+@pytest.fixture(autouse=True)
+def _default_long_pairs(request):
+    """Tests that set aw_set_wfa_long (process-wide) leave its default behind."""
+    yield
+    if request.node.get_closest_marker("gpu"):
+        from anchorwave_b200 import wfa
+        wfa.set_long(800)

@@ -1,5 +1,6 @@
-"""WFA pairs on whole CTAs in a pool that is too small for all of them at once: the ones that
-find it exhausted run again in later rounds, with unchanged results."""
+"""WFA pairs on whole CTAs in a pool that is too small for all of them at once: the next ones live on
+the chunks of those that are finished, the ones that find the pool exhausted run again in later
+rounds, with unchanged results."""
 import numpy as np
 import pytest
 
@@ -51,3 +52,23 @@ def test_pair_that_takes_the_last_of_the_pool(gpu, restatement, length, d, singl
     same += [r == restatement.wfa_align(few[i], fex[i], *PEN, singletrack, memory_mode=mode)
              for i, r in enumerate(batch[:6] + batch[7:])]
     assert all(same), (same, alone[0][:2], batch[6][:2])
+
+
+@pytest.mark.parametrize("singletrack,mode", [(False, 0), (True, 0)])
+def test_finished_pairs_give_their_chunks_back(gpu, restatement, singletrack, mode):
+    """4,000 pairs that take twice the pool and more together, a third of it at a time: one round (two
+    launches at most), which takes as many more as the pool is short of if the chunks do not come back."""
+    pool = 2000 << 20
+    ps, ts = _pairs(31, [900] * 4000, 0.12 if singletrack else 0.06)
+    al = wfa.WfaAligner(*PEN, singletrack=singletrack, memory_mode=mode, max_memory_abort=pool)
+    try:
+        wfa.set_wide(0, 0, 8)
+        res, _ = al.align_batch(ps, ts)
+        launches, total = al.launches()[0], al.memory()[1]
+    finally:
+        wfa.set_wide(8192, 1024, 8)
+        al.close()
+    assert all(r[0] == 0 for r in res)
+    assert total > 2 * pool and launches <= 2, (launches, total)
+    for i in range(0, len(ps), 100):
+        assert res[i] == restatement.wfa_align(ps[i], ts[i], *PEN, singletrack, memory_mode=mode), i
