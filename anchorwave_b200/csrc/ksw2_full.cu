@@ -370,6 +370,19 @@ __global__ void __launch_bounds__(32 * cta_warps<NP>(), NP == 8 ? 2 : 5) ksw_ful
                     ns = ns < 256 ? ns * 2 : ns;
                 }
             };
+            // past the deadline: no score and no traceback (ksw2_extd2_sse.c:136-139, :400-409), and
+            // the ends as far as the pair got.  Its last strip always comes here, as it cannot
+            // finish without those on its left; the warp of a whole pair may stop before it.
+            auto report_stop = [&]() {
+                if (lane != C.c_lane || (!last && un.y >= 0)) return;
+                const unsigned long long k = *(volatile unsigned long long *)&A.res[idx].mqe_key;
+                KswOut o;
+                o.score = AW_NEG_INF, o.max = 0, o.max_q = -1, o.max_t = -1;
+                o.mqe = k ? (int)((uint32_t)(k >> 32) ^ 0x80000000u) : AW_NEG_INF, o.mqe_t = k ? (int)(uint32_t)k : -1;
+                o.mte = last && mte_q >= 0 ? mte16 >> 4 : AW_NEG_INF, o.mte_q = last ? mte_q : -1;
+                o.n_cigar = 0, o.zdropped = 0, o.reach_end = 0, o.stopped = 1;
+                A.out[idx] = o;
+            };
             auto code_of = [&](int row) -> uint32_t { return row < qlen ? (qs[row] & 7u) << 16 : 0u; };
             // lane i holds what lane 0 needs for row (k & ~31) + i: the next group's entries and
             // the next 32 query codes are on their way while the current ones are used
@@ -411,6 +424,7 @@ __global__ void __launch_bounds__(32 * cta_warps<NP>(), NP == 8 ? 2 : 5) ksw_ful
                 }
             }
             __syncwarp();
+            if (stopped) report_stop();
             if (stopped || failed) break;
             // last row: H(qlen-1, col) = H(qlen-1, col0 - 1) + the prefix sum of the last
             // row's u (the column state after the sweep) along the strip
@@ -427,6 +441,7 @@ __global__ void __launch_bounds__(32 * cta_warps<NP>(), NP == 8 ? 2 : 5) ksw_ful
             if (s > 0) {
                 uint2 e = lane == 0 ? bnd_load(left + qlen) : make_uint2(0u, 0u);
                 await(e, lane == 0, [&]() { return bnd_load(left + qlen); });
+                if (stopped) report_stop();
                 if (stopped || failed) break;
                 __threadfence();  // what the strips on the left put into the pair's record before it
                 base16 = (int)__shfl_sync(FULLMASK, e.x, 0);
@@ -472,14 +487,6 @@ __global__ void __launch_bounds__(32 * cta_warps<NP>(), NP == 8 ? 2 : 5) ksw_ful
                 o.n_cigar = 0, o.zdropped = 0, o.reach_end = 0, o.stopped = 0;
                 A.out[idx] = o;
             }
-        }
-        if (stopped && lane == 0) {
-            // past the deadline: no score and no traceback (ksw2_extd2_sse.c:136-139, :400-409)
-            KswOut o;
-            o.score = AW_NEG_INF, o.max = 0, o.max_q = -1, o.max_t = -1;
-            o.mqe = AW_NEG_INF, o.mqe_t = -1, o.mte = AW_NEG_INF, o.mte_q = -1;
-            o.n_cigar = 0, o.zdropped = 0, o.reach_end = 0, o.stopped = 1;
-            A.out[idx] = o;
         }
         if (failed) break;
     }
