@@ -1196,7 +1196,8 @@ __device__ void cta_open(const WfaArgs &A, int idx, const HdrRing &HR, CtaShared
         }
         __syncthreads();
         const bool stop = PIG && S.retry[it % 3] != 0, end = S.at_end[it % 3] != 0 && !stop;
-        if (!end && !stop && (trimmed || S.beyond[it % 3])) {
+        // (at the end too: the backtrace reads its header and those of the null scores before it)
+        if (!stop && (trimmed || (!end && S.beyond[it % 3]))) {
             if (!trimmed) {
                 // from here on the trimmed ends count, and the plan made meanwhile is dropped
                 if (!planner) plan_trim(PR, now, tid, NT, S.part);
@@ -1214,14 +1215,11 @@ __device__ void cta_open(const WfaArgs &A, int idx, const HdrRing &HR, CtaShared
                 __syncwarp();
                 part_reset(S.part, lane);
                 commit(now.s, out);
-                plan_next(next);
+                if (!end) plan_next(next);
             }
             __syncthreads();
         }
-        if (planner && end) {
-            end_score = now.s, status = 0;
-            if (PIG && trimmed) commit(now.s, lane < 5 ? now.out[lane] : NUL);  // read by the backtrace
-        }
+        if (planner && end) end_score = now.s, status = 0;
         if (planner && stop) status = WFA_RETRY;
         op = end || stop ? WOP_DONE : next.op;
     }
@@ -1901,7 +1899,8 @@ __global__ void __launch_bounds__(WIDE_NT, 1) wfa_wide_kernel(WfaArgs A, RingSha
             // ---- 3.
             cl.sync();
             const bool end = at_end[it % 3] != 0;
-            if (!end && (trimmed || beyond[it % 3])) {
+            // (at the end too: the backtrace reads the headers of the null scores before it)
+            if (trimmed || (!end && beyond[it % 3])) {
                 if (!trimmed) {
                     if (!planner) plan_trim(PR, now, rank * 32 * WIDE_CW + tid, CL * 32 * WIDE_CW, part[2]);
                     cl.sync();
@@ -1911,7 +1910,7 @@ __global__ void __launch_bounds__(WIDE_NT, 1) wfa_wide_kernel(WfaArgs A, RingSha
                     else W.s = now.s, W.slot = now.s % W.R, W.num_null = 0, W.status = 0;  // drop the plan made meanwhile
                     take_ann(it);
                     finish_score(now, trimmed ? it & 1 : 2);
-                    plan_next(plan[(it + 1) & 1]);
+                    if (!end) plan_next(plan[(it + 1) & 1]);
                 }
                 trimmed = true;
                 __syncthreads();
