@@ -184,10 +184,15 @@ struct DeepRows {
 __host__ __device__ inline bool deep_cells(int block, int w, int qlen) { return block > 16 && w < qlen; }
 
 constexpr int BAND_WARPS = 4;  // per CTA: small CTAs spread a pair's strips over the SMs
+// CTAs per SM that the registers are sized for.  With the state bytes the edge loops want more than
+// the 128 registers of four CTAs (one 160 kb pair at w = 10% 104 against 95 ms of sweep with three, 512
+// pairs of 5 kb at 250 5.0 / 4.6), which batches of many narrow bands pay for (2,000 of 2 kb at 50: 3.8 /
+// 4.1); the tracks and the score alone do not.
+constexpr int band_ctas(int mode) { return mode == LEFT || mode == RIGHTMOST ? 3 : 4; }
 
 // STRICT: every step's values are checked, not those of every PUB-th step (band_strict).
 template <int MODE, bool STRICT>
-__global__ void __launch_bounds__(32 * BAND_WARPS, 4) ksw_band_kernel(BandArgs A) {
+__global__ void __launch_bounds__(32 * BAND_WARPS, band_ctas(MODE)) ksw_band_kernel(BandArgs A) {
     constexpr bool CIGAR = MODE != SCORES;
     constexpr int WB = MODE == TRACKS ? 8 : 4;
     using T = Tags<MODE>;
