@@ -32,10 +32,12 @@
 // Memory: per-score headers and wavefront arrays come from one device pool in 256 KiB
 // chunks (larger arrays in several), taken from its end by an atomicAdd.  A finished pair
 // gives its chunks to a free ring, from which the next pairs take theirs first, so a
-// batch needs the memory of the pairs in flight and not of all pairs (16,384 pairs of
-// 0.1-10 kb in a 20 GB pool: 672 -> 123 ms, 33 rounds -> 1).  A pair that finds
+// batch whose arrays fit a chunk needs the memory of the pairs in flight and not of all pairs
+// (16,384 pairs of 0.1-10 kb in a 20 GB pool: 672 -> 123 ms, 33 rounds -> 1).  Larger arrays (the
+// Singletrack I/D ring from 5.4 kb in sum, the piggyback rings from about 600 diagonals) always
+// come from the end, and what one gives back serves as single chunks.  A pair that finds
 // the pool empty stops with WFA_RETRY and the host re-runs it in a later round with a
-// fresh pool.
+// fresh pool, a pair alone in the least memory (WfaArgs::free_slots).
 #include "aw_internal.h"
 #include "wfa_internal.h"
 
@@ -951,8 +953,8 @@ __device__ __noinline__ void plan_trim(const WfaPairDev &PR, const WidePlan &Q, 
     fold_partials(kmin, kmax, false, pp);
 }
 
-// CTA-cooperative mode: one long pair on a CTA of NT computing threads and one planning warp.  As in the cluster kernel (below), wavefronts are not trimmed before the first
-// offset beyond the end of a sequence, so that the planner works a score ahead of the others and one
+// CTA-cooperative mode: one long pair on a CTA of NT computing threads and one planning warp.  As in
+// the cluster kernel (below), wavefronts are not trimmed before the first offset beyond the end of a sequence, so that the planner works a score ahead of the others and one
 // CTA barrier per score is left (two, with the plan between them, took 3.8 us a score at 2 kb,
 // half of it waiting for the plan; now 2.3).  A pair whose wavefront grows too wide stops with
 // WFA_WIDE for the cluster kernel; in the piggyback modes none does, and every warp reserves its own

@@ -218,7 +218,8 @@ static int run_batch(wavefront_aligner_gpu *al, int n, const char *const *patter
     W.wide_width_tail = std::min(W.wide_width, std::max(0, g_wide_tail.load()));
     W.wide_tail_pairs = std::max(1, wide_clusters);
     // a CTA's pair: eight times the tail width, as starting it over on a cluster late in its scores costs
-    // more than the CTA takes to finish it (64 pairs of 1-10 kb: 28 ms with four times, 24 with eight)
+    // more than the CTA takes to finish it (64 pairs of 1-10 kb: 28 ms with four times, 24 with eight).
+    // With the default widths that is the width which always stops it, so it counts for smaller ones.
     W.wide_width_cta = W.wide_width;
     W.wide_tail_cta = (int)std::min<int64_t>(W.wide_width, 8 * (int64_t)W.wide_width_tail);
     const int64_t long_sum = g_long_sum.load();

@@ -38,8 +38,9 @@ def set_wide(width: int = -1, tail_width: int = -1, cluster_ctas: int = 0) -> No
 
 
 def set_long(min_length_sum: int) -> None:
-    """aw_set_wfa_long: pairs whose lengths sum to at least this run first on a whole CTA each
-    (high memory; 0 = every pair on one warp).  Results are identical under every setting."""
+    """aw_set_wfa_long: pairs whose lengths sum to at least this run first on a whole CTA each, or
+    on a cluster of CTAs where a call has few (0 = every pair starts on one warp).  Results are
+    identical under every setting."""
     lib.aw_set_wfa_long(int(min_length_sum))
 
 
@@ -123,7 +124,7 @@ class WfaAligner:
         return out, ms.value
 
     def memory(self) -> Tuple[int, int]:
-        """Device bytes the last call's alignments took: (largest single alignment, sum)."""
+        """Bytes the last call's alignments allocated in the pool: (largest single alignment, sum)."""
         mx = C.c_int64(0)
         tot = C.c_int64(0)
         lib.wavefront_gpu_memory(self.h, C.byref(mx), C.byref(tot))

@@ -250,11 +250,12 @@ int wavefront_gpu_memory(const wavefront_aligner_gpu_t *aligner, int64_t *pair_m
 void aw_set_wfa_wide(int width, int tail_width, int cluster_ctas);
 /* Pairs whose pattern and text lengths sum to at least `min_length_sum` run first, each on a
  * whole CTA (the longest pairs of a batch otherwise set its duration, one warp each): four
- * warps, or sixteen for those that would outlast the batch, and in high memory a warp that plans
- * ahead of them; the others then run one per warp.  0: every pair starts on one warp.  Default
- * 800.  A CTA's pair moves to the cluster kernel by the width of aw_set_wfa_wide, as a warp's
- * does, and in the call's tail by eight times the tail width.  Results are identical.
- * Process-wide. */
+ * warps, or fifteen for those that would outlast the batch, and one that plans ahead of them;
+ * the others then run one per warp.  In high memory a call of no more pairs than clusters fit on
+ * the device starts those of 8,000 bases and more on the cluster kernel.  0: every pair starts on
+ * one warp.  Default 800.  A CTA's pair moves to the cluster kernel by the width of
+ * aw_set_wfa_wide, as a warp's does, and in the call's tail by eight times the tail width.
+ * Results are identical.  Process-wide. */
 void aw_set_wfa_long(int min_length_sum);
 /* Kernel launches of the last call (every round and phase) and, of them, the cluster
  * kernel's, with the number of pairs that moved to it. */
@@ -415,12 +416,15 @@ int aw_ksw_extd2_device_noalloc(int qlen, const uint8_t *d_query, int tlen, cons
 
 /* HBM budget (bytes) for traceback arenas per host thread; mirrors the -M
  * admission envelope (src/myImportandFunction/AlignmentResourceScheduler.cpp:706).
- * 0 = default (60% of free device memory). */
+ * 0 = default (60% of free device memory).  The strips' boundary columns count as well, but for
+ * those of the full-matrix kernel's wide strips and half of a banded pair's alone (1/64 of the
+ * traceback each). */
 void aw_set_traceback_budget(int64_t bytes);
 /* Full-matrix pairs with tlen >= threshold run their strips on a warp each (large_warps > 1:
  * 2, 4 or 8) or all on one warp (1); shorter pairs of a batch are split by the batch's work
  * unless large_warps is 1, and small batches always run on narrow strips, one warp each
- * (autotuner knobs; 0 keeps the current value).  Results are identical. */
+ * (autotuner knobs; 0 keeps the current value).  A plan keeps the threshold it was built with
+ * and follows large_warps at each execute.  Results are identical. */
 void aw_set_tuning(int large_warps, int large_tlen_threshold);
 /* Formerly the target columns per lane of the banded kernel (4, 8, or 0 to choose per batch): one
  * width is now the faster one for every batch, and the setting is accepted without effect. */
