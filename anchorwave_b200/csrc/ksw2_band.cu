@@ -918,15 +918,16 @@ BandKernel band_kernel_for(int flag, int block, bool strict) {
 
 int64_t ceil_div(int64_t a, int64_t b) { return (a + b - 1) / b; }
 
-// x, y, x2 and y2 grow by grow = qe - min(e, e2) a step at most, and a candidate adds a u or v of at
-// most qe.  Within 30 steps at the band's left edge (16 columns) they reach 30 * grow: 149 under (4, 2,
+// x, y, x2 and y2 grow by grow = M - min(e, e2) a step at most, and a candidate adds a u or v of at
+// most M (ksw2_cell.cuh).  Within 30 steps at the band's left edge (16 columns) they reach 30 * grow: 149 under (4, 2,
 // 24, 1), 989 under (30, 4, 40, 1); in the band and above it 57 was the largest value met.  A look
 // every PUB steps has room for that while grow is below 39; above, every step is checked (and a gap
 // that costs 49 to open still sends some pairs to the anti-diagonal kernel).
-int band_grow(const KswScore &S) { return S.qe - std::min(S.e, S.e2); }
-bool band_strict(const KswScore &S) { return 30 * band_grow(S) + 57 > CAND_MAX - S.qe - PUB * band_grow(S); }
+int band_uv(const KswScore &S) { return std::max(S.qe, -S.long_diff); }  // M
+int band_grow(const KswScore &S) { return band_uv(S) - std::min(S.e, S.e2); }
+bool band_strict(const KswScore &S) { return 30 * band_grow(S) + 57 > CAND_MAX - band_uv(S) - PUB * band_grow(S); }
 int band_peak_max(const KswScore &S) {
-    return 16 * std::max(CAND_MAX - S.qe - (band_strict(S) ? 1 : PUB) * band_grow(S), 0) + FB;
+    return 16 * std::max(CAND_MAX - band_uv(S) - (band_strict(S) ? 1 : PUB) * band_grow(S), 0) + FB;
 }
 
 // Device bytes of a pair's boundary columns (entries rounded as the wave packs them).

@@ -22,14 +22,15 @@ __device__ __forceinline__ int edge_diff(int r, const KswScore &S) {
 // Every 32-bit add below keeps each field inside [0, 65536), and every value a DPX op compares
 // inside [0, 32768), while no candidate is above CAND_MAX.  The other bounds hold for any cell,
 // also the ones outside a band that have no consistent neighbours, whatever x and y are: with
-// u, v in [-qe, mch + qe] before a step (qe = q + e; the initial and the boundary values are, and
-// mch < 0 moves the bounds by -mch at most),
-// z = min(max(s, a, ...), mch) is either mch, and then z - v >= -qe, or at least a = x + v >= v - qe,
-// as x >= -qe, and then z - v >= -qe as well; z - v <= mch + qe since v >= -qe; the same for
-// z - u.  x, y >= -qe and x2, y2 >= -(q2 + e2) by their max, and mch <= 0.  So by the magnitude
-// bound of full_path_ok (all of these together at most 100) no field falls below -256 * 16.
-// In a full matrix x <= q and so on; above a cell of a band they may grow by at most qe a step
-// (max(a - z - e, ..) with a = x + v, where z is clipped to mch), which the banded kernel checks.
+// u, v in [-M, mch + M] before a step (M = q + e, or the largest difference along a matrix edge,
+// -long_diff, where e = e2; the initial and the boundary values are, and mch < 0 moves the bounds
+// by -mch at most), z = min(max(s, a, ...), mch) is either mch, and then z - v >= -M, or at least
+// a = x + v >= v - (q + e), and then z - v >= -(q + e); z - v <= mch + M since v >= -M; the same for
+// z - u.  x, y >= -(q + e) and x2, y2 >= -(q2 + e2) by their max, M <= q2 + e2 and mch <= 0.  So by
+// the magnitude bound of full_path_ok (both gaps, the mismatch and the match together at most 100)
+// no field falls below -256 * 16.
+// In a full matrix x <= q and so on; at the edge of a band they may grow by M - e a step (max(a - z -
+// e, ..) with a = x + v, where z is clipped to mch), which the banded kernel checks.
 // The adds are 2-input multiply-adds by a runtime one (or minus one), so they issue on the
 // FMA pipe and leave the ALU pipe to the max/min/permute work.
 constexpr int FB = 4096;  // a multiple of 16 * 256: the byte above a field's tag is the value
