@@ -235,9 +235,12 @@ static bool full_path_ok(const Params &P, int qlen, int tlen, int w) {
 // semantics, so it takes any band and the Singletrack traceback (both entries: the AVX
 // one and ksw_extd2_singletrack_sse with its 16-byte blocks and end rules); it shares
 // the strip kernel's scoring restrictions (no z-drop or max tracking: with mat <= 0
-// every H is <= 0, so ez->max stays 0 and max_t/max_q stay -1).
-static bool band_path_ok(const Params &P, int qlen, int tlen) {
+// every H is <= 0, so ez->max stays 0 and max_t/max_q stay -1).  Not so in a band of one where the
+// extensions are equal and the second opening is larger: the edge falls by their difference at once,
+// the cells beside it rise above zero, and the maximum is theirs.
+static bool band_path_ok(const Params &P, int qlen, int tlen, int w) {
     if (exact_stop_enabled()) return false;
+    if (w == 1 && P.e == P.e2 && P.q2 > P.q) return false;
     const int allowed = AW_EZ_SCORE_ONLY | AW_EZ_RIGHT | AW_EZ_GENERIC_SC | AW_EZ_REV_CIGAR |
                         AW_EZ_SEMIGLOBAL_END | AW_EZ_SINGLETRACK | AW_EZ_SSE_SINGLETRACK;
     if (P.flag & ~allowed) return false;
@@ -386,7 +389,7 @@ static int plan_build(aw_ksw_plan_t *pl, int n, const int *qlen, const int *tlen
         if (P.m <= 1 || ql <= 0 || tl <= 0) continue;
         if (ql > INT_MAX - tl + 1) { pl->early_zdrop[i] = 1; continue; }
         if (P.early_return) continue;
-        pl->route[i] = full_path_ok(P, ql, tl, pl->w[i]) ? 1 : band_path_ok(P, ql, tl) ? 3 : 2;
+        pl->route[i] = full_path_ok(P, ql, tl, pl->w[i]) ? 1 : band_path_ok(P, ql, tl, pl->w[i]) ? 3 : 2;
         KswPair &kp = pl->pairs[i];
         kp.qoff = pl->qoff[i], kp.toff = pl->toff[i];
         kp.qlen = ql, kp.tlen = tl;
@@ -429,7 +432,7 @@ static int plan_build(aw_ksw_plan_t *pl, int n, const int *qlen, const int *tlen
         // chain outlasts the batch; Singletrack tracks are its to refuse, from the two thirds of the
         // budget that it always has for them.
         const int64_t tb = cigar ? ksw_full_tb_bytes(ql, tl, false, tracks) : 0;
-        if (!band_path_ok(P, ql, tl)) continue;
+        if (!band_path_ok(P, ql, tl, pl->w[i])) continue;
         if (tracks && tb > budget / 3 * 2) pl->route[i] = 3;
         if (!tracks && tb > budget && g_band_full_pairs.load()) {
             const double strips8 = std::ceil(std::ceil(tl / 512.0) / 8.0);

@@ -75,3 +75,24 @@ def test_padding_in_recompute_rounds(gpu, restatement, pen, mis):
         gpu.set_traceback_budget(0)
     for w, r in zip(ws, res):
         assert r.key() == restatement.ksw_extd2(q.tobytes(), t.tobytes(), mat, *pen, w=w).key(), w
+
+
+@pytest.mark.parametrize("pen", [(0, 1, 5, 1), (2, 2, 60, 2), (20, 1, 70, 1), (4, 2, 24, 1)])
+@pytest.mark.parametrize("flag", [0, RIGHT, SCORE_ONLY, ST, ST | SSE_ST])
+def test_narrowest_bands(gpu, restatement, pen, flag):
+    """Bands of 0 to 3; with equal extensions a band of one tracks a maximum above zero."""
+    rng = np.random.default_rng(pen[2] + flag)
+    mat = _matrix(-1)
+    qs, ts, ws = [], [], []
+    for i in range(160):
+        n = int(rng.integers(1, 40))
+        t = rng.integers(0, 4, n).astype(np.uint8)
+        q = np.concatenate([t, t[:1]])[int(rng.integers(0, 2)):n + int(rng.integers(0, 2))]
+        qs.append(q if len(q) else t[:1])
+        ts.append(t)
+        ws.append(i % 4)
+    res = gpu.ksw_extd2_batch(qs, ts, mat, *pen, w=ws, flag=flag)
+    more = {"block": 16} if flag & SSE_ST else {}
+    bad = [(len(q), len(t), w) for q, t, w, r in zip(qs, ts, ws, res)
+           if r.key() != restatement.ksw_extd2(q.tobytes(), t.tobytes(), mat, *pen, w=w, flag=flag & ~SSE_ST, **more).key()]
+    assert not bad, (len(bad), bad[:5])
